@@ -126,6 +126,24 @@ def test_linear_float32_row_does_not_depend_on_the_batch(ops):
         assert torch.equal(ops.linear(x[r:r + 1].contiguous(), w)[0], full[r])
 
 
+# rows around the few-row kernel's limits and the tiles' edges; N and K around a tile, a stage, and off 16-byte rows
+@pytest.mark.parametrize("M", [1, 4, 5, 16, 32, 33, 64, 65, 129])
+@pytest.mark.parametrize("N,K", [(64, 64), (68, 132), (33, 20), (9476, 36), (100, 67)])
+def test_linear_float32_adds_in_ascending_order_whatever_the_kernel(ops, M, N, K):
+    """Every float32 kernel adds an element's products over k in ascending order, one FMA each: the rows
+    of a product are the same bits however many rows it has, and within K roundings of float64."""
+    x, w = rnd(M, K), rnd(N, K, seed=1)
+    got = ops.linear(x, w)
+    want = x.double() @ w.double().T
+    bound = K * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)  # one rounding per product added
+    assert bool(((got.double() - want).abs() <= bound).all())
+    for r in (0, M // 2, M - 1):
+        assert torch.equal(ops.linear(x[r:r + 1].contiguous(), w)[0], got[r])
+    resid = rnd(M, N, seed=2)
+    total = resid + got
+    assert torch.equal(ops.linear(x, w, epilogue=ops.ADD, out=resid), total)
+
+
 @pytest.fixture(params=["fast kernels", "prompt attention in tensor memory", "warp-level attention",
                         "fallback kernels"])
 def kernel_choice(request, monkeypatch):
