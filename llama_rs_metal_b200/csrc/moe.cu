@@ -184,37 +184,59 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, const float* 
   for (int c = 0; c < top; ++c) w[c] /= mass;
 }
 
-// The router in one launch for steps of few tokens: one CTA per token forms the E float32 logits
-// (a warp per expert at a time, the lanes across the row, each lane's products in ascending order
-// and the lanes added by a butterfly: a fixed order whatever the batch), then thread 0 chooses.
-template <typename A>
+// The router in one launch: a CTA per TOK tokens forms their E float32 logits (a warp per expert at a
+// time, the lanes across the row, each lane's products in ascending order and the lanes added by a
+// butterfly: a fixed order whatever the batch), then a warp per token chooses. A lane has 16 loads of
+// a router row under way together (8 tokens, 9 outputs, width 2048: 8 us, 15 with the loads one after
+// another); prompts share every load of the router's matrix between four tokens.
+template <typename A, int TOK>
 __global__ void moe_router_kernel(const A* __restrict__ x, const float* __restrict__ w,
                                   const float* __restrict__ bias, int* __restrict__ ids,
-                                  float* __restrict__ weights, float* __restrict__ logits, int width, int E,
+                                  float* __restrict__ weights, float* __restrict__ logits, int tokens, int width, int E,
                                   int top, int scored, const float* __restrict__ correction, int groups, int keep,
-                                  int renormalize, float mass_eps, float weight_scale) {
+                                  int renormalize, float mass_eps, float weight_scale, int per_token) {
   extern __shared__ float smem[];
-  float* xs = smem;          // [width]
-  float* zs = smem + width;  // [E] (scored: also s [E], choice [E] and the groups' flags behind it)
   pdl_trigger();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   pdl_wait();
-  const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  for (int i = threadIdx.x; i < width; i += blockDim.x) xs[i] = to_f32(x[static_cast<size_t>(t) * width + i]);
+  const int t0 = blockIdx.x * TOK, live = min(TOK, tokens - t0);
+  float* xs = smem;  // [TOK][width]
+  for (int i = threadIdx.x; i < live * width; i += blockDim.x) xs[i] = to_f32(x[static_cast<size_t>(t0) * width + i]);
+  for (int i = live * width + threadIdx.x; i < TOK * width; i += blockDim.x) xs[i] = 0.f;
   __syncthreads();
   for (int e = warp; e < E; e += warps) {
     const float* row = w + static_cast<size_t>(e) * width;
-    float acc = 0.f;
-    for (int i = lane; i < width; i += 32) acc = fmaf(row[i], xs[i], acc);
-    acc = warp_sum(acc);
-    if (lane == 0) zs[e] = acc + (bias != nullptr ? bias[e] : 0.f);
+    float acc[TOK];
+#pragma unroll
+    for (int k = 0; k < TOK; ++k) acc[k] = 0.f;
+    int i = lane;
+    for (; i + 15 * 32 < width; i += 16 * 32) {
+      float r[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) r[u] = __ldg(row + i + 32 * u);
+#pragma unroll
+      for (int u = 0; u < 16; ++u)
+#pragma unroll
+        for (int k = 0; k < TOK; ++k) acc[k] = fmaf(r[u], xs[k * width + i + 32 * u], acc[k]);
+    }
+    for (; i < width; i += 32)
+#pragma unroll
+      for (int k = 0; k < TOK; ++k) acc[k] = fmaf(row[i], xs[k * width + i], acc[k]);
+#pragma unroll
+    for (int k = 0; k < TOK; ++k) {
+      const float z = warp_sum(acc[k]);
+      if (lane == 0) smem[TOK * width + k * per_token + e] = z + (bias != nullptr ? bias[e] : 0.f);
+    }
   }
   __syncthreads();
+  if (warp >= live) return;
+  const int t = t0 + warp;
+  float* zs = smem + TOK * width + warp * per_token;  // [E] (scored: also s [E], choice [E] and the groups' flags)
   if (logits != nullptr)
-    for (int e = threadIdx.x; e < E; e += blockDim.x) logits[static_cast<size_t>(t) * E + e] = zs[e];
+    for (int e = lane; e < E; e += 32) logits[static_cast<size_t>(t) * E + e] = zs[e];
   int* mine = ids + static_cast<size_t>(t) * top;
   float* out = weights + static_cast<size_t>(t) * top;
   if (scored) {
-    if (warp != 0) return;
     score_row(zs, correction, zs + E, zs + 2 * E, E, lane);
     __syncwarp();
     if (lane == 0)
@@ -222,7 +244,7 @@ __global__ void moe_router_kernel(const A* __restrict__ x, const float* __restri
                     renormalize, mass_eps, weight_scale, mine, out);
     return;
   }
-  if (threadIdx.x != 0) return;
+  if (lane != 0) return;
   float best = -INFINITY, mass = 0.f;
   for (int c = 0; c < top; ++c) {
     int arg = -1;
@@ -459,18 +481,31 @@ LRM_API int lrm_moe_router(const void* x, int x_dtype, const float* w, const flo
   if (width <= 0 || E <= 0 || top <= 0 || top > E) return LRM_BAD_ARGUMENT;
   if (scored && (groups <= 0 || E % groups || keep <= 0 || keep > groups || top > keep * (E / groups)))
     return LRM_BAD_ARGUMENT;
-  const size_t bytes = sizeof(float) * (static_cast<size_t>(width) + (scored ? 3 * E + (groups + 3) / 4 : E));
+  const size_t per_token = scored ? 3 * static_cast<size_t>(E) + (groups + 3) / 4 : E;
+  const size_t bytes = sizeof(float) * (static_cast<size_t>(width) + per_token);
   if (bytes > 48 * 1024) return LRM_UNSUPPORTED;
-  const int threads = E >= 8 ? 256 : 128;
+  // four tokens per CTA once that still leaves a CTA and more per SM; a warp per expert where few tokens leave room
+  const bool four = tokens >= 4 * 148 && 4 * bytes <= 48 * 1024;
+  const int threads = !four && E >= 32 ? 1024 : !four && E >= 16 ? 512 : E >= 8 ? 256 : 128;
+#define LRM_ROUTER(AT)                                                                                                      \
+  do {                                                                                                                      \
+    const AT* xt = static_cast<const AT*>(x);                                                                               \
+    if (four)                                                                                                               \
+      LRM_LAUNCH((moe_router_kernel<AT, 4>), (tokens + 3) / 4, threads, 4 * bytes, stream, xt, w, bias, ids, weights, logits, \
+                 tokens, width, E, top, scored, correction, groups, keep, renormalize, mass_eps, weight_scale,              \
+                 static_cast<int>(per_token));                                                                              \
+    else                                                                                                                    \
+      LRM_LAUNCH((moe_router_kernel<AT, 1>), tokens, threads, bytes, stream, xt, w, bias, ids, weights, logits, tokens,      \
+                 width, E, top, scored, correction, groups, keep, renormalize, mass_eps, weight_scale,                      \
+                 static_cast<int>(per_token));                                                                              \
+  } while (0)
   if (x_dtype == LRM_F32)
-    LRM_LAUNCH(moe_router_kernel<float>, tokens, threads, bytes, stream, static_cast<const float*>(x), w, bias, ids,
-               weights, logits, width, E, top, scored, correction, groups, keep, renormalize, mass_eps, weight_scale);
+    LRM_ROUTER(float);
   else if (x_dtype == LRM_BF16)
-    LRM_LAUNCH(moe_router_kernel<__nv_bfloat16>, tokens, threads, bytes, stream,
-               static_cast<const __nv_bfloat16*>(x), w, bias, ids, weights, logits, width, E, top, scored, correction,
-               groups, keep, renormalize, mass_eps, weight_scale);
+    LRM_ROUTER(__nv_bfloat16);
   else
     return LRM_BAD_ARGUMENT;
+#undef LRM_ROUTER
   return 0;
 }
 

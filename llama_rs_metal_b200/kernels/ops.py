@@ -1570,6 +1570,15 @@ def moe_experts_rows(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor,
         if x32.shape != x.shape:
             raise InvalidError("moe_experts_rows: x32 must match x")
     lib = _lib()
+    if (x.dtype == gate_up.dtype == torch.bfloat16 and lib.lrm_moe_experts_grouped_supports(T, width, ff, E, top)
+            and all(t.data_ptr() % 16 == 0 for t in (x, gate_up, down))):
+        # every chosen expert's matrices are read once, however many tokens chose it
+        terms = torch.empty((3, T * top, ff), dtype=torch.bfloat16, device=x.device)
+        planes = _f32((top, T, width), x.device)
+        _done(lib.lrm_moe_experts_grouped(_ptr(x), _ptr(gate_up), _ptr(down), _ptr(ids), _ptr(weights), _ptr(terms),
+                                          _ptr(planes), T, width, ff, E, top, ctypes.c_float(limit), ctypes.c_float(alpha),
+                                          act, _ptr(x32), _stream()), "moe_experts_grouped", launches=2)
+        return planes
     slices = int(lib.lrm_moe_rows_slices(T, top, ff))
     planes = _f32((top * slices, T, width), x.device)
     _done(lib.lrm_moe_experts_rows(_ptr(x), _code(x.dtype), _ptr(gate_up), _ptr(down), _code(gate_up.dtype),
