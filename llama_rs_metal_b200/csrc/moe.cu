@@ -195,13 +195,25 @@ __global__ void moe_router_kernel(const A* __restrict__ x, const float* __restri
                                   float* __restrict__ weights, float* __restrict__ logits, int tokens, int width, int E,
                                   int top, int scored, const float* __restrict__ correction, int groups, int keep,
                                   int renormalize, float mass_eps, float weight_scale, int per_token) {
-  extern __shared__ float smem[];
+  extern __shared__ __align__(16) float smem[];
   pdl_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   pdl_wait();
   const int t0 = blockIdx.x * TOK, live = min(TOK, tokens - t0);
   float* xs = smem;  // [TOK][width]
-  for (int i = threadIdx.x; i < live * width; i += blockDim.x) xs[i] = to_f32(x[static_cast<size_t>(t0) * width + i]);
+  const A* rows = x + static_cast<size_t>(t0) * width;
+  constexpr int PIECE = 16 / sizeof(A);
+  if (width % PIECE == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0) {  // 16 bytes at a time
+    for (int i = threadIdx.x * PIECE; i < live * width; i += blockDim.x * PIECE) {
+      const uint4 raw = *reinterpret_cast<const uint4*>(rows + i);
+      const A* part = reinterpret_cast<const A*>(&raw);
+#pragma unroll
+      for (int u = 0; u < PIECE; u += 4)
+        *reinterpret_cast<float4*>(xs + i + u) = make_float4(to_f32(part[u]), to_f32(part[u + 1]), to_f32(part[u + 2]), to_f32(part[u + 3]));
+    }
+  } else {
+    for (int i = threadIdx.x; i < live * width; i += blockDim.x) xs[i] = to_f32(rows[i]);
+  }
   for (int i = live * width + threadIdx.x; i < TOK * width; i += blockDim.x) xs[i] = 0.f;
   __syncthreads();
   for (int e = warp; e < E; e += warps) {
@@ -435,6 +447,45 @@ __global__ void moe_dense_gate_kernel(const G* __restrict__ gu, const int* __res
   }
 }
 
+// The same four columns at a time, a CTA per token (ff a multiple of 4, rows on 16-byte boundaries). Bound by reading
+// the chosen experts' gate and up columns and writing y.
+template <typename A>
+__global__ __launch_bounds__(256) void moe_dense_gate_wide_kernel(const float* __restrict__ gu, const int* __restrict__ ids,
+                                                                  const float* __restrict__ weights, A* __restrict__ y, int ff,
+                                                                  int experts, int top, float limit, float alpha, int act) {
+  extern __shared__ float share[];  // [experts] this token's weights
+  pdl_trigger();
+  pdl_wait();
+  const size_t t = blockIdx.x;
+  for (int e = threadIdx.x; e < experts; e += blockDim.x) {
+    float w = 0.f;
+    for (int c = 0; c < top; ++c)
+      if (ids[t * top + c] == e) w = weights[t * top + c];
+    share[e] = w;
+  }
+  __syncthreads();
+  const float* row = gu + t * experts * 2 * ff;
+  A* out = y + t * experts * ff;
+#pragma unroll 2
+  for (int item = threadIdx.x * 4; item < experts * ff; item += blockDim.x * 4) {
+    const int e = item / ff, f = item - e * ff;
+    const float w = share[e];
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (w != 0.f) {
+      const float4 g = *reinterpret_cast<const float4*>(row + static_cast<size_t>(e) * 2 * ff + f);
+      const float4 u = *reinterpret_cast<const float4*>(row + static_cast<size_t>(e) * 2 * ff + ff + f);
+      v[0] = expert_activation(g.x, u.x, act, limit, alpha) * w, v[1] = expert_activation(g.y, u.y, act, limit, alpha) * w;
+      v[2] = expert_activation(g.z, u.z, act, limit, alpha) * w, v[3] = expert_activation(g.w, u.w, act, limit, alpha) * w;
+    }
+    if constexpr (sizeof(A) == 2) {
+      __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
+      *reinterpret_cast<uint2*>(out + item) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+    } else {
+      *reinterpret_cast<float4*>(out + item) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+  }
+}
+
 }  // namespace
 
 // gu: float32 or the type of y (`gu_dtype`); y: `dtype`.
@@ -444,6 +495,18 @@ LRM_API int lrm_moe_dense_gate(const void* gu, int gu_dtype, int dtype, const in
   if (tokens <= 0) return 0;
   if (ff <= 0 || experts <= 0 || top <= 0 || (act != 0 && act != 1)) return LRM_BAD_ARGUMENT;
   const long long items = static_cast<long long>(experts) * ff;
+  const bool wide = ff % 4 == 0 && gu_dtype == LRM_F32 && experts <= 8192 && items < (1ll << 30) &&
+                    reinterpret_cast<uintptr_t>(gu) % 16 == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0;
+  if (wide && dtype == LRM_BF16) {
+    LRM_LAUNCH(moe_dense_gate_wide_kernel<__nv_bfloat16>, tokens, 256, sizeof(float) * experts, stream,
+               static_cast<const float*>(gu), ids, weights, static_cast<__nv_bfloat16*>(y), ff, experts, top, limit, alpha, act);
+    return 0;
+  }
+  if (wide && dtype == LRM_F32) {
+    LRM_LAUNCH(moe_dense_gate_wide_kernel<float>, tokens, 256, sizeof(float) * experts, stream, static_cast<const float*>(gu), ids,
+               weights, static_cast<float*>(y), ff, experts, top, limit, alpha, act);
+    return 0;
+  }
   const dim3 grid(tokens, static_cast<unsigned>((items + 1023) / 1024));
   if (dtype == LRM_BF16 && gu_dtype == LRM_BF16)
     LRM_LAUNCH((moe_dense_gate_kernel<__nv_bfloat16, __nv_bfloat16>), grid, 256, 0, stream,
