@@ -1,12 +1,13 @@
 // The state scans with a plain decay (see recurrent_scan.cuh), the read-out's norm and gate, and the
 // inputs of retention and of the gated delta rule.
-#include "recurrent_scan.cuh"
+#include "recurrent_walk.cuh"
 
 int g_scan_rows = 16;
 
 extern "C" int lrm_scan_gated_delta(const float* q, const float* k, const float* v, const float* g, const float* beta,
                                     float* state, float* out, const int* cu_seqlens, const int* slots, int seqs, int H,
-                                    int KH, int d, int dv, int tokens, cudaStream_t stream);  // recurrent_scan_delta.cu
+                                    int KH, int d, int dv, int tokens, float* workspace, cudaStream_t stream);
+extern "C" long long lrm_walk_floats_gated_delta(int seqs, int H, int KH, int d, int dv, int tokens);  // recurrent_scan_delta.cu
 
 namespace {
 
@@ -243,6 +244,14 @@ LRM_API int lrm_linear_state_scan_rows(int rows) {
   return g_scan_rows;
 }
 
+// Floats of workspace that lrm_linear_state_scan wants (0: none). rule 0: a decay per head, 1: the gated delta rule, 2: a
+// decay per head and token.
+LRM_API long long lrm_linear_state_scan_floats(int rule, int seqs, int H, int KH, int d, int dv, int tokens) {
+  return rule == 0   ? walk_floats<0>(seqs, H, KH, d, dv, tokens)
+         : rule == 1 ? lrm_walk_floats_gated_delta(seqs, H, KH, d, dv, tokens)
+                     : walk_floats<2>(seqs, H, KH, d, dv, tokens);
+}
+
 // q, k float32 [T, KH, d]; v float32 [T, H, dv]; out float32 [T, H, dv]; state float32
 // [slots, H, d, dv]. Without `g`: plain decay per head (head_decay [H]) or, when that is null, per
 // head and token (`beta` [T, H] holds the decays); with it: the gated delta rule (g [T, H, d], beta
@@ -250,18 +259,24 @@ LRM_API int lrm_linear_state_scan_rows(int rows) {
 LRM_API int lrm_linear_state_scan(const float* q, const float* k, const float* v, const float* g,
                                   const float* head_decay, const float* beta, float* state, float* out,
                                   const int* cu_seqlens, const int* slots, int seqs, int H, int KH, int d,
-                                  int dv, int tokens, cudaStream_t stream) {
+                                  int dv, int tokens, float* workspace, cudaStream_t stream) {
   if (seqs <= 0) return 0;
   if (H <= 0 || KH <= 0 || H % KH || d <= 0 || dv <= 0 || seqs > 65535 || H > 65535) return LRM_BAD_ARGUMENT;
   if (d > 2048) return LRM_UNSUPPORTED;
   if (g != nullptr) {
     if (beta == nullptr) return LRM_BAD_ARGUMENT;
-    return lrm_scan_gated_delta(q, k, v, g, beta, state, out, cu_seqlens, slots, seqs, H, KH, d, dv, tokens, stream);
+    return lrm_scan_gated_delta(q, k, v, g, beta, state, out, cu_seqlens, slots, seqs, H, KH, d, dv, tokens, workspace, stream);
   }
   if (head_decay == nullptr) {  // one decay per head and token, where beta would be
     if (beta == nullptr) return LRM_BAD_ARGUMENT;
+    if (takes_walk(seqs, d, tokens))
+      return dispatch_walk<2>(q, k, v, nullptr, nullptr, beta, nullptr, nullptr, state, out, cu_seqlens, slots, seqs, H, KH, d, dv,
+                              workspace, stream, Rows{tokens});
     return dispatch_scan<2>(q, k, v, nullptr, nullptr, beta, nullptr, nullptr, state, out, cu_seqlens, slots, seqs, H, KH, d, dv, stream, Rows{tokens});
   }
+  if (takes_walk(seqs, d, tokens))
+    return dispatch_walk<0>(q, k, v, nullptr, head_decay, nullptr, nullptr, nullptr, state, out, cu_seqlens, slots, seqs, H, KH, d,
+                            dv, workspace, stream, Rows{tokens});
   return dispatch_scan<0>(q, k, v, nullptr, head_decay, nullptr, nullptr, nullptr, state, out, cu_seqlens, slots, seqs, H, KH, d,
                           dv, stream, Rows{tokens});
 }

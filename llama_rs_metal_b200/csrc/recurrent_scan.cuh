@@ -27,9 +27,9 @@
 // which is the update above with the read-out taken after the write. Only r is waited for before the next
 // token: the sums s of four tokens are added over the parts together. Tokens are staged through
 // shared memory a chunk at a time by asynchronous copies, the next chunk under way while this
-// one is worked on, so the inner loop has no block-wide barrier and waits for no load. A step of one
-// token (decoding) and a step of a whole prompt run the same arithmetic in the same order, so
-// the state after a prompt does not depend on how it was cut.
+// one is worked on, so the inner loop has no block-wide barrier and waits for no load. This is the
+// kernel of decoding, and of prompts under the generalized rule or with heads wider than 256; the
+// other prompts take four tokens at a time (recurrent_walk.cuh).
 //
 // A sequence of padding (slot < 0) starts from zero and stores nothing.
 //

@@ -818,6 +818,11 @@ def _f32(shape, device) -> torch.Tensor:
     return torch.empty(shape, dtype=torch.float32, device=device)
 
 
+def _workspace(floats: int, device) -> Optional[torch.Tensor]:
+    """float32 scratch of a kernel that asks for `floats` numbers (None for none)."""
+    return torch.empty(floats, dtype=torch.float32, device=device) if floats else None
+
+
 def _column_ptr(t: torch.Tensor, column: int) -> ctypes.c_void_p:
     return ctypes.c_void_p(t.data_ptr() + column * t.element_size())
 
@@ -918,9 +923,11 @@ def linear_state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: 
         if head_decay.numel() != H:
             raise InvalidError("linear_state_scan: one decay per head")
     out = _f32((T, H, dv), q.device)
+    rule = 1 if g is not None else 0 if head_decay is not None else 2
+    work = _workspace(_lib().lrm_linear_state_scan_floats(rule, slots.numel(), H, KH, d, dv, T), q.device)
     _done(_lib().lrm_linear_state_scan(_ptr(q), _ptr(k), _ptr(v), _ptr(g), _ptr(head_decay), _ptr(beta), _ptr(state),
                                        _ptr(out), _ptr(cu_seqlens), _ptr(slots), slots.numel(), H, KH, d, dv, T,
-                                       _stream()), "linear_state_scan")
+                                       _ptr(work), _stream()), "linear_state_scan", launches=1 if work is None else 2)
     return out
 
 
@@ -997,10 +1004,11 @@ def bonus_state_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, g: 
     if tuple(g.shape) != (T, H * d) or max(q_off, k_off) + H * d > W or v_off + H * value_dim > W:
         raise InvalidError("bonus_state_scan: shapes do not agree")
     out = _f32((T, H, value_dim), proj.device)
+    work = _workspace(_lib().lrm_bonus_state_scan_floats(slots.numel(), H, d, value_dim, T), proj.device)
     _done(_lib().lrm_bonus_state_scan(_column_ptr(proj, q_off), _column_ptr(proj, k_off), ctypes.c_longlong(W),
                                       _column_ptr(proj, v_off), ctypes.c_longlong(W), _ptr(g), _ptr(bonus), _ptr(state),
                                       _ptr(out), _ptr(cu_seqlens), _ptr(slots), slots.numel(), H, d, value_dim, T,
-                                      _stream()), "bonus_state_scan")
+                                      _ptr(work), _stream()), "bonus_state_scan", launches=1 if work is None else 2)
     return out
 
 
@@ -1017,9 +1025,10 @@ def head_decay_delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, dec
     if k.shape != q.shape or v.shape[0] != T or H % KH or tuple(decay.shape) != (T, H) or tuple(step.shape) != (T, H):
         raise InvalidError("head_decay_delta_scan: shapes do not agree")
     out = _f32((T, H, dv), q.device)
+    work = _workspace(_lib().lrm_head_decay_delta_scan_floats(slots.numel(), H, KH, d, dv, T), q.device)
     _done(_lib().lrm_head_decay_delta_scan(_ptr(q), _ptr(k), _ptr(v), _ptr(decay), _ptr(step), _ptr(state), _ptr(out),
-                                           _ptr(cu_seqlens), _ptr(slots), slots.numel(), H, KH, d, dv, T, _stream()),
-          "head_decay_delta_scan")
+                                           _ptr(cu_seqlens), _ptr(slots), slots.numel(), H, KH, d, dv, T, _ptr(work), _stream()),
+          "head_decay_delta_scan", launches=1 if work is None else 2)
     return out
 
 
