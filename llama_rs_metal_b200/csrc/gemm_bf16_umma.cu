@@ -50,11 +50,19 @@ enum : int { kStuckEmpty = 1, kStuckFull = 2, kStuckAccumulator = 3, kStuckDrain
 // Warp 0: TMA loader. Warp 1: MMA issuer (and owner of the tensor memory). Warps 2-9: epilogue.
 // Where two sets of accumulators fit in the 512 columns of tensor memory they alternate, so the
 // epilogue of one item runs under the MMAs of the next; a 256 x 256 tile fills it alone.
-template <int BN, int STAGES, int MT>
+// EXPERTS: row tile m multiplies the W of expert tile_experts[m] (-1: no tile, nothing is done), which begins w_rows rows
+// and w_cols columns after the W of the expert before.
+struct ExpertArgs {
+  const int* tile_experts;
+  int w_rows, w_cols;
+};
+
+template <int BN, int STAGES, int MT, bool EXPERTS = false>
 __global__ __launch_bounds__(kUmmaThreads, 1) void gemm_bf16_umma_kernel(
     const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
     void* __restrict__ out, int M, int N, int K, int mode, int kb_per_split, int splits,
-    int* __restrict__ status, const QkvArgs qkv, const SplitArgs parts, int group_cols, int group_rows) {
+    int* __restrict__ status, const QkvArgs qkv, const SplitArgs parts, int group_cols, int group_rows,
+    const __grid_constant__ ExpertArgs experts) {
   constexpr uint32_t A_BYTES = MT * BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr uint32_t SET = MT * BN;                      // columns of one set of accumulators
   constexpr uint32_t NBUF = 2 * SET <= 512 ? 2 : 1;      // sets that fit in tensor memory
@@ -109,6 +117,8 @@ __global__ __launch_bounds__(kUmmaThreads, 1) void gemm_bf16_umma_kernel(
       // ---- loader: one thread feeds the ring with TMA, straight through all items
       uint32_t it = 0;  // k blocks issued so far by this CTA
       for (int item = blockIdx.x; item < items && !*bail; item += gridDim.x) {
+        const int e = EXPERTS ? experts.tile_experts[item % m_tiles] : 0;
+        if (EXPERTS && e < 0) continue;
         const int m0 = (item % m_tiles) * MT * BM, n0 = ((item / m_tiles) % n_tiles) * BN;
         const int kb_begin = (item / (m_tiles * n_tiles)) * kb_per_split;
         const int num_kb = min(k_blocks - kb_begin, kb_per_split);
@@ -125,7 +135,8 @@ __global__ __launch_bounds__(kUmmaThreads, 1) void gemm_bf16_umma_kernel(
           for (int i = 0; i < MT; ++i)  // 128 rows of X per accumulator (rows beyond M read as zero)
             tma_load_2d(tiles + s * STAGE_BYTES + i * BM * BK * 2, &map_x, full + s, (kb_begin + kb) * BK,
                         x0 + i * BM);
-          tma_load_2d(tiles + s * STAGE_BYTES + A_BYTES, &map_w, full + s, (kb_begin + kb) * BK, n0);
+          tma_load_2d(tiles + s * STAGE_BYTES + A_BYTES, &map_w, full + s, (kb_begin + kb) * BK + (EXPERTS ? e * experts.w_cols : 0),
+                      n0 + (EXPERTS ? e * experts.w_rows : 0));
         }
       }
       if (*bail) {
@@ -140,7 +151,8 @@ __global__ __launch_bounds__(kUmmaThreads, 1) void gemm_bf16_umma_kernel(
       // ---- issuer: one thread drives the tensor core
       constexpr uint32_t idesc = umma_idesc(BM, BN);  // both operands K-major
       uint32_t it = 0, local = 0;
-      for (int item = blockIdx.x; item < items && !*bail; item += gridDim.x, ++local) {
+      for (int item = blockIdx.x; item < items && !*bail; item += gridDim.x) {
+        if (EXPERTS && experts.tile_experts[item % m_tiles] < 0) continue;
         const int kb_begin = (item / (m_tiles * n_tiles)) * kb_per_split;
         const int num_kb = min(k_blocks - kb_begin, kb_per_split);
         const uint32_t acc = local % NBUF, use = local / NBUF;
@@ -168,6 +180,7 @@ __global__ __launch_bounds__(kUmmaThreads, 1) void gemm_bf16_umma_kernel(
           umma_commit(empty + s);  // arrives when these MMAs have finished reading the stage
         }
         umma_commit(acc_full + acc);  // arrives when every MMA issued so far has completed
+        ++local;
       }
     }
   } else {
@@ -175,7 +188,8 @@ __global__ __launch_bounds__(kUmmaThreads, 1) void gemm_bf16_umma_kernel(
     // may touch only the quarter of the tensor memory's lanes given by its index modulo 4
     const int quarter = warp & 3, side = (warp - 2) >> 2;
     uint32_t local = 0;
-    for (int item = blockIdx.x; item < items; item += gridDim.x, ++local) {
+    for (int item = blockIdx.x; item < items; item += gridDim.x) {
+      if (EXPERTS && experts.tile_experts[item % m_tiles] < 0) continue;
       const int m0 = (item % m_tiles) * MT * BM, n0 = ((item / m_tiles) % n_tiles) * BN;
       const int kb_begin = (item / (m_tiles * n_tiles)) * kb_per_split;
       const int num_kb = min(k_blocks - kb_begin, kb_per_split);
@@ -209,6 +223,7 @@ __global__ __launch_bounds__(kUmmaThreads, 1) void gemm_bf16_umma_kernel(
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(acc_free + acc);
+      ++local;
     }
   }
   tc_fence_before();
@@ -217,14 +232,17 @@ __global__ __launch_bounds__(kUmmaThreads, 1) void gemm_bf16_umma_kernel(
 }
 
 // ------------------------------------------------------------------------- host side
-template <int BN, int STAGES, int MT = 1>
+template <int BN, int STAGES, int MT = 1, bool EXPERTS = false>
 int launch_umma(const void* X, const void* W, void* out, int M, int x_rows, int N, int K, int mode, int splits,
                 int* status, cudaStream_t stream, const QkvArgs& qkv = QkvArgs{}, int group_cols = 0,
-                int group_rows = 0, const SplitArgs& parts = SplitArgs{}) {
+                int group_rows = 0, const SplitArgs& parts = SplitArgs{}, const ExpertArgs& experts = ExpertArgs{},
+                long long w_height = 0, long long w_width = 0) {
   CUtensorMap map_x, map_w;
-  if (!make_map_bf16(&map_x, X, x_rows, K, BM) || !make_map_bf16(&map_w, W, N, K, BN)) return LRM_UNSUPPORTED;
+  if (!make_map_bf16(&map_x, X, x_rows, K, BM) ||
+      !make_map_bf16(&map_w, W, EXPERTS ? w_height : N, EXPERTS ? w_width : K, BN))
+    return LRM_UNSUPPORTED;
   constexpr int smem = STAGES * (MT * BM * BK * 2 + BN * BK * 2) + 1024 + 256;
-  auto kernel = gemm_bf16_umma_kernel<BN, STAGES, MT>;
+  auto kernel = gemm_bf16_umma_kernel<BN, STAGES, MT, EXPERTS>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return static_cast<int>(e);
   const int k_blocks = (K + BK - 1) / BK;
@@ -240,7 +258,7 @@ int launch_umma(const void* X, const void* W, void* out, int M, int x_rows, int 
   }
   const int grid = static_cast<int>(items < sm_count ? items : sm_count);
   LRM_LAUNCH(kernel, dim3(grid), kUmmaThreads, smem, stream, map_x, map_w, out, M, N, K, mode, kb_per_split, real_splits,
-             status, qkv, parts, group_cols, group_rows);
+             status, qkv, parts, group_cols, group_rows, experts);
   return 0;
 }
 
@@ -354,4 +372,22 @@ LRM_API int lrm_gemm_bf16_umma_qkv(const void* X, const void* W, int M, int N, i
 LRM_API int lrm_gemm_bf16_umma(const void* X, const void* W, void* out, int M, int N, int K, int mode,
                                int tile, int splits, int* status, cudaStream_t stream) {
   return lrm_gemm_bf16_umma_rows(X, W, out, M, M, N, K, mode, tile, splits, status, stream);
+}
+
+// Row tiles of X [M, K] (M a multiple of 128) with a weight matrix each: out float32 [M, N] = x . W_e^T with e =
+// tile_experts[row / 128]; W_e is rows e w_rows .. e w_rows + N - 1, columns e w_cols .. e w_cols + K - 1 of W [w_height,
+// w_width]. Rows of a tile with e < 0 are left as they are. K a multiple of 64 (a column block never reaches into the next
+// expert's), w_cols and w_width of 8.
+LRM_API int lrm_gemm_bf16_umma_experts(const void* X, const void* W, void* out, int M, int N, int K, long long w_height,
+                                       long long w_width, int w_rows, int w_cols, const int* tile_experts, int* status,
+                                       cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (!lrm_gemm_bf16_umma_supports(M, N, K) || K % BK || M % BM || w_cols % 8 || w_width % 8 || w_height >= (1ll << 31) ||
+      w_width >= (1ll << 31))
+    return LRM_UNSUPPORTED;
+  if (tile_experts == nullptr || status == nullptr || w_rows < 0 || w_cols < 0) return LRM_BAD_ARGUMENT;
+  if (reinterpret_cast<uintptr_t>(X) % 16 || reinterpret_cast<uintptr_t>(W) % 16) return LRM_UNSUPPORTED;
+  const ExpertArgs experts{tile_experts, w_rows, w_cols};
+  return launch_umma<256, 4, 1, true>(X, W, out, M, M, N, K, 1, 1, status, stream, QkvArgs{}, 0, 0, SplitArgs{}, experts, w_height,
+                                      w_width);
 }

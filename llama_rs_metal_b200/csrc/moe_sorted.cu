@@ -1,0 +1,182 @@
+// A prompt's experts, rows sorted by expert, bfloat16: the passes around the two tensor-core products
+// (lrm_gemm_bf16_umma_experts, gemm_bf16_umma.cu) in which every row multiplies its own expert only.
+//
+//   sort     the (token, choice) pairs in the order of their experts, each expert's on whole tiles of 128 rows
+//   gather   x of every row's token
+//   gate     y = weight(t, c) * act(gate, up) in the products' float32, rounded to bfloat16 as on the way over all
+//            experts (moe.cu)
+//   combine  out[t] (+)= sum over a token's choices in their order
+//
+// Against the products over all experts (E / top times the arithmetic, E 2 ff float32 columns per token between them)
+// this pays from where the sorted rows are half as many as T E: see lrm_moe_sorted_tiles' caller.
+#include "common.cuh"
+
+namespace {
+
+constexpr int kTileRows = 128;
+constexpr int kSortThreads = 512;
+
+__device__ __forceinline__ float activation(float g, float u, int act, float limit, float alpha) {
+  if (act == 1) return g / (1.0f + expf(-g)) * u;
+  g = fminf(g, limit);
+  u = fminf(fmaxf(u, -limit), limit);
+  return g / (1.0f + expf(-alpha * g)) * (u + 1.0f);
+}
+
+// A CTA per expert: every CTA counts all experts' pairs, so that it knows where its own begin, then lists its own in
+// ascending order. rows[pos] = pair or -1 (padding up to whole tiles); places[pair] = pos, -1 for an identity expert;
+// tile_experts[tile] = expert, -1 behind the last tile.
+__global__ __launch_bounds__(kSortThreads) void moe_sort_kernel(const int* __restrict__ ids, int pairs, int experts,
+                                                                int* __restrict__ rows, int* __restrict__ places,
+                                                                int* __restrict__ tile_experts, int tiles) {
+  extern __shared__ int counts[];  // [experts]
+  __shared__ int warp_counts[kSortThreads / 32];
+  __shared__ int before_all, total_all;
+  pdl_trigger();
+  pdl_wait();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, mine = blockIdx.x;
+  for (int e = tid; e < experts; e += kSortThreads) counts[e] = 0;
+  if (tid == 0) before_all = total_all = 0;
+  __syncthreads();
+  for (int p = tid; p < pairs; p += kSortThreads) {
+    const int e = ids[p];
+    if (e >= 0 && e < experts) atomicAdd(counts + e, 1);
+    else if (mine == 0) places[p] = -1;
+  }
+  __syncthreads();
+  int before = 0, total = 0;
+  for (int e = tid; e < experts; e += kSortThreads) {
+    const int own = (counts[e] + kTileRows - 1) / kTileRows;
+    total += own;
+    if (e < mine) before += own;
+  }
+  atomicAdd(&before_all, before);
+  atomicAdd(&total_all, total);
+  __syncthreads();
+  const int first = before_all, count = counts[mine], own_tiles = (count + kTileRows - 1) / kTileRows;
+  for (int i = tid; i < own_tiles; i += kSortThreads) tile_experts[first + i] = mine;
+  if (mine == experts - 1)
+    for (int i = total_all + tid; i < tiles; i += kSortThreads) tile_experts[i] = -1;
+  int held = 0;
+  for (int p0 = 0; p0 < pairs; p0 += kSortThreads) {
+    const int p = p0 + tid;
+    const bool is = p < pairs && ids[p] == mine;
+    const unsigned ballot = __ballot_sync(0xffffffffu, is);
+    if (lane == 0) warp_counts[warp] = __popc(ballot);
+    __syncthreads();
+    int at = held, all = 0;
+    for (int w = 0; w < kSortThreads / 32; ++w) {
+      if (w < warp) at += warp_counts[w];
+      all += warp_counts[w];
+    }
+    if (is) {
+      const int pos = first * kTileRows + at + __popc(ballot & ((1u << lane) - 1u));
+      rows[pos] = p;
+      places[p] = pos;
+    }
+    held += all;
+    __syncthreads();
+  }
+  for (int i = count + tid; i < own_tiles * kTileRows; i += kSortThreads) rows[first * kTileRows + i] = -1;
+}
+
+// Rows behind the last tile are nobody's: not read by the products.
+__global__ __launch_bounds__(256) void moe_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ rows,
+                                                         const int* __restrict__ tile_experts, int top, int pieces,
+                                                         uint4* __restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
+  const int row = blockIdx.x;
+  if (tile_experts[row / kTileRows] < 0) return;
+  const int p = rows[row];
+  for (int i = threadIdx.x; i < pieces; i += blockDim.x)
+    out[static_cast<size_t>(row) * pieces + i] = p < 0 ? make_uint4(0u, 0u, 0u, 0u) : x[static_cast<size_t>(p / top) * pieces + i];
+}
+
+__global__ __launch_bounds__(256) void moe_sorted_gate_kernel(const float* __restrict__ gu, const int* __restrict__ rows,
+                                                              const int* __restrict__ tile_experts, const float* __restrict__ weights,
+                                                              int ff, float limit, float alpha, int act,
+                                                              __nv_bfloat16* __restrict__ y) {
+  pdl_trigger();
+  pdl_wait();
+  const int row = blockIdx.x;
+  if (tile_experts[row / kTileRows] < 0) return;
+  const int p = rows[row];
+  const float w = p < 0 ? 0.f : weights[p];
+  const float* g = gu + static_cast<size_t>(row) * 2 * ff;
+  for (int f = threadIdx.x * 4; f < ff; f += blockDim.x * 4) {
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (w != 0.f) {
+      const float4 a = *reinterpret_cast<const float4*>(g + f), b = *reinterpret_cast<const float4*>(g + ff + f);
+      v[0] = activation(a.x, b.x, act, limit, alpha) * w, v[1] = activation(a.y, b.y, act, limit, alpha) * w;
+      v[2] = activation(a.z, b.z, act, limit, alpha) * w, v[3] = activation(a.w, b.w, act, limit, alpha) * w;
+    }
+    __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
+    *reinterpret_cast<uint2*>(y + static_cast<size_t>(row) * ff + f) =
+        make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+  }
+}
+
+__global__ __launch_bounds__(256) void moe_combine_kernel(const float* __restrict__ part, const int* __restrict__ places, int top,
+                                                          int width, int add, float* __restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
+  const size_t t = blockIdx.x;
+  for (int i = threadIdx.x * 4; i < width; i += blockDim.x * 4) {
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int c = 0; c < top; ++c) {
+      const int pos = places[t * top + c];
+      if (pos < 0) continue;
+      const float4 v = *reinterpret_cast<const float4*>(part + static_cast<size_t>(pos) * width + i);
+      sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w;
+    }
+    float4* to = reinterpret_cast<float4*>(out + t * width + i);
+    if (add) {
+      const float4 old = *to;
+      sum.x += old.x, sum.y += old.y, sum.z += old.z, sum.w += old.w;
+    }
+    *to = sum;
+  }
+}
+
+}  // namespace
+
+// Tiles of 128 rows that hold any choice of `pairs` pairs among `experts` experts.
+LRM_API int lrm_moe_sorted_tiles_room(int pairs, int experts) { return pairs / kTileRows + experts; }
+
+// ids int32 [pairs] -> rows int32 [tiles * 128], places int32 [pairs], tile_experts int32 [tiles].
+LRM_API int lrm_moe_sort(const int* ids, int pairs, int experts, int* rows, int* places, int* tile_experts, int tiles,
+                         cudaStream_t stream) {
+  if (pairs <= 0) return 0;
+  if (experts <= 0 || experts > 8192 || tiles < lrm_moe_sorted_tiles_room(pairs, experts)) return LRM_BAD_ARGUMENT;
+  LRM_LAUNCH(moe_sort_kernel, experts, kSortThreads, sizeof(int) * experts, stream, ids, pairs, experts, rows, places, tile_experts,
+             tiles);
+  return 0;
+}
+
+// x bfloat16 [T, width] -> out [tiles * 128, width] (width a multiple of 8, rows 16-byte aligned).
+LRM_API int lrm_moe_gather(const void* x, const int* rows, const int* tile_experts, int top, int width, int tiles, void* out,
+                           cudaStream_t stream) {
+  if (width <= 0 || width % 8 || top <= 0 || tiles <= 0) return LRM_BAD_ARGUMENT;
+  LRM_LAUNCH(moe_gather_kernel, tiles * kTileRows, 256, 0, stream, static_cast<const uint4*>(x), rows, tile_experts, top, width / 8,
+             static_cast<uint4*>(out));
+  return 0;
+}
+
+// gu float32 [tiles * 128, 2 ff] (gate columns, then up columns) -> y bfloat16 [tiles * 128, ff]; ff a multiple of 4.
+LRM_API int lrm_moe_sorted_gate(const float* gu, const int* rows, const int* tile_experts, const float* weights, int ff, int tiles,
+                                float limit, float alpha, int act, void* y, cudaStream_t stream) {
+  if (ff <= 0 || ff % 4 || tiles <= 0 || (act != 0 && act != 1)) return LRM_BAD_ARGUMENT;
+  LRM_LAUNCH(moe_sorted_gate_kernel, tiles * kTileRows, 256, 0, stream, gu, rows, tile_experts, weights, ff, limit, alpha, act,
+             static_cast<__nv_bfloat16*>(y));
+  return 0;
+}
+
+// part float32 [tiles * 128, width], places int32 [T * top]; out float32 [T, width], added to with `add`.
+LRM_API int lrm_moe_combine(const float* part, const int* places, int tokens, int top, int width, int add, float* out,
+                            cudaStream_t stream) {
+  if (tokens <= 0) return 0;
+  if (width <= 0 || width % 4 || top <= 0) return LRM_BAD_ARGUMENT;
+  LRM_LAUNCH(moe_combine_kernel, tokens, 256, 0, stream, part, places, top, width, add, out);
+  return 0;
+}

@@ -103,6 +103,8 @@ WORK: Dict[str, Callable[..., Tuple[float, float]]] = {
     "lrm_attention_decode_tiled": lambda a: (2.0 * hints["kv_tokens"] * _v(a[11]) * _v(a[12]) * 2, 0),
     "lrm_attention_decode_cluster": lambda a: (2.0 * hints["kv_tokens"] * _v(a[14]) * _v(a[15]) * 2, 0),
     "lrm_attention_paged_rowwise": lambda a: (2.0 * hints["kv_tokens"] * _v(a[13]) * _v(a[14]) * _ELEM[_v(a[4])], 0),
+    "lrm_attention_extend_umma": lambda a: (2.0 * hints["kv_tokens"] * _v(a[14]) * _v(a[15]) * 2,
+                                            4.0 * hints["pairs"] * _v(a[13]) * _v(a[15])),
     "lrm_attention_extend_tiled": lambda a: (2.0 * hints["kv_tokens"] * _v(a[12]) * _v(a[13]) * 2,
                                              4.0 * hints["pairs"] * _v(a[11]) * _v(a[13])),
     # one shared key head whose rows hold the values: the keys once per sequence; per (query, key) pair and
@@ -135,6 +137,10 @@ WORK: Dict[str, Callable[..., Tuple[float, float]]] = {
     "lrm_moe_experts_grouped": lambda a: (
         min(_v(a[7]) * _v(a[11]), _v(a[10])) * 6.0 * _v(a[9]) * _v(a[8]) + 4.0 * _v(a[7]) * _v(a[11]) * _v(a[8]),
         6.0 * _v(a[7]) * _v(a[11]) * _v(a[9]) * _v(a[8])),
+    "lrm_gemm_bf16_umma_experts": lambda a: _gemm(_v(a[3]), _v(a[4]), _v(a[5]), 4, 2),
+    "lrm_moe_gather": lambda a: (_v(a[5]) * 128.0 * _v(a[4]) * 4.0, 0),
+    "lrm_moe_sorted_gate": lambda a: (_v(a[5]) * 128.0 * _v(a[4]) * 10.0, 0),
+    "lrm_moe_combine": lambda a: (_v(a[2]) * (_v(a[3]) + 1.0) * _v(a[4]) * 4.0, 0),
     "lrm_moe_dense_gate": lambda a: (_v(a[6]) * _v(a[7]) * _v(a[8]) * (2.0 * _ELEM[_v(a[1])] + _ELEM[_v(a[2])]), 0),
     "lrm_moe_router": lambda a: (_v(a[7]) * _v(a[8]) * _ELEM[_v(a[1])] + 4.0 * _v(a[9]) * _v(a[8]), 2.0 * _v(a[7]) * _v(a[8]) * _v(a[9])),
     "lrm_moe_route": lambda a: (_v(a[4]) * (_v(a[5]) * 4.0 + _v(a[6]) * 8.0), 0),

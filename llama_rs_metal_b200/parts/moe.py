@@ -24,13 +24,15 @@ class MixtureOfExperts(FeedForward):
 
     The router's matrix is kept in float32 whatever the runtime, so its product runs on the
     float32 kernel. The experts' matrices are stacked, gate_up [E, 2 ff, h] and down [h, E, ff],
-    and serve two ways of computing (csrc/moe.cu). Token by token (decoding, float32, many
-    experts per choice): one launch reads, for every token, only the experts it chose; their
-    outputs come back as float32 planes that are added to the stream in a fixed order (by the
-    next norm where it folds them). All experts at once (bfloat16 steps of DENSE_ROWS tokens and
-    more when at most DENSE_RATIO experts exist per chosen one): two tensor-core products over
-    every expert, with the weights of the experts a token did not choose set to zero between
-    them.
+    and serve three ways of computing. Token by token (decoding, float32, many experts per choice):
+    only the experts somebody chose are read, in bfloat16 once per step (csrc/moe_rows.cu), else once
+    per token that chose them (csrc/moe.cu); their outputs come back as float32 planes that are added
+    to the stream in a fixed order (by the next norm where it folds them). All experts at once
+    (bfloat16 steps of DENSE_ROWS tokens and more when at most DENSE_RATIO experts exist per chosen
+    one): two tensor-core products over every expert, with the weights of the experts a token did not
+    choose set to zero between them. Sorted (such steps once they have tokens enough to fill tiles of
+    128 rows per expert, csrc/moe_sorted.cu): the same two products with every row in its own expert's
+    tile.
 
     Options beyond that router and that expert. `activation` "silu": an expert is W_down (silu(W_gate
     x) * (W_up x)). `scoring` "softmax_all": the scores are s = softmax(z) over all outputs; the
@@ -134,6 +136,13 @@ class MixtureOfExperts(FeedForward):
                 else ops.moe_route(logits, self.bias, self.top)
         return routed
 
+    def _sorted(self, x, ids, weights, out):
+        """The experts of a prompt on rows sorted by expert, added to `out` (None: returned), or None where all experts
+        for every token are the faster way or the only one."""
+        if not ops.moe_prefers_sorted(x.shape[0], self.hidden_size, self.intermediate_size, self.num_experts, self.top):
+            return None
+        return ops.moe_experts_sorted(x, self.gate_up, self.down, ids, weights, self.limit, self.alpha, self.act, out)
+
     def forward(self, x, ctx, residual):
         ids, weights = self.route(x)
         # identity experts pass the input on: the float32 stream itself where x is its rounding
@@ -151,6 +160,11 @@ class MixtureOfExperts(FeedForward):
             if self.shared_gate:
                 ops.row_gate_(out, x, self.shared_gate_weight)
             if dense:
+                added = self._sorted(x, ids, weights, out)
+                if added is not None:
+                    if self.identity:
+                        ops.moe_identity_add_(added, x32 if x32 is not None else x, ids, weights, self.num_experts)
+                    return added
                 both = self.gate_up_all(x, out_dtype=torch.float32)
                 y = ops.moe_dense_gate(both, ids, weights, self.num_experts, self.limit, self.alpha, out_dtype=x.dtype,
                                        act=self.act)
@@ -170,6 +184,12 @@ class MixtureOfExperts(FeedForward):
             residual = self.shared.forward(x, ctx, residual=residual)
             ctx.settle(residual)
         if dense:
+            if ctx.pending is None:
+                added = self._sorted(x, ids, weights, residual)
+                if added is not None:
+                    if self.identity:
+                        ops.moe_identity_add_(residual, x32 if x32 is not None else x, ids, weights, self.num_experts)
+                    return residual
             # gate and up stay float32 up to the activation, as they do token by token
             both = self.gate_up_all(x, out_dtype=torch.float32)
             y = ops.moe_dense_gate(both, ids, weights, self.num_experts, self.limit, self.alpha, out_dtype=x.dtype,
