@@ -25,6 +25,11 @@
 //
 // Rows and keys outside a sequence are zero-filled by TMA or belong to a neighbouring sequence
 // of the packed batch; the causal mask hides such keys and such rows are never stored.
+// PAGED: several queries per started sequence over its paged cache, which already holds the step's keys. A key tile is a
+// page (64 keys, one piece of memory per head); the queries stand at the last positions of their sequence. The rows of a
+// sequence's last page that hold no key of it are whatever an earlier owner left: their scores are masked, and their
+// values are zeroed in shared memory before the tensor core may multiply them (0 x NaN).
+//
 // Every mbarrier wait is bounded; a wait that gives up records a code in `status`, and the CTA
 // winds down and frees its tensor memory. No cluster multicast. Head sizes 64 and 128.
 // (Reference: crates/metal-backend/src/shaders/attention.metal:28-57, the streaming softmax.)
@@ -50,13 +55,21 @@ template <int D, int BKV> struct Shape {
 // Shared memory (1024-byte aligned): Q [2][128][D] | stages of (K [128][D] | V [128][D]) |
 // barriers. A [128][D] tile with D = 128 is two [128][64] blocks of 16 KB one after the other
 // (a swizzle row is 128 bytes = 64 elements).
-template <int D, int NQ, int BKV>
+// The cache of a PAGED launch.
+struct Pages {
+  const int* table;    // [slots][stride]
+  int stride;
+  const int* slots;    // per sequence
+  const int* kv_lens;  // keys per sequence, the step's own included
+};
+
+template <int D, int NQ, int BKV, bool PAGED>
 __global__ __launch_bounds__(threads_per_cta(NQ), NQ == 1 ? Shape<D, BKV>::kCtasPerSm : 1)
 void attention_prefill_pingpong_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out,
     const int* __restrict__ cu_seqlens, int q_heads, int kv_heads, float scale_log2, int window,
-    int* __restrict__ status) {
+    int* __restrict__ status, Pages pages) {
   constexpr uint32_t TILE = BQ * D * 2;       // bytes of one [128][D] query tile
   constexpr uint32_t BLOCK = BQ * 64 * 2;     // bytes of one [128][64] block of it
   constexpr uint32_t KV_TILE = BKV * D * 2;   // bytes of one [BKV][D] key or value tile
@@ -64,6 +77,7 @@ void attention_prefill_pingpong_kernel(
   constexpr int DB = D / 64;                  // 64-column blocks per tile
   constexpr int STAGES = Shape<D, BKV>::kStages;
   static_assert(BKV == 128 || (BKV == 64 && NQ == 1), "tiles of 64 keys go with one query tile per CTA");
+  static_assert(!PAGED || BKV == 64, "a page has 64 keys");
   constexpr int kLoaderWarp = 4 * NQ, kIssuerWarp = 4 * NQ + 1;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   if ((smem_u32(smem_raw) & 1023u) != 0) {  // the swizzled tiles need it; give up rather than compute nonsense
@@ -79,7 +93,8 @@ void attention_prefill_pingpong_kernel(
   uint64_t* s_full = kv_free + STAGES;        // [2] scores of tile i written
   uint64_t* p_ready = s_full + 2;             // [2] probabilities of tile i written (4 warps arrive)
   uint64_t* o_done = p_ready + 2;             // [2] the last P V of tile i is complete
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2);
+  uint64_t* tail = o_done + 2;                // PAGED: the last page has arrived
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail + 1);
   volatile int* bail = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   // CTAs are handed out in the order x, y, z: all heads and sequences of the last pair of query
@@ -91,9 +106,11 @@ void attention_prefill_pingpong_kernel(
   if (q0 >= len) return;
   const int kh = h / (q_heads / kv_heads);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kt_first = window > 0 ? max(0, q0 - window + 1) / BKV : 0;
+  // position of the sequence's first query, and the keys there are (PAGED: no key tile beyond them exists)
+  const int base = PAGED ? pages.kv_lens[b] - len : 0, keys = base + len;
+  const int kt_first = window > 0 ? max(0, base + q0 - window + 1) / BKV : 0;
   // key tiles per query tile: up to its diagonal tile; the second tile may not exist
-  const int n0 = (q0 + BQ - 1) / BKV - kt_first + 1;
+  const int n0 = (PAGED ? min(base + q0 + BQ, keys) - 1 : q0 + BQ - 1) / BKV - kt_first + 1;
   const int n1 = NQ == 2 && q0 + BQ < len ? n0 + 1 : 0;
   const int n_tiles = max(n0, n1);
 
@@ -108,6 +125,7 @@ void attention_prefill_pingpong_kernel(
       mbar_init(p_ready + i, 4);
       mbar_init(o_done + i, 1);
     }
+    mbar_init(tail, 1);
     *bail = 0;
     mbar_fence_init();
   }
@@ -128,27 +146,59 @@ void attention_prefill_pingpong_kernel(
   pdl_wait();
 
   if (warp == kLoaderWarp) {
+    // ---- one thread brings the query tiles once and the key/value tiles through the ring
     if (lane == 0) {
-      // ---- one thread brings the query tiles once and the key/value tiles through the ring
       mbar_expect_tx(q_full, (n1 > 0 ? 2 : 1) * TILE);
       for (int i = 0; i < (n1 > 0 ? 2 : 1); ++i)
 #pragma unroll
         for (int db = 0; db < DB; ++db)
           tma_load_2d(q_tiles + i * TILE + db * BLOCK, &map_q, q_full, h * D + db * 64, start + q0 + i * BQ);
-      for (int j = 0; j < n_tiles && !*bail; ++j) {
-        const int s = j % STAGES;
-        if (j >= STAGES && !mbar_wait(kv_free + s, ((j / STAGES) - 1) & 1, status, kStuckStage)) {
-          *bail = 1;
-          break;
-        }
-        const int row = start + (kt_first + j) * BKV;
-        unsigned char* kdst = kv_tiles + s * 2 * KV_TILE;
-        mbar_expect_tx(kv_full + s, 2 * KV_TILE);
+    }
+    auto bring = [&](int j, uint64_t* arrives, int column, int row) {
+      unsigned char* kdst = kv_tiles + j % STAGES * 2 * KV_TILE;
+      mbar_expect_tx(arrives, 2 * KV_TILE);
 #pragma unroll
-        for (int db = 0; db < DB; ++db) {
-          tma_load_2d(kdst + db * KV_BLOCK, &map_k, kv_full + s, kh * D + db * 64, row);
-          tma_load_2d(kdst + KV_TILE + db * KV_BLOCK, &map_v, kv_full + s, kh * D + db * 64, row);
+      for (int db = 0; db < DB; ++db) {
+        tma_load_2d(kdst + db * KV_BLOCK, &map_k, arrives, column + db * 64, row);
+        tma_load_2d(kdst + KV_TILE + db * KV_BLOCK, &map_v, arrives, column + db * 64, row);
+      }
+    };
+    if constexpr (!PAGED) {
+      if (lane == 0) {
+        for (int j = 0; j < n_tiles && !*bail; ++j) {
+          const int s = j % STAGES;
+          if (j >= STAGES && !mbar_wait(kv_free + s, ((j / STAGES) - 1) & 1, status, kStuckStage)) {
+            *bail = 1;
+            break;
+          }
+          bring(j, kv_full + s, kh * D, start + (kt_first + j) * BKV);
         }
+      }
+    } else {
+      const int* table = pages.table + static_cast<size_t>(pages.slots[b]) * pages.stride;
+      const int tail_tile = keys % BKV != 0 ? keys / BKV - kt_first : -1;  // the page with rows that hold no key
+      for (int j = 0; j < n_tiles; ++j) {
+        const int s = j % STAGES;
+        bool ok = true;  // (every decision is lane 0's: the warp stays together)
+        if (lane == 0) {
+          ok = !*bail && (j < STAGES || mbar_wait(kv_free + s, ((j / STAGES) - 1) & 1, status, kStuckStage));
+          if (ok) bring(j, j == tail_tile ? tail : kv_full + s, 0, (table[kt_first + j] * kv_heads + kh) * BKV);
+          if (ok && j == tail_tile) ok = mbar_wait(tail, 0, status, kStuckKV);
+          if (!ok) *bail = 1;
+        }
+        if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+        if (j != tail_tile) continue;
+        mbar_wait(tail, 0, status, kStuckKV);  // (lane 0 saw it complete) makes the copies visible to every lane
+        // whole rows of 128 bytes, so the swizzle within a row does not matter
+        unsigned char* values = kv_tiles + s * 2 * KV_TILE + KV_TILE;
+        const int first = keys % BKV;
+        for (int i = lane; i < (BKV - first) * 8; i += 32)
+#pragma unroll
+          for (int db = 0; db < DB; ++db)
+            *reinterpret_cast<uint4*>(values + db * KV_BLOCK + first * 128 + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(kv_full + s);
       }
     }
   } else if (warp == kIssuerWarp) {
@@ -211,7 +261,8 @@ void attention_prefill_pingpong_kernel(
     // a warp may touch the quarter of the tensor memory's lanes given by its index modulo 4.
     const int i = warp >> 2, quad = warp & 3;
     const int n_mine = i == 0 ? n0 : n1;
-    const int row = q0 + i * BQ + quad * 32 + lane;  // position in the sequence
+    const int query = q0 + i * BQ + quad * 32 + lane;  // of the sequence's queries
+    const int row = base + query;                      // position in the sequence
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
     const uint32_t my_s = tmem_s[i] + lane_base, my_o = tmem_o[i] + lane_base;
     float m_run = -INFINITY;   // the row's true running maximum (log2 domain)
@@ -226,7 +277,7 @@ void attention_prefill_pingpong_kernel(
       }
       tc_fence_after();
       const int key0 = (kt_first + j) * BKV;
-      const int first_row = q0 + i * BQ;
+      const int first_row = base + q0 + i * BQ;
       const bool edge = key0 + BKV - 1 > first_row || (window > 0 && key0 <= first_row + BQ - 1 - window);
       // pass 1: the row's maximum over this tile; the whole row comes into registers at once (four
       // loads in flight, one wait) and is dropped again (only tiles on the diagonal or the window's
@@ -326,12 +377,12 @@ void attention_prefill_pingpong_kernel(
     if (ok && n_mine > 0) {
       // the mass belongs to m_ref, and so does O: their quotient is the row's attention output
       const float inv = 1.0f / l;
-      __nv_bfloat16* dst = out + (static_cast<size_t>(start + row) * q_heads + h) * D;
+      __nv_bfloat16* dst = out + (static_cast<size_t>(start + query) * q_heads + h) * D;
 #pragma unroll 1
       for (int c = 0; c < D / 32; ++c) {
         uint32_t r[32];
         tmem_load32(my_o + c * 32, r);
-        if (row < len) {
+        if (query < len) {
 #pragma unroll
           for (int e = 0; e < 32; e += 8)
             *reinterpret_cast<uint4*>(dst + c * 32 + e) = make_uint4(
@@ -358,7 +409,7 @@ int launch(const void* q, const void* k, const void* v, void* out, const int* cu
       !make_map_bf16(&map_v, v, tokens, static_cast<long long>(kv_heads) * D, BKV))
     return LRM_UNSUPPORTED;
   constexpr int smem = NQ * BQ * D * 2 + 2 * Shape<D, BKV>::kStages * BKV * D * 2 + 256;
-  auto kernel = attention_prefill_pingpong_kernel<D, NQ, BKV>;
+  auto kernel = attention_prefill_pingpong_kernel<D, NQ, BKV, false>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return static_cast<int>(e);
   const int pairs = (max_seq_len + NQ * BQ - 1) / (NQ * BQ);
@@ -366,7 +417,27 @@ int launch(const void* q, const void* k, const void* v, void* out, const int* cu
   const dim3 grid(q_heads, seqs, pairs);
   LRM_LAUNCH(kernel, grid, dim3(threads_per_cta(NQ)), smem, stream, map_q, map_k, map_v,
              static_cast<__nv_bfloat16*>(out), cu_seqlens, q_heads, kv_heads, scale * 1.4426950408889634f, window,
-             status);
+             status, Pages{});
+  return 0;
+}
+
+template <int D>
+int launch_paged(const void* q, const void* k_pages, const void* v_pages, long long page_rows, void* out, const int* cu_seqlens,
+                 const Pages& pages, int tokens, int seqs, int max_seq_len, int q_heads, int kv_heads, float scale, int window,
+                 int* status, cudaStream_t stream) {
+  constexpr int BKV = 64;
+  CUtensorMap map_q, map_k, map_v;
+  if (!make_map_bf16(&map_q, q, tokens, static_cast<long long>(q_heads) * D, BQ) ||
+      !make_map_bf16(&map_k, k_pages, page_rows, D, BKV) || !make_map_bf16(&map_v, v_pages, page_rows, D, BKV))
+    return LRM_UNSUPPORTED;
+  constexpr int smem = BQ * D * 2 + 2 * Shape<D, BKV>::kStages * BKV * D * 2 + 256;
+  auto kernel = attention_prefill_pingpong_kernel<D, 1, BKV, true>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  const int tiles = (max_seq_len + BQ - 1) / BQ;
+  if (seqs > 65535 || tiles > 65535) return LRM_UNSUPPORTED;
+  LRM_LAUNCH(kernel, dim3(q_heads, seqs, tiles), dim3(threads_per_cta(1)), smem, stream, map_q, map_k, map_v,
+             static_cast<__nv_bfloat16*>(out), cu_seqlens, q_heads, kv_heads, scale * 1.4426950408889634f, window, status, pages);
   return 0;
 }
 
@@ -410,5 +481,27 @@ LRM_API int lrm_attention_prefill_pingpong(const void* q, const void* k, const v
   if (d == 128)
     return launch<128, 2>(q, k, v, out, cu_seqlens, tokens, seqs, max_seq_len, q_heads, kv_heads, scale, window,
                           status, stream);
+  return LRM_UNSUPPORTED;
+}
+
+// Several queries per sequence over the paged cache: q [tokens, q_heads, d] packed by cu_seqlens, the queries of sequence b at
+// its last positions of kv_lens[b]; pages [n_pages][kv_heads][64][d] of keys and of values, page_table [slots][table_stride].
+LRM_API int lrm_attention_extend_umma(const void* q, const void* k_pages, const void* v_pages, int n_pages, void* out,
+                                      const int* cu_seqlens, const int* page_table, int table_stride, const int* slots,
+                                      const int* kv_lens, int tokens, int seqs, int max_seq_len, int q_heads, int kv_heads, int d,
+                                      int page_size, float scale, int window, int* status, cudaStream_t stream) {
+  if (seqs <= 0 || max_seq_len <= 0 || tokens <= 0) return 0;
+  if (q_heads <= 0 || kv_heads <= 0 || q_heads % kv_heads != 0 || n_pages <= 0 || status == nullptr) return LRM_BAD_ARGUMENT;
+  const long long rows = static_cast<long long>(n_pages) * kv_heads * 64;
+  if (page_size != 64 || window < 0 || q_heads > 65535 || rows >= (1ll << 31)) return LRM_UNSUPPORTED;
+  for (const void* p : {q, k_pages, v_pages, static_cast<const void*>(out)})
+    if (reinterpret_cast<uintptr_t>(p) % 16) return LRM_UNSUPPORTED;
+  const Pages pages{page_table, table_stride, slots, kv_lens};
+  if (d == 64)
+    return launch_paged<64>(q, k_pages, v_pages, rows, out, cu_seqlens, pages, tokens, seqs, max_seq_len, q_heads, kv_heads, scale,
+                            window, status, stream);
+  if (d == 128)
+    return launch_paged<128>(q, k_pages, v_pages, rows, out, cu_seqlens, pages, tokens, seqs, max_seq_len, q_heads, kv_heads, scale,
+                             window, status, stream);
   return LRM_UNSUPPORTED;
 }

@@ -8,9 +8,10 @@ prompts with head size 64 or 128 run the TMA + tcgen05 kernel
 A bfloat16 decode step of a layer that writes its own unwindowed cache runs rotation,
 cache write, attention and the merge of the splits as one cluster kernel
 (csrc/attention_decode_cluster.cu). A step that appends several tokens to started
-sequences stores its keys first and attends over the cache (row-wise, or the tiled
-extend kernel in bfloat16). bfloat16 attention over one key head whose rows also hold the
-values (latent attention's cache) runs csrc/attention_shared_keys.cu in every phase.
+sequences stores its keys first and attends over the cache (row-wise, or in bfloat16 the
+tiled extend kernel or, with head size 64 or 128, the tcgen05 prompt kernel over pages).
+bfloat16 attention over one key head whose rows also hold the values (latent attention's
+cache) runs csrc/attention_shared_keys.cu in every phase.
 Attention without a softmax (a key's weight is the sigmoid of its score) has kernels of its own in
 csrc/attention_sigmoid.cu: tiled in bfloat16 for head sizes 32, 64, 96 and 128, row-wise otherwise.
 Softmax attention with a cap on its scores, kept first keys or an output gate (and then also with sinks and
@@ -255,6 +256,26 @@ def decode(q, kv, out, slots, kv_lens, max_kv_len: int, scale: float, window: in
           "attention_paged_rowwise")
 
 
+EXTEND_UMMA_CTAS = 128
+
+
+def extends_on_tcgen05(q, kv, dv: int, seqs: int, max_seq_len: int, window: int, slopes, out_scale: float, extras, out) -> bool:
+    """True when a portion's attention over the paged cache runs on the tcgen05 kernel: at head size 128 whatever the
+    portion, at 64 where there are query tiles enough (a tile of 128 queries of one head walks its pages one after another,
+    two of them the warp-level kernel's). 32 heads on 8, us, warp-level against tcgen05: head size 128, 3,000 keys and 16
+    new tokens 95 and 69, 400 and 129 onto 3,000 and 1,111 keys 143 and 86, 1,000 onto 5,000 462 and 146, 2,000 onto 16,000
+    2796 and 785; head size 64, 65 onto 3,000 keys (32 CTAs) 53 and 63, eight times 16 onto 3,000 (256) 75 and 72, 400 and
+    129 onto 3,000 and 1,111 (256) 89 and 78, 1,000 onto 5,000 289 and 133."""
+    d = q.shape[2]
+    return (not force_rowwise and not force_warp_level and q.dtype == torch.bfloat16 and window >= 0 and extras.plain
+            and (d == 128 or q.shape[1] * seqs * -(-max_seq_len // 128) >= EXTEND_UMMA_CTAS)
+            and _plain(q, dv, slopes, out_scale) and kv.page_size == 64
+            and not getattr(kv, "values_in_keys", False) and kv.k.dtype == torch.bfloat16
+            and all(t.data_ptr() % 16 == 0 for t in (q, kv.k, kv.v, out))
+            and kv.k.shape[0] * kv.kv_heads * 64 < 2 ** 31 and seqs <= 65535
+            and bool(library.load().lrm_attention_prefill_pingpong_supports(d)))
+
+
 def extend(q, kv, out, cu_seqlens, seq_of_token, positions, slots, kv_lens, max_seq_len: int, scale: float,
            window: int, slopes=None, out_scale: float = 1.0, extras=None) -> None:
     """Packed queries, several per sequence, over the cache that already holds the step's keys."""
@@ -270,6 +291,15 @@ def extend(q, kv, out, cu_seqlens, seq_of_token, positions, slots, kv_lens, max_
                                             cu_seqlens.numel() - 1, max_seq_len, Hq, d, dv, ctypes.c_float(scale),
                                             window, None, 1, _ptr(extras.sinks), _stream()),
               "attention_shared_keys")
+        return
+    if extends_on_tcgen05(q, kv, dv, cu_seqlens.numel() - 1, max_seq_len, window, slopes, out_scale, extras, out):
+        from . import gemm_dispatch
+        gemm_dispatch.mark_status_dirty()
+        _done(lib.lrm_attention_extend_umma(_ptr(q), _ptr(kv.k), _ptr(kv.v), kv.k.shape[0], _ptr(out), _ptr(cu_seqlens),
+                                            _ptr(kv.page_table), kv.page_table.shape[1], _ptr(slots), _ptr(kv_lens), T,
+                                            cu_seqlens.numel() - 1, max_seq_len, Hq, kv.kv_heads, d, kv.page_size,
+                                            ctypes.c_float(scale), window, _ptr(gemm_dispatch._status_word(q.device)),
+                                            _stream()), "attention_extend_umma")
         return
     if dv == d and _tiled(q, kv.page_size):
         _done(lib.lrm_attention_extend_tiled(_ptr(q), _ptr(kv.k), _ptr(kv.v), _ptr(out), _ptr(cu_seqlens),
