@@ -69,13 +69,12 @@ __global__ __launch_bounds__(256) void gemm_f32_kernel(const float* __restrict__
   }
 }
 
-// The tiled kernel for prompts: BM x BN outputs per CTA, 8 x 8 per thread (a warp covers 32 x 64), K in
+// The tiled kernel for prompts: BM x BN outputs per CTA, 8 x TN per thread (a warp covers 32 x 8 TN), K in
 // blocks of 16 through two shared-memory buffers laid out [k][row]. Blocks are on their way to registers two
 // ahead of the multiplications, the fragments of the next k one ahead. Two neighbouring columns are one
 // fma.rn.f32x2, two IEEE float32 FMAs in one instruction; an element still adds its products over k in
-// ascending order, so all tile sizes give the same bits. A tile of 128 x 64 or two of 64 x 64 keep one warp
-// on each of an SM's schedulers, which is what bounds it (an issue every 2.9 cycles, 2 of them the FMAs
-// themselves). 384 rows, us, 64 x 64 tiles of 4 x 4 per thread and scalar loads before: 3072 x 2048 126
+// ascending order, so all tile sizes give the same bits. A tile of 128 x 64 keeps one warp on each of an SM's
+// schedulers, which is what bounds it (an issue every 2.9 cycles, 2 of them the FMAs themselves). 384 rows, us, 64 x 64 tiles of 4 x 4 per thread and scalar loads before: 3072 x 2048 126
 // (252), 16384 x 2048 607 (1248), 2048 x 8192 488 (1045); blocks one ahead only: 139, 637, 673.
 constexpr int TK = 16, PAD = 4;
 
@@ -89,23 +88,23 @@ __device__ __forceinline__ unsigned long long twice(float v) {
 }
 
 // VEC: rows of X, W and C start on 16-byte boundaries (K and N multiples of 4).
-template <int BM_, int BN_, bool VEC>
-__global__ __launch_bounds__(BM_ * BN_ / 64, BM_ == 128 ? 2 : 4) void gemm_f32_tiled_kernel(
+template <int BM_, int BN_, int TN, bool VEC>
+__global__ __launch_bounds__(BM_ * BN_ / (8 * TN), BM_ == 128 ? 2 : 4) void gemm_f32_tiled_kernel(
     const float* __restrict__ X, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K, int mode,
     int group_cols, int group_rows) {
-  constexpr int THREADS = BM_ * BN_ / 64, XL = BM_ * TK / 4 / THREADS, WL = BN_ * TK / 4 / THREADS;
+  constexpr int THREADS = BM_ * BN_ / (8 * TN), XL = BM_ * TK / 4 / THREADS, WL = BN_ * TK / 4 / THREADS;
   __shared__ __align__(16) float Xs[2][TK][BM_ + PAD];
   __shared__ __align__(16) float Ws[2][TK][BN_ + PAD];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  static_assert(BN_ == 64, "a warp covers the tile's columns");
-  const int m_in = warp * 32 + (lane >> 3) * 4, n_in = (lane & 7) * 4;
+  constexpr int WARPS_N = BN_ / (8 * TN), HALVES = TN / 4;  // warps side by side, pieces of 4 columns a thread has
+  const int m_in = warp / WARPS_N * 32 + (lane >> 3) * 4, n_in = warp % WARPS_N * 8 * TN + (lane & 7) * 4;
   const int m0 = blockIdx.y * BM_, n0 = blockIdx.x * BN_;
   if (group_cols > 0) X += static_cast<size_t>(n0 / group_cols) * group_rows * K;
-  unsigned long long acc[8][4];
+  unsigned long long acc[8][2 * HALVES];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+    for (int j = 0; j < 2 * HALVES; ++j) acc[i][j] = 0ull;
 
   float4 x0[XL], w0[WL], x1[XL], w1[WL];  // two blocks under way
   auto piece = [&](const float* __restrict__ base, int row, int rows, int k) {
@@ -147,12 +146,12 @@ __global__ __launch_bounds__(BM_ * BN_ / 64, BM_ == 128 ? 2 : 4) void gemm_f32_t
     }
   };
   float4 a[2][2];
-  ulonglong2 b[2][2];
+  ulonglong2 b[2][HALVES];
   auto fragments = [&](int slot, int buffer, int kk) {
     a[slot][0] = *reinterpret_cast<const float4*>(&Xs[buffer][kk][m_in]);
     a[slot][1] = *reinterpret_cast<const float4*>(&Xs[buffer][kk][m_in + 16]);
-    b[slot][0] = *reinterpret_cast<const ulonglong2*>(&Ws[buffer][kk][n_in]);
-    b[slot][1] = *reinterpret_cast<const ulonglong2*>(&Ws[buffer][kk][n_in + 32]);
+#pragma unroll
+    for (int j = 0; j < HALVES; ++j) b[slot][j] = *reinterpret_cast<const ulonglong2*>(&Ws[buffer][kk][n_in + 32 * j]);
   };
   // Block k0 lies in `buffer`; block k0 + TK is in `xn`, `wn` and goes to the other buffer (all threads are past the
   // barrier behind that buffer's last reads); block k0 + 2 TK is asked for into `xm`, `wm`.
@@ -172,10 +171,8 @@ __global__ __launch_bounds__(BM_ * BN_ / 64, BM_ == 128 ? 2 : 4) void gemm_f32_t
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const unsigned long long aa = twice(rows[i]);
-        fma2(acc[i][0], aa, b[kk & 1][0].x);
-        fma2(acc[i][1], aa, b[kk & 1][0].y);
-        fma2(acc[i][2], aa, b[kk & 1][1].x);
-        fma2(acc[i][3], aa, b[kk & 1][1].y);
+#pragma unroll
+        for (int j = 0; j < HALVES; ++j) fma2(acc[i][2 * j], aa, b[kk & 1][j].x), fma2(acc[i][2 * j + 1], aa, b[kk & 1][j].y);
       }
     }
   };
@@ -193,7 +190,7 @@ __global__ __launch_bounds__(BM_ * BN_ / 64, BM_ == 128 ? 2 : 4) void gemm_f32_t
     const int m = m0 + m_in + (i & 3) + (i >> 2) * 16;
     if (m >= M) continue;
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
+    for (int half = 0; half < HALVES; ++half) {
       const int n = n0 + n_in + half * 32;
       float* dst = C + static_cast<size_t>(m) * N + n;
       float v[4];
@@ -217,27 +214,27 @@ __global__ __launch_bounds__(BM_ * BN_ / 64, BM_ == 128 ? 2 : 4) void gemm_f32_t
   }
 }
 
-template <int BM_, int BN_>
+template <int BM_, int BN_, int TN>
 int launch_tiled(const float* X, const float* W, float* C, int M, int N, int K, int mode, int group_cols, int group_rows,
                  bool vec, cudaStream_t stream) {
   const dim3 grid((N + BN_ - 1) / BN_, (M + BM_ - 1) / BM_);
   // Launched behind the kernel before, not beside it: let in early, CTAs pile up on the SMs that kernel leaves first,
   // and a step whose tiles fill the SMs once then takes two rounds (384 x 3072 x 2048: 203 us against 126).
   if (vec)
-    gemm_f32_tiled_kernel<BM_, BN_, true><<<grid, BM_ * BN_ / 64, 0, stream>>>(X, W, C, M, N, K, mode, group_cols, group_rows);
+    gemm_f32_tiled_kernel<BM_, BN_, TN, true><<<grid, BM_ * BN_ / (8 * TN), 0, stream>>>(X, W, C, M, N, K, mode, group_cols, group_rows);
   else
-    gemm_f32_tiled_kernel<BM_, BN_, false><<<grid, BM_ * BN_ / 64, 0, stream>>>(X, W, C, M, N, K, mode, group_cols, group_rows);
+    gemm_f32_tiled_kernel<BM_, BN_, TN, false><<<grid, BM_ * BN_ / (8 * TN), 0, stream>>>(X, W, C, M, N, K, mode, group_cols, group_rows);
   LRM_LAUNCH_CHECK();
   return 0;
 }
 
-// Tiles of the busiest SM times a tile's size: 128 x 64 where that is no more work than in 64 x 64 tiles, whose
-// operands are read more often (but a lone 64 x 64 tile has only two warps for the four schedulers).
+// 128 x 64 tiles (8 x 8 outputs per thread) where the busiest SM has no more work with them than with 64 x 64 tiles of 8 x 4,
+// which read their operands more often. us, 128 x 64 against 64 x 64: 512 rows of 16384 x 2048 702 and 757, 384 rows of
+// 3072 x 2048 127 and 125; 128 rows of 2048 x 8192 (32 and 64 tiles) 491 and 306, 64 rows of 3072 x 2048 121 and 78.
 bool prefers_wide_tile(int M, int N) {
   const long long wide = static_cast<long long>((M + 127) / 128) * ((N + 63) / 64);
   const long long small = static_cast<long long>((M + 63) / 64) * ((N + 63) / 64);
-  const long long rounds = (small + 147) / 148;
-  return 2 * ((wide + 147) / 148) <= (rounds > 2 ? rounds : 2);
+  return 2 * ((wide + 147) / 148) <= (small + 147) / 148;
 }
 
 // Few rows (a head's logits, decoding): bound by reading W. A CTA owns 32 columns, a lane each, and its warps
@@ -329,8 +326,8 @@ LRM_API int lrm_gemm_f32_grouped(const float* X, const float* W, float* C, int M
   const bool rows_aligned = K % 4 == 0 && aligned(X) && aligned(W);
   if (M > kFewRows) {
     const bool vec = rows_aligned && N % 4 == 0 && aligned(C);
-    if (prefers_wide_tile(M, N)) return launch_tiled<128, 64>(X, W, C, M, N, K, mode, group_cols, group_rows, vec, stream);
-    return launch_tiled<64, 64>(X, W, C, M, N, K, mode, group_cols, group_rows, vec, stream);
+    if (prefers_wide_tile(M, N)) return launch_tiled<128, 64, 8>(X, W, C, M, N, K, mode, group_cols, group_rows, vec, stream);
+    return launch_tiled<64, 64, 4>(X, W, C, M, N, K, mode, group_cols, group_rows, vec, stream);
   }
   if (rows_aligned) {
     if (M <= 4) return launch_few<1>(X, W, C, M, N, K, mode, group_cols, group_rows, stream);
