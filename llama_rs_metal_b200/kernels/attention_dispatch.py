@@ -3,7 +3,7 @@
 The row-wise kernel (csrc/attention_rowwise.cu) takes every head size up to
 512 and both dtypes, and is the only attention of the float32 path. bfloat16
 prompts with head size 64 or 128 run the TMA + tcgen05 kernel
-(csrc/attention_prefill_umma.cu); bfloat16 with head size 32, 64 or 128 and
+(csrc/attention_prefill_pingpong.cu); bfloat16 with head size 32, 64 or 128 and
 64-token pages otherwise runs the warp-level tiled kernels (csrc/attention_tiled.cu).
 A bfloat16 decode step of a layer that writes its own unwindowed cache runs rotation,
 cache write, attention and the merge of the splits as one cluster kernel
@@ -42,7 +42,8 @@ force_shared_key_splits = None  # tests fix the splits of the shared-key kernel'
 force_sigmoid_ranks = None  # tests fix the CTAs per cluster of the sigmoid decode kernel
 force_gated_split = False  # tests keep decode steps of that kernel behind a split of the projection in its own launch
 force_gated_ranks = None  # tests fix the CTAs per cluster of the gated softmax kernel's decode step
-prefill_kernel = None  # tests pin the tcgen05 prompt kernel: "pingpong" or "single" (None: the rule in prefill())
+prefill_kernel = None  # tests pin the form of the tcgen05 prompt kernel: "single" (two chains per query tile), "pingpong" (a
+# chain per query tile, two tiles at head size 128) or "chain" (one chain); None: the rule beside the kernel
 
 
 @dataclass(frozen=True)
@@ -158,35 +159,15 @@ def prefill(q, k, v, out, cu_seqlens, seq_of_token, max_seq_len: int, scale: flo
     dv = v.shape[2]
     aligned = all(t.data_ptr() % 16 == 0 for t in (q, k, v, out))
     if (not force_rowwise and not force_warp_level and q.dtype == torch.bfloat16 and aligned and window >= 0
-            and _plain(q, dv, slopes, out_scale) and lib.lrm_attention_prefill_umma_supports(d)):
+            and _plain(q, dv, slopes, out_scale) and lib.lrm_attention_prefill_pingpong_supports(d)):
         from . import gemm_dispatch
         gemm_dispatch.mark_status_dirty()
-        # Two tcgen05 kernels. The one that keeps probabilities and output in tensor memory wins on
-        # long prompts and on batches of prompts: at head size 128 (one query tile per CTA on key tiles
-        # of 64 up to 2,304 tokens, two query tiles taking turns beyond) from 1,536 tokens on (2,048
-        # tokens 60 against 86 us, 953 against 582 TFLOP/s at 32,768); at head size 64 (four CTAs per SM on key tiles of 64) beyond 2,048 tokens (3,072
-        # tokens 78 against 100 us, 681 against 534 TFLOP/s at 32,768) and whenever several prompts
-        # are packed (four of 512 tokens 20 against 29 us, eight of 128 tokens 9.5 against 11.1). A
-        # single short prompt is bound by the chain of key tiles of its last query tile, which the
-        # older kernel, with two threads per row, walks a little faster (1,024 tokens 24 against 26 us).
-        # Packed prompts go to the newer kernel at head size 128 too (four of 512 tokens 33 against 46 us).
-        # (several prompts: the packed tokens are well more than the longest prompt; a short prompt
-        # filled up to whole rows with a few tokens of padding does not count)
-        pingpong = (max_seq_len >= 1536 if d == 128 else max_seq_len > 2048) or 4 * T >= 5 * max_seq_len
-        if prefill_kernel is not None:
-            pingpong = prefill_kernel == "pingpong"
-        if pingpong:
-            _done(lib.lrm_attention_prefill_pingpong(_ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(cu_seqlens), T,
-                                                     cu_seqlens.numel() - 1, max_seq_len, Hq, k.shape[1], d,
-                                                     ctypes.c_float(scale), window,
-                                                     _ptr(gemm_dispatch._status_word(q.device)), _stream()),
-                  "attention_prefill_pingpong")
-            return
-        _done(lib.lrm_attention_prefill_umma(_ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(cu_seqlens), T,
-                                             cu_seqlens.numel() - 1, max_seq_len, Hq, k.shape[1], d,
-                                             ctypes.c_float(scale), window,
-                                             _ptr(gemm_dispatch._status_word(q.device)), _stream()),
-              "attention_prefill_umma")
+        form = {None: 0, "chain": 1, "single": 2, "pingpong": 3 if d == 128 else 1}[prefill_kernel]
+        _done(lib.lrm_attention_prefill_pingpong(_ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(cu_seqlens), T,
+                                                 cu_seqlens.numel() - 1, max_seq_len, Hq, k.shape[1], d,
+                                                 ctypes.c_float(scale), window, form,
+                                                 _ptr(gemm_dispatch._status_word(q.device)), _stream()),
+              "attention_prefill_pingpong")
         return
     if dv == d and _tiled(q, 64):
         _done(lib.lrm_attention_prefill_tiled(_ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(cu_seqlens),

@@ -93,8 +93,6 @@ WORK: Dict[str, Callable[..., Tuple[float, float]]] = {
     "lrm_silu_mul": lambda a: (3.0 * _v(a[3]) * _v(a[4]) * _ELEM[_v(a[2])], 0),
     "lrm_add_planes": lambda a: ((_v(a[2]) + 2.0) * _v(a[3]) * 4, 0),
     # prompts: q, k, v, out once; 4 flops per (query, key, head dimension) pair of the causal triangle
-    "lrm_attention_prefill_umma": lambda a: (2.0 * _v(a[5]) * 2 * (_v(a[8]) + _v(a[9])) * _v(a[10]),
-                                             4.0 * hints["pairs"] * _v(a[8]) * _v(a[10])),
     "lrm_attention_prefill_pingpong": lambda a: (2.0 * _v(a[5]) * 2 * (_v(a[8]) + _v(a[9])) * _v(a[10]),
                                                  4.0 * hints["pairs"] * _v(a[8]) * _v(a[10])),
     "lrm_attention_prefill_tiled": lambda a: (0, 4.0 * hints["pairs"] * _v(a[7]) * _v(a[9])),
