@@ -11,7 +11,9 @@
 //   O += P V_j     tcgen05.mma with P read from tensor memory as the A operand and V from
 //                  shared memory as an MN-major operand exactly as TMA laid it down; O stays
 //                  in tensor memory for the whole row of key tiles
-// Every step waits for the one before it, some 3,000 cycles per 64 keys, so what bounds a prompt is
+// Every step waits for the one before it, some 2,500 cycles per 64 keys (of a lone CTA: 310 until the issuer sees the
+// probabilities, 180 and 175 to issue the two products, 285 until the scores are there, 120 for the load, 180 for the
+// maximum, 400 for a rescaling, 740 for the probabilities, which the 2^x unit needs 512 for), so what bounds a prompt is
 // how many such chains an SM has under way and how long the longest is. Three forms:
 //   two chains per query tile   key tiles of 64, the even ones one chain and the odd ones the other,
 //                               each with its own maximum, mass and O; at the end the two threads of a
@@ -245,82 +247,86 @@ void attention_prefill_pingpong_kernel(
       }
     }
   } else if (warp == kIssuerWarp) {
-    if (lane == 0) {
-      // ---- one thread drives the tensor core
-      constexpr uint32_t idesc_s = umma_idesc(BQ, BKV);            // both K-major
-      constexpr uint32_t idesc_pv = umma_idesc(BQ, D, true);       // V is MN-major
-      auto scores = [&](int i, int j) {  // S_i = Q_i K_j^T
-        const uint32_t qa = smem_u32(q_tiles + (NQ == 2 ? i * TILE : 0)), ka = smem_u32(kv_tiles + (j % STAGES) * 2 * KV_TILE);
+    // ---- one thread drives the tensor core. The warp stays together around it, so that descriptors are computed once per
+    // warp: with a branch of one lane around the loop a product's four MMAs took 340 cycles to issue.
+    constexpr uint32_t idesc_s = umma_idesc(BQ, BKV);            // both K-major
+    constexpr uint32_t idesc_pv = umma_idesc(BQ, D, true);       // V is MN-major
+    const uint32_t q_at = smem_u32(q_tiles), kv_at = smem_u32(kv_tiles);
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+    const int tiles = __shfl_sync(0xffffffffu, n_tiles, 0), last0 = __shfl_sync(0xffffffffu, n0, 0) - 1,
+              last1 = __shfl_sync(0xffffffffu, n1, 0) - 1;
+    const bool leader = elect_one();
+    auto wait = [&](uint64_t* bar, int parity, int where) {
+      const bool ok = __all_sync(0xffffffffu, mbar_wait(bar, parity, status, where));
+      tc_fence_after();
+      return ok;
+    };
+    auto scores = [&](int i, int j) {  // S_i = Q_i K_j^T
+      const uint32_t qa = q_at + (NQ == 2 ? i * TILE : 0), ka = kv_at + (j % STAGES) * 2 * KV_TILE;
+      if (leader) {
 #pragma unroll
         for (int k = 0; k < D / UMMA_K; ++k) {  // 64-column block, then 32 bytes per step
           const uint32_t step = (k % 4) * UMMA_K * 2;
-          umma_bf16(tmem_s(i), smem_desc(qa + (k / 4) * BLOCK + step), smem_desc(ka + (k / 4) * KV_BLOCK + step),
+          umma_bf16(tmem + i * BKV, smem_desc(qa + (k / 4) * BLOCK + step), smem_desc(ka + (k / 4) * KV_BLOCK + step),
                     idesc_s, k > 0 ? 1u : 0u);
         }
         umma_commit(s_full + i);
-      };
-      auto weighted = [&](int i, int j) {  // O_i (+)= P_i V_j, P from tensor memory (8 columns per 16 keys)
-        const uint32_t va = smem_u32(kv_tiles + (j % STAGES) * 2 * KV_TILE + KV_TILE);
+      }
+    };
+    auto weighted = [&](int i, int j) {  // O_i (+)= P_i V_j, P from tensor memory (8 columns per 16 keys)
+      const uint32_t va = kv_at + (j % STAGES) * 2 * KV_TILE + KV_TILE;
+      if (leader) {
 #pragma unroll
         for (int k = 0; k < BKV / UMMA_K; ++k)
-          umma_bf16_a_tmem(tmem_o(i), tmem_s(i) + k * (UMMA_K / 2), smem_desc(va + k * UMMA_K * 128, KV_BLOCK),
-                           idesc_pv, (j >= CHAINS / NQ || k > 0) ? 1u : 0u);
-      };
-      bool ok = mbar_wait(q_full, 0, status, kStuckQ) && mbar_wait(kv_full, 0, status, kStuckKV);
-      if (ok) {
-        tc_fence_after();
-        scores(0, 0);
-        if (NQ == 2 && n1 > 0) scores(1, 0);
+          umma_bf16_a_tmem(tmem + CHAINS * BKV + i * D, tmem + i * BKV + k * (UMMA_K / 2),
+                           smem_desc(va + k * UMMA_K * 128, KV_BLOCK), idesc_pv, (j >= CHAINS / NQ || k > 0) ? 1u : 0u);
       }
-      if constexpr (NQ == 1) {  // key tile t belongs to chain t % CHAINS
-        if (CHAINS == 2 && ok && n_tiles > 1) {
-          ok = mbar_wait(kv_full + 1, 0, status, kStuckKV);
-          tc_fence_after();
-          if (ok) scores(1, 1);
-        }
-        for (int t = 0; t < n_tiles && ok; ++t) {
-          const int i = t % CHAINS, next = t + CHAINS;
-          ok = mbar_wait(p_ready + i, (t / CHAINS) & 1, status, kStuckProbabilities);
-          if (!ok) break;
-          tc_fence_after();
-          weighted(i, t);
-          if (next >= n_tiles) umma_commit(o_done + i);
-          umma_commit(kv_free + t % STAGES);
-          if (next < n_tiles) {
-            ok = mbar_wait(kv_full + next % STAGES, (next / STAGES) & 1, status, kStuckKV);
-            if (!ok) break;
-            tc_fence_after();
-            scores(i, next);
-          }
-        }
+    };
+    auto commit = [&](uint64_t* bar) {
+      if (leader) umma_commit(bar);
+    };
+    bool ok = wait(q_full, 0, kStuckQ) && wait(kv_full, 0, kStuckKV);
+    if (ok) scores(0, 0);
+    if constexpr (NQ == 1) {  // key tile t belongs to chain t % CHAINS
+      if (CHAINS == 2 && ok && tiles > 1) {
+        ok = wait(kv_full + 1, 0, kStuckKV);
+        if (ok) scores(1, 1);
       }
-      for (int j = 0; NQ == 2 && j < n_tiles && ok; ++j) {
-        const bool more0 = j + 1 < n0, more1 = j + 1 < n1;
-        if (j < n0) {
-          ok = mbar_wait(p_ready + 0, j & 1, status, kStuckProbabilities);
+      for (int t = 0; t < tiles && ok; ++t) {
+        const int i = t % CHAINS, next = t + CHAINS;
+        if (next < tiles) ok = wait(kv_full + next % STAGES, (next / STAGES) & 1, kStuckKV);
+        ok = ok && wait(p_ready + i, (t / CHAINS) & 1, kStuckProbabilities);
+        if (!ok) break;
+        weighted(i, t);
+        if (next < tiles) scores(i, next);
+        else commit(o_done + i);
+        commit(kv_free + t % STAGES);
+      }
+    } else {
+      if (ok && last1 >= 0) scores(1, 0);
+      for (int j = 0; j < tiles && ok; ++j) {
+        if (j <= last0) {
+          ok = wait(p_ready + 0, j & 1, kStuckProbabilities);
           if (!ok) break;
-          tc_fence_after();
           weighted(0, j);
-          if (j == n0 - 1) umma_commit(o_done + 0);
+          if (j == last0) commit(o_done + 0);
         }
-        if (more0 || more1) {  // the next key tile has to be here for the next scores
-          ok = mbar_wait(kv_full + (j + 1) % STAGES, ((j + 1) / STAGES) & 1, status, kStuckKV);
+        if (j < last0 || j < last1) {  // the next key tile has to be here for the next scores
+          ok = wait(kv_full + (j + 1) % STAGES, ((j + 1) / STAGES) & 1, kStuckKV);
           if (!ok) break;
-          tc_fence_after();
         }
-        if (more0) scores(0, j + 1);
-        if (j < n1) {
-          ok = mbar_wait(p_ready + 1, j & 1, status, kStuckProbabilities);
+        if (j < last0) scores(0, j + 1);
+        if (j <= last1) {
+          ok = wait(p_ready + 1, j & 1, kStuckProbabilities);
           if (!ok) break;
-          tc_fence_after();
           weighted(1, j);
-          if (j == n1 - 1) umma_commit(o_done + 1);
+          if (j == last1) commit(o_done + 1);
         }
-        umma_commit(kv_free + j % STAGES);  // every product that reads stage j has been issued
-        if (more1) scores(1, j + 1);
+        commit(kv_free + j % STAGES);  // every product that reads stage j has been issued
+        if (j < last1) scores(1, j + 1);
       }
-      if (!ok) *bail = 1;
     }
+    if (!ok) *bail = 1;
   } else {
     // ---- softmax and output: one thread per query row and chain. Warps 0-3 own chain 0, warps 4-7 chain 1;
     // a warp may touch the quarter of the tensor memory's lanes given by its index modulo 4.
@@ -373,7 +379,8 @@ void attention_prefill_pingpong_kernel(
       const float mx = fmaxf(fmaxf(most[0], most[1]), fmaxf(most[2], most[3]));
       m_run = fmaxf(m_run, mx * scale_log2);
       // bring O and the mass to the new maximum only when it has moved far (always for the first
-      // tile, where O holds nothing yet and only the reference is set)
+      // tile, where O holds nothing yet and only the reference is set); here, since behind the probabilities it was slower
+      // (8,192 tokens of head size 64 378 us, here 366)
       const bool far = m_run > m_ref + rescale_step;
       if (j == 0) {
         m_ref = m_run;
@@ -598,7 +605,8 @@ LRM_API int lrm_attention_prefill_pingpong(const void* q, const void* k, const v
   const float step = single && max_seq_len <= (d == 64 ? 2048 : 1535) ? 0.f : 8.f;
   if (form == 0) {
     if (d == 64) {
-      // us, one chain and two: 2,048 tokens of 32 heads 52 and 41, 8,192 422 and 388, two prompts of 1,000 31 and 28; but
+      // us, one chain and two (the issuing thread then a lane's branch): 2,048 tokens of 32 heads 52 and 41, 8,192 422 and 388,
+      // two prompts of 1,000 31 and 28; but
       // four of 512 18.6 and 20.2, sixteen of 256 26 and 29 (more CTAs than two rounds' worth, short ones).
       form = !single && max_seq_len <= 768 && ctas > 2 * 148 ? 1 : 2;
     } else {

@@ -57,6 +57,12 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
       ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
 }
+// True in one lane of a whole warp, the same every time.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
+}
 // Tensor memory is handed out in powers of two of at least 32 columns.
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst, uint32_t columns) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst)),
