@@ -3,6 +3,8 @@
 * up to 8 rows (small decode batches): the weight-streaming kernel
   (csrc/gemm_bf16_stream.cu); it also takes 9-64 rows when the tensor-core kernel would
   leave most SMs idle and cannot split K (few output columns, epilogue other than "add");
+* up to 64 rows of products large enough: tcgen05 with the weights as its wide operand
+  (csrc/gemm_bf16_few.cu; few_takes says where it is the faster one);
 * more rows (prompts, larger decode batches): the TMA + tcgen05 kernel
   (csrc/gemm_bf16_umma.cu), with 128 x 128, 128 x 256 or 256 x 256 tiles, whichever needs less
   time by a count of rounds over the SMs and the measured cost of a tile;
@@ -69,8 +71,10 @@ def check_status() -> None:
                           35: "a free accumulator"})
             names.update({41: "the query tile", 42: "a key/value tile", 43: "scores", 44: "probabilities", 45: "the output",
                           46: "a free key/value stage", 47: "aligned shared memory"})
-            kernel = "attention_gated_umma" if code >= 41 else "gemm_bf16_umma_pair" if code >= 31 else "attention_prefill_pingpong" if code >= 21 else \
-                "gemm_bf16_umma"
+            names.update({51: "a free stage", 52: "operand tiles", 53: "the accumulator", 54: "copies in flight",
+                          55: "a free accumulator"})
+            kernel = "gemm_bf16_few" if code >= 51 else "attention_gated_umma" if code >= 41 else "gemm_bf16_umma_pair" \
+                if code >= 31 else "attention_prefill_pingpong" if code >= 21 else "gemm_bf16_umma"
             raise LlamaError(f"{kernel} gave up waiting for {names.get(code, code)}; its result is invalid")
 
 
@@ -154,6 +158,49 @@ def _few_rows_plan(M: int, N: int, K: int, mode: int):
         k_blocks = -(-K // 64)
         return True, max(1, min(k_blocks, 64, SM_COUNT // tiles))
     return False, 1
+
+
+def few_takes(M: int, N: int, K: int, mode: int) -> bool:
+    """Where the kernel with the weights as the wide tcgen05 operand is the faster one for up to 64 rows. Its ring holds
+    200 KB per SM on their way and reads at 6.2 TB/s, but it takes about 2 us to begin and to drain its accumulator, more
+    where a cluster shares a tile. In a chain of products, us, against the kernels it replaces: 28672 x 4096 with the SiLU
+    gate 8 rows 44.4 (49.5), 32 rows 48.7 (51.7), 64 rows 55.3 (52.2); 32768 x 4096 in float32 16 rows 46.0 (51.7), 32 rows
+    48.3 (52.4), 64 rows the same; 128256 x 2048 32 rows 86.0 (92.8), 64 rows 91.7 (96.9); 16384 x 2048 gated 8 rows 14.3
+    (13.7), 16 rows 15.4 (17.2), 32 rows 17.9 (17.2); 6144 x 4096 16 rows 16.8 (16.9), 32 rows 20.6 (22.2), 64 rows 28.0
+    (41.0); 3072 x 2048 32 rows 11.4 (8.8). A decode step of 32 sequences, two layers of the 8B shape:
+    541 us, 550 without. float32 results whose sums over K the streaming kernel cuts among its warps stay
+    there: here one sum runs over all of K in the tensor core."""
+    elements = N * K
+    if -(-N // 128) >= SM_COUNT // 2:  # no clusters
+        if M <= 12:
+            return mode in (0, 3) and elements >= 60e6
+        return mode in (0, 1, 3) and elements >= (30e6 if M <= 16 else 100e6 if M <= 32 else 200e6)
+    return mode == 0 and M > 16 and elements >= 15e6
+
+
+def _few(x: torch.Tensor, weight: torch.Tensor, mode: int, lib) -> bool:
+    M, K = x.shape
+    N = weight.shape[0]
+    return (M <= 64 and not force_tiled and not force_stream and stream_shape is None and umma_width is None
+            and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0 and few_takes(M, N, K, mode)
+            and bool(lib.lrm_gemm_bf16_few_supports(M, N, K)))
+
+
+def _held_rows(x: torch.Tensor) -> int:
+    """Rows of x, beyond its own, that its storage holds, up to 32 (they may be named in a tensor map)."""
+    M, K = x.shape
+    held = (x.untyped_storage().nbytes() // x.element_size() - x.storage_offset()) // K
+    return min(max(M, 32), max(M, held))
+
+
+def gemm_bf16_few(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, mode: int, ranks: int = 0) -> None:
+    """gemm_bf16 for up to 64 rows on the kernel with the weights as the wide operand; `ranks` CTAs share a tile of 128
+    weight rows (0: the kernel's rule)."""
+    M, K = x.shape
+    lib = library.load()
+    mark_status_dirty()
+    _done(lib.lrm_gemm_bf16_few(_ptr(x), _ptr(weight), _ptr(out), M, _held_rows(x), weight.shape[0], K, mode, ranks,
+                                _ptr(_status_word(x.device)), _stream()), "gemm_bf16_few")
 
 
 def _fast_kernels(x: torch.Tensor, weight: torch.Tensor, lib):
@@ -280,6 +327,9 @@ def gemm_bf16(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, mode: in
     M, K = x.shape
     N = weight.shape[0]
     lib = library.load()
+    if _few(x, weight, mode, lib):
+        gemm_bf16_few(x, weight, out, mode)
+        return
     stream_ok, umma_ok = _fast_kernels(x, weight, lib)
     tile, splits = tile_choice(M, N, K, mode, pair_room() if umma_ok and M > 64 else 0), 1
     if stream_ok and umma_ok and M > STREAM_ROWS and not force_stream:
