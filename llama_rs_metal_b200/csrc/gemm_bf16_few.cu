@@ -7,17 +7,14 @@
 // accumulator's lanes are weight rows: a thread has one output column for all activation rows, and neighbouring threads
 // neighbouring columns.
 //
-// Many column tiles: persistent, CTA b works on tiles b, b + gridDim.x, ..., two accumulators in turn. Few of them: a cluster
-// of CTAs shares a tile, each a contiguous range of K; the partial sums go through distributed shared memory to the CTA
-// that finishes their activation rows, which adds them in rank order. No atomics: the result is the same every time.
+// Persistent: CTA b works on tiles b, b + gridDim.x, ..., two accumulators in turn, so a tile's epilogue runs under the next
+// tile's reads. No atomics: the result is the same every time. (Narrow products, a cluster of CTAs to a tile with the partial
+// sums meeting in distributed shared memory: 6144 x 4096, 32 rows, 20.6 us against the streaming kernel's 22.2 alone, but a
+// whole step got slower, since the streaming kernels beside it need the shared memory for their L1.)
 //
 // Epilogues as in gemm_bf16_stream.cu: 0 bf16, 1 f32, 3 SiLU gate (blocks of 8 gate / 8 up rows alternate). Every mbarrier wait
 // is bounded. Its times beside those of the kernels it replaces stand at gemm_dispatch.few_takes.
-#include <cooperative_groups.h>
-
 #include "umma.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace {
 
@@ -30,8 +27,7 @@ struct Few {
   static constexpr int STAGES = NC == 16 ? 11 : NC == 32 ? 9 : 7;
   static constexpr uint32_t W_BYTES = kTileRows * BK * 2, STAGE_BYTES = W_BYTES + NC * BK * 2;
   static constexpr uint32_t SET = NC < 32 ? 32 : NC;                 // tensor memory columns of an accumulator
-  static constexpr int REGION = (NC + 8) * kTileRows;                // floats that a cluster's partial sums are sent into
-  static constexpr size_t BYTES = 1024 + STAGES * STAGE_BYTES + REGION * 4 + 256;
+  static constexpr size_t BYTES = 1024 + STAGES * STAGE_BYTES + 256;
 };
 
 __device__ __forceinline__ float silu_f32(float g) { return g / (1.0f + expf(-g)); }
@@ -59,20 +55,15 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
   pdl_trigger();
   extern __shared__ unsigned char smem_raw[];
   unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  float* region = reinterpret_cast<float*>(ring + STAGES * F::STAGE_BYTES);  // [CTA of the cluster][its rows][128]
-  uint64_t* full = reinterpret_cast<uint64_t*>(region + F::REGION);
+  uint64_t* full = reinterpret_cast<uint64_t*>(ring + STAGES * F::STAGE_BYTES);
   uint64_t* empty = full + STAGES;
   uint64_t* acc_full = empty + STAGES;  // [2]
   uint64_t* acc_free = acc_full + 2;    // [2] four warps arrive
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 2);
   volatile int* bail = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  cg::cluster_group cluster = cg::this_cluster();
-  const int ranks = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles = (N + kTileRows - 1) / kTileRows, k_blocks = (K + BK - 1) / BK;
-  const int first_tile = blockIdx.x / ranks, stride = gridDim.x / ranks;
-  const int per_rank = (k_blocks + ranks - 1) / ranks;  // (the host leaves no rank without a block)
-  const int kb_begin = rank * per_rank, num_kb = min(k_blocks, kb_begin + per_rank) - kb_begin;
+  const int first_tile = blockIdx.x, stride = gridDim.x, num_kb = k_blocks;
   const int early = min(num_kb, STAGES);  // stages of the first tile's weights asked for ahead of the wait
 
   if (threadIdx.x == 0) {
@@ -88,7 +79,7 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
     mbar_fence_init();
     for (int kb = 0; kb < early; ++kb) {
       mbar_expect_tx(full + kb, F::STAGE_BYTES);
-      tma_load_2d(ring + kb * F::STAGE_BYTES, &map_w, full + kb, (kb_begin + kb) * BK, first_tile * kTileRows);
+      tma_load_2d(ring + kb * F::STAGE_BYTES, &map_w, full + kb, kb * BK, first_tile * kTileRows);
     }
   }
   if (warp == 1) {
@@ -99,15 +90,13 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (ranks > 1) cluster.sync();  // everybody has started before anybody writes into a peer's region
-  pdl_wait();                     // X is read from here on
+  pdl_wait();  // X is read from here on
 
-  const int rows_each = (M + ranks - 1) / ranks;  // activation rows a CTA of a cluster finishes
   if (warp == 0) {
     if (lane == 0) {
       // The early stages' activations first, whatever happens: copies into those stages are under way.
       for (int kb = 0; kb < early; ++kb)
-        tma_load_2d(ring + kb * F::STAGE_BYTES + F::W_BYTES, &map_x, full + kb, (kb_begin + kb) * BK, 0);
+        tma_load_2d(ring + kb * F::STAGE_BYTES + F::W_BYTES, &map_x, full + kb, kb * BK, 0);
       uint32_t it = early;  // blocks asked for so far
       int from = early;
       for (int tile = first_tile; tile < tiles && !*bail; tile += stride, from = 0) {
@@ -118,8 +107,8 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
             break;
           }
           mbar_expect_tx(full + s, F::STAGE_BYTES);
-          tma_load_2d(ring + s * F::STAGE_BYTES, &map_w, full + s, (kb_begin + kb) * BK, tile * kTileRows);
-          tma_load_2d(ring + s * F::STAGE_BYTES + F::W_BYTES, &map_x, full + s, (kb_begin + kb) * BK, 0);
+          tma_load_2d(ring + s * F::STAGE_BYTES, &map_w, full + s, kb * BK, tile * kTileRows);
+          tma_load_2d(ring + s * F::STAGE_BYTES + F::W_BYTES, &map_x, full + s, kb * BK, 0);
         }
       }
       if (*bail) {  // wait (bounded) for the copies already in flight before the CTA may exit
@@ -175,12 +164,7 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
           const int m = c * 32 + i;
           if (m >= M) break;
           const float v = __uint_as_float(r[i]);
-          if (ranks == 1) {
-            finish(v, m, n, out, N, mode);
-          } else {
-            float* to = cluster.map_shared_rank(region, m / rows_each);
-            to[(rank * rows_each + m % rows_each) * kTileRows + place] = v;
-          }
+          finish(v, m, n, out, N, mode);
         }
       }
       tc_fence_before();
@@ -191,80 +175,19 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_base, 2 * F::SET);
-  if (ranks > 1) {
-    cluster.sync();  // every part has arrived
-    if (warp >= 2 && !*bail) {
-      const int place = (warp & 3) * 32 + lane, n = first_tile * kTileRows + place;
-      for (int i = 0; i < rows_each && rank * rows_each + i < M; ++i) {
-        float sum = 0.f;
-        for (int u = 0; u < ranks; ++u) sum += region[(u * rows_each + i) * kTileRows + place];
-        finish(sum, rank * rows_each + i, n, out, N, mode);
-      }
-    }
-  }
 }
 
 template <int NC>
-cudaError_t prepare() {
-  cudaError_t e = cudaFuncSetAttribute(gemm_bf16_few_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(Few<NC>::BYTES));
-  return e;
-}
-
-template <int NC>
-void fill_config(cudaLaunchConfig_t& config, cudaLaunchAttribute* attributes, int ctas, int ranks, cudaStream_t stream) {
-  config.gridDim = dim3(ctas);
-  config.blockDim = dim3(kThreads);
-  config.dynamicSmemBytes = Few<NC>::BYTES;
-  config.stream = stream;
-  attributes[0].id = cudaLaunchAttributeClusterDimension;
-  attributes[0].val.clusterDim.x = ranks;
-  attributes[0].val.clusterDim.y = 1;
-  attributes[0].val.clusterDim.z = 1;
-  attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attributes[1].val.programmaticStreamSerializationAllowed = 1;
-  config.attrs = attributes;
-  config.numAttrs = g_lrm_pdl ? 2 : 1;
-}
-
-// Clusters of `ranks` CTAs that the device holds at once.
-template <int NC>
-int room(int ranks) {
-  static int held[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  if (held[ranks] == 0) {
-    cudaLaunchConfig_t config = {};
-    cudaLaunchAttribute attributes[2];
-    fill_config<NC>(config, attributes, ranks, ranks, nullptr);
-    config.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_bf16_few_kernel<NC>, &config) != cudaSuccess) {
-      cudaGetLastError();
-      n = 0;
-    }
-    held[ranks] = n > 0 ? n : -1;
-  }
-  return held[ranks];
-}
-
-template <int NC>
-int launch(const void* X, const void* W, void* out, int M, int x_rows, int N, int K, int mode, int ranks, int* status,
-           cudaStream_t stream) {
+int launch(const void* X, const void* W, void* out, int M, int x_rows, int N, int K, int mode, int* status, cudaStream_t stream) {
   CUtensorMap map_w, map_x;
   if (!make_map_bf16(&map_w, W, N, K, kTileRows) || !make_map_bf16(&map_x, X, x_rows, K, NC)) return LRM_UNSUPPORTED;
-  cudaError_t e = prepare<NC>();
+  auto kernel = gemm_bf16_few_kernel<NC>;
+  constexpr int smem = static_cast<int>(Few<NC>::BYTES);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return static_cast<int>(e);
-  const int tiles = (N + kTileRows - 1) / kTileRows, k_blocks = (K + BK - 1) / BK;
-  if (ranks == 0) {  // as many CTAs to a tile as let all tiles run at once, none with less than four blocks of K
-    ranks = 1;
-    for (int r = 2; r <= 8; ++r)
-      if (tiles <= room<NC>(r) && k_blocks >= 4 * r && (r - 1) * ((k_blocks + r - 1) / r) < k_blocks) ranks = r;
-  }
-  if (ranks > 1 && (tiles > room<NC>(ranks) || (ranks - 1) * ((k_blocks + ranks - 1) / ranks) >= k_blocks)) return LRM_BAD_ARGUMENT;
-  cudaLaunchConfig_t config = {};
-  cudaLaunchAttribute attributes[2];
-  fill_config<NC>(config, attributes, ranks > 1 ? tiles * ranks : (tiles < 148 ? tiles : 148), ranks, stream);
-  e = cudaLaunchKernelEx(&config, gemm_bf16_few_kernel<NC>, map_w, map_x, out, M, N, K, mode, status);
-  return e == cudaSuccess ? 0 : static_cast<int>(e);
+  const int tiles = (N + kTileRows - 1) / kTileRows;
+  LRM_LAUNCH(kernel, dim3(tiles < 148 ? tiles : 148), kThreads, smem, stream, map_w, map_x, out, M, N, K, mode, status);
+  return 0;
 }
 
 }  // namespace
@@ -274,21 +197,15 @@ LRM_API int lrm_gemm_bf16_few_supports(int M, int N, int K) {
   return M >= 1 && M <= 64 && N >= 1 && K >= 8 && K % 8 == 0 && encode_tiled() != nullptr ? 1 : 0;
 }
 
-static int launch_rows(const void* X, const void* W, void* out, int M, int x_rows, int N, int K, int mode, int ranks, int* status,
-                       cudaStream_t stream) {
-  if (M <= 16) return launch<16>(X, W, out, M, x_rows, N, K, mode, ranks, status, stream);
-  if (M <= 32) return launch<32>(X, W, out, M, x_rows, N, K, mode, ranks, status, stream);
-  return launch<64>(X, W, out, M, x_rows, N, K, mode, ranks, status, stream);
-}
-
-// `x_rows` >= M: rows of X that may be read (TMA was measured slower on maps of fewer than 32 rows). `ranks`: CTAs that share a
-// tile of 128 weight rows (0: the kernel's rule). `status`: one int in device memory, 0 before the launch.
-LRM_API int lrm_gemm_bf16_few(const void* X, const void* W, void* out, int M, int x_rows, int N, int K, int mode, int ranks,
+// `x_rows` >= M: rows of X that may be read (TMA was measured slower on maps of fewer than 32 rows). `status`: one int in device memory, 0 before the launch.
+LRM_API int lrm_gemm_bf16_few(const void* X, const void* W, void* out, int M, int x_rows, int N, int K, int mode,
                               int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (!lrm_gemm_bf16_few_supports(M, N, K)) return LRM_UNSUPPORTED;
-  if ((mode != 0 && mode != 1 && mode != 3) || (mode == 3 && N % 16 != 0) || x_rows < M || ranks < 0 || ranks > 8 || status == nullptr)
+  if ((mode != 0 && mode != 1 && mode != 3) || (mode == 3 && N % 16 != 0) || x_rows < M || status == nullptr)
     return LRM_BAD_ARGUMENT;
   if (reinterpret_cast<uintptr_t>(X) % 16 || reinterpret_cast<uintptr_t>(W) % 16) return LRM_UNSUPPORTED;
-  return launch_rows(X, W, out, M, x_rows, N, K, mode, ranks, status, stream);
+  if (M <= 16) return launch<16>(X, W, out, M, x_rows, N, K, mode, status, stream);
+  if (M <= 32) return launch<32>(X, W, out, M, x_rows, N, K, mode, status, stream);
+  return launch<64>(X, W, out, M, x_rows, N, K, mode, status, stream);
 }

@@ -3,7 +3,7 @@
 * up to 8 rows (small decode batches): the weight-streaming kernel
   (csrc/gemm_bf16_stream.cu); it also takes 9-64 rows when the tensor-core kernel would
   leave most SMs idle and cannot split K (few output columns, epilogue other than "add");
-* up to 64 rows of products large enough: tcgen05 with the weights as its wide operand
+* 13 to 64 rows of products large enough: tcgen05 with the weights as its wide operand
   (csrc/gemm_bf16_few.cu; few_takes says where it is the faster one);
 * more rows (prompts, larger decode batches): the TMA + tcgen05 kernel
   (csrc/gemm_bf16_umma.cu), with 128 x 128, 128 x 256 or 256 x 256 tiles, whichever needs less
@@ -161,29 +161,25 @@ def _few_rows_plan(M: int, N: int, K: int, mode: int):
 
 
 def few_takes(M: int, N: int, K: int, mode: int) -> bool:
-    """Where the kernel with the weights as the wide tcgen05 operand is the faster one for up to 64 rows. Its ring holds
-    200 KB per SM on their way and reads at 6.2 TB/s, but it takes about 2 us to begin and to drain its accumulator, more
-    where a cluster shares a tile. In a chain of products, us, against the kernels it replaces: 28672 x 4096 with the SiLU
-    gate 8 rows 44.4 (49.5), 32 rows 48.7 (51.7), 64 rows 55.3 (52.2); 32768 x 4096 in float32 16 rows 46.0 (51.7), 32 rows
-    48.3 (52.4), 64 rows the same; 128256 x 2048 32 rows 86.0 (92.8), 64 rows 91.7 (96.9); 16384 x 2048 gated 8 rows 14.3
-    (13.7), 16 rows 15.4 (17.2), 32 rows 17.9 (17.2); 6144 x 4096 16 rows 16.8 (16.9), 32 rows 20.6 (22.2), 64 rows 28.0
-    (41.0); 3072 x 2048 32 rows 11.4 (8.8). A decode step of 32 sequences, two layers of the 8B shape:
-    541 us, 550 without. float32 results whose sums over K the streaming kernel cuts among its warps stay
-    there: here one sum runs over all of K in the tensor core."""
-    elements = N * K
-    if -(-N // 128) >= SM_COUNT // 2:  # no clusters
-        if M <= 12:
-            return mode in (0, 3) and elements >= 60e6
-        return mode in (0, 1, 3) and elements >= (30e6 if M <= 16 else 100e6 if M <= 32 else 200e6)
-    return mode == 0 and M > 16 and elements >= 15e6
+    """Where the kernel with the weights as the wide tcgen05 operand is the faster one: 13 to 64 rows of products with tiles
+    enough, which the tile kernel read at 5.5 TB/s; its ring holds 200 KB per SM on their way and reads at 6.2, but its
+    epilogue grows with the rows. In a chain of products, us, against the tile kernel: 28672 x 4096 with the SiLU gate 32
+    rows 48.7 (51.7), 64 rows 55.3 (52.2); 32768 x 4096 in float32 16 rows 46.0 (51.7), 32 rows 48.3 (52.4), 64 rows the
+    same; 128256 x 2048 32 rows 86.0 (92.8), 64 rows 91.7 (96.9); 16384 x 2048 gated 16 rows 15.4 (17.2), 32 rows 17.9
+    (17.2). A decode step of 32 sequences, two layers of the 8B shape: 543 us (554). Up to 12 rows the streaming kernel
+    stays although 28672 x 4096 alone is faster here (8 rows 44.4 against 49.5): its like beside it live off the L1 that this
+    kernel's ring takes from them (3 sequences, one layer of the 8B shape: 231 us a step against 177)."""
+    if not 12 < M <= 64:
+        return False
+    least = 30e6 if M <= 16 else 100e6 if M <= 32 else 200e6
+    return mode in (0, 1, 3) and -(-N // 128) >= SM_COUNT // 2 and N * K >= least
 
 
 def _few(x: torch.Tensor, weight: torch.Tensor, mode: int, lib) -> bool:
     M, K = x.shape
     N = weight.shape[0]
-    return (M <= 64 and not force_tiled and not force_stream and stream_shape is None and umma_width is None
-            and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0 and few_takes(M, N, K, mode)
-            and bool(lib.lrm_gemm_bf16_few_supports(M, N, K)))
+    return (few_takes(M, N, K, mode) and not force_tiled and not force_stream and stream_shape is None and umma_width is None
+            and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0 and bool(lib.lrm_gemm_bf16_few_supports(M, N, K)))
 
 
 def _held_rows(x: torch.Tensor) -> int:
@@ -193,13 +189,12 @@ def _held_rows(x: torch.Tensor) -> int:
     return min(max(M, 32), max(M, held))
 
 
-def gemm_bf16_few(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, mode: int, ranks: int = 0) -> None:
-    """gemm_bf16 for up to 64 rows on the kernel with the weights as the wide operand; `ranks` CTAs share a tile of 128
-    weight rows (0: the kernel's rule)."""
+def gemm_bf16_few(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, mode: int) -> None:
+    """gemm_bf16 (modes 0, 1, 3) for up to 64 rows on the kernel with the weights as the wide operand."""
     M, K = x.shape
     lib = library.load()
     mark_status_dirty()
-    _done(lib.lrm_gemm_bf16_few(_ptr(x), _ptr(weight), _ptr(out), M, _held_rows(x), weight.shape[0], K, mode, ranks,
+    _done(lib.lrm_gemm_bf16_few(_ptr(x), _ptr(weight), _ptr(out), M, _held_rows(x), weight.shape[0], K, mode,
                                 _ptr(_status_word(x.device)), _stream()), "gemm_bf16_few")
 
 
@@ -327,7 +322,7 @@ def gemm_bf16(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, mode: in
     M, K = x.shape
     N = weight.shape[0]
     lib = library.load()
-    if _few(x, weight, mode, lib):
+    if 12 < M <= 64 and _few(x, weight, mode, lib):
         gemm_bf16_few(x, weight, out, mode)
         return
     stream_ok, umma_ok = _fast_kernels(x, weight, lib)

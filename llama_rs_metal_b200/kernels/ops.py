@@ -818,8 +818,13 @@ def _f32(shape, device) -> torch.Tensor:
     return torch.empty(shape, dtype=torch.float32, device=device)
 
 
-def _workspace(floats: int, device) -> Optional[torch.Tensor]:
-    """float32 scratch of a kernel that asks for `floats` numbers (None for none)."""
+WALK_TOKENS = 96  # the state scans go in blocks from this many tokens per sequence on (kWalkTokens in csrc/recurrent_walk.cuh)
+
+
+def _walk_workspace(entry: str, tokens: int, device, *sizes) -> Optional[torch.Tensor]:
+    """float32 scratch of a state scan's blocked form (None where it does not go in blocks; steps of fewer than WALK_TOKENS
+    tokens need not ask)."""
+    floats = getattr(_lib(), entry)(*sizes, tokens)
     return torch.empty(floats, dtype=torch.float32, device=device) if floats else None
 
 
@@ -924,7 +929,7 @@ def linear_state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: 
             raise InvalidError("linear_state_scan: one decay per head")
     out = _f32((T, H, dv), q.device)
     rule = 1 if g is not None else 0 if head_decay is not None else 2
-    work = _workspace(_lib().lrm_linear_state_scan_floats(rule, slots.numel(), H, KH, d, dv, T), q.device)
+    work = None if T < WALK_TOKENS else _walk_workspace("lrm_linear_state_scan_floats", T, q.device, rule, slots.numel(), H, KH, d, dv)
     _done(_lib().lrm_linear_state_scan(_ptr(q), _ptr(k), _ptr(v), _ptr(g), _ptr(head_decay), _ptr(beta), _ptr(state),
                                        _ptr(out), _ptr(cu_seqlens), _ptr(slots), slots.numel(), H, KH, d, dv, T,
                                        _ptr(work), _stream()), "linear_state_scan", launches=1 if work is None else 2)
@@ -1004,7 +1009,7 @@ def bonus_state_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, g: 
     if tuple(g.shape) != (T, H * d) or max(q_off, k_off) + H * d > W or v_off + H * value_dim > W:
         raise InvalidError("bonus_state_scan: shapes do not agree")
     out = _f32((T, H, value_dim), proj.device)
-    work = _workspace(_lib().lrm_bonus_state_scan_floats(slots.numel(), H, d, value_dim, T), proj.device)
+    work = None if T < WALK_TOKENS else _walk_workspace("lrm_bonus_state_scan_floats", T, proj.device, slots.numel(), H, d, value_dim)
     _done(_lib().lrm_bonus_state_scan(_column_ptr(proj, q_off), _column_ptr(proj, k_off), ctypes.c_longlong(W),
                                       _column_ptr(proj, v_off), ctypes.c_longlong(W), _ptr(g), _ptr(bonus), _ptr(state),
                                       _ptr(out), _ptr(cu_seqlens), _ptr(slots), slots.numel(), H, d, value_dim, T,
@@ -1025,7 +1030,7 @@ def head_decay_delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, dec
     if k.shape != q.shape or v.shape[0] != T or H % KH or tuple(decay.shape) != (T, H) or tuple(step.shape) != (T, H):
         raise InvalidError("head_decay_delta_scan: shapes do not agree")
     out = _f32((T, H, dv), q.device)
-    work = _workspace(_lib().lrm_head_decay_delta_scan_floats(slots.numel(), H, KH, d, dv, T), q.device)
+    work = None if T < WALK_TOKENS else _walk_workspace("lrm_head_decay_delta_scan_floats", T, q.device, slots.numel(), H, KH, d, dv)
     _done(_lib().lrm_head_decay_delta_scan(_ptr(q), _ptr(k), _ptr(v), _ptr(decay), _ptr(step), _ptr(state), _ptr(out),
                                            _ptr(cu_seqlens), _ptr(slots), slots.numel(), H, KH, d, dv, T, _ptr(work), _stream()),
           "head_decay_delta_scan", launches=1 if work is None else 2)
