@@ -605,9 +605,9 @@ LRM_API int lrm_attention_prefill_pingpong(const void* q, const void* k, const v
   const float step = single && max_seq_len <= (d == 64 ? 2048 : 1535) ? 0.f : 8.f;
   if (form == 0) {
     if (d == 64) {
-      // us, one chain and two (the issuing thread then a lane's branch): 2,048 tokens of 32 heads 52 and 41, 8,192 422 and 388,
-      // two prompts of 1,000 31 and 28; but
-      // four of 512 18.6 and 20.2, sixteen of 256 26 and 29 (more CTAs than two rounds' worth, short ones).
+      // us, one chain and two (measured before the issuing warp stayed together, some 7 % more): 2,048 tokens of 32 heads 52 and
+      // 41, 8,192 422 and 388, two prompts of 1,000 31 and 28; but four of 512 18.6 and 20.2, sixteen of 256 26 and 29 (more
+      // than two CTAs per SM, and short ones).
       form = !single && max_seq_len <= 768 && ctas > 2 * 148 ? 1 : 2;
     } else {
       // us, one chain, two, two query tiles (24 heads): 1,024 tokens 26, 19, 25; 1,500 36, 32, 33; 2,048 47, 53, 41; 8,192

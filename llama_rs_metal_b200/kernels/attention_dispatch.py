@@ -244,9 +244,9 @@ def extends_on_tcgen05(q, kv, dv: int, seqs: int, max_seq_len: int, window: int,
     """True when a portion's attention over the paged cache runs on the tcgen05 kernel: at head size 128 whatever the
     portion, at 64 where there are query tiles enough (a tile of 128 queries of one head walks its pages one after another,
     two of them the warp-level kernel's). 32 heads on 8, us, warp-level against tcgen05: head size 128, 3,000 keys and 16
-    new tokens 95 and 69, 400 and 129 onto 3,000 and 1,111 keys 143 and 86, 1,000 onto 5,000 462 and 146, 2,000 onto 16,000
-    2796 and 785; head size 64, 65 onto 3,000 keys (32 CTAs) 53 and 63, eight times 16 onto 3,000 (256) 75 and 72, 400 and
-    129 onto 3,000 and 1,111 (256) 89 and 78, 1,000 onto 5,000 289 and 133."""
+    new tokens 96 and 41, 400 and 129 onto 3,000 and 1,111 143 and 65, 1,000 onto 5,000 461 and 164, 2,000 onto 16,000
+    2791 and 873; head size 64, eight times 16 onto 3,000 (256 CTAs) 77 and 52, 400 and 129 onto 3,000 and 1,111 (256) 90 and
+    55, 1,000 onto 5,000 315 and 91; with one chain per tile, 65 onto 3,000 (32) 53 and 63."""
     d = q.shape[2]
     return (not force_rowwise and not force_warp_level and q.dtype == torch.bfloat16 and window >= 0 and extras.plain
             and (d == 128 or q.shape[1] * seqs * -(-max_seq_len // 128) >= EXTEND_UMMA_CTAS)
