@@ -190,7 +190,7 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, const float* 
 // a router row under way together (8 tokens, 9 outputs, width 2048: 8 us, 15 with the loads one after
 // another); prompts share every load of the router's matrix between four tokens.
 template <typename A, int TOK>
-__global__ void moe_router_kernel(const A* __restrict__ x, const float* __restrict__ w,
+__global__ void moe_router_kernel(const A* x, const float* __restrict__ w,
                                   const float* __restrict__ bias, int* __restrict__ ids,
                                   float* __restrict__ weights, float* __restrict__ logits, int tokens, int width, int E,
                                   int top, int scored, const float* __restrict__ correction, int groups, int keep,
@@ -450,8 +450,8 @@ __global__ void moe_dense_gate_kernel(const G* __restrict__ gu, const int* __res
 // The same four columns at a time, a CTA per token (ff a multiple of 4, rows on 16-byte boundaries). Bound by reading
 // the chosen experts' gate and up columns and writing y.
 template <typename A>
-__global__ __launch_bounds__(256) void moe_dense_gate_wide_kernel(const float* __restrict__ gu, const int* __restrict__ ids,
-                                                                  const float* __restrict__ weights, A* __restrict__ y, int ff,
+__global__ __launch_bounds__(256) void moe_dense_gate_wide_kernel(const float* gu, const int* ids, const float* weights,
+                                                                  A* __restrict__ y, int ff,
                                                                   int experts, int top, float limit, float alpha, int act) {
   extern __shared__ float share[];  // [experts] this token's weights
   pdl_trigger();

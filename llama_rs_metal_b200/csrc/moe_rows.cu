@@ -43,7 +43,7 @@ __device__ __forceinline__ float activation(float g, float u, int act, float lim
 
 // For at most 32 pairs, by every warp for itself: the `nth` distinct expert among ids[0 .. n) (identity experts, >=
 // experts, not counted; numbered by their first pair) and its pairs in ascending order; -1 when there are fewer.
-__device__ __forceinline__ int chosen_expert_of_few(const int* __restrict__ ids, int n, int experts, int nth, int* list, int* count) {
+__device__ __forceinline__ int chosen_expert_of_few(const int* ids, int n, int experts, int nth, int* list, int* count) {
   const int lane = threadIdx.x & 31;
   const int id = lane < n ? ids[lane] : -1;
   const unsigned same = __match_any_sync(0xffffffffu, id);
@@ -59,7 +59,7 @@ __device__ __forceinline__ int chosen_expert_of_few(const int* __restrict__ ids,
 }
 
 // The same for any number, by the whole block (experts numbered by their ids). words: [32] shared, list: [n] shared.
-__device__ int chosen_expert(const int* __restrict__ ids, int n, int experts, int nth, unsigned* words, int* list, int* count,
+__device__ int chosen_expert(const int* ids, int n, int experts, int nth, unsigned* words, int* list, int* count,
                              int* picked) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid < 32) words[tid] = 0u;
@@ -109,11 +109,12 @@ __device__ int chosen_expert(const int* __restrict__ ids, int n, int experts, in
 
 // DOWN false: rows f (gate) and ff + f (up) of gate_up, right operand x rows [tokens, width], K = width;
 // DOWN true: rows r and r + 8 of down, right operand the three terms of y [3][pairs, ff], K = ff.
+// Only W is read ahead of the wait and through the read-only path; what the launches before write (x, x32, ids, weights, y3)
+// is read through plain pointers, so that no load of it can be moved ahead of the wait.
 template <int NT, int WARPS, bool DOWN>
 __global__ __launch_bounds__(WARPS * 32, 16 / WARPS) void moe_grouped_kernel(
-    const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ W, const int* __restrict__ ids,
-    const float* __restrict__ weights, __nv_bfloat16* __restrict__ y3, float* __restrict__ planes, int tokens, int width,
-    int ff, int experts, int top, float limit, float alpha, int act, const float* __restrict__ x32) {
+    const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ W, const int* ids, const float* weights, __nv_bfloat16* y3,
+    float* planes, int tokens, int width, int ff, int experts, int top, float limit, float alpha, int act, const float* x32) {
   extern __shared__ __align__(16) unsigned char shared[];
   __shared__ unsigned words[32];
   __shared__ int count_of, picked;
@@ -202,7 +203,7 @@ __global__ __launch_bounds__(WARPS * 32, 16 / WARPS) void moe_grouped_kernel(
 #pragma unroll
             for (int part = DOWN ? 2 : 0; part >= 0; --part) {  // the smallest term of y first
               const __nv_bfloat16* from = DOWN ? y3 + part * term : x;
-              const uint4 v = in ? __ldg(reinterpret_cast<const uint4*>(from + right[j] + k)) : zero;
+              const uint4 v = in ? *reinterpret_cast<const uint4*>(from + right[j] + k) : zero;
               mma16816(sum, wa_at[i][s].x, wb_at[i][s].x, wa_at[i][s].y, wb_at[i][s].y, v.x, v.y);
               mma16816(sum, wa_at[i][s].z, wb_at[i][s].z, wa_at[i][s].w, wb_at[i][s].w, v.z, v.w);
             }

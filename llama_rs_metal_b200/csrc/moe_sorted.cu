@@ -9,6 +9,8 @@
 //
 // Against the products over all experts (E / top times the arithmetic, E 2 ff float32 columns per token between them)
 // this pays from where the sorted rows are half as many as T E: see lrm_moe_sorted_tiles' caller.
+// What the launches before write is read through plain pointers: loads through `const __restrict__` ones may be moved ahead of
+// the wait for those launches.
 #include "common.cuh"
 
 namespace {
@@ -26,7 +28,7 @@ __device__ __forceinline__ float activation(float g, float u, int act, float lim
 // A CTA per expert: every CTA counts all experts' pairs, so that it knows where its own begin, then lists its own in
 // ascending order. rows[pos] = pair or -1 (padding up to whole tiles); places[pair] = pos, -1 for an identity expert;
 // tile_experts[tile] = expert, -1 behind the last tile.
-__global__ __launch_bounds__(kSortThreads) void moe_sort_kernel(const int* __restrict__ ids, int pairs, int experts,
+__global__ __launch_bounds__(kSortThreads) void moe_sort_kernel(const int* ids, int pairs, int experts,
                                                                 int* __restrict__ rows, int* __restrict__ places,
                                                                 int* __restrict__ tile_experts, int tiles) {
   extern __shared__ int counts[];  // [experts]
@@ -81,8 +83,8 @@ __global__ __launch_bounds__(kSortThreads) void moe_sort_kernel(const int* __res
 }
 
 // Rows behind the last tile are nobody's: not read by the products.
-__global__ __launch_bounds__(256) void moe_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ rows,
-                                                         const int* __restrict__ tile_experts, int top, int pieces,
+__global__ __launch_bounds__(256) void moe_gather_kernel(const uint4* x, const int* rows,
+                                                         const int* tile_experts, int top, int pieces,
                                                          uint4* __restrict__ out) {
   pdl_trigger();
   pdl_wait();
@@ -93,8 +95,8 @@ __global__ __launch_bounds__(256) void moe_gather_kernel(const uint4* __restrict
     out[static_cast<size_t>(row) * pieces + i] = p < 0 ? make_uint4(0u, 0u, 0u, 0u) : x[static_cast<size_t>(p / top) * pieces + i];
 }
 
-__global__ __launch_bounds__(256) void moe_sorted_gate_kernel(const float* __restrict__ gu, const int* __restrict__ rows,
-                                                              const int* __restrict__ tile_experts, const float* __restrict__ weights,
+__global__ __launch_bounds__(256) void moe_sorted_gate_kernel(const float* gu, const int* rows,
+                                                              const int* tile_experts, const float* weights,
                                                               int ff, float limit, float alpha, int act,
                                                               __nv_bfloat16* __restrict__ y) {
   pdl_trigger();
@@ -117,7 +119,7 @@ __global__ __launch_bounds__(256) void moe_sorted_gate_kernel(const float* __res
   }
 }
 
-__global__ __launch_bounds__(256) void moe_combine_kernel(const float* __restrict__ part, const int* __restrict__ places, int top,
+__global__ __launch_bounds__(256) void moe_combine_kernel(const float* part, const int* places, int top,
                                                           int width, int add, float* __restrict__ out) {
   pdl_trigger();
   pdl_wait();

@@ -52,9 +52,9 @@ __device__ __forceinline__ int walk_base(const int* cu_seqlens, int b) { return 
 // A CTA per stage and head (row decays) or key head.
 template <int DP, int MODE, int L>
 __global__ __launch_bounds__(128) void walk_prepare_kernel(
-    const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ g, const float* __restrict__ head_decay,
-    const float* __restrict__ beta, const float* __restrict__ look, const float* __restrict__ put, float* __restrict__ vectors_at,
-    float* __restrict__ scalars_at, const int* __restrict__ cu_seqlens, int seqs, int H, int KH, int d, long long q_stride) {
+    const float* q, const float* k, const float* g, const float* __restrict__ head_decay, const float* beta,
+    const float* __restrict__ look, const float* put, float* __restrict__ vectors_at, float* __restrict__ scalars_at,
+    const int* __restrict__ cu_seqlens, int seqs, int H, int KH, int d, long long q_stride) {
   using W = WalkShape<DP, MODE, L>;
   constexpr bool DELTA = W::DELTA, ROW_DECAY = W::ROW_DECAY, BONUS = W::BONUS;
   constexpr int BLOCKS = W::BLOCKS, SUMS = L * L;
