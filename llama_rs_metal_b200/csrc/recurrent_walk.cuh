@@ -374,6 +374,16 @@ __global__ __launch_bounds__(128) void walk_scan_kernel(
           for (int c = 0; c < C; ++c) u[j][c] = walk_pair(x[c] * rest[j], x[c] * rest[j]);
         }
       }
+      // A state that is not finite keeps no lost part (infinity times nothing is not a number); it shows in the read-outs, to
+      // which every row of the thread's columns has been added.
+      bool finite = true;
+      if (!ROW_DECAY) {
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          const float2 sums = walk_parts(reads_out[c][0]);
+          finite &= isfinite(sums.x + sums.y);
+        }
+      }
 #pragma unroll
       for (int a = 0; a < NQ; ++a) {
         unsigned long long next[2][C];
@@ -385,6 +395,15 @@ __global__ __launch_bounds__(128) void walk_scan_kernel(
           decay.x = decay.y = walk_pair(scalars[W::AT_ALL], scalars[W::AT_ALL]);
 #pragma unroll
           for (int c = 0; c < C; ++c) next[0][c] = walk_mul2(S[a][0][c], lost), next[1][c] = walk_mul2(S[a][1][c], lost);
+          if (!finite) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+              for (int c = 0; c < C; ++c) {
+                const float2 held = walk_parts(S[a][e][c]), part = walk_parts(next[e][c]);
+                next[e][c] = walk_pair(isfinite(held.x) ? part.x : 0.f, isfinite(held.y) ? part.y : 0.f);
+              }
+          }
         }
 #pragma unroll
         for (int m = 0; m < L; ++m) {

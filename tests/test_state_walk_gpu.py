@@ -102,3 +102,22 @@ def test_a_token_takes_nothing_from_the_tokens_behind_it(rule):
     assert torch.equal(spoilt[:21], clean[:21]) and torch.equal(spoilt[112:], clean[112:])
     assert bool(spoilt[22:112].isnan().all()) and bool(state[0].isnan().all())
     assert torch.equal(state[1:], x["state"][1:])
+
+
+@pytest.mark.parametrize("rule", ["token_decay", "head_decay", "bonus"])
+@pytest.mark.parametrize("H,d,dv", [(2, 64, 32), (16, 128, 144), (40, 128, 96)])
+def test_an_infinite_state_stays_infinite_and_alone(rule, H, d, dv):
+    """Without a delta rule an infinity in the state stays where it is, under decays of one and below, and shows in the
+    read-outs of its column only."""
+    lengths, slots = [101, 112], [1, 2]
+    x = _inputs(H, H, d, dv, lengths, seed=5)
+    x["g"].clamp_(min=0.5)  # no block's decays underflow: infinity times nothing would not be a number
+    for name in ("g", "decay"):
+        x[name][::3] = 1.0
+    x["head"][0] = 1.0
+    x["state"][1, 0, 3, 5], x["state"][2, H - 1, d - 1, dv - 1] = float("inf"), float("-inf")
+    got, want = _run(rule, x, lengths, slots), _reference(rule, x, lengths, slots)
+    for a, b in zip(got, want):
+        whole = b.isfinite()
+        assert bool((~whole).any()) and torch.equal(a[~whole].double(), b[~whole])
+        assert float((a[whole].double() - b[whole]).norm() / b[whole].norm()) <= 2e-6
