@@ -244,7 +244,7 @@ LRM_API int lrm_linear_state_scan_rows(int rows) {
   return g_scan_rows;
 }
 
-// Floats of workspace that lrm_linear_state_scan wants (0: none). rule 0: a decay per head, 1: the gated delta rule, 2: a
+// Floats of workspace that lrm_linear_state_scan wants to go in blocks (0: it does not; without one it goes token by token). rule 0: a decay per head, 1: the gated delta rule, 2: a
 // decay per head and token.
 LRM_API long long lrm_linear_state_scan_floats(int rule, int seqs, int H, int KH, int d, int dv, int tokens) {
   return rule == 0   ? walk_floats<0>(seqs, H, KH, d, dv, tokens)
@@ -269,12 +269,12 @@ LRM_API int lrm_linear_state_scan(const float* q, const float* k, const float* v
   }
   if (head_decay == nullptr) {  // one decay per head and token, where beta would be
     if (beta == nullptr) return LRM_BAD_ARGUMENT;
-    if (takes_walk(seqs, d, tokens))
+    if (workspace != nullptr && takes_walk(seqs, d, tokens))
       return dispatch_walk<2>(q, k, v, nullptr, nullptr, beta, nullptr, nullptr, state, out, cu_seqlens, slots, seqs, H, KH, d, dv,
                               workspace, stream, Rows{tokens});
     return dispatch_scan<2>(q, k, v, nullptr, nullptr, beta, nullptr, nullptr, state, out, cu_seqlens, slots, seqs, H, KH, d, dv, stream, Rows{tokens});
   }
-  if (takes_walk(seqs, d, tokens))
+  if (workspace != nullptr && takes_walk(seqs, d, tokens))
     return dispatch_walk<0>(q, k, v, nullptr, head_decay, nullptr, nullptr, nullptr, state, out, cu_seqlens, slots, seqs, H, KH, d,
                             dv, workspace, stream, Rows{tokens});
   return dispatch_scan<0>(q, k, v, nullptr, head_decay, nullptr, nullptr, nullptr, state, out, cu_seqlens, slots, seqs, H, KH, d,

@@ -527,7 +527,7 @@ template <int MODE>
 int dispatch_walk(const float* q, const float* k, const float* v, const float* g, const float* head_decay, const float* beta,
                   const float* look, const float* put, float* state, float* out, const int* cu_seqlens, const int* slots, int seqs,
                   int H, int KH, int d, int dv, float* workspace, cudaStream_t stream, const Rows& rows) {
-  if (workspace == nullptr || reinterpret_cast<uintptr_t>(workspace) % 16) return LRM_BAD_ARGUMENT;
+  if (reinterpret_cast<uintptr_t>(workspace) % 16) return LRM_BAD_ARGUMENT;
   const WalkArgs a{q, k, v, g, head_decay, beta, look, put, state, out, cu_seqlens, slots, seqs, H, KH, d, dv, workspace, stream, rows};
   const WalkPlan plan = walk_plan<MODE>(seqs, H, d, dv);
   constexpr int LONG = WalkShape<64, MODE, 4>::DELTA ? 8 : 4;

@@ -192,6 +192,17 @@ def test_portions_of_any_size_give_the_whole_prompt(engine, folders, plain, name
               f"{name} sequence {b} in portions {sizes}")
 
 
+@pytest.mark.parametrize("name", NAMES)
+def test_float32_gives_the_same_bits_whole_and_in_long_portions(engine, folders, name):
+    tokens = helpers.random_tokens(70, 256, vocab_of(name))
+    rows = []
+    for cuts in ([0, 256], [0, 100, 256], [0, 130, 133, 256]):
+        runner, cache, _ = open_runner(engine, folders[name, "float32"], "float32")
+        slot = cache.open_slot()
+        rows.append(torch.cat([runner.step([entry(slot, tokens[a:b])]).clone() for a, b in zip(cuts, cuts[1:])]))
+    assert all(torch.equal(rows[0], other) for other in rows[1:])
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_company_in_the_batch_changes_nothing_beyond_rounding(engine, folders, plain, dtype):
     name = "K2"

@@ -1,4 +1,4 @@
-"""State scans of long sequences, four tokens at a time (csrc/recurrent_walk.cuh), against float64 token by token."""
+"""State scans of long sequences, eight or four tokens at a time (csrc/recurrent_walk.cuh), against float64 token by token."""
 import pytest
 import torch
 
@@ -56,7 +56,7 @@ def _reference(rule, x, lengths, slots):
     return out, state
 
 
-def _run(rule, x, lengths, slots):
+def _run(rule, x, lengths, slots, **options):
     from llama_rs_metal_b200.kernels import ops
     state, cu = x["state"].clone(), _int32([sum(lengths[:i]) for i in range(len(lengths) + 1)])
     H, d, dv = x["bonus"].shape[0], x["bonus"].shape[1], x["v"].shape[2]
@@ -64,13 +64,13 @@ def _run(rule, x, lengths, slots):
         T = x["q"].shape[0]
         proj = torch.cat([x["q"].reshape(T, -1), torch.zeros(T, 3, device=DEV), x["k"].reshape(T, -1), x["v"].reshape(T, -1)], dim=1)
         out = ops.bonus_state_scan(proj.contiguous(), 0, H * d + 3, 2 * H * d + 3, x["g"].reshape(T, -1).contiguous(), x["bonus"],
-                                   state, cu, _int32(slots), dv)
+                                   state, cu, _int32(slots), dv, **options)
     elif rule == "head_delta":
-        out = ops.head_decay_delta_scan(x["q"], x["k"], x["v"], x["decay"], x["step"], state, cu, _int32(slots))
+        out = ops.head_decay_delta_scan(x["q"], x["k"], x["v"], x["decay"], x["step"], state, cu, _int32(slots), **options)
     else:
         more = {"delta": dict(g=x["g"], beta=x["step"]), "token_decay": dict(token_decay=x["decay"]),
                 "head_decay": dict(head_decay=x["head"])}[rule]
-        out = ops.linear_state_scan(x["q"], x["k"], x["v"], state, cu, _int32(slots), **more)
+        out = ops.linear_state_scan(x["q"], x["k"], x["v"], state, cu, _int32(slots), **more, **options)
     return out, state
 
 
@@ -121,3 +121,22 @@ def test_an_infinite_state_stays_infinite_and_alone(rule, H, d, dv):
         whole = b.isfinite()
         assert bool((~whole).any()) and torch.equal(a[~whole].double(), b[~whole])
         assert float((a[whole].double() - b[whole]).norm() / b[whole].norm()) <= 2e-6
+
+
+def _cut(x, begin, end):
+    return {name: t if name in ("head", "bonus", "state") else t[begin:end].contiguous() for name, t in x.items()}
+
+
+@pytest.mark.parametrize("rule", ["delta", "head_delta", "token_decay", "head_decay", "bonus"])
+def test_without_blocks_cuts_and_company_change_no_bit(rule):
+    """Whole, in portions on both sides of the line to the blocked form, and beside other sequences."""
+    x = _inputs(40, 40, 64, 80, [300, 40, 129], seed=3)
+    (out, state), (alone, alone_state) = (_run(rule, y, n, s, blocks=False) for y, n, s in
+                                          ((x, [300, 40, 129], [1, 2, 3]), (_cut(x, 0, 300), [300], [1])))
+    assert torch.equal(out[:300], alone) and torch.equal(state[1], alone_state[1])
+    held, parts = x, []
+    for begin, end in ((0, 97), (97, 98), (98, 300)):
+        o, s = _run(rule, dict(_cut(held, begin, end)), [end - begin], [1], blocks=False)
+        held = dict(held, state=s)
+        parts.append(o)
+    assert torch.equal(torch.cat(parts), alone) and torch.equal(held["state"][1], alone_state[1])
