@@ -269,12 +269,12 @@ LRM_API int lrm_linear_state_scan(const float* q, const float* k, const float* v
   }
   if (head_decay == nullptr) {  // one decay per head and token, where beta would be
     if (beta == nullptr) return LRM_BAD_ARGUMENT;
-    if (workspace != nullptr && takes_walk(seqs, d, tokens))
+    if (workspace != nullptr && takes_walk(d, tokens))
       return dispatch_walk<2>(q, k, v, nullptr, nullptr, beta, nullptr, nullptr, state, out, cu_seqlens, slots, seqs, H, KH, d, dv,
                               workspace, stream, Rows{tokens});
     return dispatch_scan<2>(q, k, v, nullptr, nullptr, beta, nullptr, nullptr, state, out, cu_seqlens, slots, seqs, H, KH, d, dv, stream, Rows{tokens});
   }
-  if (workspace != nullptr && takes_walk(seqs, d, tokens))
+  if (workspace != nullptr && takes_walk(d, tokens))
     return dispatch_walk<0>(q, k, v, nullptr, head_decay, nullptr, nullptr, nullptr, state, out, cu_seqlens, slots, seqs, H, KH, d,
                             dv, workspace, stream, Rows{tokens});
   return dispatch_scan<0>(q, k, v, nullptr, head_decay, nullptr, nullptr, nullptr, state, out, cu_seqlens, slots, seqs, H, KH, d,

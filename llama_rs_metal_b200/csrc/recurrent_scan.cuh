@@ -28,14 +28,17 @@
 // token: the sums s of four tokens are added over the parts together. Tokens are staged through
 // shared memory a chunk at a time by asynchronous copies, the next chunk under way while this
 // one is worked on, so the inner loop has no block-wide barrier and waits for no load. This is the
-// kernel of decoding, and of prompts under the generalized rule or with heads wider than 256; the
-// other prompts take four tokens at a time (recurrent_walk.cuh).
+// kernel of decoding, of sequences that bring few tokens, of the float32 runtime, and of the generalized
+// rule and heads wider than 256; the other sequences go eight or four tokens at a time
+// (recurrent_walk.cuh).
 //
 // A sequence of padding (slot < 0) starts from zero and stores nothing.
 //
 // The scan's kernels; each mode is built in a source file of its own kind (recurrent_scan.cu and
 // recurrent_scan_*.cu).
 #pragma once
+#include <climits>
+
 #include "common.cuh"
 
 extern int g_scan_rows;  // most rows a thread holds (tuning: lrm_linear_state_scan_rows); recurrent_scan.cu
@@ -72,7 +75,7 @@ __global__ __launch_bounds__(kScanThreads) void linear_scan_kernel(
     const float* __restrict__ look, const float* __restrict__ put,
     float* __restrict__ state, float* __restrict__ out, const int* __restrict__ cu_seqlens,
     const int* __restrict__ slots, int H, int KH, int d, int dv, int P_any, int chunk, long long q_stride,
-    long long v_stride, int wide_rows) {
+    long long v_stride, int wide_rows, int below) {
   extern __shared__ __align__(16) float smem[];
   constexpr bool DELTA = MODE == 1 || MODE == 5;
   constexpr bool GEN = MODE == 3;
@@ -91,6 +94,7 @@ __global__ __launch_bounds__(kScanThreads) void linear_scan_kernel(
   const int j = blockIdx.x * COLS + jl;
   pdl_wait();
   const int start = cu_seqlens[b], n = cu_seqlens[b + 1] - start;
+  if (n >= below) return;  // the blocked walk's
   const int slot = slots[b];
   float S[ROWS];
   float* mine = slot >= 0 ? state + (static_cast<size_t>(slot) * H + h) * d * dv : nullptr;
@@ -315,6 +319,7 @@ __global__ __launch_bounds__(kScanThreads) void linear_scan_kernel(
 struct Rows {
   int tokens;
   long long q = 0, v = 0;
+  int below = INT_MAX;  // sequences of as many tokens and more are left alone
 };
 
 constexpr int kLongWalk = 16;  // tokens per sequence from which a scan is a long walk
@@ -346,10 +351,10 @@ int launch_scan(const float* q, const float* k, const float* v, const float* g, 
   // still runs, its CTAs pile up on the SMs that kernel leaves first (one prompt of 2,048 tokens: 800
   // us in the middle of a step against 260 alone), so it starts when that kernel is done.
   const int pdl = g_lrm_pdl;
-  if (rows.tokens >= static_cast<long long>(seqs) * kLongWalk) g_lrm_pdl = 0;
+  if (rows.below == INT_MAX && rows.tokens >= static_cast<long long>(seqs) * kLongWalk) g_lrm_pdl = 0;
   const cudaError_t launched = lrm_launch(linear_scan_kernel<ROWS, MODE, PT>, grid, kScanThreads, bytes, stream, q, k, v, g,
                                           head_decay, beta, look, put, state, out, cu_seqlens, slots, H, KH, d, dv, P,
-                                          chunk, q_stride, v_stride, wide);
+                                          chunk, q_stride, v_stride, wide, rows.below);
   g_lrm_pdl = pdl;
   if (launched != cudaSuccess) return static_cast<int>(launched);
   return 0;

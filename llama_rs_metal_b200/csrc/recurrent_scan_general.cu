@@ -26,7 +26,7 @@ LRM_API int lrm_bonus_state_scan(const float* q, const float* k, long long q_str
   if (g == nullptr || bonus == nullptr || q_stride < static_cast<long long>(H) * d || v_stride < static_cast<long long>(H) * dv)
     return LRM_BAD_ARGUMENT;
   if (d > 2048) return LRM_UNSUPPORTED;
-  if (workspace != nullptr && takes_walk(seqs, d, tokens))
+  if (workspace != nullptr && takes_walk(d, tokens))
     return dispatch_walk<4>(q, k, v, g, nullptr, nullptr, bonus, nullptr, state, out, cu_seqlens, slots, seqs, H, H, d, dv,
                             workspace, stream, Rows{tokens, q_stride, v_stride});
   return dispatch_scan<4>(q, k, v, g, nullptr, nullptr, bonus, nullptr, state, out, cu_seqlens, slots, seqs, H, H, d,

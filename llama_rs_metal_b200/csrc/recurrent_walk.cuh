@@ -24,7 +24,7 @@
 // register for the packed FMAs. Bound by the shared-memory pipe (a vector goes to every warp: the wider a thread's tile,
 // the less) and, under the delta rules, by the chain through a block.
 //
-// The line to the token-by-token kernel (decoding) is a sequence's average of kWalkTokens tokens: below it the first
+// The line to the token-by-token kernel (decoding) is a sequence of kWalkTokens tokens: below it the first
 // launch and the padding of blocks cost more than the chain they shorten (17 tokens of 16 heads 27 against 22 us, three
 // sequences of 30 on average 31 against 28; 250 tokens on average 84 against 142).
 #pragma once
@@ -33,7 +33,7 @@
 namespace {
 
 constexpr int kWalkStage = 16;   // tokens of a stage
-constexpr int kWalkTokens = 96;  // tokens per sequence from which this way of computing pays
+constexpr int kWalkTokens = 96;  // tokens of a sequence from which this way of computing pays
 
 template <int DP, int MODE, int L>
 struct WalkShape {
@@ -54,7 +54,7 @@ template <int DP, int MODE, int L>
 __global__ __launch_bounds__(128) void walk_prepare_kernel(
     const float* q, const float* k, const float* g, const float* __restrict__ head_decay, const float* beta,
     const float* __restrict__ look, const float* put, float* __restrict__ vectors_at, float* __restrict__ scalars_at,
-    const int* __restrict__ cu_seqlens, int seqs, int H, int KH, int d, long long q_stride) {
+    const int* __restrict__ cu_seqlens, int seqs, int H, int KH, int d, long long q_stride, int least) {
   using W = WalkShape<DP, MODE, L>;
   constexpr bool DELTA = W::DELTA, ROW_DECAY = W::ROW_DECAY, BONUS = W::BONUS;
   constexpr int BLOCKS = W::BLOCKS, SUMS = L * L;
@@ -67,7 +67,7 @@ __global__ __launch_bounds__(128) void walk_prepare_kernel(
   while (b + 1 < seqs && walk_base(cu_seqlens, b + 1) <= stage) ++b;
   const int first = (stage - walk_base(cu_seqlens, b)) * kWalkStage;  // token of the sequence
   const int start = cu_seqlens[b] + first, cn = min(kWalkStage, cu_seqlens[b + 1] - start);
-  if (cn <= 0) return;
+  if (cn <= 0 || cu_seqlens[b + 1] - cu_seqlens[b] < least) return;
   const int tid = threadIdx.x, lane = tid & 31;
   constexpr int TPB = DP < 128 ? DP : 128, AT_ONCE = 128 / TPB, RPT = DP / TPB;  // threads per block, blocks at once, rows per thread
   float* to = vectors_at + (static_cast<size_t>(stage) * (ROW_DECAY ? H : KH) + vh) * W::STAGE;
@@ -222,7 +222,7 @@ template <int NQ, int C, int DP, int MODE, int L>
 __global__ __launch_bounds__(128) void walk_scan_kernel(
     const float* __restrict__ vectors_at, const float* __restrict__ scalars_at, const float* __restrict__ v,
     float* __restrict__ state, float* __restrict__ out, const int* __restrict__ cu_seqlens, const int* __restrict__ slots, int H,
-    int KH, int d, int dv, long long v_stride, int wide) {
+    int KH, int d, int dv, long long v_stride, int wide, int least) {
   using W = WalkShape<DP, MODE, L>;
   using K = Walk<NQ, C, DP, MODE, L>;
   constexpr int P = K::P, COLS = K::COLS, BLOCKS = W::BLOCKS, SCALARS = W::SCALARS, SPARE = K::SPARE;
@@ -230,6 +230,7 @@ __global__ __launch_bounds__(128) void walk_scan_kernel(
   extern __shared__ __align__(16) float smem[];
   const int h = blockIdx.y, b = blockIdx.z, vh = ROW_DECAY ? h : h / (H / KH), VH = ROW_DECAY ? H : KH, col0 = blockIdx.x * COLS;
   const int start = cu_seqlens[b], n = cu_seqlens[b + 1] - start, slot = slots[b], base_stage = walk_base(cu_seqlens, b);
+  if (n < least) return;
   const int stages = (n + kWalkStage - 1) / kWalkStage;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
@@ -449,8 +450,10 @@ __global__ __launch_bounds__(128) void walk_scan_kernel(
 inline long long walk_stages(int tokens, int seqs) { return tokens / kWalkStage + seqs; }
 inline int walk_padded(int d) { return d > 128 ? 256 : d > 64 ? 128 : 64; }
 
-// Whether a step is one this way of computing takes: sequences of kWalkTokens tokens on average, heads of up to 256.
-inline bool takes_walk(int seqs, int d, int tokens) { return tokens >= static_cast<long long>(seqs) * kWalkTokens && d <= 256; }
+// Whether a step may hold sequences that go this way: heads of up to 256. Which ones do is decided by each sequence's own
+// tokens, in the kernels, so that its bits do not hang on the lengths of the others.
+inline bool takes_walk(int d, int tokens) { return tokens >= kWalkTokens && d <= 256; }
+inline int walking(int seqs, int tokens) { return seqs < tokens / kWalkTokens ? seqs : tokens / kWalkTokens; }  // at most
 
 // How a step's walks are cut: tokens of a block, quads of rows and columns a thread holds.
 struct WalkPlan {
@@ -463,9 +466,9 @@ struct WalkPlan {
 // registers for them). A decay per token: 64 CTAs 183 with one quad and two columns, 206 with two quads; 256 CTAs (32
 // heads of 128 x 64, 1,500 and 777 tokens) 249, 187 and 218 with two quads and four columns; 1,024 CTAs 678, 524, 428.
 template <int MODE>
-WalkPlan walk_plan(int seqs, int H, int d, int dv) {
+WalkPlan walk_plan(int seqs, int H, int d, int dv, int tokens) {
   constexpr bool DELTA = WalkShape<64, MODE, 4>::DELTA;
-  const long long ctas = static_cast<long long>((dv + 15) / 16) * H * seqs;
+  const long long ctas = static_cast<long long>((dv + 15) / 16) * H * walking(seqs, tokens);
   const bool few = 2 * ctas <= 148, many = ctas > (DELTA ? 2 : 3) * 148;
   if (d <= 64) return many ? WalkPlan{4, 1, 4} : WalkPlan{DELTA ? 8 : 4, 1, 2};
   if (d <= 128) return many ? WalkPlan{4, 2, 4} : WalkPlan{DELTA ? 8 : 4, few ? 1 : 2, 2};
@@ -483,8 +486,8 @@ long long walk_floats_of(int seqs, int H, int KH, int d, int tokens, long long* 
 template <int MODE>
 long long walk_floats(int seqs, int H, int KH, int d, int dv, int tokens) {
   long long vectors;
-  if (!takes_walk(seqs, d, tokens)) return 0;
-  return walk_plan<MODE>(seqs, H, d, dv).L == 8 ? walk_floats_of<MODE, 8>(seqs, H, KH, d, tokens, &vectors)
+  if (!takes_walk(d, tokens)) return 0;
+  return walk_plan<MODE>(seqs, H, d, dv, tokens).L == 8 ? walk_floats_of<MODE, 8>(seqs, H, KH, d, tokens, &vectors)
                                                 : walk_floats_of<MODE, 4>(seqs, H, KH, d, tokens, &vectors);
 }
 
@@ -497,6 +500,7 @@ struct WalkArgs {
   float* workspace;
   cudaStream_t stream;
   Rows rows;
+  int least;  // tokens of a sequence from which it walks (0: a step of one sequence, which has them)
 };
 
 template <int NQ, int C, int DP, int MODE, int L>
@@ -513,11 +517,11 @@ int launch_walk(const WalkArgs& a) {
   walk_floats_of<MODE, L>(a.seqs, a.H, a.KH, a.d, a.rows.tokens, &vectors);
   const dim3 grid(static_cast<unsigned>(walk_stages(a.rows.tokens, a.seqs)), K::W::ROW_DECAY ? a.H : a.KH);
   LRM_LAUNCH((walk_prepare_kernel<DP, MODE, L>), grid, 128, 0, a.stream, a.q, a.k, a.g, a.head_decay, a.beta, a.look, a.put,
-             a.workspace, a.workspace + vectors, a.cu_seqlens, a.seqs, a.H, a.KH, a.d, q_stride);
+             a.workspace, a.workspace + vectors, a.cu_seqlens, a.seqs, a.H, a.KH, a.d, q_stride, a.least);
   const int wide = a.dv % 4 == 0 && v_stride % 4 == 0 && reinterpret_cast<uintptr_t>(a.v) % 16 == 0;
   // launched behind the kernel before, not beside it: let in early its CTAs pile up on the SMs that kernel leaves first
   kernel<<<dim3((a.dv + K::COLS - 1) / K::COLS, a.H, a.seqs), 128, K::BYTES, a.stream>>>(
-      a.workspace, a.workspace + vectors, a.v, a.state, a.out, a.cu_seqlens, a.slots, a.H, a.KH, a.d, a.dv, v_stride, wide);
+      a.workspace, a.workspace + vectors, a.v, a.state, a.out, a.cu_seqlens, a.slots, a.H, a.KH, a.d, a.dv, v_stride, wide, a.least);
   LRM_LAUNCH_CHECK();
   return 0;
 }
@@ -528,8 +532,16 @@ int dispatch_walk(const float* q, const float* k, const float* v, const float* g
                   const float* look, const float* put, float* state, float* out, const int* cu_seqlens, const int* slots, int seqs,
                   int H, int KH, int d, int dv, float* workspace, cudaStream_t stream, const Rows& rows) {
   if (reinterpret_cast<uintptr_t>(workspace) % 16) return LRM_BAD_ARGUMENT;
-  const WalkArgs a{q, k, v, g, head_decay, beta, look, put, state, out, cu_seqlens, slots, seqs, H, KH, d, dv, workspace, stream, rows};
-  const WalkPlan plan = walk_plan<MODE>(seqs, H, d, dv);
+  WalkArgs a{q, k, v, g, head_decay, beta, look, put, state, out, cu_seqlens, slots, seqs, H, KH, d, dv, workspace, stream, rows, 0};
+  if (seqs > 1) {  // the sequences that bring fewer tokens, one after another
+    a.least = kWalkTokens;
+    Rows few = rows;
+    few.below = kWalkTokens;
+    const int code = dispatch_scan<MODE>(q, k, v, g, head_decay, beta, look, put, state, out, cu_seqlens, slots, seqs, H, KH, d, dv,
+                                         stream, few);
+    if (code != 0) return code;
+  }
+  const WalkPlan plan = walk_plan<MODE>(seqs, H, d, dv, rows.tokens);
   constexpr int LONG = WalkShape<64, MODE, 4>::DELTA ? 8 : 4;
   if (d > 128) return launch_walk<(LONG == 8 ? 4 : 2), (LONG == 8 ? 2 : 4), 256, MODE, LONG>(a);
   if (d > 64) {

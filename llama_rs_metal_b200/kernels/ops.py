@@ -818,15 +818,21 @@ def _f32(shape, device) -> torch.Tensor:
     return torch.empty(shape, dtype=torch.float32, device=device)
 
 
-WALK_TOKENS = 96  # the state scans go in blocks from this many tokens per sequence on (kWalkTokens in csrc/recurrent_walk.cuh)
+WALK_TOKENS = 96  # the state scans' sequences of as many tokens go in blocks (kWalkTokens in csrc/recurrent_walk.cuh)
 
 
-def _walk_workspace(entry: str, blocks: bool, tokens: int, device, *sizes) -> Optional[torch.Tensor]:
-    """float32 scratch of a state scan's blocked form; None where it goes token by token."""
-    if not blocks or tokens < WALK_TOKENS:
+def _walk_workspace(entry: str, blocks: bool, tokens: int, longest: Optional[int], device, *sizes) -> Optional[torch.Tensor]:
+    """float32 scratch of a state scan's blocked form; None where it goes token by token. `longest`: tokens of the longest
+    sequence, where the caller knows (no kernel is launched for long ones that a step cannot hold)."""
+    if not blocks or min(tokens, tokens if longest is None else longest) < WALK_TOKENS:
         return None
     floats = getattr(_lib(), entry)(*sizes, tokens)
     return torch.empty(floats, dtype=torch.float32, device=device) if floats else None
+
+
+def _walk_launches(work: Optional[torch.Tensor], seqs: int) -> int:
+    """Short sequences token by token (where there may be any), and two for the blocks."""
+    return 1 if work is None else 2 + (seqs > 1)
 
 
 def _column_ptr(t: torch.Tensor, column: int) -> ctypes.c_void_p:
@@ -897,15 +903,17 @@ def delta_prepare(proj: torch.Tensor, conv_off: int, b_off: int, a: torch.Tensor
 def linear_state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor,
                       cu_seqlens: torch.Tensor, slots: torch.Tensor, head_decay: Optional[torch.Tensor] = None,
                       g: Optional[torch.Tensor] = None, beta: Optional[torch.Tensor] = None,
-                      token_decay: Optional[torch.Tensor] = None, blocks: bool = True) -> torch.Tensor:
+                      token_decay: Optional[torch.Tensor] = None, blocks: bool = True,
+                      longest: Optional[int] = None) -> torch.Tensor:
     """Update and read-out of a per-sequence, per-head matrix state (float32
     [slots, H, d, dv], updated in place), every token in order. With `head_decay` [H]: S <- a S + k v^T. With `token_decay`
     [T,H]: S <- a_t S + k v^T, one decay per head and token. With `g` [T,H,d]
     and `beta` [T,H]: S <- diag(g) S, then S <- S + k (beta (v - S^T k))^T. o = S^T q after the
     update. q, k float32 [T,KH,d] (query head h reads q/k head h // (H/KH)), v float32 [T,H,dv].
-    -> o float32 [T,H,dv]. With `blocks` a step of many tokens goes several of them at a time, in float32 too,
-    but its sums are added in another order than token by token: without it a sequence gives the same bits
-    however its tokens are cut into steps."""
+    -> o float32 [T,H,dv]. With `blocks` a sequence that brings many tokens goes several of them at a time, in
+    float32 too, but its sums are added in another order than token by token, and in one that depends on how
+    many tokens and sequences the step has: without it a sequence gives the same bits however its tokens are
+    cut into steps. `longest`: the most tokens a sequence brings, or more, where the caller knows."""
     for name, t, dims in (("q", q, 3), ("k", k, 3), ("v", v, 3), ("state", state, 4)):
         _check(t, name, torch.float32, dims)
     _check(cu_seqlens, "cu_seqlens", torch.int32, 1)
@@ -932,10 +940,10 @@ def linear_state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: 
             raise InvalidError("linear_state_scan: one decay per head")
     out = _f32((T, H, dv), q.device)
     rule = 1 if g is not None else 0 if head_decay is not None else 2
-    work = _walk_workspace("lrm_linear_state_scan_floats", blocks, T, q.device, rule, slots.numel(), H, KH, d, dv)
+    work = _walk_workspace("lrm_linear_state_scan_floats", blocks, T, longest, q.device, rule, slots.numel(), H, KH, d, dv)
     _done(_lib().lrm_linear_state_scan(_ptr(q), _ptr(k), _ptr(v), _ptr(g), _ptr(head_decay), _ptr(beta), _ptr(state),
                                        _ptr(out), _ptr(cu_seqlens), _ptr(slots), slots.numel(), H, KH, d, dv, T,
-                                       _ptr(work), _stream()), "linear_state_scan", launches=1 if work is None else 2)
+                                       _ptr(work), _stream()), "linear_state_scan", launches=_walk_launches(work, slots.numel()))
     return out
 
 
@@ -1000,11 +1008,11 @@ def _check_scan(state: torch.Tensor, cu_seqlens: torch.Tensor, slots: torch.Tens
 
 def bonus_state_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, g: torch.Tensor, bonus: torch.Tensor,
                      state: torch.Tensor, cu_seqlens: torch.Tensor, slots: torch.Tensor, value_dim: int,
-                     blocks: bool = True) -> torch.Tensor:
+                     blocks: bool = True, longest: Optional[int] = None) -> torch.Tensor:
     """A state that is read before it is written: o = (S + diag(bonus) k v^T)^T q, then S <- diag(g) S + k v^T
     (float32 [slots, H, d, dv], updated in place). q, k [H*d] and v [H*dv] are the columns at q_off, k_off
     and v_off of a float32 activation proj [T, W]; g float32 [T, H*d]; bonus float32 [H, d]. -> o [T,H,dv].
-    `blocks` as in linear_state_scan."""
+    `blocks`, `longest` as in linear_state_scan."""
     _check(proj, "proj", torch.float32, 2)
     _check(g, "g", torch.float32, 2)
     _check(bonus, "bonus", torch.float32, 2)
@@ -1014,21 +1022,21 @@ def bonus_state_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, g: 
     if tuple(g.shape) != (T, H * d) or max(q_off, k_off) + H * d > W or v_off + H * value_dim > W:
         raise InvalidError("bonus_state_scan: shapes do not agree")
     out = _f32((T, H, value_dim), proj.device)
-    work = _walk_workspace("lrm_bonus_state_scan_floats", blocks, T, proj.device, slots.numel(), H, d, value_dim)
+    work = _walk_workspace("lrm_bonus_state_scan_floats", blocks, T, longest, proj.device, slots.numel(), H, d, value_dim)
     _done(_lib().lrm_bonus_state_scan(_column_ptr(proj, q_off), _column_ptr(proj, k_off), ctypes.c_longlong(W),
                                       _column_ptr(proj, v_off), ctypes.c_longlong(W), _ptr(g), _ptr(bonus), _ptr(state),
                                       _ptr(out), _ptr(cu_seqlens), _ptr(slots), slots.numel(), H, d, value_dim, T,
-                                      _ptr(work), _stream()), "bonus_state_scan", launches=1 if work is None else 2)
+                                      _ptr(work), _stream()), "bonus_state_scan", launches=_walk_launches(work, slots.numel()))
     return out
 
 
 def head_decay_delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, step: torch.Tensor,
                           state: torch.Tensor, cu_seqlens: torch.Tensor, slots: torch.Tensor,
-                          blocks: bool = True) -> torch.Tensor:
+                          blocks: bool = True, longest: Optional[int] = None) -> torch.Tensor:
     """The delta rule with one decay per head and token on the per-sequence, per-head state (float32
     [slots, H, d, dv], updated in place): S <- decay S; S <- S + k (step (v - S^T k))^T; o = S^T q. q, k
     float32 [T,KH,d] (head h reads head h // (H/KH)), v [T,H,dv], decay and step [T,H]. -> o [T,H,dv].
-    `blocks` as in linear_state_scan."""
+    `blocks`, `longest` as in linear_state_scan."""
     for name, t, dims in (("q", q, 3), ("k", k, 3), ("v", v, 3), ("decay", decay, 2), ("step", step, 2)):
         _check(t, name, torch.float32, dims)
     T, KH, d = q.shape
@@ -1037,10 +1045,10 @@ def head_decay_delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, dec
     if k.shape != q.shape or v.shape[0] != T or H % KH or tuple(decay.shape) != (T, H) or tuple(step.shape) != (T, H):
         raise InvalidError("head_decay_delta_scan: shapes do not agree")
     out = _f32((T, H, dv), q.device)
-    work = _walk_workspace("lrm_head_decay_delta_scan_floats", blocks, T, q.device, slots.numel(), H, KH, d, dv)
+    work = _walk_workspace("lrm_head_decay_delta_scan_floats", blocks, T, longest, q.device, slots.numel(), H, KH, d, dv)
     _done(_lib().lrm_head_decay_delta_scan(_ptr(q), _ptr(k), _ptr(v), _ptr(decay), _ptr(step), _ptr(state), _ptr(out),
                                            _ptr(cu_seqlens), _ptr(slots), slots.numel(), H, KH, d, dv, T, _ptr(work), _stream()),
-          "head_decay_delta_scan", launches=1 if work is None else 2)
+          "head_decay_delta_scan", launches=_walk_launches(work, slots.numel()))
     return out
 
 

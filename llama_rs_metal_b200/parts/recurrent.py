@@ -55,10 +55,10 @@ def _needs_own_state(ctx) -> None:
         raise UnsupportedError("a mixer with a fixed-size state cannot read another layer's state")
 
 
-def _in_blocks(ctx) -> bool:
-    """Whether a state scan may take several tokens at a time: not in the float32 runtime, where a sequence gives the same
-    bits however its tokens are cut into steps."""
-    return not ctx.runtime.float32
+def _blocks(ctx) -> dict:
+    """How a state scan may take its tokens: several at a time, but in the float32 runtime, where a sequence gives the same
+    bits however its tokens are cut into steps; and the most that a sequence brings."""
+    return dict(blocks=not ctx.runtime.float32, longest=ctx.max_seq_len)
 
 
 @register_mixer("retention")
@@ -115,7 +115,7 @@ class Retention(Mixer):
         q, k, v = ops.retention_prepare(projected, 0, H * d, 2 * H * d, H, d, dv, ctx.positions, inv_freq, rotary,
                                         self.key_scale)
         o = ops.linear_state_scan(q, k, v, cache.state, ctx.cu_seqlens, ctx.slots, head_decay=self.head_decay,
-                                  blocks=_in_blocks(ctx))
+                                  **_blocks(ctx))
         mixed = ops.head_norm_gate(o, self.eps, projected.dtype, gate=projected, gate_column=2 * H * d + H * dv,
                                    gate_act=ops.GATE_SILU, out_scale=self.output_scale)
         return self.out(mixed, epilogue=ops.ADD, out=residual, ctx=ctx)
@@ -200,7 +200,7 @@ class GatedDeltaRule(Mixer):
         q, k, v, g, beta = ops.delta_prepare(projected, 0, self.channels, both, self.dt_bias, self.rate, self.taps,
                                              tails.state, ctx.cu_seqlens, ctx.seq_of_token, ctx.slots, H, G, d, dv,
                                              self.unit_eps, d ** -0.5)
-        o = ops.linear_state_scan(q, k, v, state.state, ctx.cu_seqlens, ctx.slots, g=g, beta=beta, blocks=_in_blocks(ctx))
+        o = ops.linear_state_scan(q, k, v, state.state, ctx.cu_seqlens, ctx.slots, g=g, beta=beta, **_blocks(ctx))
         mixed = ops.head_norm_gate(o, self.eps, projected.dtype, weight=self.norm_weight, gate=both,
                                    gate_column=H * d, gate_act=ops.GATE_SIGMOID, out_scale=self.output_scale)
         return self.out(mixed, epilogue=ops.ADD, out=residual, ctx=ctx)
@@ -336,7 +336,7 @@ class HeadDecayDeltaRule(Mixer):
             projected, 0, at_b, at_b + H, self.dt_bias, self.rate, self.taps, tails.state if tails is not None else None,
             ctx.cu_seqlens, ctx.seq_of_token, ctx.slots, H, G, d, dv, self.unit_eps, d ** -0.5,
             one_each=ctx.phase == "decode")
-        o = ops.head_decay_delta_scan(q, k, v, decay, step, state.state, ctx.cu_seqlens, ctx.slots, blocks=_in_blocks(ctx))
+        o = ops.head_decay_delta_scan(q, k, v, decay, step, state.state, ctx.cu_seqlens, ctx.slots, **_blocks(ctx))
         return ops.head_norm_gate(o, self.eps, x.dtype, weight=self.norm_weight, gate=projected, gate_column=at_g,
                                   gate_act=ops.GATE_SILU, out_scale=self.output_scale, out=out, out_column=column)
 
@@ -404,7 +404,7 @@ class TimeMix(Mixer):
         projected = self.fused(mixes)                                    # [T, r | k | v | g | low], float32
         w = ops.decay_product(projected, at(4), self.up, self.w_bias)    # [T, heads * head_dim], float32
         o = ops.bonus_state_scan(projected, at(0), at(1), at(2), w, self.bonus, state.state, ctx.cu_seqlens, ctx.slots,
-                                 self.head_dim, blocks=_in_blocks(ctx))
+                                 self.head_dim, **_blocks(ctx))
         return ops.head_norm_gate(o, self.eps, x.dtype, weight=self.norm_weight, gate=projected, gate_column=at(3),
                                   gate_act=ops.GATE_SILU, out_scale=self.output_scale, out=out, out_column=column)
 
@@ -534,7 +534,7 @@ class StateSpaceDuality(Mixer):
                                              ctx.slots, H, G, N, dv)
         ops.conv_tail_update_(projected, self.inner, self.channels, self.conv_taps, tails.state, ctx.cu_seqlens,
                               ctx.slots)
-        o = ops.linear_state_scan(q, k, v, state.state, ctx.cu_seqlens, ctx.slots, token_decay=decay, blocks=_in_blocks(ctx))
+        o = ops.linear_state_scan(q, k, v, state.state, ctx.cu_seqlens, ctx.slots, token_decay=decay, **_blocks(ctx))
         mixed = ops.skip_gate_part_norm(o, xf, self.skip, projected, 0, self.norm_weight, self.norm_parts, self.eps,
                                         x.dtype)
         return self.out(mixed, epilogue=ops.ADD, out=residual, ctx=ctx)
@@ -597,7 +597,7 @@ class MatrixMemory(Mixer):
         decay, take, floor = ops.capped_gates(projected, gates_at, gates_at + H, self.i_bias, self.f_bias,
                                               self.gate_cap, top.state, ctx.cu_seqlens, ctx.slots)
         q, k, v = ops.memory_prepare(projected, 0, H * d, 2 * H * d, take, d ** -0.5, H, d, dv, self.padded)
-        o = ops.linear_state_scan(q, k, v, state.state, ctx.cu_seqlens, ctx.slots, token_decay=decay, blocks=_in_blocks(ctx))
+        o = ops.linear_state_scan(q, k, v, state.state, ctx.cu_seqlens, ctx.slots, token_decay=decay, **_blocks(ctx))
         mixed = ops.head_norm_gate(o, self.eps, x.dtype, weight=self.norm_weight, gate=projected,
                                    gate_column=2 * H * d + H * dv, gate_act=ops.GATE_SIGMOID, value_dim=dv,
                                    floor=floor, floor_eps=self.floor_eps)
