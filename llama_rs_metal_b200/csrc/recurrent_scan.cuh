@@ -75,7 +75,7 @@ __global__ __launch_bounds__(kScanThreads) void linear_scan_kernel(
     const float* __restrict__ look, const float* __restrict__ put,
     float* __restrict__ state, float* __restrict__ out, const int* __restrict__ cu_seqlens,
     const int* __restrict__ slots, int H, int KH, int d, int dv, int P_any, int chunk, long long q_stride,
-    long long v_stride, int wide_rows, int below) {
+    long long v_stride, int wide_rows, int below, int below_padding) {
   extern __shared__ __align__(16) float smem[];
   constexpr bool DELTA = MODE == 1 || MODE == 5;
   constexpr bool GEN = MODE == 3;
@@ -94,8 +94,8 @@ __global__ __launch_bounds__(kScanThreads) void linear_scan_kernel(
   const int j = blockIdx.x * COLS + jl;
   pdl_wait();
   const int start = cu_seqlens[b], n = cu_seqlens[b + 1] - start;
-  if (n >= below) return;  // the blocked walk's
   const int slot = slots[b];
+  if (n >= (slot < 0 ? below_padding : below)) return;  // the blocked walk's
   float S[ROWS];
   float* mine = slot >= 0 ? state + (static_cast<size_t>(slot) * H + h) * d * dv : nullptr;
 #pragma unroll
@@ -319,7 +319,7 @@ __global__ __launch_bounds__(kScanThreads) void linear_scan_kernel(
 struct Rows {
   int tokens;
   long long q = 0, v = 0;
-  int below = INT_MAX;  // sequences of as many tokens and more are left alone
+  int below = INT_MAX, below_padding = INT_MAX;  // sequences (of padding) of as many tokens and more are left alone
 };
 
 constexpr int kLongWalk = 16;  // tokens per sequence from which a scan is a long walk
@@ -354,7 +354,7 @@ int launch_scan(const float* q, const float* k, const float* v, const float* g, 
   if (rows.below == INT_MAX && rows.tokens >= static_cast<long long>(seqs) * kLongWalk) g_lrm_pdl = 0;
   const cudaError_t launched = lrm_launch(linear_scan_kernel<ROWS, MODE, PT>, grid, kScanThreads, bytes, stream, q, k, v, g,
                                           head_decay, beta, look, put, state, out, cu_seqlens, slots, H, KH, d, dv, P,
-                                          chunk, q_stride, v_stride, wide, rows.below);
+                                          chunk, q_stride, v_stride, wide, rows.below, rows.below_padding);
   g_lrm_pdl = pdl;
   if (launched != cudaSuccess) return static_cast<int>(launched);
   return 0;

@@ -46,7 +46,12 @@ struct WalkShape {
   static constexpr int AT_T = L * L, AT_UPTO = 2 * L * L, AT_REST = AT_UPTO + L, AT_ALL = AT_REST + L, SCALARS = AT_ALL + 4;
 };
 
-// Stages of sequence b lie from walk_base(b) on: a whole number of stages each, none shared.
+// Stages of sequence b are numbered from walk_base(b) on: a whole number of stages each, none shared. A launch takes a run of
+// them: all, or as many as the workspace has room for.
+struct WalkPiece {
+  int first, count;
+  bool whole;
+};
 __device__ __forceinline__ int walk_base(const int* cu_seqlens, int b) { return cu_seqlens[b] / kWalkStage + b; }
 
 // A CTA per stage and head (row decays) or key head.
@@ -54,7 +59,7 @@ template <int DP, int MODE, int L>
 __global__ __launch_bounds__(128) void walk_prepare_kernel(
     const float* q, const float* k, const float* g, const float* __restrict__ head_decay, const float* beta,
     const float* __restrict__ look, const float* put, float* __restrict__ vectors_at, float* __restrict__ scalars_at,
-    const int* __restrict__ cu_seqlens, int seqs, int H, int KH, int d, long long q_stride, int least) {
+    const int* __restrict__ cu_seqlens, int seqs, int H, int KH, int d, long long q_stride, int least, WalkPiece piece) {
   using W = WalkShape<DP, MODE, L>;
   constexpr bool DELTA = W::DELTA, ROW_DECAY = W::ROW_DECAY, BONUS = W::BONUS;
   constexpr int BLOCKS = W::BLOCKS, SUMS = L * L;
@@ -64,8 +69,8 @@ __global__ __launch_bounds__(128) void walk_prepare_kernel(
   pdl_wait();
   const int stage = blockIdx.x, vh = blockIdx.y, per_key = H / KH, kh = ROW_DECAY ? vh / per_key : vh;
   int b = 0;
-  while (b + 1 < seqs && walk_base(cu_seqlens, b + 1) <= stage) ++b;
-  const int first = (stage - walk_base(cu_seqlens, b)) * kWalkStage;  // token of the sequence
+  while (b + 1 < seqs && walk_base(cu_seqlens, b + 1) <= piece.first + stage) ++b;
+  const int first = (piece.first + stage - walk_base(cu_seqlens, b)) * kWalkStage;  // token of the sequence
   const int start = cu_seqlens[b] + first, cn = min(kWalkStage, cu_seqlens[b + 1] - start);
   if (cn <= 0 || cu_seqlens[b + 1] - cu_seqlens[b] < least) return;
   const int tid = threadIdx.x, lane = tid & 31;
@@ -222,16 +227,17 @@ template <int NQ, int C, int DP, int MODE, int L>
 __global__ __launch_bounds__(128) void walk_scan_kernel(
     const float* __restrict__ vectors_at, const float* __restrict__ scalars_at, const float* __restrict__ v,
     float* __restrict__ state, float* __restrict__ out, const int* __restrict__ cu_seqlens, const int* __restrict__ slots, int H,
-    int KH, int d, int dv, long long v_stride, int wide, int least) {
+    int KH, int d, int dv, long long v_stride, int wide, int least, WalkPiece piece) {
   using W = WalkShape<DP, MODE, L>;
   using K = Walk<NQ, C, DP, MODE, L>;
   constexpr int P = K::P, COLS = K::COLS, BLOCKS = W::BLOCKS, SCALARS = W::SCALARS, SPARE = K::SPARE;
   constexpr bool DELTA = W::DELTA, ROW_DECAY = W::ROW_DECAY;
   extern __shared__ __align__(16) float smem[];
   const int h = blockIdx.y, b = blockIdx.z, vh = ROW_DECAY ? h : h / (H / KH), VH = ROW_DECAY ? H : KH, col0 = blockIdx.x * COLS;
-  const int start = cu_seqlens[b], n = cu_seqlens[b + 1] - start, slot = slots[b], base_stage = walk_base(cu_seqlens, b);
-  if (n < least) return;
-  const int stages = (n + kWalkStage - 1) / kWalkStage;
+  const int start = cu_seqlens[b], n = cu_seqlens[b + 1] - start, slot = slots[b];
+  const int base_stage = walk_base(cu_seqlens, b) - piece.first;  // where the sequence's first stage lies, or would
+  const int begin = max(0, -base_stage), stages = min((n + kWalkStage - 1) / kWalkStage, piece.count - base_stage);
+  if (n < least || begin >= stages || (!piece.whole && slot < 0)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
   auto issue = [&](int stage) {
@@ -260,7 +266,7 @@ __global__ __launch_bounds__(128) void walk_scan_kernel(
   unsigned long long S[NQ][2][C];                                   // [quad of rows][pair of them][column]
   float* mine = slot >= 0 ? state + (static_cast<size_t>(slot) * H + h) * d * dv : nullptr;
 #pragma unroll
-  for (int i = 0; i < K::BUFFERS - 1; ++i) issue(i);
+  for (int i = 0; i < K::BUFFERS - 1; ++i) issue(begin + i);
 #pragma unroll
   for (int a = 0; a < NQ; ++a)
 #pragma unroll
@@ -297,7 +303,7 @@ __global__ __launch_bounds__(128) void walk_scan_kernel(
   const bool writes = p % SPARE == 0 && col0 + col + my_col < dv;
   float* rows = out + (static_cast<size_t>(start) * H + h) * dv + col0 + col + my_col;
 
-  for (int stage = 0; stage < stages; ++stage) {
+  for (int stage = begin; stage < stages; ++stage) {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(K::BUFFERS - 2));
     __syncthreads();  // this stage is here for every thread, and everyone is done with the one before
     issue(stage + K::BUFFERS - 1);
@@ -475,21 +481,31 @@ WalkPlan walk_plan(int seqs, int H, int d, int dv, int tokens) {
   return DELTA ? WalkPlan{8, 4, 2} : WalkPlan{4, 2, 4};
 }
 
-// Floats of a workspace (vectors, then the numbers per head), 0 where the token-by-token kernel runs.
+// Floats of a stage in the workspace: its vectors, and its numbers per head (behind the vectors of all stages).
 template <int MODE, int L>
-long long walk_floats_of(int seqs, int H, int KH, int d, int tokens, long long* vectors) {
+long long walk_vectors(int H, int KH, int d) {
   using W = WalkShape<64, MODE, L>;
-  const long long blocks = walk_stages(tokens, seqs) * W::BLOCKS;
-  *vectors = blocks * (W::ROW_DECAY ? H : KH) * W::VECTORS * walk_padded(d);
-  return *vectors + blocks * H * W::SCALARS;
+  return static_cast<long long>(W::BLOCKS) * (W::ROW_DECAY ? H : KH) * W::VECTORS * walk_padded(d);
 }
+template <int MODE, int L>
+long long walk_stage_floats(int H, int KH, int d) {
+  using W = WalkShape<64, MODE, L>;
+  return walk_vectors<MODE, L>(H, KH, d) + static_cast<long long>(W::BLOCKS) * H * W::SCALARS;
+}
+
+// Floats of a workspace that holds a step whole, 0 where the token-by-token kernel runs.
 template <int MODE>
 long long walk_floats(int seqs, int H, int KH, int d, int dv, int tokens) {
-  long long vectors;
   if (!takes_walk(d, tokens)) return 0;
-  return walk_plan<MODE>(seqs, H, d, dv, tokens).L == 8 ? walk_floats_of<MODE, 8>(seqs, H, KH, d, tokens, &vectors)
-                                                : walk_floats_of<MODE, 4>(seqs, H, KH, d, tokens, &vectors);
+  return walk_plan<MODE>(seqs, H, d, dv, tokens).L == 8 ? walk_stages(tokens, seqs) * walk_stage_floats<MODE, 8>(H, KH, d)
+                                                        : walk_stages(tokens, seqs) * walk_stage_floats<MODE, 4>(H, KH, d);
 }
+
+// Scratch of `floats` floats, 16-byte aligned.
+struct Workspace {
+  float* at;
+  long long floats;
+};
 
 // Everything a walk is launched with.
 struct WalkArgs {
@@ -497,7 +513,7 @@ struct WalkArgs {
   float *state, *out;
   const int *cu_seqlens, *slots;
   int seqs, H, KH, d, dv;
-  float* workspace;
+  Workspace workspace;
   cudaStream_t stream;
   Rows rows;
   int least;  // tokens of a sequence from which it walks (0: a step of one sequence, which has them)
@@ -513,36 +529,44 @@ int launch_walk(const WalkArgs& a) {
   }
   const long long q_stride = a.rows.q > 0 ? a.rows.q : static_cast<long long>(a.KH) * a.d;
   const long long v_stride = a.rows.v > 0 ? a.rows.v : static_cast<long long>(a.H) * a.dv;
-  long long vectors;
-  walk_floats_of<MODE, L>(a.seqs, a.H, a.KH, a.d, a.rows.tokens, &vectors);
-  const dim3 grid(static_cast<unsigned>(walk_stages(a.rows.tokens, a.seqs)), K::W::ROW_DECAY ? a.H : a.KH);
-  LRM_LAUNCH((walk_prepare_kernel<DP, MODE, L>), grid, 128, 0, a.stream, a.q, a.k, a.g, a.head_decay, a.beta, a.look, a.put,
-             a.workspace, a.workspace + vectors, a.cu_seqlens, a.seqs, a.H, a.KH, a.d, q_stride, a.least);
   const int wide = a.dv % 4 == 0 && v_stride % 4 == 0 && reinterpret_cast<uintptr_t>(a.v) % 16 == 0;
   // launched behind the kernel before, not beside it: let in early its CTAs pile up on the SMs that kernel leaves first
-  kernel<<<dim3((a.dv + K::COLS - 1) / K::COLS, a.H, a.seqs), 128, K::BYTES, a.stream>>>(
-      a.workspace, a.workspace + vectors, a.v, a.state, a.out, a.cu_seqlens, a.slots, a.H, a.KH, a.d, a.dv, v_stride, wide, a.least);
-  LRM_LAUNCH_CHECK();
+  const long long all = walk_stages(a.rows.tokens, a.seqs), room = a.workspace.floats / walk_stage_floats<MODE, L>(a.H, a.KH, a.d);
+  const long long pieces = (all + room - 1) / room, per = (all + pieces - 1) / pieces;
+  float* scalars = a.workspace.at + per * walk_vectors<MODE, L>(a.H, a.KH, a.d);
+  for (long long first = 0; first < all; first += per) {
+    const WalkPiece piece{static_cast<int>(first), static_cast<int>(min(per, all - first)), pieces == 1};
+    LRM_LAUNCH((walk_prepare_kernel<DP, MODE, L>), dim3(piece.count, K::W::ROW_DECAY ? a.H : a.KH), 128, 0, a.stream, a.q, a.k, a.g,
+               a.head_decay, a.beta, a.look, a.put, a.workspace.at, scalars, a.cu_seqlens, a.seqs, a.H, a.KH, a.d, q_stride, a.least,
+               piece);
+    kernel<<<dim3((a.dv + K::COLS - 1) / K::COLS, a.H, a.seqs), 128, K::BYTES, a.stream>>>(
+        a.workspace.at, scalars, a.v, a.state, a.out, a.cu_seqlens, a.slots, a.H, a.KH, a.d, a.dv, v_stride, wide, a.least, piece);
+    LRM_LAUNCH_CHECK();
+  }
   return 0;
 }
 
-// `workspace`: walk_floats<MODE>(...) floats, 16-byte aligned.
+// A step that the workspace does not hold whole goes in pieces, a run of stages at a time: a state is float32 on the way from
+// piece to piece as it is within one, so the bits are the same. Padding has no state to go on from, so there it goes token by
+// token. `workspace`: as many floats as a stage has at least.
 template <int MODE>
 int dispatch_walk(const float* q, const float* k, const float* v, const float* g, const float* head_decay, const float* beta,
                   const float* look, const float* put, float* state, float* out, const int* cu_seqlens, const int* slots, int seqs,
-                  int H, int KH, int d, int dv, float* workspace, cudaStream_t stream, const Rows& rows) {
-  if (reinterpret_cast<uintptr_t>(workspace) % 16) return LRM_BAD_ARGUMENT;
+                  int H, int KH, int d, int dv, const Workspace& workspace, cudaStream_t stream, const Rows& rows) {
   WalkArgs a{q, k, v, g, head_decay, beta, look, put, state, out, cu_seqlens, slots, seqs, H, KH, d, dv, workspace, stream, rows, 0};
-  if (seqs > 1) {  // the sequences that bring fewer tokens, one after another
-    a.least = kWalkTokens;
+  const WalkPlan plan = walk_plan<MODE>(seqs, H, d, dv, rows.tokens);
+  constexpr int LONG = WalkShape<64, MODE, 4>::DELTA ? 8 : 4;
+  const long long stage = plan.L == 8 ? walk_stage_floats<MODE, 8>(H, KH, d) : walk_stage_floats<MODE, 4>(H, KH, d);
+  if (reinterpret_cast<uintptr_t>(workspace.at) % 16 || workspace.floats < stage) return LRM_BAD_ARGUMENT;
+  const bool pieces = workspace.floats / stage < walk_stages(rows.tokens, seqs);
+  if (seqs > 1 || pieces) {  // the sequences that bring fewer tokens, one after another
+    a.least = seqs > 1 ? kWalkTokens : 0;
     Rows few = rows;
-    few.below = kWalkTokens;
+    few.below = a.least, few.below_padding = pieces ? INT_MAX : kWalkTokens;
     const int code = dispatch_scan<MODE>(q, k, v, g, head_decay, beta, look, put, state, out, cu_seqlens, slots, seqs, H, KH, d, dv,
                                          stream, few);
     if (code != 0) return code;
   }
-  const WalkPlan plan = walk_plan<MODE>(seqs, H, d, dv, rows.tokens);
-  constexpr int LONG = WalkShape<64, MODE, 4>::DELTA ? 8 : 4;
   if (d > 128) return launch_walk<(LONG == 8 ? 4 : 2), (LONG == 8 ? 2 : 4), 256, MODE, LONG>(a);
   if (d > 64) {
     if (plan.C == 4) return launch_walk<2, 4, 128, MODE, 4>(a);

@@ -158,3 +158,24 @@ def test_a_sequence_goes_its_way_whatever_the_others_bring(rule):
     few = _cut(x, 530, 721)  # no sequence in blocks, with the launches for them and without
     assert all(torch.equal(a, b) for a, b in zip(_run(rule, few, [95, 90, 6], [3, 4, 0]),
                                                  _run(rule, few, [95, 90, 6], [3, 4, 0], longest=95)))
+
+
+@pytest.mark.parametrize("rule", ["delta", "head_delta", "token_decay", "head_decay", "bonus"])
+@pytest.mark.parametrize("H,d,dv", [(4, 64, 32), (3, 128, 40), (2, 200, 24)])
+def test_a_bounded_workspace_changes_no_bit(monkeypatch, rule, H, d, dv):
+    """In pieces of several sequences and of one, of many stages and of one; with padding, a short sequence and an empty one
+    among them. The scratch is no larger than allowed, or than a stage."""
+    from llama_rs_metal_b200.kernels import ops
+    lengths, slots = [130, 0, 400, 20, 112, 97], [1, 2, 3, 4, -1, 5]
+    x = _inputs(H, H, d, dv, lengths, seed=6)
+    want, held = _run(rule, x, lengths, slots), []
+    made = ops._walk_workspace
+    monkeypatch.setattr(ops, "_walk_workspace", lambda *a: held.append(made(*a)) or held[-1])
+    _run(rule, x, lengths, slots)
+    whole, stages = held[-1].numel(), sum(lengths) // 16 + len(lengths)
+    for room in (stages - 1, 20, 7, 1, 0):
+        monkeypatch.setattr(ops, "SCAN_FLOATS", room * (whole // stages) + 3)
+        out, state = _run(rule, x, lengths, slots)
+        assert torch.equal(state, want[1]) and torch.equal(out[:550], want[0][:550]) and torch.equal(out[662:], want[0][662:])
+        assert float((out[550:662] - want[0][550:662]).norm() / want[0][550:662].norm()) <= 2e-6  # padding: token by token
+        assert held[-1].numel() <= max(1, room) * (whole // stages) + 3
