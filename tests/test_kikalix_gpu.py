@@ -192,7 +192,7 @@ def test_portions_of_any_size_give_the_whole_prompt(engine, folders, plain, name
               f"{name} sequence {b} in portions {sizes}")
 
 
-@pytest.mark.parametrize("name", NAMES)
+@pytest.mark.parametrize("name", ["K1", "K3"])  # (K2's experts cut their sums by the number of rows in a step)
 def test_float32_gives_the_same_bits_whole_and_in_long_portions(engine, folders, name):
     """(First portions of whole rows of 64: the sequence of padding that others get lays out the state scan anew.)"""
     tokens = helpers.random_tokens(70, 256, vocab_of(name))
