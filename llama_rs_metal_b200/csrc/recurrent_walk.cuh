@@ -54,6 +54,24 @@ struct WalkPiece {
 };
 __device__ __forceinline__ int walk_base(const int* cu_seqlens, int b) { return cu_seqlens[b] / kWalkStage + b; }
 
+// The z-th sequence of at least `least` tokens, or -1. A warp per call, all with the same z. (A walk's grid has as many as the
+// step's tokens can make, not all sequences: 128 of one token each would else be 16,384 CTAs of 16 heads that end at once, 35 us.)
+__device__ __forceinline__ int walking_sequence(const int* cu_seqlens, int seqs, int least, int z) {
+  const int lane = threadIdx.x & 31;
+  for (int b0 = 0; b0 < seqs; b0 += 32) {
+    const int b = b0 + lane;
+    unsigned which = __ballot_sync(0xffffffffu, b < seqs && cu_seqlens[b + 1] - cu_seqlens[b] >= least);
+    const int here = __popc(which);
+    if (z >= here) {
+      z -= here;
+      continue;
+    }
+    for (; z > 0; --z) which &= which - 1;
+    return b0 + __ffs(which) - 1;
+  }
+  return -1;
+}
+
 // A CTA per stage and head (row decays) or key head.
 template <int DP, int MODE, int L>
 __global__ __launch_bounds__(128) void walk_prepare_kernel(
@@ -68,8 +86,12 @@ __global__ __launch_bounds__(128) void walk_prepare_kernel(
   pdl_trigger();
   pdl_wait();
   const int stage = blockIdx.x, vh = blockIdx.y, per_key = H / KH, kh = ROW_DECAY ? vh / per_key : vh;
-  int b = 0;
-  while (b + 1 < seqs && walk_base(cu_seqlens, b + 1) <= piece.first + stage) ++b;
+  int b = 0;  // the last sequence whose stages begin no later
+  for (int high = seqs; high - b > 1;) {
+    const int middle = (b + high) >> 1;
+    if (walk_base(cu_seqlens, middle) <= piece.first + stage) b = middle;
+    else high = middle;
+  }
   const int first = (piece.first + stage - walk_base(cu_seqlens, b)) * kWalkStage;  // token of the sequence
   const int start = cu_seqlens[b] + first, cn = min(kWalkStage, cu_seqlens[b + 1] - start);
   if (cn <= 0 || cu_seqlens[b + 1] - cu_seqlens[b] < least) return;
@@ -226,18 +248,21 @@ struct Walk {
 template <int NQ, int C, int DP, int MODE, int L>
 __global__ __launch_bounds__(128) void walk_scan_kernel(
     const float* __restrict__ vectors_at, const float* __restrict__ scalars_at, const float* __restrict__ v,
-    float* __restrict__ state, float* __restrict__ out, const int* __restrict__ cu_seqlens, const int* __restrict__ slots, int H,
-    int KH, int d, int dv, long long v_stride, int wide, int least, WalkPiece piece) {
+    float* __restrict__ state, float* __restrict__ out, const int* __restrict__ cu_seqlens, const int* __restrict__ slots,
+    int seqs, int H, int KH, int d, int dv, long long v_stride, int wide, int least, WalkPiece piece) {
   using W = WalkShape<DP, MODE, L>;
   using K = Walk<NQ, C, DP, MODE, L>;
   constexpr int P = K::P, COLS = K::COLS, BLOCKS = W::BLOCKS, SCALARS = W::SCALARS, SPARE = K::SPARE;
   constexpr bool DELTA = W::DELTA, ROW_DECAY = W::ROW_DECAY;
   extern __shared__ __align__(16) float smem[];
-  const int h = blockIdx.y, b = blockIdx.z, vh = ROW_DECAY ? h : h / (H / KH), VH = ROW_DECAY ? H : KH, col0 = blockIdx.x * COLS;
-  const int start = cu_seqlens[b], n = cu_seqlens[b + 1] - start, slot = slots[b];
-  const int base_stage = walk_base(cu_seqlens, b) - piece.first;  // where the sequence's first stage lies, or would
-  const int begin = max(0, -base_stage), stages = min((n + kWalkStage - 1) / kWalkStage, piece.count - base_stage);
-  if (n < least || begin >= stages || (!piece.whole && slot < 0)) return;
+  const int h = blockIdx.y, b = walking_sequence(cu_seqlens, seqs, least, blockIdx.z), vh = ROW_DECAY ? h : h / (H / KH), VH = ROW_DECAY ? H : KH, col0 = blockIdx.x * COLS;
+  if (b < 0) return;
+  // the part of the sequence in this launch, as a sequence of its own whose first stage lies at base_stage
+  const int from_piece = walk_base(cu_seqlens, b) - piece.first, base_stage = max(0, from_piece);
+  const int skipped = max(0, -from_piece) * kWalkStage, start = cu_seqlens[b] + skipped, slot = slots[b];
+  const int n = min(cu_seqlens[b + 1] - start, (piece.count - base_stage) * kWalkStage);
+  const int stages = (n + kWalkStage - 1) / kWalkStage;
+  if (n <= 0 || (!piece.whole && slot < 0)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
   auto issue = [&](int stage) {
@@ -266,7 +291,7 @@ __global__ __launch_bounds__(128) void walk_scan_kernel(
   unsigned long long S[NQ][2][C];                                   // [quad of rows][pair of them][column]
   float* mine = slot >= 0 ? state + (static_cast<size_t>(slot) * H + h) * d * dv : nullptr;
 #pragma unroll
-  for (int i = 0; i < K::BUFFERS - 1; ++i) issue(begin + i);
+  for (int i = 0; i < K::BUFFERS - 1; ++i) issue(i);
 #pragma unroll
   for (int a = 0; a < NQ; ++a)
 #pragma unroll
@@ -303,7 +328,7 @@ __global__ __launch_bounds__(128) void walk_scan_kernel(
   const bool writes = p % SPARE == 0 && col0 + col + my_col < dv;
   float* rows = out + (static_cast<size_t>(start) * H + h) * dv + col0 + col + my_col;
 
-  for (int stage = begin; stage < stages; ++stage) {
+  for (int stage = 0; stage < stages; ++stage) {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(K::BUFFERS - 2));
     __syncthreads();  // this stage is here for every thread, and everyone is done with the one before
     issue(stage + K::BUFFERS - 1);
@@ -460,6 +485,10 @@ inline int walk_padded(int d) { return d > 128 ? 256 : d > 64 ? 128 : 64; }
 // tokens, in the kernels, so that its bits do not hang on the lengths of the others.
 inline bool takes_walk(int d, int tokens) { return tokens >= kWalkTokens && d <= 256; }
 inline int walking(int seqs, int tokens) { return seqs < tokens / kWalkTokens ? seqs : tokens / kWalkTokens; }  // at most
+// A guess at how many, for the layout: all where they bring kWalkTokens on average; else their lengths differ a lot, and the
+// longest is what a step waits for. (2,048 tokens beside 31 sequences of one, 8 heads of 128: 493 us laid out for many, 204
+// for one.)
+inline int walking_guess(int seqs, int tokens) { return tokens >= static_cast<long long>(seqs) * kWalkTokens ? seqs : 1; }
 
 // How a step's walks are cut: tokens of a block, quads of rows and columns a thread holds.
 struct WalkPlan {
@@ -474,7 +503,7 @@ struct WalkPlan {
 template <int MODE>
 WalkPlan walk_plan(int seqs, int H, int d, int dv, int tokens) {
   constexpr bool DELTA = WalkShape<64, MODE, 4>::DELTA;
-  const long long ctas = static_cast<long long>((dv + 15) / 16) * H * walking(seqs, tokens);
+  const long long ctas = static_cast<long long>((dv + 15) / 16) * H * walking_guess(seqs, tokens);
   const bool few = 2 * ctas <= 148, many = ctas > (DELTA ? 2 : 3) * 148;
   if (d <= 64) return many ? WalkPlan{4, 1, 4} : WalkPlan{DELTA ? 8 : 4, 1, 2};
   if (d <= 128) return many ? WalkPlan{4, 2, 4} : WalkPlan{DELTA ? 8 : 4, few ? 1 : 2, 2};
@@ -539,8 +568,8 @@ int launch_walk(const WalkArgs& a) {
     LRM_LAUNCH((walk_prepare_kernel<DP, MODE, L>), dim3(piece.count, K::W::ROW_DECAY ? a.H : a.KH), 128, 0, a.stream, a.q, a.k, a.g,
                a.head_decay, a.beta, a.look, a.put, a.workspace.at, scalars, a.cu_seqlens, a.seqs, a.H, a.KH, a.d, q_stride, a.least,
                piece);
-    kernel<<<dim3((a.dv + K::COLS - 1) / K::COLS, a.H, a.seqs), 128, K::BYTES, a.stream>>>(
-        a.workspace.at, scalars, a.v, a.state, a.out, a.cu_seqlens, a.slots, a.H, a.KH, a.d, a.dv, v_stride, wide, a.least, piece);
+    kernel<<<dim3((a.dv + K::COLS - 1) / K::COLS, a.H, walking(a.seqs, a.rows.tokens)), 128, K::BYTES, a.stream>>>(
+        a.workspace.at, scalars, a.v, a.state, a.out, a.cu_seqlens, a.slots, a.seqs, a.H, a.KH, a.d, a.dv, v_stride, wide, a.least, piece);
     LRM_LAUNCH_CHECK();
   }
   return 0;
