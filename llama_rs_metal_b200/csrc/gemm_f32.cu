@@ -304,9 +304,9 @@ template <int PER>
 int launch_few(const float* X, const float* W, float* C, int M, int N, int K, int mode, int group_cols, int group_rows,
                cudaStream_t stream) {
   const size_t bytes = sizeof(float) * kFewStages * (32 + M) * kFewPitch;
-  if (bytes > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<PER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               static_cast<int>(bytes));
+  constexpr int most = sizeof(float) * kFewStages * (32 + PER * kFewWarps) * kFewPitch;
+  if (most > 48 * 1024) {  // the same for every M: a smaller one would take back what another thread's launch counts on
+    const cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<PER>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     if (e != cudaSuccess) return static_cast<int>(e);
   }
   LRM_LAUNCH((gemm_f32_few_kernel<PER>), (N + 31) / 32, kFewWarps * 32, bytes, stream, X, W, C, M, N, K, mode, group_cols,

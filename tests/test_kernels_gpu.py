@@ -144,6 +144,31 @@ def test_linear_float32_adds_in_ascending_order_whatever_the_kernel(ops, M, N, K
     assert torch.equal(ops.linear(x, w, epilogue=ops.ADD, out=resid), total)
 
 
+def test_linear_float32_of_few_rows_from_several_threads(ops):
+    """One kernel serves 17 to 32 rows with shared memory of several sizes: a launch counts on no other thread's."""
+    import threading
+    w, faults = rnd(64, 256, seed=1), []
+
+    def work(rows):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                x = rnd(rows, 256, seed=rows)
+                want = ops.linear(x, w)
+                for _ in range(2000):
+                    got = ops.linear(x, w)
+                assert torch.equal(got, want)
+        except Exception as error:  # noqa: BLE001
+            faults.append(error)
+
+    threads = [threading.Thread(target=work, args=(rows,)) for rows in (17, 32, 18, 31)]
+    for thread in threads:
+        thread.start()
+    for thread in threads:
+        thread.join()
+    torch.cuda.synchronize()
+    assert not faults
+
+
 @pytest.fixture(params=["fast kernels", "prompt attention in tensor memory", "warp-level attention",
                         "fallback kernels"])
 def kernel_choice(request, monkeypatch):
