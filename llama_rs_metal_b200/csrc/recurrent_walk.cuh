@@ -245,7 +245,10 @@ struct Walk {
   static constexpr size_t BYTES = sizeof(float) * BUFFERS * BUFFER;
 };
 
-template <int NQ, int C, int DP, int MODE, int L>
+// ALL: of a step in one piece whose tokens let every sequence walk, sequence z; else the z-th that walks, and what of it the
+// piece holds. (Finding them in the plain case too cost up to 12 % by the code around it: 16 heads of 128 with a bonus, 2,048
+// tokens, 274 us against 245.)
+template <int NQ, int C, int DP, int MODE, int L, bool ALL>
 __global__ __launch_bounds__(128) void walk_scan_kernel(
     const float* __restrict__ vectors_at, const float* __restrict__ scalars_at, const float* __restrict__ v,
     float* __restrict__ state, float* __restrict__ out, const int* __restrict__ cu_seqlens, const int* __restrict__ slots,
@@ -255,14 +258,19 @@ __global__ __launch_bounds__(128) void walk_scan_kernel(
   constexpr int P = K::P, COLS = K::COLS, BLOCKS = W::BLOCKS, SCALARS = W::SCALARS, SPARE = K::SPARE;
   constexpr bool DELTA = W::DELTA, ROW_DECAY = W::ROW_DECAY;
   extern __shared__ __align__(16) float smem[];
-  const int h = blockIdx.y, b = walking_sequence(cu_seqlens, seqs, least, blockIdx.z), vh = ROW_DECAY ? h : h / (H / KH), VH = ROW_DECAY ? H : KH, col0 = blockIdx.x * COLS;
-  if (b < 0) return;
-  // the part of the sequence in this launch, as a sequence of its own whose first stage lies at base_stage
-  const int from_piece = walk_base(cu_seqlens, b) - piece.first, base_stage = max(0, from_piece);
-  const int skipped = max(0, -from_piece) * kWalkStage, start = cu_seqlens[b] + skipped, slot = slots[b];
-  const int n = min(cu_seqlens[b + 1] - start, (piece.count - base_stage) * kWalkStage);
+  const int h = blockIdx.y, b = ALL ? blockIdx.z : walking_sequence(cu_seqlens, seqs, least, blockIdx.z);
+  const int vh = ROW_DECAY ? h : h / (H / KH), VH = ROW_DECAY ? H : KH, col0 = blockIdx.x * COLS;
+  if (!ALL && b < 0) return;
+  int start = cu_seqlens[b], n = cu_seqlens[b + 1] - start, base_stage = walk_base(cu_seqlens, b);
+  const int slot = slots[b];
+  if (n < least) return;
+  if (!ALL) {  // the part of the sequence in this launch, as a sequence of its own whose first stage lies at base_stage
+    const int skipped = max(0, piece.first - base_stage) * kWalkStage;
+    base_stage = max(0, base_stage - piece.first), start += skipped;
+    n = min(n - skipped, (piece.count - base_stage) * kWalkStage);
+    if (n <= 0 || (!piece.whole && slot < 0)) return;
+  }
   const int stages = (n + kWalkStage - 1) / kWalkStage;
-  if (n <= 0 || (!piece.whole && slot < 0)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
   auto issue = [&](int stage) {
@@ -551,7 +559,10 @@ struct WalkArgs {
 template <int NQ, int C, int DP, int MODE, int L>
 int launch_walk(const WalkArgs& a) {
   using K = Walk<NQ, C, DP, MODE, L>;
-  auto kernel = walk_scan_kernel<NQ, C, DP, MODE, L>;
+  const long long all = walk_stages(a.rows.tokens, a.seqs), room = a.workspace.floats / walk_stage_floats<MODE, L>(a.H, a.KH, a.d);
+  const int walkers = walking(a.seqs, a.rows.tokens);
+  auto kernel = room >= all && walkers == a.seqs ? walk_scan_kernel<NQ, C, DP, MODE, L, true>
+                                                 : walk_scan_kernel<NQ, C, DP, MODE, L, false>;
   if (K::BYTES > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(K::BYTES));
     if (e != cudaSuccess) return static_cast<int>(e);
@@ -560,7 +571,6 @@ int launch_walk(const WalkArgs& a) {
   const long long v_stride = a.rows.v > 0 ? a.rows.v : static_cast<long long>(a.H) * a.dv;
   const int wide = a.dv % 4 == 0 && v_stride % 4 == 0 && reinterpret_cast<uintptr_t>(a.v) % 16 == 0;
   // launched behind the kernel before, not beside it: let in early its CTAs pile up on the SMs that kernel leaves first
-  const long long all = walk_stages(a.rows.tokens, a.seqs), room = a.workspace.floats / walk_stage_floats<MODE, L>(a.H, a.KH, a.d);
   const long long pieces = (all + room - 1) / room, per = (all + pieces - 1) / pieces;
   float* scalars = a.workspace.at + per * walk_vectors<MODE, L>(a.H, a.KH, a.d);
   for (long long first = 0; first < all; first += per) {
@@ -568,7 +578,7 @@ int launch_walk(const WalkArgs& a) {
     LRM_LAUNCH((walk_prepare_kernel<DP, MODE, L>), dim3(piece.count, K::W::ROW_DECAY ? a.H : a.KH), 128, 0, a.stream, a.q, a.k, a.g,
                a.head_decay, a.beta, a.look, a.put, a.workspace.at, scalars, a.cu_seqlens, a.seqs, a.H, a.KH, a.d, q_stride, a.least,
                piece);
-    kernel<<<dim3((a.dv + K::COLS - 1) / K::COLS, a.H, walking(a.seqs, a.rows.tokens)), 128, K::BYTES, a.stream>>>(
+    kernel<<<dim3((a.dv + K::COLS - 1) / K::COLS, a.H, walkers), 128, K::BYTES, a.stream>>>(
         a.workspace.at, scalars, a.v, a.state, a.out, a.cu_seqlens, a.slots, a.seqs, a.H, a.KH, a.d, a.dv, v_stride, wide, a.least, piece);
     LRM_LAUNCH_CHECK();
   }

@@ -143,19 +143,20 @@ def test_without_blocks_cuts_and_company_change_no_bit(rule):
 
 
 @pytest.mark.parametrize("rule", ["delta", "head_delta", "token_decay", "head_decay", "bonus"])
-def test_a_sequence_goes_its_way_whatever_the_others_bring(rule):
+@pytest.mark.parametrize("lengths", [[30, 500, 95, 96], [3, 200, 1, 2, 96, 5, 1] + [1] * 30 + [97]])
+def test_a_sequence_goes_its_way_whatever_the_others_bring(rule, lengths):
     """Each sequence's own tokens decide between blocks and token by token (96 tokens; heads enough for one layout either
-    way), and a hint of the longest only saves launches."""
-    lengths = [30, 500, 95, 96]
+    way), where the tokens let all walk and where the kernel finds those that do; a hint of the longest only saves launches."""
     x = _inputs(80, 80, 64, 96, lengths, seed=4)
-    out, state = _run(rule, x, lengths, [1, 2, 3, 4])
+    slots = list(range(1, len(lengths) + 1))
+    out, state = _run(rule, x, lengths, slots)
     at = 0
-    for n, slot in zip(lengths, (1, 2, 3, 4)):
+    for n, slot in zip(lengths, slots):
         for options in ({}, dict(longest=n)):
             alone, alone_state = _run(rule, _cut(x, at, at + n), [n], [slot], **options)
             assert torch.equal(out[at:at + n], alone) and torch.equal(state[slot], alone_state[slot])
         at += n
-    few = _cut(x, 530, 721)  # no sequence in blocks, with the launches for them and without
+    few = _cut(x, at - 191, at)  # no sequence in blocks, with the launches for them and without
     assert all(torch.equal(a, b) for a, b in zip(_run(rule, few, [95, 90, 6], [3, 4, 0]),
                                                  _run(rule, few, [95, 90, 6], [3, 4, 0], longest=95)))
 
