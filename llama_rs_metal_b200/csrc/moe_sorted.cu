@@ -8,7 +8,8 @@
 //   combine  out[t] (+)= sum over a token's choices in their order
 //
 // Against the products over all experts (E / top times the arithmetic, E 2 ff float32 columns per token between them)
-// this pays from where the sorted rows are half as many as T E: see lrm_moe_sorted_tiles' caller.
+// this pays where the sorted rows are half as many as T E and the products large: ops.moe_prefers_sorted has the line and
+// what both sides measured.
 // What the launches before write is read through plain pointers: loads through `const __restrict__` ones may be moved ahead of
 // the wait for those launches.
 #include "common.cuh"

@@ -120,3 +120,14 @@ def test_unequal_sequences_get_a_cluster_size_more():
     assert size(8, 8, 4, 64, 4096, fill=3) == 7
     assert size(1, 8, 4, 64, 4096, fill=1) == 14                                        # one sequence is never unequal
     assert size(64, 8, 4, 64, 4096, fill=2) == 1                                        # 1,024 CTAs would be two full rounds
+
+
+def test_prompts_experts_are_sorted_only_where_that_was_the_faster_way():
+    """(tokens, width, inner width, experts, chosen): both ways were timed at these sizes."""
+    from llama_rs_metal_b200.kernels import ops
+    faster = [(500, 2048, 1024, 8, 2), (600, 2048, 1024, 3, 1), (4096, 2048, 1024, 32, 8), (500, 1024, 512, 8, 2),
+              (1500, 1024, 512, 4, 1), (2048, 1024, 512, 3, 1)]
+    slower = [(1000, 2048, 1024, 8, 4), (500, 1024, 512, 4, 1), (1500, 1024, 512, 3, 1), (2048, 512, 256, 8, 2),
+              (4096, 512, 256, 4, 1), (4096, 512, 256, 32, 8), (2048, 512, 256, 16, 4)]
+    assert all(ops.moe_prefers_sorted(*sizes) for sizes in faster)
+    assert not any(ops.moe_prefers_sorted(*sizes) for sizes in slower)
