@@ -162,17 +162,21 @@ def _few_rows_plan(M: int, N: int, K: int, mode: int):
 
 def few_takes(M: int, N: int, K: int, mode: int) -> bool:
     """Where the kernel with the weights as the wide tcgen05 operand is the faster one: 13 to 64 rows of products with tiles
-    enough, which the tile kernel read at 5.5 TB/s; its ring holds 200 KB per SM on their way and reads at 6.2, but its
-    epilogue grows with the rows. In a chain of products, us, against the tile kernel: 28672 x 4096 with the SiLU gate 32
-    rows 48.7 (51.7), 64 rows 55.3 (52.2); 32768 x 4096 in float32 16 rows 46.0 (51.7), 32 rows 48.3 (52.4), 64 rows the
-    same; 128256 x 2048 32 rows 86.0 (92.8), 64 rows 91.7 (96.9); 16384 x 2048 gated 16 rows 15.4 (17.2), 32 rows 17.9
-    (17.2). A decode step of 32 sequences, two layers of the 8B shape: 543 us (554). Up to 12 rows the streaming kernel
-    stays although 28672 x 4096 alone is faster here (8 rows 44.4 against 49.5): its like beside it live off the L1 that this
-    kernel's ring takes from them (3 sequences, one layer of the 8B shape: 231 us a step against 177)."""
-    if not 12 < M <= 64:
+    enough, which the tile kernel reads at 5.5 TB/s; its ring holds 200 KB per SM on their way and reads at 6.2, but its
+    epilogue grows with the rows, most of all the SiLU gate's. us in a chain of products over more weights than L2 holds, in
+    brackets the kernel that else runs. bfloat16 results: 16384 x 2048 16 rows 13.7 (21.3), 28672 x 4096 16 rows 44.7
+    (50.4), 32 rows 45.6 (51.4), 49408 x 4096 33 rows 71.8 (78.4), 64 rows 73.8 (79.1), 128256 x 2048 64 rows 87.0 (94.4).
+    Gated: 16384 x 2048 16 rows 16.4 (24.4), 28672 x 4096 32 rows 53.3 (57.8), 49408 x 4096 33 rows 79.5 (84.1), 48 rows 84.1
+    (85.4), 64 rows 87.8 (85.2), 128256 x 2048 64 rows 101.1 (96.4). A tile for half the SMs only, 9472 x 22000: 32 rows
+    103.4 (105.3), 48 rows 107.2 (106.3), gated 118.4 (111.8). Smaller products of more rows would gain too (28672 x 4096 64
+    rows 48.1 against 51.7; gated 63.2 against 59.2). Up to 12 rows the streaming kernel stays although 28672 x 4096 alone
+    is faster here (8 rows 44.4 against 49.5): its like beside it live off the L1 that this kernel's ring takes from them (3
+    sequences, one layer of the 8B shape: 231 us a step against 177)."""
+    if not 12 < M <= (48 if mode == 3 else 64):
         return False
     least = 30e6 if M <= 16 else 100e6 if M <= 32 else 200e6
-    return mode in (0, 1, 3) and -(-N // 128) >= SM_COUNT // 2 and N * K >= least
+    tiles = -(-N // 128)
+    return mode in (0, 1, 3) and tiles >= (SM_COUNT // 2 if M <= 32 else SM_COUNT) and N * K >= least
 
 
 def _few(x: torch.Tensor, weight: torch.Tensor, mode: int, lib) -> bool:

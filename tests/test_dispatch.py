@@ -131,3 +131,13 @@ def test_prompts_experts_are_sorted_only_where_that_was_the_faster_way():
               (4096, 512, 256, 4, 1), (4096, 512, 256, 32, 8), (2048, 512, 256, 16, 4)]
     assert all(ops.moe_prefers_sorted(*sizes) for sizes in faster)
     assert not any(ops.moe_prefers_sorted(*sizes) for sizes in slower)
+
+
+def test_products_of_few_rows_take_the_wide_weight_kernel_only_where_it_was_the_faster_one():
+    """(rows, N, K, mode): both kernels were timed at these sizes."""
+    faster = [(13, 16384, 2048, 0), (16, 16384, 2048, 3), (32, 28672, 4096, 0), (32, 28672, 4096, 3), (64, 49408, 4096, 0),
+              (64, 128256, 2048, 0), (48, 49408, 4096, 3), (32, 9472, 22000, 0)]
+    slower = [(64, 49408, 4096, 3), (64, 128256, 2048, 3), (64, 65536, 4096, 3), (48, 9472, 22000, 0), (33, 9472, 22000, 3),
+              (64, 28672, 4096, 3)]
+    assert all(gemm_dispatch.few_takes(*sizes) for sizes in faster)
+    assert not any(gemm_dispatch.few_takes(*sizes) for sizes in slower)
