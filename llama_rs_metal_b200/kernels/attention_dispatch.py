@@ -240,16 +240,27 @@ def decode(q, kv, out, slots, kv_lens, max_kv_len: int, scale: float, window: in
 EXTEND_UMMA_CTAS = 128
 
 
-def extends_on_tcgen05(q, kv, dv: int, seqs: int, max_seq_len: int, window: int, slopes, out_scale: float, extras, out) -> bool:
-    """True when a portion's attention over the paged cache runs on the tcgen05 kernel: at head size 128 whatever the
-    portion, at 64 where there are query tiles enough (a tile of 128 queries of one head walks its pages one after another,
-    two of them the warp-level kernel's). 32 heads on 8, us, warp-level against tcgen05: head size 128, 3,000 keys and 16
-    new tokens 96 and 41, 400 and 129 onto 3,000 and 1,111 143 and 65, 1,000 onto 5,000 461 and 164, 2,000 onto 16,000
-    2791 and 873; head size 64, eight times 16 onto 3,000 (256 CTAs) 77 and 52, 400 and 129 onto 3,000 and 1,111 (256) 90 and
-    55, 1,000 onto 5,000 315 and 91; with one chain per tile, 65 onto 3,000 (32) 53 and 63."""
+def extend_prefers_tcgen05(d: int, ctas: int, reach: Optional[int]) -> bool:
+    """Where a portion's attention over `reach` keys (None: not known, taken as many) is faster on the tcgen05 kernel than on the
+    warp-level one. us, warp-level and tcgen05, tokens onto a context that ends at `reach` keys. Head size 128, 32 heads on 8:
+    2 tokens to 66 keys 5.2 and 6.4, to 130 7.2 and 7.1, to 200 9.1 and 7.6, to 800 26.7 and 13.7; 16 times 2 of 24 heads to 130
+    keys 17.5 and 20.0, to 200 22.8 and 21.3; 400 and 129 onto 3,000 and 1,111 143 and 65, 2,000 onto 16,000 2791 and 873. Head
+    size 64, 128 CTAs and more: 4 times 16 to 66 keys 3.9 and 6.4, to 320 7.1 and 8.2, to 500 10.0 and 9.9, to 800 15.4 and
+    13.1; 8 times 64 to 400 keys 13.7 and 13.8, to 600 17.8 and 16.5; 1,000 onto 5,000 315 and 91. The line of CTAs is from a
+    form of one chain per query tile; with the two chains there are now, 128 tokens of 32 heads (32 CTAs) to 500 keys take 10.4
+    and 11.1, to 800 15.6 and 14.3, onto 3,000 52 and 33."""
+    return (reach is None or reach >= (192 if d == 128 else 512)) and (d == 128 or ctas >= EXTEND_UMMA_CTAS)
+
+
+def extends_on_tcgen05(q, kv, dv: int, seqs: int, max_seq_len: int, window: int, slopes, out_scale: float, extras, out,
+                       max_kv_len: Optional[int] = None) -> bool:
+    """True when a portion's attention over the paged cache runs on the tcgen05 kernel: forms and alignments it takes, and where
+    it is the faster one (a tile of 128 queries of one head walks its pages one after another, two of them the warp-level
+    kernel's). `max_kv_len`: keys of the longest sequence, where known."""
     d = q.shape[2]
+    reach = max_kv_len if max_kv_len is None or window <= 0 else min(max_kv_len, window + max_seq_len)
     return (not force_rowwise and not force_warp_level and q.dtype == torch.bfloat16 and window >= 0 and extras.plain
-            and (d == 128 or q.shape[1] * seqs * -(-max_seq_len // 128) >= EXTEND_UMMA_CTAS)
+            and extend_prefers_tcgen05(d, q.shape[1] * seqs * -(-max_seq_len // 128), reach)
             and _plain(q, dv, slopes, out_scale) and kv.page_size == 64
             and not getattr(kv, "values_in_keys", False) and kv.k.dtype == torch.bfloat16
             and all(t.data_ptr() % 16 == 0 for t in (q, kv.k, kv.v, out))
@@ -258,8 +269,9 @@ def extends_on_tcgen05(q, kv, dv: int, seqs: int, max_seq_len: int, window: int,
 
 
 def extend(q, kv, out, cu_seqlens, seq_of_token, positions, slots, kv_lens, max_seq_len: int, scale: float,
-           window: int, slopes=None, out_scale: float = 1.0, extras=None) -> None:
-    """Packed queries, several per sequence, over the cache that already holds the step's keys."""
+           window: int, slopes=None, out_scale: float = 1.0, extras=None, max_kv_len: Optional[int] = None) -> None:
+    """Packed queries, several per sequence, over the cache that already holds the step's keys. `max_kv_len`: the most keys a
+    sequence has, where known (it only decides between kernels)."""
     from .ops import _value_dim
     T, Hq, d = q.shape
     dv = _value_dim(kv)
@@ -273,7 +285,7 @@ def extend(q, kv, out, cu_seqlens, seq_of_token, positions, slots, kv_lens, max_
                                             window, None, 1, _ptr(extras.sinks), _stream()),
               "attention_shared_keys")
         return
-    if extends_on_tcgen05(q, kv, dv, cu_seqlens.numel() - 1, max_seq_len, window, slopes, out_scale, extras, out):
+    if extends_on_tcgen05(q, kv, dv, cu_seqlens.numel() - 1, max_seq_len, window, slopes, out_scale, extras, out, max_kv_len):
         from . import gemm_dispatch
         gemm_dispatch.mark_status_dirty()
         _done(lib.lrm_attention_extend_umma(_ptr(q), _ptr(kv.k), _ptr(kv.v), kv.k.shape[0], _ptr(out), _ptr(cu_seqlens),
@@ -578,7 +590,7 @@ def attend(projected, *, q_heads: int, kv_heads: int, head_dim: int, rotary, ctx
             return ops.attention_decode(q, cache, ctx.slots, ctx.kv_lens, ctx.max_kv_len, scale, window, slopes,
                                         out_scale, extras)
         return ops.attention_extend(q, cache, ctx.cu_seqlens, ctx.seq_of_token, ctx.positions, ctx.slots,
-                                    ctx.kv_lens, ctx.max_seq_len, scale, window, slopes, out_scale, extras)
+                                    ctx.kv_lens, ctx.max_seq_len, scale, window, slopes, out_scale, extras, ctx.max_kv_len)
     if projection is not None:
         x, weight = projection
         if (phase == "prefill" and writes_cache and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
@@ -623,4 +635,4 @@ def attend(projected, *, q_heads: int, kv_heads: int, head_dim: int, rotary, ctx
     if phase == "decode":
         return ops.attention_decode(q, cache, ctx.slots, ctx.kv_lens, ctx.max_kv_len, scale, window)
     return ops.attention_extend(q, cache, ctx.cu_seqlens, ctx.seq_of_token, ctx.positions, ctx.slots,
-                                ctx.kv_lens, ctx.max_seq_len, scale, window)
+                                ctx.kv_lens, ctx.max_seq_len, scale, window, max_kv_len=ctx.max_kv_len)

@@ -1806,9 +1806,10 @@ def attention_decode(q: torch.Tensor, kv, slots: torch.Tensor, kv_lens: torch.Te
 def attention_extend(q: torch.Tensor, kv, cu_seqlens: torch.Tensor, seq_of_token: torch.Tensor,
                      positions: torch.Tensor, slots: torch.Tensor, kv_lens: torch.Tensor, max_seq_len: int,
                      scale: float, window: Optional[int] = None, slopes: Optional[torch.Tensor] = None,
-                     out_scale: float = 1.0, extras=None) -> torch.Tensor:
+                     out_scale: float = 1.0, extras=None, max_kv_len: Optional[int] = None) -> torch.Tensor:
     """Several queries per sequence over the cache, which already holds the step's own keys:
-    query t (packed, of sequence seq_of_token[t]) sees the keys up to positions[t]. -> [T, Hq*d]"""
+    query t (packed, of sequence seq_of_token[t]) sees the keys up to positions[t]. `max_kv_len`: the most
+    keys a sequence has, where the caller knows (it only decides between kernels). -> [T, Hq*d]"""
     _check(q, "q", dims=3)
     _check(kv.k, "k pages", q.dtype, 4)
     _check(kv.v, "v pages", q.dtype, 4)
@@ -1827,7 +1828,7 @@ def attention_extend(q: torch.Tensor, kv, cu_seqlens: torch.Tensor, seq_of_token
     from . import attention_dispatch
     _check_extras(extras, Hq)
     attention_dispatch.extend(q, kv, out, cu_seqlens, seq_of_token, positions, slots, kv_lens, max_seq_len,
-                              scale, window or 0, slopes, out_scale, extras)
+                              scale, window or 0, slopes, out_scale, extras, max_kv_len)
     return out
 
 

@@ -141,3 +141,11 @@ def test_products_of_few_rows_take_the_wide_weight_kernel_only_where_it_was_the_
               (64, 28672, 4096, 3)]
     assert all(gemm_dispatch.few_takes(*sizes) for sizes in faster)
     assert not any(gemm_dispatch.few_takes(*sizes) for sizes in slower)
+
+
+def test_portions_go_to_the_tcgen05_kernel_only_where_it_was_the_faster_one():
+    """(head size, query tiles of all heads, keys): both kernels were timed at these."""
+    prefers = attention_dispatch.extend_prefers_tcgen05
+    assert all(prefers(*at) for at in [(128, 32, 200), (128, 384, 200), (128, 32, 3000), (64, 128, 600), (64, 512, 600), (64, 128, 3000),
+                                       (128, 4, None), (64, 128, None)])
+    assert not any(prefers(*at) for at in [(128, 32, 66), (128, 384, 130), (128, 32, 100), (64, 128, 66), (64, 512, 320), (64, 32, 300)])
