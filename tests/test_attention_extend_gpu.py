@@ -16,8 +16,10 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("window", [None, 64, 100])
 def test_portions_match_float64(monkeypatch, held, new, heads, kv_heads, d, window):
     from llama_rs_metal_b200.cache.cache import KeyValueView
-    from llama_rs_metal_b200.kernels import attention_dispatch, ops
+    from llama_rs_metal_b200.kernels import attention_dispatch, gemm_dispatch, ops
     monkeypatch.setattr(attention_dispatch, "EXTEND_UMMA_CTAS", 1)
+    took, rule = [], attention_dispatch.extends_on_tcgen05
+    monkeypatch.setattr(attention_dispatch, "extends_on_tcgen05", lambda *a: took.append(rule(*a)) or took[-1])
     gen = torch.Generator().manual_seed(sum(held) + d)
     lengths = [h + n for h, n in zip(held, new)]
     per = max(-(-n // 64) for n in lengths)
@@ -53,6 +55,8 @@ def test_portions_match_float64(monkeypatch, held, new, heads, kv_heads, d, wind
                                int32([b for b, n in enumerate(new) for _ in range(n)]),
                                int32([p for h, n in zip(held, new) for p in range(h, h + n)]), int32(slots), int32(lengths),
                                max(new), 1 / math.sqrt(d), window).view(-1, heads, d).double().cpu()
+    assert took == [True]
+    gemm_dispatch.check_status()
     at, left = 0, iter(want)
     for n in new:
         expected = torch.stack([next(left) for _ in range(heads)], 1)

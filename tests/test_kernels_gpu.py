@@ -127,11 +127,16 @@ def test_linear_float32_row_does_not_depend_on_the_batch(ops):
 
 
 # rows around the few-row kernel's limits and the tiles' edges; N and K around a tile, a stage, and off 16-byte rows
-@pytest.mark.parametrize("M", [1, 4, 5, 16, 32, 33, 64, 65, 129])
-@pytest.mark.parametrize("N,K", [(64, 64), (68, 132), (33, 20), (9476, 36), (100, 67)])
+# (and the tiles of 128 x 64, which run where they give the busiest SM no more work: from 257 rows of 3072 outputs, say, with
+# rows on 16 bytes and off)
+@pytest.mark.parametrize("M,N,K", [(M, N, K) for M in (1, 4, 5, 16, 32, 33, 64, 65, 129)
+                                   for N, K in ((64, 64), (68, 132), (33, 20), (9476, 36), (100, 67))]
+                         + [(257, 3072, 36), (300, 3068, 52), (384, 3070, 67), (513, 1533, 33)])
 def test_linear_float32_adds_in_ascending_order_whatever_the_kernel(ops, M, N, K):
     """Every float32 kernel adds an element's products over k in ascending order, one FMA each: the rows
     of a product are the same bits however many rows it has, and within K roundings of float64."""
+    wide, small = (-(-(-(-M // rows) * -(-N // 64)) // 148) for rows in (128, 64))  # tiles of the busiest SM
+    assert (2 * wide <= small) == (M > 129)
     x, w = rnd(M, K), rnd(N, K, seed=1)
     got = ops.linear(x, w)
     want = x.double() @ w.double().T

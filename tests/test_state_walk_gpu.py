@@ -11,10 +11,10 @@ def _int32(values):
 
 
 # head sizes on both sides of 64, 128 and 256, value widths off a CTA's columns and off 16 bytes, few and many heads
-# (four and eight rows per thread, two and four columns); lengths on both sides of a block of 4 or 8 and a stage of 16, none, and
+# (four and eight rows per thread, two and four columns, of each padded size); lengths on both sides of a block of 4 or 8 and a stage of 16, none, and
 # one token among long ones
 SHAPES = [(2, 1, 64, 32), (3, 3, 33, 17), (12, 4, 65, 50), (4, 2, 128, 128), (16, 4, 128, 144), (2, 2, 129, 9), (1, 1, 256, 24),
-          (24, 24, 64, 64), (40, 8, 128, 96)]
+          (24, 24, 64, 64), (40, 8, 128, 96), (48, 48, 64, 64), (64, 8, 33, 50)]
 LENGTHS = [[96], [97, 191, 1], [200, 0, 107], [95, 111]]
 
 
