@@ -65,9 +65,6 @@ template <int D, int NQ, int CHAINS> struct Shape {
   static constexpr int kSmem = NQ * BQ * D * 2 + 2 * kStages * BKV * D * 2 + 256 + (CHAINS > NQ ? 2 * BQ * 8 : 0);
 };
 
-// Shared memory (1024-byte aligned): Q [2][128][D] | stages of (K [128][D] | V [128][D]) |
-// barriers. A [128][D] tile with D = 128 is two [128][64] blocks of 16 KB one after the other
-// (a swizzle row is 128 bytes = 64 elements).
 // The cache of a PAGED launch.
 struct Pages {
   const int* table;    // [slots][stride]
@@ -117,7 +114,9 @@ void attention_prefill_pingpong_kernel(
     if (threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0, kMisaligned);
     return;
   }
-  unsigned char* q_tiles = smem_raw;                        // [NQ] tiles
+  // NQ query tiles [BQ][D], STAGES pairs of a key and a value tile [BKV][D], barriers. A tile with D = 128 is two blocks of 64
+  // columns one after the other (a swizzle row is 128 bytes = 64 elements).
+  unsigned char* q_tiles = smem_raw;
   unsigned char* kv_tiles = q_tiles + NQ * TILE;            // stage s: K at s * 2 * KV_TILE, V right after
   uint64_t* bars = reinterpret_cast<uint64_t*>(kv_tiles + STAGES * 2 * KV_TILE);
   uint64_t* q_full = bars;
@@ -605,15 +604,17 @@ LRM_API int lrm_attention_prefill_pingpong(const void* q, const void* k, const v
   const float step = single && max_seq_len <= (d == 64 ? 2048 : 1535) ? 0.f : 8.f;
   if (form == 0) {
     if (d == 64) {
-      // us, one chain and two (measured before the issuing warp stayed together, some 7 % more): 2,048 tokens of 32 heads 52 and
-      // 41, 8,192 422 and 388, two prompts of 1,000 31 and 28; but four of 512 18.6 and 20.2, sixteen of 256 26 and 29 (more
-      // than two CTAs per SM, and short ones).
-      form = !single && max_seq_len <= 768 && ctas > 2 * 148 ? 1 : 2;
+      // us, one chain and two, 32 heads: one prompt of 512 tokens 14.6 and 10.5, 2,048 51 and 41, 8,192 384 and 366; packed two of
+      // 1,000 28.5 and 26.2, four of 768 32.3 and 31.1, four of 800 36.4 and 37.9, unequal ones the same within 3 %; but four of
+      // 512 19.3 and 19.6, sixteen of 256 28.1 and 29.1, 32 of 128 22.9 and 26.7, eight of 700 53 and 56 (more than two CTAs per
+      // SM, and short ones).
+      form = !single && max_seq_len <= 768 && ctas > 2 * kSmCount ? 1 : 2;
     } else {
-      // us, one chain, two, two query tiles (24 heads): 1,024 tokens 26, 19, 25; 1,500 36, 32, 33; 2,048 47, 53, 41; 8,192
-      // 495, 575, 380; packed 700, 1,333, 64, 257 and 1,999 78, 91, 75; four of 512 23, 27, 27; two of 1,000 29, 35, 31;
-      // 2,048 within a window of 512 37, 39, 41.
-      form = max_seq_len > 1535 && reach >= 1024 ? 3 : (single ? max_seq_len <= 1535 : ctas <= 148) ? 2 : 1;
+      // us, one chain, two, two query tiles, 24 heads: one prompt of 512 tokens 18, 14, 20, 1,024 28, 20, 30, 1,500 38, 31, 37,
+      // 2,048 44, 50, 41, 8,192 450, 522, 374; packed two of 1,000 28, 35, 32, four of 512 23, 28, 28, sixteen of 256 33, 44, 39,
+      // eight of 700 64, 81, 68; 700, 1,333, 64, 257 and 1,999 68, 85, 74, 3,001, 517 and 1,200 98, 121, 97; 2,048 within a window
+      // of 512 37, 39, 41 (before the issuing warp stayed together).
+      form = max_seq_len > 1535 && reach >= 1024 ? 3 : (single ? max_seq_len <= 1535 : ctas <= kSmCount) ? 2 : 1;
     }
   }
   const auto run = d == 64 ? (form == 1 ? launch<64, 1, 1> : launch<64, 1, 2>)
@@ -640,7 +641,7 @@ LRM_API int lrm_attention_extend_umma(const void* q, const void* k_pages, const 
   // 78 and 63, 1,000 onto 5,000 136 and 143, eight times 16 onto 3,000 75 and 84, 2,000 onto 16,000 742 and 814, of 24 heads
   // 717 and 616.
   const long long ctas = q_heads * max(static_cast<long long>(seqs), static_cast<long long>(tokens / BQ));
-  const bool two = d == 64 || (ctas + 147) / 148 < 2 * ((ctas + 295) / 296);
+  const bool two = d == 64 || (ctas + kSmCount - 1) / kSmCount < 2 * ((ctas + 2 * kSmCount - 1) / (2 * kSmCount));
   const auto run = d == 64 ? launch_paged<64, 2> : two ? launch_paged<128, 2> : launch_paged<128, 1>;
   return run(q, k_pages, v_pages, rows, out, cu_seqlens, pages, tokens, seqs, max_seq_len, q_heads, kv_heads, scale, window,
              status, stream);

@@ -30,6 +30,8 @@ enum : int { LRM_BAD_ARGUMENT = -1, LRM_UNSUPPORTED = -2, LRM_DEVICE_STATUS = -3
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+constexpr int kSmCount = 148;  // SMs of a B200: grids and layouts are chosen for them
+
 extern int g_lrm_pdl;  // 1: launch with programmatic stream serialization (set by lrm_set_pdl)
 
 template <typename... KArgs, typename... Args>

@@ -186,7 +186,7 @@ int launch(const void* X, const void* W, void* out, int M, int x_rows, int N, in
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return static_cast<int>(e);
   const int tiles = (N + kTileRows - 1) / kTileRows;
-  LRM_LAUNCH(kernel, dim3(tiles < 148 ? tiles : 148), kThreads, smem, stream, map_w, map_x, out, M, N, K, mode, status);
+  LRM_LAUNCH(kernel, dim3(tiles < kSmCount ? tiles : kSmCount), kThreads, smem, stream, map_w, map_x, out, M, N, K, mode, status);
   return 0;
 }
 

@@ -12,7 +12,7 @@ namespace {
 constexpr int BM = 64, BN = 64, BK = 16;
 constexpr int kFewRows = 32;
 
-// Few rows whose operands do not start on 16-byte boundaries.
+// Up to kFewRows rows whose operands do not start on 16-byte boundaries.
 // mode 0: C = acc;  mode 1: C += acc (the residual add folded into the epilogue)
 __global__ __launch_bounds__(256) void gemm_f32_kernel(const float* __restrict__ X,
                                                        const float* __restrict__ W,
@@ -234,7 +234,7 @@ int launch_tiled(const float* X, const float* W, float* C, int M, int N, int K, 
 bool prefers_wide_tile(int M, int N) {
   const long long wide = static_cast<long long>((M + 127) / 128) * ((N + 63) / 64);
   const long long small = static_cast<long long>((M + 63) / 64) * ((N + 63) / 64);
-  return 2 * ((wide + 147) / 148) <= (small + 147) / 148;
+  return 2 * ((wide + kSmCount - 1) / kSmCount) <= (small + kSmCount - 1) / kSmCount;
 }
 
 // Few rows (a head's logits, decoding): bound by reading W. A CTA owns 32 columns, a lane each, and its warps

@@ -20,16 +20,16 @@
 // and that slice's share of W_down y, scaled by the expert's weight, as one float32 plane
 // [T, width] per (choice, slice): the planes are added to the residual stream in plane order by
 // the caller (or by the next norm), so the sum has a fixed order and no atomics meet in memory.
-// A row's result depends on nothing else in the batch. This is the kernel of decoding and of
-// the float32 path; it reads an expert's matrices once per token that chose it.
+// This is the kernel of the float32 path and of small experts; it reads an expert's matrices once per
+// token that chose it. bfloat16 steps of few rows of larger experts read them once (moe_rows.cu).
 //
 // Experts, all at once (prompts in bfloat16, few experts per choice): the matrices are laid out so
 // that every expert's gate and up rows form one [E * 2 ff, width] matrix and the down matrices one
 // [width, E * ff] matrix. One tensor-core product gives every expert's gate and up for every
 // token; lrm_moe_dense_gate turns them into y, multiplied by the expert's weight for the token
 // (zero for an expert the token did not choose); a second product with the down matrix sums the
-// chosen experts' outputs in its K loop. It does E / top times the arithmetic a grouped product
-// would, on kernels several times faster than a grouped product on the warp-level tensor path.
+// chosen experts' outputs in its K loop. It does E / top times the arithmetic of products on rows sorted
+// by expert (moe_sorted.cu), which larger prompts take.
 //
 // Layout of the matrices for both: gate_up [E][2 ff][width] (an expert's gate rows, then its up
 // rows), down [width][E][ff].
@@ -548,7 +548,7 @@ LRM_API int lrm_moe_router(const void* x, int x_dtype, const float* w, const flo
   const size_t bytes = sizeof(float) * (static_cast<size_t>(width) + per_token);
   if (bytes > 48 * 1024) return LRM_UNSUPPORTED;
   // four tokens per CTA once that still leaves a CTA and more per SM; a warp per expert where few tokens leave room
-  const bool four = tokens >= 4 * 148 && 4 * bytes <= 48 * 1024;
+  const bool four = tokens >= 4 * kSmCount && 4 * bytes <= 48 * 1024;
   const int threads = !four && E >= 32 ? 1024 : !four && E >= 16 ? 512 : E >= 8 ? 256 : 128;
 #define LRM_ROUTER(AT)                                                                                                      \
   do {                                                                                                                      \

@@ -24,9 +24,16 @@
 // register for the packed FMAs. Bound by the shared-memory pipe (a vector goes to every warp: the wider a thread's tile,
 // the less) and, under the delta rules, by the chain through a block.
 //
-// The line to the token-by-token kernel (decoding) is a sequence of kWalkTokens tokens: below it the first
-// launch and the padding of blocks cost more than the chain they shorten (17 tokens of 16 heads 27 against 22 us, three
-// sequences of 30 on average 31 against 28; 250 tokens on average 84 against 142).
+// The line to the token-by-token kernel (decoding) is a sequence of kWalkTokens tokens: below it the launches and the padding
+// of blocks cost more than the chain they shorten. Blocks and token by token, us, delta rule and a decay per token: 16 heads of
+// 128 x 128, one sequence of 96 25 and 26, 23 and 21, of 128 25 and 34, 23 and 25, of 512 71 and 120, 59 and 88, of 2,048 260
+// and 463, 203 and 337; four of 100 46 and 98, 36 and 48; 100 of 96 753 and 1307, 494 and 887. 16 heads of 64 x 64, one of 96 23
+// and 21, 22 and 16, of 128 24 and 27, 23 and 19, of 192 28 and 38, 23 and 28; 8 heads of 256 x 64, one of 96 35 and 52, 28 and
+// 38. So it is early for a lone sequence of small heads by a few us, and right for several.
+//
+// Which sequences walk is each one's own matter, but the tokens of a block and the rows of a thread follow the step's size
+// (walk_plan), and with them the order of the sums: the same sequence gives other bits, within float32 rounding, in another
+// step. Who needs the bits goes without a workspace, token by token.
 #pragma once
 #include "recurrent_scan.cuh"
 
@@ -512,7 +519,7 @@ template <int MODE>
 WalkPlan walk_plan(int seqs, int H, int d, int dv, int tokens) {
   constexpr bool DELTA = WalkShape<64, MODE, 4>::DELTA;
   const long long ctas = static_cast<long long>((dv + 15) / 16) * H * walking_guess(seqs, tokens);
-  const bool few = 2 * ctas <= 148, many = ctas > (DELTA ? 2 : 3) * 148;
+  const bool few = 2 * ctas <= kSmCount, many = ctas > (DELTA ? 2 : 3) * kSmCount;
   if (d <= 64) return many ? WalkPlan{4, 1, 4} : WalkPlan{DELTA ? 8 : 4, 1, 2};
   if (d <= 128) return many ? WalkPlan{4, 2, 4} : WalkPlan{DELTA ? 8 : 4, few ? 1 : 2, 2};
   return DELTA ? WalkPlan{8, 4, 2} : WalkPlan{4, 2, 4};

@@ -1556,8 +1556,8 @@ def moe_identity_add_(out: torch.Tensor, x: torch.Tensor, ids: torch.Tensor, wei
 def moe_router(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], top: int,
                scoring: Optional[Scoring] = None):
     """moe_route(x . weight^T, bias, top) in one launch: float32 logits from x [T, width] (float32, or
-    bfloat16 widened exactly) and float32 weight [E, width], a CTA per token. For steps of few
-    tokens; None where the kernel does not take the sizes (the caller makes the product and routes).
+    bfloat16 widened exactly) and float32 weight [E, width], a CTA per token (per four tokens from 592 on). For
+    steps of few tokens or few outputs; None where the kernel does not take the sizes (the caller makes the product and routes).
     With `scoring` the choice is the scored router's (moe_route_scored) and `bias` is not used."""
     _check(x, "x", dims=2)
     _check(weight, "weight", torch.float32, 2)

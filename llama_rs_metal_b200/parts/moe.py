@@ -30,9 +30,9 @@ class MixtureOfExperts(FeedForward):
     to the stream in a fixed order (by the next norm where it folds them). All experts at once
     (bfloat16 steps of DENSE_ROWS tokens and more when at most DENSE_RATIO experts exist per chosen
     one): two tensor-core products over every expert, with the weights of the experts a token did not
-    choose set to zero between them. Sorted (such steps once they have tokens enough to fill tiles of
-    128 rows per expert, csrc/moe_sorted.cu): the same two products with every row in its own expert's
-    tile.
+    choose set to zero between them. Sorted (such steps of large experts once they have tokens enough to
+    fill tiles of 128 rows per expert, csrc/moe_sorted.cu): the same two products with every row in its
+    own expert's tile.
 
     Options beyond that router and that expert. `activation` "silu": an expert is W_down (silu(W_gate
     x) * (W_up x)). `scoring` "softmax_all": the scores are s = softmax(z) over all outputs; the
@@ -48,7 +48,7 @@ class MixtureOfExperts(FeedForward):
     by, `weight_scale` multiplies the weights afterwards."""
 
     graph_safe = True
-    ROUTER_ROWS = 256  # up to this many tokens the router always runs as one launch, a CTA per token
+    ROUTER_ROWS = 256  # up to this many tokens the router always runs as one launch
     DENSE_ROWS = 64   # from this many tokens on a step is a prompt: the tensor-core products pay
     DENSE_RATIO = 4   # experts per chosen expert up to which computing all of them is the faster way
 
