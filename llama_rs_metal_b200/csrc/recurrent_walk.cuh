@@ -15,7 +15,7 @@
 // every product and sum is float32. u is T (v - p) with the triangular T = (I + diag(b) C)^-1 diag(b). The p of a block
 // are added over the parts together: one exchange in place of L, and the read-outs' exchange overlaps it.
 //
-// Two launches. What does not depend on the column is made first, for all blocks at once, into a workspace: the
+// Two launches (behind one for a step's sequences that go token by token). What does not depend on the column is made first, for all blocks at once, into a workspace: the
 // vectors k G, q G, k (G_L / G_m) and G_L per head where decays differ by row, the bare k and q per key head where a
 // token has one decay (which then multiplies sums instead of vectors), and D, T and the other numbers per head. G_L of
 // one decay comes with the rounding it lost: a decay that is the same for every token would lose it the same way in
