@@ -1,6 +1,6 @@
 // The state scans with a plain decay (see recurrent_scan.cuh), the read-out's norm and gate, and the
 // inputs of retention and of the gated delta rule.
-#include "recurrent_walk.cuh"
+#include "recurrent_block.cuh"
 
 int g_scan_rows = 16;
 

@@ -29,8 +29,8 @@
 // shared memory a chunk at a time by asynchronous copies, the next chunk under way while this
 // one is worked on, so the inner loop has no block-wide barrier and waits for no load. This is the
 // kernel of decoding, of sequences that bring few tokens, of the float32 runtime, and of the generalized
-// rule and heads wider than 256; the other sequences go eight or four tokens at a time
-// (recurrent_walk.cuh).
+// rule and heads wider than 256; the other sequences go in blocks, 16 tokens at a time on the tensor cores
+// (recurrent_block.cuh) or eight or four (recurrent_walk.cuh).
 //
 // A sequence of padding (slot < 0) starts from zero and stores nothing.
 //

@@ -1,5 +1,5 @@
 // The gated delta rule with a decay per key channel, and with one decay per head (see recurrent_scan.cuh).
-#include "recurrent_walk.cuh"
+#include "recurrent_block.cuh"
 
 // Called by lrm_linear_state_scan, which has checked the arguments.
 extern "C" int lrm_scan_gated_delta(const float* q, const float* k, const float* v, const float* g, const float* beta,

@@ -1,5 +1,5 @@
 // The generalized delta rule and the scan with a bonus for the current token (see recurrent_scan.cuh).
-#include "recurrent_walk.cuh"
+#include "recurrent_block.cuh"
 
 // The generalized delta rule: q, k, v, g as above (one key head per head), look and put float32
 // [T, H, d]: S <- diag(g) S + put (look^T S) + k v^T with both terms reading the old S; o = S^T q.

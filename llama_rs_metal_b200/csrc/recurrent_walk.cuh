@@ -1,57 +1,22 @@
-// The state scan of recurrent_scan.cuh for long sequences (prompts), a block of L tokens at a time (8 under the delta
-// rules, else 4).
+// State scans of long sequences with float32 FMAs, a block of L tokens at a time (the formulas of recurrent_block.cuh): the way
+// of steps whose sequences and heads make more CTAs than the SMs hold at once, where the tensor path of recurrent_block.cuh
+// pays more for its preparation, once per head, than it gains in the walk (block_takes_fma says where the line lies).
 //
-// A sequence's tokens form a chain through its state. Taken one by one, every token of a delta rule waits for
-// a sum over the state's rows that is spread over threads: 430 cycles a token. Here a block of tokens
-// reads the state once. With G_j the product of the decays of the block's first j tokens (per row i of the
-// state) and S the state ahead of the block,
-//   p_j = sum_i k_ji G_ji S_i                              what token j reads, but for its block's own writes
-//   u_j = b_j (v_j - p_j - sum_{m<j} C_jm u_m)             C_jm = sum_i k_ji (G_j / G_m)_i k_mi      (delta rules)
-//   u_j = v_j                                                                                        (the others)
-//   o_j = sum_i q_ji G_ji S_i + sum_{m<=j} D_jm u_m        D_jm = sum_i q_ji (G_j / G_m)_i k_mi
-//   S_i <- G_Li S_i + sum_m k_mi (G_L / G_m)_i u_m
-// (with a bonus m for the newest, read before the write: G_{j-1} for q_j's G_j, and D_jj = sum_i q_ji m_i k_ji.)
-// Quotients of decays are made as products of the decays between, so nothing is divided by a small number;
-// every product and sum is float32. u is T (v - p) with the triangular T = (I + diag(b) C)^-1 diag(b). The p of a block
-// are added over the parts together: one exchange in place of L, and the read-outs' exchange overlaps it.
-//
-// Two launches (behind one for a step's sequences that go token by token). What does not depend on the column is made first, for all blocks at once, into a workspace: the
-// vectors k G, q G, k (G_L / G_m) and G_L per head where decays differ by row, the bare k and q per key head where a
-// token has one decay (which then multiplies sums instead of vectors), and D, T and the other numbers per head. G_L of
-// one decay comes with the rounding it lost: a decay that is the same for every token would lose it the same way in
-// every block. Then a CTA per (sequence, head, tile of columns) walks the blocks; stages of 16 tokens come as contiguous
-// pieces through asynchronous copies. A walking thread holds 4 NQ rows of C columns, two rows of a column in one 64-bit
-// register for the packed FMAs. Bound by the shared-memory pipe (a vector goes to every warp: the wider a thread's tile,
-// the less) and, under the delta rules, by the chain through a block.
-//
-// The line to the token-by-token kernel (decoding) is a sequence of kWalkTokens tokens: below it the launches and the padding
-// of blocks cost more than the chain they shorten. Blocks and token by token, us, delta rule and a decay per token: 16 heads of
-// 128 x 128, one sequence of 96 25 and 26, 23 and 21, of 128 25 and 34, 23 and 25, of 512 71 and 120, 59 and 88, of 2,048 260
-// and 463, 203 and 337; four of 100 46 and 98, 36 and 48; 100 of 96 753 and 1307, 494 and 887. 16 heads of 64 x 64, one of 96 23
-// and 21, 22 and 16, of 128 24 and 27, 23 and 19, of 192 28 and 38, 23 and 28; 8 heads of 256 x 64, one of 96 35 and 52, 28 and
-// 38. So it is early for a lone sequence of small heads by a few us, and right for several.
-//
-// Which sequences walk is each one's own matter, but the tokens of a block and the rows of a thread follow the step's size
-// (walk_plan), and with them the order of the sums: the same sequence gives other bits, within float32 rounding, in another
-// step. Who needs the bits goes without a workspace, token by token.
+// Quotients of decays are made as products of the decays between; every product and sum is float32. What does not depend on
+// the column is made first, for all blocks at once: the vectors k G, q G, k (G_L / G_m) and G_L per head where decays differ by
+// row, the bare k and q per key head where a token has one decay, and D, T and the other numbers per head. Then a CTA per
+// (sequence, head, tile of columns) walks the blocks; a walking thread holds 4 NQ rows of C columns, two rows of a column in one
+// 64-bit register for the packed FMAs. Bound by the shared-memory pipe (a vector goes to every warp: the wider a thread's
+// tile, the less). 16 heads of 128 x 128, eight sequences of 1,024 tokens (1,024 CTAs at 16 columns): two quads of rows and two
+// columns a thread 890 us, and 609 with four columns and 4 tokens a block (which leaves registers for them); a decay per
+// token 524 and 428.
 #pragma once
 #include "recurrent_scan.cuh"
 
 namespace {
 
 constexpr int kWalkStage = 16;   // tokens of a stage
-constexpr int kWalkTokens = 96;  // tokens of a sequence from which this way of computing pays
-
-template <int DP, int MODE, int L>
-struct WalkShape {
-  static constexpr bool DELTA = MODE == 1 || MODE == 5, ROW_DECAY = MODE == 1 || MODE == 4, BONUS = MODE == 4;
-  static constexpr int BLOCKS = kWalkStage / L;                               // of a stage
-  static constexpr int VECTORS = !ROW_DECAY ? 2 * L : DELTA ? 3 * L + 1 : 2 * L + 1;  // of DP floats, in a block
-  static constexpr int AT_Q = DELTA || !ROW_DECAY ? L * DP : 0, AT_W = ROW_DECAY ? AT_Q + L * DP : 0, AT_G = AT_W + L * DP;
-  static constexpr int STAGE = BLOCKS * VECTORS * DP;                        // floats of a stage's vectors
-  // numbers of a block and head: D [L][L] | T [L][L] | G_j [L] | G_L / G_j [L] | G_L and what its rounding lost
-  static constexpr int AT_T = L * L, AT_UPTO = 2 * L * L, AT_REST = AT_UPTO + L, AT_ALL = AT_REST + L, SCALARS = AT_ALL + 4;
-};
+constexpr int kWalkTokens = 96;  // tokens of a sequence from which going in blocks pays
 
 // Stages of sequence b are numbered from walk_base(b) on: a whole number of stages each, none shared. A launch takes a run of
 // them: all, or as many as the workspace has room for.
@@ -78,6 +43,39 @@ __device__ __forceinline__ int walking_sequence(const int* cu_seqlens, int seqs,
   }
   return -1;
 }
+
+inline long long walk_stages(int tokens, int seqs) { return tokens / kWalkStage + seqs; }
+inline int walk_padded(int d) { return d > 128 ? 256 : d > 64 ? 128 : 64; }
+
+// Scratch of `floats` floats, 16-byte aligned.
+struct Workspace {
+  float* at;
+  long long floats;
+};
+
+// Everything a walk is launched with.
+struct WalkArgs {
+  const float *q, *k, *v, *g, *head_decay, *beta, *look, *put;
+  float *state, *out;
+  const int *cu_seqlens, *slots;
+  int seqs, H, KH, d, dv;
+  Workspace workspace;
+  cudaStream_t stream;
+  Rows rows;
+  int least;     // tokens of a sequence from which it walks (0: a step of one sequence, which has them)
+  int walkers;   // sequences that may
+};
+
+template <int DP, int MODE, int L>
+struct WalkShape {
+  static constexpr bool DELTA = MODE == 1 || MODE == 5, ROW_DECAY = MODE == 1 || MODE == 4, BONUS = MODE == 4;
+  static constexpr int BLOCKS = kWalkStage / L;                               // of a stage
+  static constexpr int VECTORS = !ROW_DECAY ? 2 * L : DELTA ? 3 * L + 1 : 2 * L + 1;  // of DP floats, in a block
+  static constexpr int AT_Q = DELTA || !ROW_DECAY ? L * DP : 0, AT_W = ROW_DECAY ? AT_Q + L * DP : 0, AT_G = AT_W + L * DP;
+  static constexpr int STAGE = BLOCKS * VECTORS * DP;                        // floats of a stage's vectors
+  // numbers of a block and head: D [L][L] | T [L][L] | G_j [L] | G_L / G_j [L] | G_L and what its rounding lost
+  static constexpr int AT_T = L * L, AT_UPTO = 2 * L * L, AT_REST = AT_UPTO + L, AT_ALL = AT_REST + L, SCALARS = AT_ALL + 4;
+};
 
 // A CTA per stage and head (row decays) or key head.
 template <int DP, int MODE, int L>
@@ -493,38 +491,6 @@ __global__ __launch_bounds__(128) void walk_scan_kernel(
   }
 }
 
-inline long long walk_stages(int tokens, int seqs) { return tokens / kWalkStage + seqs; }
-inline int walk_padded(int d) { return d > 128 ? 256 : d > 64 ? 128 : 64; }
-
-// Whether a step may hold sequences that go this way: heads of up to 256. Which ones do is decided by each sequence's own
-// tokens, in the kernels, so that its bits do not hang on the lengths of the others.
-inline bool takes_walk(int d, int tokens) { return tokens >= kWalkTokens && d <= 256; }
-inline int walking(int seqs, int tokens) { return seqs < tokens / kWalkTokens ? seqs : tokens / kWalkTokens; }  // at most
-// A guess at how many, for the layout: all where they bring kWalkTokens on average; else their lengths differ a lot, and the
-// longest is what a step waits for. (2,048 tokens beside 31 sequences of one, 8 heads of 128: 493 us laid out for many, 204
-// for one.)
-inline int walking_guess(int seqs, int tokens) { return tokens >= static_cast<long long>(seqs) * kWalkTokens ? seqs : 1; }
-
-// How a step's walks are cut: tokens of a block, quads of rows and columns a thread holds.
-struct WalkPlan {
-  int L, NQ, C;
-};
-
-// Measured for heads of 128 x 128 (CTAs counted at 16 columns each), us. Delta rule: 8 heads (64 CTAs), 2,048 tokens, 8 tokens
-// a block: a quad and two columns a thread 224, two quads 252; 16 heads (128 CTAs) 320 and 261; 16 heads, eight sequences
-// of 1,024 tokens (1,024 CTAs): two quads, two columns 890, and 609 with four columns and 4 tokens a block (which leaves
-// registers for them). A decay per token: 64 CTAs 183 with one quad and two columns, 206 with two quads; 256 CTAs (32
-// heads of 128 x 64, 1,500 and 777 tokens) 249, 187 and 218 with two quads and four columns; 1,024 CTAs 678, 524, 428.
-template <int MODE>
-WalkPlan walk_plan(int seqs, int H, int d, int dv, int tokens) {
-  constexpr bool DELTA = WalkShape<64, MODE, 4>::DELTA;
-  const long long ctas = static_cast<long long>((dv + 15) / 16) * H * walking_guess(seqs, tokens);
-  const bool few = 2 * ctas <= kSmCount, many = ctas > (DELTA ? 2 : 3) * kSmCount;
-  if (d <= 64) return many ? WalkPlan{4, 1, 4} : WalkPlan{DELTA ? 8 : 4, 1, 2};
-  if (d <= 128) return many ? WalkPlan{4, 2, 4} : WalkPlan{DELTA ? 8 : 4, few ? 1 : 2, 2};
-  return DELTA ? WalkPlan{8, 4, 2} : WalkPlan{4, 2, 4};
-}
-
 // Floats of a stage in the workspace: its vectors, and its numbers per head (behind the vectors of all stages).
 template <int MODE, int L>
 long long walk_vectors(int H, int KH, int d) {
@@ -532,43 +498,16 @@ long long walk_vectors(int H, int KH, int d) {
   return static_cast<long long>(W::BLOCKS) * (W::ROW_DECAY ? H : KH) * W::VECTORS * walk_padded(d);
 }
 template <int MODE, int L>
-long long walk_stage_floats(int H, int KH, int d) {
+long long walk_block_floats(int H, int KH, int d) {
   using W = WalkShape<64, MODE, L>;
   return walk_vectors<MODE, L>(H, KH, d) + static_cast<long long>(W::BLOCKS) * H * W::SCALARS;
 }
 
-// Floats of a workspace that holds a step whole, 0 where the token-by-token kernel runs.
-template <int MODE>
-long long walk_floats(int seqs, int H, int KH, int d, int dv, int tokens) {
-  if (!takes_walk(d, tokens)) return 0;
-  return walk_plan<MODE>(seqs, H, d, dv, tokens).L == 8 ? walk_stages(tokens, seqs) * walk_stage_floats<MODE, 8>(H, KH, d)
-                                                        : walk_stages(tokens, seqs) * walk_stage_floats<MODE, 4>(H, KH, d);
-}
-
-// Scratch of `floats` floats, 16-byte aligned.
-struct Workspace {
-  float* at;
-  long long floats;
-};
-
-// Everything a walk is launched with.
-struct WalkArgs {
-  const float *q, *k, *v, *g, *head_decay, *beta, *look, *put;
-  float *state, *out;
-  const int *cu_seqlens, *slots;
-  int seqs, H, KH, d, dv;
-  Workspace workspace;
-  cudaStream_t stream;
-  Rows rows;
-  int least;  // tokens of a sequence from which it walks (0: a step of one sequence, which has them)
-};
-
 template <int NQ, int C, int DP, int MODE, int L>
 int launch_walk(const WalkArgs& a) {
   using K = Walk<NQ, C, DP, MODE, L>;
-  const long long all = walk_stages(a.rows.tokens, a.seqs), room = a.workspace.floats / walk_stage_floats<MODE, L>(a.H, a.KH, a.d);
-  const int walkers = walking(a.seqs, a.rows.tokens);
-  auto kernel = room >= all && walkers == a.seqs ? walk_scan_kernel<NQ, C, DP, MODE, L, true>
+  const long long all = walk_stages(a.rows.tokens, a.seqs), room = a.workspace.floats / walk_block_floats<MODE, L>(a.H, a.KH, a.d);
+  auto kernel = room >= all && a.walkers == a.seqs ? walk_scan_kernel<NQ, C, DP, MODE, L, true>
                                                  : walk_scan_kernel<NQ, C, DP, MODE, L, false>;
   if (K::BYTES > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(K::BYTES));
@@ -585,42 +524,30 @@ int launch_walk(const WalkArgs& a) {
     LRM_LAUNCH((walk_prepare_kernel<DP, MODE, L>), dim3(piece.count, K::W::ROW_DECAY ? a.H : a.KH), 128, 0, a.stream, a.q, a.k, a.g,
                a.head_decay, a.beta, a.look, a.put, a.workspace.at, scalars, a.cu_seqlens, a.seqs, a.H, a.KH, a.d, q_stride, a.least,
                piece);
-    kernel<<<dim3((a.dv + K::COLS - 1) / K::COLS, a.H, walkers), 128, K::BYTES, a.stream>>>(
+    kernel<<<dim3((a.dv + K::COLS - 1) / K::COLS, a.H, a.walkers), 128, K::BYTES, a.stream>>>(
         a.workspace.at, scalars, a.v, a.state, a.out, a.cu_seqlens, a.slots, a.seqs, a.H, a.KH, a.d, a.dv, v_stride, wide, a.least, piece);
     LRM_LAUNCH_CHECK();
   }
   return 0;
 }
 
-// A step that the workspace does not hold whole goes in pieces, a run of stages at a time: a state is float32 on the way from
-// piece to piece as it is within one, so the bits are the same. Padding has no state to go on from, so there it goes token by
-// token. `workspace`: as many floats as a stage has at least.
 template <int MODE>
-int dispatch_walk(const float* q, const float* k, const float* v, const float* g, const float* head_decay, const float* beta,
-                  const float* look, const float* put, float* state, float* out, const int* cu_seqlens, const int* slots, int seqs,
-                  int H, int KH, int d, int dv, const Workspace& workspace, cudaStream_t stream, const Rows& rows) {
-  WalkArgs a{q, k, v, g, head_decay, beta, look, put, state, out, cu_seqlens, slots, seqs, H, KH, d, dv, workspace, stream, rows, 0};
-  const WalkPlan plan = walk_plan<MODE>(seqs, H, d, dv, rows.tokens);
-  constexpr int LONG = WalkShape<64, MODE, 4>::DELTA ? 8 : 4;
-  const long long stage = plan.L == 8 ? walk_stage_floats<MODE, 8>(H, KH, d) : walk_stage_floats<MODE, 4>(H, KH, d);
-  if (reinterpret_cast<uintptr_t>(workspace.at) % 16 || workspace.floats < stage) return LRM_BAD_ARGUMENT;
-  const bool pieces = workspace.floats / stage < walk_stages(rows.tokens, seqs);
-  if (seqs > 1 || pieces) {  // the sequences that bring fewer tokens, one after another
-    a.least = seqs > 1 ? kWalkTokens : 0;
-    Rows few = rows;
-    few.below = a.least, few.below_padding = pieces ? INT_MAX : kWalkTokens;
-    const int code = dispatch_scan<MODE>(q, k, v, g, head_decay, beta, look, put, state, out, cu_seqlens, slots, seqs, H, KH, d, dv,
-                                         stream, few);
-    if (code != 0) return code;
+constexpr int walk_block(int padded) {  // tokens of a block
+  return padded == 256 && WalkShape<64, MODE, 4>::DELTA ? 8 : 4;
+}
+template <int MODE>
+long long walk_stage_floats(int H, int KH, int d) {
+  return walk_block<MODE>(walk_padded(d)) == 8 ? walk_block_floats<MODE, 8>(H, KH, d) : walk_block_floats<MODE, 4>(H, KH, d);
+}
+template <int MODE>
+int launch_walk(const WalkArgs& a) {
+  constexpr int LONG = walk_block<MODE>(256);
+  if (a.d > 128) return launch_walk<(LONG == 8 ? 4 : 2), (LONG == 8 ? 2 : 4), 256, MODE, LONG>(a);
+  if constexpr (MODE != 0 && MODE != 2) {  // (where the tensor path is always the faster one)
+    if (a.d > 64) return launch_walk<2, 4, 128, MODE, 4>(a);
+    return launch_walk<1, 4, 64, MODE, 4>(a);
   }
-  if (d > 128) return launch_walk<(LONG == 8 ? 4 : 2), (LONG == 8 ? 2 : 4), 256, MODE, LONG>(a);
-  if (d > 64) {
-    if (plan.C == 4) return launch_walk<2, 4, 128, MODE, 4>(a);
-    if (plan.NQ == 1) return launch_walk<1, 2, 128, MODE, LONG>(a);
-    return launch_walk<2, 2, 128, MODE, LONG>(a);
-  }
-  if (plan.C == 4) return launch_walk<1, 4, 64, MODE, 4>(a);
-  return launch_walk<1, 2, 64, MODE, LONG>(a);
+  return LRM_UNSUPPORTED;
 }
 
 }  // namespace

@@ -1,0 +1,71 @@
+"""State scans of long sequences in blocks of 16 tokens on the tensor cores (csrc/recurrent_block.cuh), at the edges of its blocks, its
+tiles of 16 columns, its rows per warp, and of the line to the blocks with FMAs (csrc/recurrent_walk.cuh)."""
+import pytest
+import torch
+
+from test_state_walk_gpu import DEV, _inputs, _int32, _reference, _run
+
+pytestmark = pytest.mark.gpu
+
+RULES = ["delta", "head_delta", "token_decay", "head_decay", "bonus"]
+
+
+def _distance(a, b):
+    return float((a.double() - b).norm() / b.norm())
+
+
+# 16 to 1 rows of the last piece of a warp, columns of a whole tile, one more, one; blocks of 16, 15 and one token at the end
+@pytest.mark.parametrize("lengths", [[96, 111], [112, 113, 0, 7]])
+@pytest.mark.parametrize("H,G,d,dv", [(2, 2, 64, 16), (4, 2, 49, 17), (2, 1, 128, 1), (2, 2, 113, 33), (2, 1, 256, 16), (1, 1, 193, 31),
+                                      (6, 1, 16, 8)])
+@pytest.mark.parametrize("rule", RULES)
+def test_edges_match_the_recurrence_no_further_off_than_token_by_token(rule, H, G, d, dv, lengths):
+    G = H if rule == "bonus" else G
+    x = _inputs(H, G, d, dv, lengths, seed=d + dv)
+    slots = list(range(len(lengths)))
+    want, single = _reference(rule, x, lengths, slots), _run(rule, x, lengths, slots, blocks=False)
+    for a, b, c in zip(_run(rule, x, lengths, slots), want, single):
+        assert _distance(a, b) <= 2e-6                             # float32 sums, forgotten at the decays' rate
+        assert _distance(a, b) <= 2 * _distance(c, b) + 2.0 ** -24  # both are sums of roundings of 2^-24
+
+
+# CTAs (tiles x heads x sequences) on both sides of the line: 370 for delta rules, 444 with a bonus, 222 for heads beyond 128
+@pytest.mark.parametrize("H,d,dv,seqs", [(46, 64, 64, 2), (47, 64, 64, 2), (55, 64, 64, 2), (56, 64, 64, 2), (37, 160, 48, 2), (38, 160, 48, 2)])
+@pytest.mark.parametrize("rule", RULES)
+def test_both_sides_of_the_line_to_the_blocks_with_fmas(rule, H, d, dv, seqs):
+    lengths = [97 + 16 * i for i in range(seqs)]
+    x = _inputs(H, H, d, dv, lengths, seed=H)
+    for a, b in zip(_run(rule, x, lengths, [1, 0]), _reference(rule, x, lengths, [1, 0])):
+        assert _distance(a, b) <= 2e-6
+
+
+@pytest.mark.parametrize("rule", RULES)
+def test_inputs_off_16_bytes(rule):
+    x = _inputs(3, 3, 64, 24, [130], seed=2)
+    moved = {}
+    for name, t in x.items():
+        room = torch.empty(t.numel() + 1, device=DEV)
+        moved[name] = room[1:].view(t.shape).copy_(t)
+    for a, b in zip(_run(rule, moved, [130], [0]), _run(rule, x, [130], [0])):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("name,value", [("q", float("inf")), ("k", float("nan")), ("v", float("-inf")), ("g", float("nan"))])
+@pytest.mark.parametrize("rule", RULES)
+def test_what_is_not_finite_shows_where_it_does_token_by_token(rule, name, value):
+    """In the second block of eight, in one head and sequence: what comes ahead of it, other heads and the other sequence stay as
+    they are, and no read-out that is finite token by token is not."""
+    lengths, token = [130, 100], 27
+    x = _inputs(2, 2, 64, 20, lengths, seed=7)
+    clean, _ = _run(rule, x, lengths, [1, 0])
+    x[name][token, 1, 3] = value
+    if name == "g":
+        x["decay"][token, 1] = value
+    got, state = _run(rule, x, lengths, [1, 0])
+    want, want_state = _run(rule, x, lengths, [1, 0], blocks=False)
+    for a, b in ((got, want), (state, want_state)):
+        whole = b.isfinite()
+        assert bool(a[whole].isfinite().all()) and _distance(a[whole], b[whole].double()) <= 2e-6
+        assert not bool(a[~whole].isfinite().any())
+    assert torch.equal(got[:16], clean[:16]) and torch.equal(got[130:], clean[130:])
+    assert _distance(got[16:token], clean[16:token].double()) <= 2e-6
