@@ -1,4 +1,5 @@
-// True 32-bit matrix product on the CUDA cores: C[M,N] = X[M,K] . W[N,K]^T.
+// True 32-bit matrix product on the CUDA cores: C[M,N] = X[M,K] . W[N,K]^T, for the smaller matrices and for operands off 16 bytes
+// (gemm_f32_umma.cu has the others).
 // W is a Linear weight as stored ([out][in]); every product and sum is an
 // IEEE float32 fused multiply-add, with no tensor-core or reduced-precision
 // mode anywhere. Each output element is accumulated over k = 0..K-1 in

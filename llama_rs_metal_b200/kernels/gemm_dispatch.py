@@ -73,7 +73,9 @@ def check_status() -> None:
                           46: "a free key/value stage", 47: "aligned shared memory"})
             names.update({51: "a free stage", 52: "operand tiles", 53: "the accumulator", 54: "copies in flight",
                           55: "a free accumulator"})
-            kernel = "gemm_bf16_few" if code >= 51 else "attention_gated_umma" if code >= 41 else "gemm_bf16_umma_pair" \
+            names.update({61: "a free stage", 62: "operand parts", 63: "the accumulator", 64: "operand tiles", 65: "copies in flight",
+                          66: "a free tile"})
+            kernel = "gemm_f32_umma" if code >= 61 else "gemm_bf16_few" if code >= 51 else "attention_gated_umma" if code >= 41 else "gemm_bf16_umma_pair" \
                 if code >= 31 else "attention_prefill_pingpong" if code >= 21 else "gemm_bf16_umma"
             raise LlamaError(f"{kernel} gave up waiting for {names.get(code, code)}; its result is invalid")
 
@@ -355,6 +357,35 @@ def gemm_bf16(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, mode: in
         return
     _done(lib.lrm_gemm_bf16_mma(_ptr(x), _ptr(weight), _ptr(out), M, N, K, mode, _stream()),
           "gemm_bf16_mma")
+
+
+def f32_takes_umma(N: int, K: int) -> bool:
+    """Whether a float32 product goes to the tensor cores in three-part splits (csrc/gemm_f32_umma.cu) or to the FMA kernels
+    (csrc/gemm_f32.cu). A matter of the matrix alone, so that a row gives the same bits however many there are. us for 1, 32 and 333
+    rows, in brackets the FMA kernels: 1024 x 1024 9.3 (12.7), 10.7 (28.8), 14.9 (39.4); 512 x 2048 9.7 (23.9), 11.3 (56.3), 16.6
+    (76.9); 2048 x 512, below the line, 9.1 (6.9), 9.7 (15.3), 21.0 (32.7). Of larger matrices a single row of 128256 x 2048 alone is slower
+    (193 against 177). Rows on 32 bytes (K a multiple of 8), as the parts' copies want them."""
+    return K % 8 == 0 and K >= 1024 and N >= 512
+
+
+def gemm_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, mode: int, rows: int, group_cols: int = 0) -> None:
+    """float32 out [rows, N] (mode 0: =, 1: +=) x . weight^T. group_cols > 0: columns i * group_cols .. belong to the input that begins
+    i * rows rows into x. The kernel follows from the matrix and the addresses alone, never from `rows`."""
+    N, K = weight.shape
+    lib = library.load()
+    if (f32_takes_umma(N, K) and not force_tiled and group_cols % 128 == 0 and x.data_ptr() % 16 == 0
+            and weight.data_ptr() % 16 == 0):
+        mark_status_dirty()
+        scratch = lib.lrm_gemm_f32_umma_scratch(rows, x.numel() // K, K)
+        parts = torch.empty(scratch, dtype=torch.uint8, device=x.device) if scratch else None
+        _done(lib.lrm_gemm_f32_umma(_ptr(x), _ptr(weight), _ptr(out), rows, N, K, mode, group_cols, rows, _ptr(parts),
+                                    _ptr(_status_word(x.device)), _stream()), "gemm_f32_umma", launches=2 if scratch else 1)
+        return
+    if group_cols:
+        _done(lib.lrm_gemm_f32_grouped(_ptr(x), _ptr(weight), _ptr(out), rows, N, K, mode, group_cols, rows, _stream()),
+              "gemm_f32_grouped")
+    else:
+        _done(lib.lrm_gemm_f32(_ptr(x), _ptr(weight), _ptr(out), rows, N, K, mode, _stream()), "gemm_f32")
 
 
 def gemm_bf16_split(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, gated: torch.Tensor) -> None:

@@ -301,8 +301,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, epilogue: str = STORE,
             if out_dtype not in (None, torch.float32):
                 raise InvalidError("linear: float32 inputs give float32 outputs")
             out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-        _done(lib.lrm_gemm_f32(_ptr(x), _ptr(weight), _ptr(out), M, N, K,
-                               1 if epilogue == ADD else 0, _stream()), "gemm_f32")
+        from . import gemm_dispatch
+        gemm_dispatch.gemm_f32(x, weight, out, 1 if epilogue == ADD else 0, M)
         return out
     if x.dtype != torch.bfloat16:
         raise UnsupportedError(f"linear: dtype {x.dtype}")
@@ -365,8 +365,8 @@ def linear_grouped(x: torch.Tensor, weight: torch.Tensor, group_cols: int) -> to
         raise InvalidError("linear_grouped: whole tiles per input, and rows of weight for every input")
     out = torch.empty((T, N), dtype=torch.float32, device=x.device)
     if x.dtype == torch.float32:
-        _done(_lib().lrm_gemm_f32_grouped(_ptr(x), _ptr(weight), _ptr(out), T, N, K, 0, group_cols, T, _stream()),
-              "gemm_f32_grouped")
+        from . import gemm_dispatch
+        gemm_dispatch.gemm_f32(x, weight, out, 0, T, group_cols)
         return out
     from . import gemm_dispatch
     gemm_dispatch.gemm_bf16_grouped(x, weight, out, group_cols)

@@ -79,6 +79,7 @@ WORK: Dict[str, Callable[..., Tuple[float, float]]] = {
     "lrm_rms_norm": lambda a: (_v(a[9]) * _v(a[10]) * (4 + _ELEM[_v(a[4])] + 4 * _v(a[7]) + (4 if _v(a[7]) else 0)),
                                3.0 * _v(a[9]) * _v(a[10])),
     "lrm_gemm_f32": lambda a: _gemm(_v(a[3]), _v(a[4]), _v(a[5]), 8 if _v(a[6]) else 4, 4),
+    "lrm_gemm_f32_umma": lambda a: _gemm(_v(a[3]), _v(a[4]), _v(a[5]), 8 if _v(a[6]) else 4, 4),
     "lrm_gemm_bf16_stream_shaped": lambda a: _gemm(_v(a[3]), _v(a[4]), _v(a[5]), _out_elem(_v(a[6]))),
     "lrm_gemm_bf16_mma": lambda a: _gemm(_v(a[3]), _v(a[4]), _v(a[5]), _out_elem(_v(a[6]))),
     "lrm_gemm_bf16_umma_rows": lambda a: _gemm(_v(a[3]), _v(a[5]), _v(a[6]), _out_elem(_v(a[7]))),

@@ -1,0 +1,77 @@
+"""float32 products on the tensor cores (csrc/gemm_f32_umma.cu) against float64: rows around its tiles and the kernel for few, matrices off
+its tiles of 128 rows and blocks of 64 of K, with one to four slices of K."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+MATRICES = [(512, 1024), (520, 1032), (1000, 2056), (1537, 4096), (12416, 1088)]  # slices: 2, 2, 4, 4, 1
+ROWS = [1, 16, 17, 32, 33, 47, 128, 129, 257]
+
+
+def _randn(*shape, seed=0):
+    return torch.randn(shape, generator=torch.Generator(device=DEV).manual_seed(seed), device=DEV)
+
+
+def _bound(x, w):
+    """Left-out products 2^-22 of the numbers' (2^-7 2^-16 twice), four large truncated additions a block at 2^-22 each, and a rounding
+    of 2^-24 for each of the K / 64 additions between blocks."""
+    K = x.shape[1]
+    return (5 * 2.0 ** -22 + K * 2.0 ** -30) * (x.double().abs() @ w.double().abs().T)
+
+
+@pytest.mark.parametrize("N,K", MATRICES)
+@pytest.mark.parametrize("M", ROWS)
+def test_products_match_float64_and_a_row_does_not_depend_on_the_batch(M, N, K):
+    from llama_rs_metal_b200.kernels import gemm_dispatch, ops
+    assert gemm_dispatch.f32_takes_umma(N, K)
+    x, w = _randn(M, K), _randn(N, K, seed=1)
+    got = ops.linear(x, w)
+    assert bool(((got.double() - x.double() @ w.double().T).abs() <= _bound(x, w)).all())
+    for r in {0, M // 2, M - 1}:
+        assert torch.equal(ops.linear(x[r:r + 1].contiguous(), w)[0], got[r])
+    total = _randn(M, N, seed=2)
+    want = total + got
+    assert torch.equal(ops.linear(x, w, epilogue=ops.ADD, out=total), want)
+    gemm_dispatch.check_status()
+
+
+@pytest.mark.parametrize("T", [5, 40])
+def test_grouped_inputs_match_single_ones(T):
+    from llama_rs_metal_b200.kernels import ops
+    x, w = _randn(3, T, 1024), _randn(2 * 384 + 200, 1024, seed=1)
+    got = ops.linear_grouped(x, w, 384)
+    for i, (begin, end) in enumerate(((0, 384), (384, 768), (768, 968))):
+        want = x[i].double() @ w[begin:end].double().T
+        assert bool(((got[:, begin:end].double() - want).abs() <= _bound(x[i], w[begin:end])).all())
+
+
+@pytest.mark.parametrize("M", [20, 140])
+def test_numbers_out_of_the_parts_range(M):
+    """Infinities, NaNs and numbers of 2^40 and more are added with float32 FMAs, in their row and column alone; the smallest numbers
+    keep their bits."""
+    from llama_rs_metal_b200.kernels import ops
+    x, w = _randn(M, 1024), _randn(640, 1024, seed=1)
+    clean = ops.linear(x, w)
+    x[3, 100], x[5, 7], x[6, 1023], x[M - 1, 512] = float("inf"), float("nan"), 3e38, 2.0 ** 41
+    w[2, 9], w[600, 64] = float("-inf"), 1e30
+    x[8] *= 2.0 ** -118
+    got, want = ops.linear(x, w), x.double() @ w.double().T
+    rows = torch.tensor([r for r in range(M) if r not in (3, 5, 6, 8, M - 1)], device=DEV)
+    cols = torch.tensor([c for c in range(640) if c not in (2, 600)], device=DEV)
+    assert torch.equal(got[rows][:, cols], clean[rows][:, cols])
+    single = want.float()                                    # what float32 can hold
+    assert torch.equal(got.isnan(), single.isnan()) and torch.equal(got.isinf(), single.isinf())
+    assert torch.equal(got[got.isinf()], single[got.isinf()])
+    whole = single.isfinite()
+    x[5, 7], x[3, 100], w[2, 9] = 0.0, 0.0, 0.0
+    bound = 1024 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T) + 1024 * 2.0 ** -149  # a rounding per FMA, and of the smallest
+    assert bool(((got.double() - want).abs() <= bound)[whole].all())
+
+
+def test_rows_off_16_bytes_go_to_the_other_kernels():
+    from llama_rs_metal_b200.kernels import ops
+    room = torch.empty(9 * 1024 + 1, device=DEV)
+    x, w = room[1:].view(9, 1024).copy_(_randn(9, 1024)), _randn(512, 1024, seed=1)
+    assert bool(((ops.linear(x, w).double() - x.double() @ w.double().T).abs() <= 1024 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)).all())
