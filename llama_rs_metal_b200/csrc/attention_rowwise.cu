@@ -1,8 +1,16 @@
-// Causal grouped-query attention, one warp per (query, head), keys visited one
-// at a time with a streaming softmax in float32:
-//   s = (q.k) * scale;  m' = max(m, s);  l = l e^(m-m') + e^(s-m');
-//   acc = acc e^(m-m') + e^(s-m') v;  out = acc / l
+// Causal grouped-query attention, a warp per (query, head), with a streaming softmax in float32 over blocks of 32 keys (heads of up
+// to 128) or single keys (wider ones):
+//   s = (q.k) * scale;  m' = max(m, s);  l = l e^(m-m') + sum e^(s-m');
+//   acc = acc e^(m-m') + sum e^(s-m') v;  out = acc / l
 // (reference: crates/metal-backend/src/shaders/attention.metal:28-57).
+//
+// A block's keys lie at multiples of 32 of their positions, a lane per key for the scores and a lane per column for the values, both
+// added in ascending order, so a row's sums depend on nothing but the row. A CTA has up to 16 rows of a key/value head (queries and
+// the heads that share it) and brings a block's keys and values to shared memory once for all of them, the next block's on their way
+// meanwhile. Bound by a CTA's chain of blocks. The 1B shape in float32, us: a prompt of 333 tokens 62 (160 key by key, each of which
+// waited for the sum of its dot product over the warp), a decode step of two layers with 3,000 keys, four sequences, 593 (6,287),
+// 300 tokens onto 1,000 1,207 (7,570). 32 rows a CTA 509 a layer's prompt against 495, 8 rows 494 and 1,247 for the portion.
+//
 // It is the attention of the float32 path for prompts and for decoding, and
 // the bfloat16 path's fallback for sizes its tiled kernels refuse (head sizes up to 1024). The two
 // entry points differ only in where keys come from (the step's packed k/v, or
@@ -22,6 +30,8 @@
 // 1 + temp_coef * ln(floor((p + 1) / temp_every) + 1) times (the factor goes into the score's
 // scale, in float32). `v_stride` is the distance between two value rows in elements: values
 // that are the first dv columns of the key rows are read from the keys' storage with the keys' d.
+#include <climits>
+
 #include "common.cuh"
 
 constexpr int kWidest = 32;  // elements of a row one lane holds at most: head sizes up to 1024
@@ -147,6 +157,218 @@ __global__ void attention_paged_kernel(const A* __restrict__ q, const A* __restr
                 slopes != nullptr ? slopes[h] : 0.f, out_scale, sinks != nullptr ? sinks[h] : -INFINITY);
 }
 
+// --------------------------------------------------------------------------- blocks of 32 keys
+constexpr int kKeys = 32, kBlocked = 128;  // keys of a block; widest head that goes so
+
+struct RowsArgs {
+  const void *q, *k, *v;
+  void* out;
+  const int *cu_seqlens, *seq_of_token, *page_table, *slots, *kv_lens, *positions;
+  int queries, q_heads, kv_heads, d, dv, page_size, table_stride, window, temp_every, v_stride;
+  float scale, out_scale, temp_coef;
+  const float *slopes, *sinks;
+  int aligned;  // rows of q, k and v begin on four elements
+};
+
+template <typename A>
+__device__ __forceinline__ float4 load_four(const A* from, int count, bool aligned) {
+  float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (count >= 4 && aligned) {
+    if constexpr (sizeof(A) == 4) {
+      x = *reinterpret_cast<const float4*>(from);
+    } else {
+      const uint2 raw = *reinterpret_cast<const uint2*>(from);
+      x.x = __uint_as_float(raw.x << 16), x.y = __uint_as_float(raw.x & 0xffff0000u);
+      x.z = __uint_as_float(raw.y << 16), x.w = __uint_as_float(raw.y & 0xffff0000u);
+    }
+  } else {
+    if (count > 0) x.x = to_f32(from[0]);
+    if (count > 1) x.y = to_f32(from[1]);
+    if (count > 2) x.z = to_f32(from[2]);
+    if (count > 3) x.w = to_f32(from[3]);
+  }
+  return x;
+}
+
+// WARPS * RW rows of key/value head blockIdx.y, RW a warp, the last ones first (in a prompt they see the most keys); row i is query
+// i / group, head i % group of the group. The next block's keys and values are on their way to registers under a block's work.
+template <typename A, int DP, int RW, int WARPS, bool PAGED>
+__global__ __launch_bounds__(WARPS * 32) void attention_rows_kernel(const RowsArgs a) {
+  constexpr int ROWS = RW * WARPS, THREADS = WARPS * 32, PER = DP / 32, KP = DP + 4;
+  static_assert(ROWS <= 32, "a lane per row");
+  extern __shared__ __align__(16) float rows_smem[];
+  float(*qs)[DP] = reinterpret_cast<float(*)[DP]>(rows_smem);
+  float(*ks)[KP] = reinterpret_cast<float(*)[KP]>(rows_smem + ROWS * DP);
+  float(*vs)[DP] = reinterpret_cast<float(*)[DP]>(rows_smem + ROWS * DP + kKeys * KP);
+  float(*ps)[kKeys] = reinterpret_cast<float(*)[kKeys]>(rows_smem + ROWS * DP + kKeys * KP + kKeys * DP);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kh = blockIdx.y, group = a.q_heads / a.kv_heads;
+  const int row0 = static_cast<int>(gridDim.x - 1 - blockIdx.x) * ROWS, count = min(ROWS, a.queries * group - row0);
+  const bool aligned = a.aligned != 0;
+
+  // Lane r of every warp knows row r: its sequence, position and first key.
+  int seq = -1, pos = -1, first = 0;
+  if (lane < count) {
+    const int t = (row0 + lane) / group;
+    seq = a.seq_of_token != nullptr ? a.seq_of_token[t] : t;
+    pos = PAGED ? (a.positions != nullptr ? a.positions[t] : a.kv_lens[seq] - 1) : t - a.cu_seqlens[seq];
+    first = first_visible_key(pos, a.window);
+  }
+  for (int i = tid; i < ROWS * (DP / 4); i += THREADS) {
+    const int r = i / (DP / 4), c = i % (DP / 4) * 4, idx = row0 + r;
+    const A* from = static_cast<const A*>(a.q) + (static_cast<size_t>(idx / group) * a.q_heads + kh * group + idx % group) * a.d + c;
+    *reinterpret_cast<float4*>(&qs[r][c]) = load_four<A>(from, r < count ? a.d - c : 0, aligned);
+  }
+  float m[RW], l[RW], scale[RW], slope[RW], acc[RW][PER];
+  int my_seq[RW], my_pos[RW], my_first[RW];
+#pragma unroll
+  for (int i = 0; i < RW; ++i) {
+    const int r = warp * RW + i, h = kh * group + (row0 + r) % group;
+    my_seq[i] = __shfl_sync(0xffffffffu, seq, r), my_pos[i] = __shfl_sync(0xffffffffu, pos, r), my_first[i] = __shfl_sync(0xffffffffu, first, r);
+    // a sink is a key met before all others: score `sink`, weight 1 at its own maximum, no value
+    m[i] = a.sinks != nullptr && r < count ? a.sinks[h] : -INFINITY, l[i] = m[i] > -INFINITY ? 1.f : 0.f;
+    scale[i] = a.scale * query_temperature(my_pos[i], a.temp_coef, a.temp_every), slope[i] = a.slopes != nullptr && r < count ? a.slopes[h] : 0.f;
+#pragma unroll
+    for (int e = 0; e < PER; ++e) acc[i][e] = 0.f;
+  }
+
+  for (int begin = 0; begin < count;) {  // the rows of one sequence after another
+    const int b = __shfl_sync(0xffffffffu, seq, begin);
+    const unsigned same = __ballot_sync(0xffffffffu, lane >= begin && lane < count && seq == b);
+    const int end = begin + __popc(same);  // (a step's tokens lie sequence after sequence)
+    const bool in = lane >= begin && lane < end;
+    int low = in ? first : INT_MAX, high = in ? pos : -1;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) low = min(low, __shfl_xor_sync(0xffffffffu, low, o)), high = max(high, __shfl_xor_sync(0xffffffffu, high, o));
+    const size_t base = PAGED ? 0 : static_cast<size_t>(a.cu_seqlens[b]);
+    const int* table = PAGED ? a.page_table + static_cast<size_t>(a.slots[b]) * a.table_stride : nullptr;
+    constexpr int PIECES = kKeys * (DP / 4) / THREADS;
+    float4 next_k[PIECES], next_v[PIECES];
+    auto fetch = [&](int block) {
+#pragma unroll
+      for (int n = 0; n < PIECES; ++n) {
+        const int i = tid + n * THREADS, c = i % (DP / 4) * 4, p = block + i / (DP / 4);
+        const bool there = p >= low && p <= high;
+        size_t line = 0;
+        if (there && PAGED) line = (static_cast<size_t>(table[p / a.page_size]) * a.kv_heads + kh) * a.page_size + p % a.page_size;
+        else if (there) line = (base + p) * a.kv_heads + kh;
+        next_k[n] = load_four<A>(static_cast<const A*>(a.k) + line * a.d + c, there ? a.d - c : 0, aligned);
+        next_v[n] = load_four<A>(static_cast<const A*>(a.v) + line * a.v_stride + c, there ? a.dv - c : 0, aligned);
+      }
+    };
+    int block = low / kKeys * kKeys;
+    fetch(block);
+    for (; block <= high; block += kKeys) {
+      __syncthreads();  // everyone is done with the block before (and the queries are here)
+#pragma unroll
+      for (int n = 0; n < PIECES; ++n) {
+        const int i = tid + n * THREADS, r = i / (DP / 4), c = i % (DP / 4) * 4;
+        *reinterpret_cast<float4*>(&ks[r][c]) = next_k[n], *reinterpret_cast<float4*>(&vs[r][c]) = next_v[n];
+      }
+      __syncthreads();
+      if (block + kKeys <= high) fetch(block + kKeys);
+      bool active[RW], any = false, whole = true;  // rows that see a key of the block; whether all see all of them
+#pragma unroll
+      for (int i = 0; i < RW; ++i) {
+        active[i] = my_seq[i] == b && warp * RW + i < count && my_pos[i] >= block && my_first[i] < block + kKeys;
+        any = any || active[i];
+        whole = whole && (!active[i] || (my_first[i] <= block && my_pos[i] >= block + kKeys - 1));
+      }
+      if (!any) continue;
+      float2 dot[RW][2];
+#pragma unroll
+      for (int i = 0; i < RW; ++i) dot[i][0] = dot[i][1] = make_float2(0.f, 0.f);
+#pragma unroll 4
+      for (int c = 0; c < a.d; c += 4) {
+        const float4 key = *reinterpret_cast<const float4*>(&ks[lane][c]);
+#pragma unroll
+        for (int i = 0; i < RW; ++i) {
+          const float4 query = *reinterpret_cast<const float4*>(&qs[warp * RW + i][c]);
+          dot[i][0].x = fmaf(query.x, key.x, dot[i][0].x), dot[i][0].y = fmaf(query.y, key.y, dot[i][0].y);
+          dot[i][1].x = fmaf(query.z, key.z, dot[i][1].x), dot[i][1].y = fmaf(query.w, key.w, dot[i][1].y);
+        }
+      }
+      const int p = block + lane;
+#pragma unroll
+      for (int i = 0; i < RW; ++i) {
+        if (!active[i]) continue;
+        float score = ((dot[i][0].x + dot[i][0].y) + (dot[i][1].x + dot[i][1].y)) * scale[i];
+        if (slope[i] != 0.f) score -= slope[i] * static_cast<float>(my_pos[i] - p);
+        const bool seen = p >= my_first[i] && p <= my_pos[i];
+        const float nm = fmaxf(m[i], warp_max(seen ? score : -INFINITY)), old = expf(m[i] - nm), prob = seen ? expf(score - nm) : 0.f;
+        l[i] = fmaf(l[i], old, warp_sum(prob)), m[i] = nm;
+        ps[warp * RW + i][lane] = prob;
+#pragma unroll
+        for (int e = 0; e < PER; ++e) acc[i][e] *= old;
+      }
+      __syncwarp();
+#pragma unroll 2
+      for (int j = 0; j < kKeys; j += 4) {
+        float prob[RW][4];
+#pragma unroll
+        for (int i = 0; i < RW; ++i) {
+          const float4 x = *reinterpret_cast<const float4*>(&ps[warp * RW + i][j]);
+          prob[i][0] = x.x, prob[i][1] = x.y, prob[i][2] = x.z, prob[i][3] = x.w;
+        }
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+          float value[PER];
+#pragma unroll
+          for (int e = 0; e < PER; ++e) value[e] = vs[j + n][lane + 32 * e];
+#pragma unroll
+          for (int i = 0; i < RW; ++i) {  // (what a row does not see adds nothing, not even a NaN)
+            if (active[i] && (whole || (block + j + n >= my_first[i] && block + j + n <= my_pos[i]))) {
+#pragma unroll
+              for (int e = 0; e < PER; ++e) acc[i][e] = fmaf(prob[i][n], value[e], acc[i][e]);
+            }
+          }
+        }
+      }
+      __syncwarp();
+    }
+    begin = end;
+  }
+#pragma unroll
+  for (int i = 0; i < RW; ++i) {
+    const int r = warp * RW + i, idx = row0 + r;
+    if (r >= count) continue;
+    A* to = static_cast<A*>(a.out) + (static_cast<size_t>(idx / group) * a.q_heads + kh * group + idx % group) * a.dv;
+#pragma unroll
+    for (int e = 0; e < PER; ++e) {
+      const int j = lane + 32 * e;
+      if (j < a.dv) to[j] = from_f32<A>(a.out_scale == 1.0f ? acc[i][e] / l[i] : (acc[i][e] / l[i]) * a.out_scale);
+    }
+  }
+}
+
+template <typename A, int DP, int RW, int WARPS, bool PAGED>
+int launch_rows(const RowsArgs& a, cudaStream_t stream) {
+  constexpr int ROWS = RW * WARPS;
+  constexpr size_t bytes = sizeof(float) * (ROWS * DP + kKeys * (DP + 4) + kKeys * DP + ROWS * kKeys);
+  if (bytes > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(attention_rows_kernel<A, DP, RW, WARPS, PAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+    if (e != cudaSuccess) return static_cast<int>(e);
+  }
+  const long long rows = static_cast<long long>(a.queries) * (a.q_heads / a.kv_heads);
+  attention_rows_kernel<A, DP, RW, WARPS, PAGED><<<dim3(static_cast<unsigned>((rows + ROWS - 1) / ROWS), a.kv_heads), WARPS * 32, bytes, stream>>>(a);
+  LRM_LAUNCH_CHECK();
+  return 0;
+}
+
+// 16 rows a CTA for prompts, which share their keys; 4 where a query is its sequence's only one, or few may be.
+template <typename A, bool PAGED>
+int dispatch_rows(const RowsArgs& a, cudaStream_t stream) {
+  const bool many = PAGED ? a.positions != nullptr && a.queries >= 128 : true;
+  if (a.d <= 64 && a.dv <= 64)
+    return many ? launch_rows<A, 64, 2, 8, PAGED>(a, stream) : launch_rows<A, 64, 1, 4, PAGED>(a, stream);
+  return many ? launch_rows<A, 128, 2, 8, PAGED>(a, stream) : launch_rows<A, 128, 1, 4, PAGED>(a, stream);
+}
+
+static int rows_alignment(const RowsArgs& a, int dtype) {
+  const uintptr_t bytes = dtype == LRM_F32 ? 16 : 8;
+  return a.d % 4 == 0 && a.v_stride % 4 == 0 && a.dv % 4 == 0 && reinterpret_cast<uintptr_t>(a.q) % bytes == 0 &&
+         reinterpret_cast<uintptr_t>(a.k) % bytes == 0 && reinterpret_cast<uintptr_t>(a.v) % bytes == 0;
+}
+
 static bool bad_geometry(int q_heads, int kv_heads, int d, int dv) {
   return q_heads <= 0 || kv_heads <= 0 || q_heads % kv_heads != 0 || d <= 0 ||
          d > 32 * kWidest || dv <= 0 || dv > 32 * kWidest;
@@ -164,6 +386,14 @@ LRM_API int lrm_attention_packed_rowwise(const void* q, const void* k, const voi
   if (q_heads > 65535) return LRM_UNSUPPORTED;
   const dim3 grid(tokens, q_heads);
   const int widest = d > dv ? d : dv;
+  if (widest <= kBlocked) {
+    RowsArgs a{q, k, v, out, cu_seqlens, seq_of_token, nullptr, nullptr, nullptr, nullptr, tokens, q_heads, kv_heads, d, dv, 1, 0, window,
+               temp_every, v_stride, scale, out_scale, temp_coef, slopes, sinks, 0};
+    a.aligned = rows_alignment(a, dtype);
+    return dtype == LRM_F32    ? dispatch_rows<float, false>(a, stream)
+           : dtype == LRM_BF16 ? dispatch_rows<__nv_bfloat16, false>(a, stream)
+                               : LRM_BAD_ARGUMENT;
+  }
 #define LRM_PACKED(AT, PER)                                                                                      \
   attention_packed_kernel<AT, PER><<<grid, 32, 0, stream>>>(                                                     \
       static_cast<const AT*>(q), static_cast<const AT*>(k), static_cast<const AT*>(v), static_cast<AT*>(out),    \
@@ -171,8 +401,7 @@ LRM_API int lrm_attention_packed_rowwise(const void* q, const void* k, const voi
       temp_every, v_stride)
 #define LRM_PACKED_BY_WIDTH(AT)                  \
   do {                                           \
-    if (widest <= 128) LRM_PACKED(AT, 4);        \
-    else if (widest <= 512) LRM_PACKED(AT, 16);  \
+    if (widest <= 512) LRM_PACKED(AT, 16);  \
     else LRM_PACKED(AT, 32);                     \
   } while (0)
   if (dtype == LRM_F32)
@@ -206,6 +435,14 @@ LRM_API int lrm_attention_paged_rowwise(const void* q, const void* k_pages, cons
   if (q_heads > 65535) return LRM_UNSUPPORTED;
   const dim3 grid(queries, q_heads);
   const int widest = d > dv ? d : dv;
+  if (widest <= kBlocked) {
+    RowsArgs a{q, k_pages, v_pages, out, nullptr, seq_of_token, page_table, slots, kv_lens, positions, queries, q_heads, kv_heads, d, dv,
+               page_size, table_stride, window, temp_every, v_stride, scale, out_scale, temp_coef, slopes, sinks, 0};
+    a.aligned = rows_alignment(a, dtype);
+    return dtype == LRM_F32    ? dispatch_rows<float, true>(a, stream)
+           : dtype == LRM_BF16 ? dispatch_rows<__nv_bfloat16, true>(a, stream)
+                               : LRM_BAD_ARGUMENT;
+  }
 #define LRM_PAGED(AT, PER)                                                                                       \
   attention_paged_kernel<AT, PER><<<grid, 32, 0, stream>>>(                                                      \
       static_cast<const AT*>(q), static_cast<const AT*>(k_pages), static_cast<const AT*>(v_pages),               \
@@ -213,8 +450,7 @@ LRM_API int lrm_attention_paged_rowwise(const void* q, const void* k_pages, cons
       kv_heads, d, dv, page_size, scale, window, slopes, out_scale, sinks, temp_coef, temp_every, v_stride)
 #define LRM_PAGED_BY_WIDTH(AT)                  \
   do {                                          \
-    if (widest <= 128) LRM_PAGED(AT, 4);        \
-    else if (widest <= 512) LRM_PAGED(AT, 16);  \
+    if (widest <= 512) LRM_PAGED(AT, 16);  \
     else LRM_PAGED(AT, 32);                     \
   } while (0)
   if (dtype == LRM_F32)
