@@ -82,6 +82,7 @@ __global__ __launch_bounds__(kUmmaThreads, 1) void gemm_bf16_umma_kernel(
   uint64_t* acc_free = acc_full + 2;     // [2] accumulators read back by all four epilogue warps
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 2);
   volatile int* bail = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  unsigned char* const stages = tiles + STAGES * STAGE_BYTES + 256;  // [8 epilogue warps][kStageBytes]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m_tiles = (M + MT * BM - 1) / (MT * BM), n_tiles = (N + BN - 1) / BN;
@@ -187,6 +188,7 @@ __global__ __launch_bounds__(kUmmaThreads, 1) void gemm_bf16_umma_kernel(
     // ---- epilogue: eight warps, one accumulator row per thread and half of its columns; a warp
     // may touch only the quarter of the tensor memory's lanes given by its index modulo 4
     const int quarter = warp & 3, side = (warp - 2) >> 2;
+    unsigned char* const stage = stages + (warp - 2) * kStageBytes;
     uint32_t local = 0;
     for (int item = blockIdx.x; item < items; item += gridDim.x) {
       if (EXPERTS && experts.tile_experts[item % m_tiles] < 0) continue;
@@ -208,16 +210,15 @@ __global__ __launch_bounds__(kUmmaThreads, 1) void gemm_bf16_umma_kernel(
         const int heads = BN / qkv.head_dim, cut = ((heads + 1) >> 1) * qkv.head_dim;
 #pragma unroll 1
         for (int i = 0; i < MT; ++i)
-          store_heads<BN>(tmem_base + acc * SET + i * BN + (static_cast<uint32_t>(quarter * 32) << 16),
-                          m0 + i * BM + quarter * 32 + lane, n0, M, N, qkv, side == 0 ? 0 : cut, side == 0 ? cut : BN);
+          store_heads<BN>(tmem_base + acc * SET + i * BN + (static_cast<uint32_t>(quarter * 32) << 16), stage,
+                          m0 + i * BM + quarter * 32, lane, n0, M, N, qkv, side == 0 ? 0 : cut, side == 0 ? cut : BN);
       } else if (num_kb > 0) {
         constexpr int kPieces = MT * BN / 32;
 #pragma unroll 1
         for (int c = side * (kPieces / 2); c < (side + 1) * (kPieces / 2); ++c) {  // accumulator c / (BN / 32) holds rows 128 (c / (BN / 32)) ...
-          const int m = m0 + (c / (BN / 32)) * BM + quarter * 32 + lane;
           uint32_t r[32];
           tmem_load32(tmem_base + acc * SET + (static_cast<uint32_t>(quarter * 32) << 16) + c * 32, r);
-          store_piece(r, plane, m, n0 + (c % (BN / 32)) * 32, M, N, mode, parts);
+          store_piece(r, stage, plane, m0 + (c / (BN / 32)) * BM + quarter * 32, lane, n0 + (c % (BN / 32)) * 32, M, N, mode, parts);
         }
       }
       tc_fence_before();
@@ -241,7 +242,7 @@ int launch_umma(const void* X, const void* W, void* out, int M, int x_rows, int 
   if (!make_map_bf16(&map_x, X, x_rows, K, BM) ||
       !make_map_bf16(&map_w, W, EXPERTS ? w_height : N, EXPERTS ? w_width : K, BN))
     return LRM_UNSUPPORTED;
-  constexpr int smem = STAGES * (MT * BM * BK * 2 + BN * BK * 2) + 1024 + 256;
+  constexpr int smem = STAGES * (MT * BM * BK * 2 + BN * BK * 2) + 1024 + 256 + 8 * kStageBytes;
   auto kernel = gemm_bf16_umma_kernel<BN, STAGES, MT, EXPERTS>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return static_cast<int>(e);

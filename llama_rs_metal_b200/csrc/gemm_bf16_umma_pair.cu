@@ -110,6 +110,7 @@ __global__ __launch_bounds__(kPairThreads, 1) void gemm_bf16_umma_pair_kernel(
   uint64_t* acc_free = acc_full + 2;     // [2] the leader's: read back by the epilogue warps of both CTAs
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 2);
   volatile int* bail = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  unsigned char* const stages = tiles + STAGES * STAGE_BYTES + 256;  // [8 epilogue warps][kStageBytes]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
@@ -204,6 +205,7 @@ __global__ __launch_bounds__(kPairThreads, 1) void gemm_bf16_umma_pair_kernel(
     // ---- epilogue: eight warps, one accumulator row and half of its columns per thread, this
     // CTA's 128 rows of the tile
     const int quarter = warp & 3, side = (warp - 2) >> 2;
+    unsigned char* const stage = stages + (warp - 2) * kStageBytes;
     uint32_t local = 0;
     for (int item = pair; item < items; item += pairs, ++local) {
       const int m0 = (item % m_tiles) * 2 * PM + static_cast<int>(rank) * PM, n0 = (item / m_tiles) * BN;
@@ -215,14 +217,14 @@ __global__ __launch_bounds__(kPairThreads, 1) void gemm_bf16_umma_pair_kernel(
       tc_fence_after();
       if (mode == 5) {
         const int heads = BN / qkv.head_dim, cut = ((heads + 1) >> 1) * qkv.head_dim;
-        store_heads<BN>(tmem_base + acc * SET + (static_cast<uint32_t>(quarter * 32) << 16),
-                        m0 + quarter * 32 + lane, n0, M, N, qkv, side == 0 ? 0 : cut, side == 0 ? cut : BN);
+        store_heads<BN>(tmem_base + acc * SET + (static_cast<uint32_t>(quarter * 32) << 16), stage,
+                        m0 + quarter * 32, lane, n0, M, N, qkv, side == 0 ? 0 : cut, side == 0 ? cut : BN);
       } else {
 #pragma unroll 1
         for (int c = side * (BN / 64); c < (side + 1) * (BN / 64); ++c) {
           uint32_t r[32];
           tmem_load32(tmem_base + acc * SET + (static_cast<uint32_t>(quarter * 32) << 16) + c * 32, r);
-          store_piece(r, out, m0 + quarter * 32 + lane, n0 + c * 32, M, N, mode, parts);
+          store_piece(r, stage, out, m0 + quarter * 32, lane, n0 + c * 32, M, N, mode, parts);
         }
       }
       tc_fence_before();
@@ -237,7 +239,7 @@ __global__ __launch_bounds__(kPairThreads, 1) void gemm_bf16_umma_pair_kernel(
 }
 
 template <int BN, int STAGES> constexpr int pair_smem() {
-  return STAGES * (PM * PK * 2 + (BN / 2) * PK * 2) + 1024 + 256;
+  return STAGES * (PM * PK * 2 + (BN / 2) * PK * 2) + 1024 + 256 + 8 * kStageBytes;
 }
 
 template <int BN, int STAGES>

@@ -5,11 +5,39 @@
 //   6 columns below a split as 1, the columns from it on as 3, each into a tensor of its own (SplitArgs),
 // and epilogue 5, which works on whole heads of a fused q|k|v projection (store_heads).
 #pragma once
+#include <type_traits>
+
 #include "umma.cuh"
 
 namespace {
 
-__device__ __forceinline__ float silu_f32(float g) { return g / (1.0f + expf(-g)); }
+// g / (1 + exp(-g)) of COUNT values. A division of its own for each, with its test for the rare operands, leaves a warp with
+// one chain of some 80 cycles after the other (5.6 us for a 128 x 256 tile, staged 5.7); here the quotients of a thread go side by side:
+// Newton's step for the reciprocal of a denominator between 1 and 2^116, then Markstein's correction of the quotient by its
+// remainder (IBM J. Res. Dev. 34, 1990), which rounds as the division does. Beyond 80 the denominator is 1, and below -80 one
+// plus it is it.
+template <int COUNT>
+__device__ __forceinline__ void silu_all(float (&g)[COUNT]) {
+  float v[COUNT];
+  bool plain = true;
+#pragma unroll
+  for (int i = 0; i < COUNT; ++i) plain &= fabsf(g[i]) <= 80.f;  // not for NaN
+#pragma unroll
+  for (int i = 0; i < COUNT; ++i) {
+    const float d = 1.0f + expf(-g[i]);
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    r = fmaf(r, fmaf(-d, r, 1.0f), r);
+    const float q = g[i] * r;
+    v[i] = fmaf(fmaf(-d, q, g[i]), r, q);
+  }
+  if (!__all_sync(0xffffffffu, plain)) {
+#pragma unroll
+    for (int i = 0; i < COUNT; ++i) v[i] = g[i] > 80.f ? g[i] : g[i] < -80.f ? g[i] * expf(g[i]) : v[i];
+  }
+#pragma unroll
+  for (int i = 0; i < COUNT; ++i) g[i] = v[i];
+}
 
 // What epilogue 6 needs: two products with the same input in one launch. Columns [0, split) are stored in
 // float32 to `out` [M, split]; columns from `split` (a multiple of 32) on are gate and up rows, and the
@@ -20,10 +48,44 @@ struct SplitArgs {
   int split;
 };
 
-// The epilogue of one 32-column piece of an accumulator row held in registers.
-__device__ __forceinline__ void store_piece(const uint32_t (&r)[32], void* __restrict__ out, int m, int n,
-                                            int M, int N, int mode, const SplitArgs& parts) {
-  if (m >= M || n >= N) return;
+// A warp's 32 accumulator rows on their way to memory. A thread that stores its own row touches 32 rows with every
+// instruction, 16 bytes of each; through this piece of shared memory (2 KB per warp) the same bytes leave as runs of 64 bytes
+// (32 for gated values): BYTES of every row, 16-byte pieces swapped about so that neither way meets a bank twice.
+// us of a 128 x 256 tile's epilogue (1,536 x 9,472, K = 64: what a further round of tiles adds), in brackets each thread on its
+// own row: bfloat16 2.4 (6.0), float32 4.1 (9.3), added 4.3 (8.7), gated 3.3 (5.6). It is not hidden behind the last tile, and
+// only partly behind others: with K = 2048 the whole product is 42.3 (51.7), gated 45.7 (52.5).
+constexpr int kStageBytes = 32 * 64;
+
+template <int BYTES>
+__device__ __forceinline__ void stage_row(unsigned char* stage, int lane, const uint32_t* v) {
+  static_assert(BYTES == 32 || BYTES == 64, "");
+#pragma unroll
+  for (int c = 0; c < BYTES / 16; ++c) {
+    const int at = BYTES == 64 ? c ^ ((lane >> 1) & 3) : c ^ ((lane >> 2) & 1);
+    *reinterpret_cast<uint4*>(stage + lane * BYTES + at * 16) = make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+  }
+}
+
+// f(row, byte of the row, 16 bytes) for all that the warp's lanes staged.
+template <int BYTES, class F>
+__device__ __forceinline__ void unstage(const unsigned char* stage, int lane, F f) {
+  constexpr int PER = BYTES / 16, ROWS = 32 / PER;  // pieces of a row, rows per step
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 32 / ROWS; ++i) {
+    const int row = i * ROWS + lane / PER, c = lane % PER;
+    const int at = BYTES == 64 ? c ^ ((row >> 1) & 3) : c ^ ((row >> 2) & 1);
+    f(row, c * 16, *reinterpret_cast<const uint4*>(stage + row * BYTES + at * 16));
+  }
+  __syncwarp();
+}
+
+// The epilogue of a 32-column piece of a warp's 32 accumulator rows (rows m0 .. of the product), a row per lane in registers.
+// Every lane of the warp calls it.
+__device__ __forceinline__ void store_piece(const uint32_t (&r)[32], unsigned char* stage, void* __restrict__ out, int m0,
+                                            int lane, int n, int M, int N, int mode, const SplitArgs& parts) {
+  if (n >= N) return;
+  const int m = m0 + lane;
   size_t pitch = N >> 1;  // of the gated values
   if (mode == 6) {
     if (n < parts.split) {
@@ -40,52 +102,71 @@ __device__ __forceinline__ void store_piece(const uint32_t (&r)[32], void* __res
   const bool whole = n + 32 <= N;
   if (mode == 3) {
     // [8 gate | 8 up | 8 gate | 8 up] -> 16 gated values
-    __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(out) + static_cast<size_t>(m) * pitch + (n >> 1);
+    __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(out) + (n >> 1);
+    float gate[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) gate[i] = __uint_as_float(r[(i >> 3) * 16 + (i & 7)]);
+    silu_all(gate);
     uint32_t packed[8];
 #pragma unroll
     for (int i = 0; i < 16; i += 2) {
-      const int a = (i >> 3) * 16 + (i & 7);
-      const float v0 = silu_f32(__uint_as_float(r[a])) * __uint_as_float(r[a + 8]);
-      const float v1 = silu_f32(__uint_as_float(r[a + 1])) * __uint_as_float(r[a + 9]);
-      packed[i >> 1] = pack_bf16(v0, v1);
+      const int up = (i >> 3) * 16 + (i & 7) + 8;
+      packed[i >> 1] = pack_bf16(gate[i] * __uint_as_float(r[up]), gate[i + 1] * __uint_as_float(r[up + 1]));
     }
     if (whole) {
-      *reinterpret_cast<uint4*>(dst) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-      *reinterpret_cast<uint4*>(dst + 8) = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-    } else {
-      const __nv_bfloat16* vals = reinterpret_cast<const __nv_bfloat16*>(packed);
-      for (int i = 0; i < 16 && n + (i >> 3) * 16 + 8 + (i & 7) < N; ++i) dst[i] = vals[i];
+      stage_row<32>(stage, lane, packed);
+      unstage<32>(stage, lane, [&](int row, int byte, const uint4& v) {
+        if (m0 + row < M) *reinterpret_cast<uint4*>(dst + static_cast<size_t>(m0 + row) * pitch + byte / 2) = v;
+      });
+    } else if (m < M) {
+      __nv_bfloat16* mine = dst + static_cast<size_t>(m) * pitch;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const uint32_t two = packed[i >> 1];
+        const uint16_t bits = static_cast<uint16_t>((i & 1) ? two >> 16 : two);
+        if (n + (i >> 3) * 16 + 8 + (i & 7) < N) mine[i] = __ushort_as_bfloat16(bits);
+      }
     }
   } else if (mode == 0) {
-    __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(out) + static_cast<size_t>(m) * N + n;
+    __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(out) + n;
     if (whole && (N & 7) == 0) {
+      uint32_t packed[16];
 #pragma unroll
-      for (int i = 0; i < 32; i += 8)
-        *reinterpret_cast<uint4*>(dst + i) = make_uint4(
-            pack_bf16(__uint_as_float(r[i]), __uint_as_float(r[i + 1])),
-            pack_bf16(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])),
-            pack_bf16(__uint_as_float(r[i + 4]), __uint_as_float(r[i + 5])),
-            pack_bf16(__uint_as_float(r[i + 6]), __uint_as_float(r[i + 7])));
-    } else {
-      for (int i = 0; i < 32 && n + i < N; ++i) dst[i] = __float2bfloat16_rn(__uint_as_float(r[i]));
+      for (int i = 0; i < 16; ++i) packed[i] = pack_bf16(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+      stage_row<64>(stage, lane, packed);
+      unstage<64>(stage, lane, [&](int row, int byte, const uint4& v) {
+        if (m0 + row < M) *reinterpret_cast<uint4*>(dst + static_cast<size_t>(m0 + row) * N + byte / 2) = v;
+      });
+    } else if (m < M) {
+      __nv_bfloat16* mine = dst + static_cast<size_t>(m) * N;
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (n + i < N) mine[i] = __float2bfloat16_rn(__uint_as_float(r[i]));
     }
   } else {
-    float* dst = static_cast<float*>(out) + static_cast<size_t>(m) * N + n;
+    float* dst = static_cast<float*>(out) + n;
     if (whole && (N & 3) == 0) {
 #pragma unroll
-      for (int i = 0; i < 32; i += 4) {
-        float4 v = make_float4(__uint_as_float(r[i]), __uint_as_float(r[i + 1]), __uint_as_float(r[i + 2]),
-                               __uint_as_float(r[i + 3]));
-        // Adding goes through a vector reduction in L2 (no value comes back, so the thread does
-        // not wait for the old contents). Each element gets exactly one add per launch, so the
-        // result is as deterministic as a read-modify-write.
-        if (mode == 2) atomicAdd(reinterpret_cast<float4*>(dst + i), v);
-        else *reinterpret_cast<float4*>(dst + i) = v;
+      for (int half = 0; half < 2; ++half) {
+        stage_row<64>(stage, lane, r + 16 * half);
+        unstage<64>(stage, lane, [&](int row, int byte, const uint4& raw) {
+          if (m0 + row >= M) return;
+          float4* to = reinterpret_cast<float4*>(dst + static_cast<size_t>(m0 + row) * N + 16 * half + byte / 4);
+          const float4 v = make_float4(__uint_as_float(raw.x), __uint_as_float(raw.y), __uint_as_float(raw.z), __uint_as_float(raw.w));
+          // Adding goes through a vector reduction in L2 (no value comes back, so the thread does
+          // not wait for the old contents). Each element gets exactly one add per launch, so the
+          // result is as deterministic as a read-modify-write.
+          if (mode == 2) atomicAdd(to, v);
+          else *to = v;
+        });
       }
-    } else {
-      for (int i = 0; i < 32 && n + i < N; ++i) {
-        if (mode == 2) atomicAdd(dst + i, __uint_as_float(r[i]));
-        else dst[i] = __uint_as_float(r[i]);
+    } else if (m < M) {
+      float* mine = dst + static_cast<size_t>(m) * N;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        if (n + i >= N) continue;
+        if (mode == 2) atomicAdd(mine + i, __uint_as_float(r[i]));
+        else mine[i] = __uint_as_float(r[i]);
       }
     }
   }
@@ -108,59 +189,76 @@ struct QkvArgs {
   int q_heads, kv_heads, head_dim, page_size;
 };
 
-__device__ __forceinline__ void store_32_bf16(__nv_bfloat16* dst, const uint32_t (&packed)[16]) {
-#pragma unroll
-  for (int i = 0; i < 16; i += 4)
-    *reinterpret_cast<uint4*>(dst + 2 * i) = make_uint4(packed[i], packed[i + 1], packed[i + 2], packed[i + 3]);
-}
-
-// One accumulator row (token m) of a tile whose first column n0 is the first of a head and whose
-// width BN is a whole number of heads: `tmem_row` addresses the row's first column in tensor
-// memory. Every lane of the warp must call it (the loads are warp-wide); rows beyond M only load.
+// One warp's 32 accumulator rows (tokens m0 ..) of a tile whose first column n0 is the first of a head and whose
+// width BN is a whole number of heads: `tmem_row` addresses the rows' first column in tensor
+// memory. Every lane of the warp must call it; rows beyond M only load.
 // Of the tile's heads this call takes those that begin in columns [first, last).
 template <int BN>
-__device__ __forceinline__ void store_heads(uint32_t tmem_row, int m, int n0, int M, int N, const QkvArgs& a,
-                                            int first = 0, int last = BN) {
+__device__ __forceinline__ void store_heads(uint32_t tmem_row, unsigned char* stage, int m0, int lane, int n0, int M, int N,
+                                            const QkvArgs& a, int first = 0, int last = BN) {
   const int d = a.head_dim, half = d >> 1;
-  const bool live = m < M;
-  const int dest = live && a.k_pages != nullptr ? a.dest_rows[m] : -1;
-  const size_t page = dest >= 0 ? static_cast<size_t>(dest / a.page_size) : 0;
-  const int in_page = dest >= 0 ? dest % a.page_size : 0;
+  // where this lane's row goes in the cache (head 0); the lanes that store it ask for it
+  uint32_t place = 0xffffffffu;  // in rows of d
+  if (m0 + lane < M && a.k_pages != nullptr) {
+    const int dest = a.dest_rows[m0 + lane];
+    if (dest >= 0) place = static_cast<uint32_t>(dest / a.page_size) * a.kv_heads * a.page_size + dest % a.page_size;
+  }
   for (int c0 = first; c0 < last && n0 + c0 < N; c0 += d) {
     const int head = (n0 + c0) / d;
     const bool is_q = head < a.q_heads, is_v = head >= a.q_heads + a.kv_heads;
     const int kh = is_q ? 0 : head - a.q_heads - (is_v ? a.kv_heads : 0);
-    __nv_bfloat16* packed_dst = is_q ? a.q + (static_cast<size_t>(m) * a.q_heads + head) * d
-                                     : (is_v ? a.v : a.k) + (static_cast<size_t>(m) * a.kv_heads + kh) * d;
-    __nv_bfloat16* cache_dst = (is_q || dest < 0) ? nullptr
-        : (is_v ? a.v_pages : a.k_pages) + ((page * a.kv_heads + kh) * a.page_size + in_page) * d;
+    __nv_bfloat16* packed_dst = is_q ? a.q + static_cast<size_t>(head) * d : (is_v ? a.v : a.k) + static_cast<size_t>(kh) * d;
+    const size_t pitch = static_cast<size_t>(is_q ? a.q_heads : a.kv_heads) * d;
+    __nv_bfloat16* cache_dst = is_q || a.k_pages == nullptr ? nullptr
+        : (is_v ? a.v_pages : a.k_pages) + static_cast<size_t>(kh) * a.page_size * d;
+    const auto put = [&](auto bytes, int c, const uint32_t* packed) {  // columns c .. of the head
+      stage_row<decltype(bytes)::value>(stage, lane, packed);
+      unstage<decltype(bytes)::value>(stage, lane, [&](int row, int byte, const uint4& v) {
+        const uint32_t at = __shfl_sync(0xffffffffu, place, row);
+        if (m0 + row >= M) return;
+        *reinterpret_cast<uint4*>(packed_dst + (m0 + row) * pitch + c + byte / 2) = v;
+        if (cache_dst != nullptr && at != 0xffffffffu)
+          *reinterpret_cast<uint4*>(cache_dst + static_cast<size_t>(at) * d + c + byte / 2) = v;
+      });
+    };
     if (is_v || a.table == nullptr) {
       for (int c = 0; c < d; c += 32) {
         uint32_t r[32];
         tmem_load32(tmem_row + c0 + c, r);
-        if (live) {
-          uint32_t packed[16];
+        uint32_t packed[16];
 #pragma unroll
-          for (int i = 0; i < 16; ++i) packed[i] = pack_bf16(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-          store_32_bf16(packed_dst + c, packed);
-          if (cache_dst != nullptr) store_32_bf16(cache_dst + c, packed);
-        }
+        for (int i = 0; i < 16; ++i) packed[i] = pack_bf16(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+        put(std::integral_constant<int, 64>(), c, packed);
       }
       continue;
     }
-    for (int c = 0; c < half; c += 32) {  // columns c.. pair with columns half + c..
-      uint32_t lo[32], hi[32];
-      tmem_load32_async(tmem_row + c0 + c, lo);
-      tmem_load32_async(tmem_row + c0 + half + c, hi);
-      tmem_load_wait();
-      tmem_pin(lo);
-      tmem_pin(hi);
-      if (live) {
-        const float4* cs = reinterpret_cast<const float4*>(a.table + static_cast<size_t>(m) * half + c);
-        uint32_t out_lo[16], out_hi[16];
+    for (int c = 0; c < half; c += 16) {  // columns c.. pair with columns half + c..
+      // The angles come as runs of 64 bytes of a row too and reach the rows' lanes through the staging area: every lane loading
+      // its own row's cost as much as the stores.
+      uint4 angles[2][4];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {  // two pairs at a time: (cos, sin) of columns c + 2i and c + 2i + 1
-          const float4 t = __ldg(cs + i);
+      for (int part = 0; part < 2; ++part)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int row = min(m0 + i * 8 + (lane >> 2), M - 1);
+          angles[part][i] = __ldg(reinterpret_cast<const uint4*>(a.table + static_cast<size_t>(row) * half + c + part * 8) +
+                                  (lane & 3));
+        }
+      uint32_t lo[16], hi[16], out_lo[8], out_hi[8];
+      tmem_load16(tmem_row + c0 + c, lo);
+      tmem_load16(tmem_row + c0 + half + c, hi);
+#pragma unroll
+      for (int part = 0; part < 2; ++part) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int row = i * 8 + (lane >> 2), at = (lane & 3) ^ ((row >> 1) & 3);
+          *reinterpret_cast<uint4*>(stage + row * 64 + at * 16) = angles[part][i];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {  // (cos, sin) of two columns
+          const int i = part * 4 + u;
+          const float4 t = *reinterpret_cast<const float4*>(stage + lane * 64 + (u ^ ((lane >> 1) & 3)) * 16);
           // the projection is rounded to bfloat16 first, as where it is stored before it is rotated
           const float xa0 = __bfloat162float(__float2bfloat16_rn(__uint_as_float(lo[2 * i])));
           const float xa1 = __bfloat162float(__float2bfloat16_rn(__uint_as_float(lo[2 * i + 1])));
@@ -169,13 +267,10 @@ __device__ __forceinline__ void store_heads(uint32_t tmem_row, int m, int n0, in
           out_lo[i] = pack_bf16(fmaf(xa0, t.x, -__fmul_rn(xb0, t.y)), fmaf(xa1, t.z, -__fmul_rn(xb1, t.w)));
           out_hi[i] = pack_bf16(fmaf(xa0, t.y, __fmul_rn(xb0, t.x)), fmaf(xa1, t.w, __fmul_rn(xb1, t.z)));
         }
-        store_32_bf16(packed_dst + c, out_lo);
-        store_32_bf16(packed_dst + half + c, out_hi);
-        if (cache_dst != nullptr) {
-          store_32_bf16(cache_dst + c, out_lo);
-          store_32_bf16(cache_dst + half + c, out_hi);
-        }
+        __syncwarp();
       }
+      put(std::integral_constant<int, 32>(), c, out_lo);
+      put(std::integral_constant<int, 32>(), half + c, out_hi);
     }
   }
 }
