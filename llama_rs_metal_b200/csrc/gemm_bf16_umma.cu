@@ -148,7 +148,58 @@ __global__ __launch_bounds__(kUmmaThreads, 1) void gemm_bf16_umma_kernel(
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if constexpr (STAGES >= 5) {
+      // ---- issuer: the warp stays together around the lane that drives the tensor core, on numbers the same in all lanes, so that
+      // descriptors are made in uniform registers, and goes through all blocks that are there with one question. What a lane of
+      // its own spends on a block (a wait, 200 cycles, and four products of 52) is more than the 256 cycles of a 128 x 128 tile's
+      // products: 2048 x 8192 of 900 rows 38 us (44), 3072 x 2048 of 3,300 44 (54). A 128 x 192 tile gains 5 %. A 128 x 256 one
+      // loses 7 %: its ring of four stages does not cover the few steps more between a block's arrival and its products, which
+      // take 512 cycles anyway, so it keeps the lane of its own.
+      constexpr uint32_t idesc = umma_idesc(BM, BN);  // both operands K-major
+      const uint32_t ring = __shfl_sync(0xffffffffu, smem_u32(tiles), 0), tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+      const bool chosen = elect_one();
+      uint32_t it = 0, local = 0;
+      bool going = true;
+      for (int item = blockIdx.x; item < items && going; item += gridDim.x) {
+        if (EXPERTS && experts.tile_experts[item % m_tiles] < 0) continue;
+        const int kb_begin = (item / (m_tiles * n_tiles)) * kb_per_split;
+        const int num_kb = min(k_blocks - kb_begin, kb_per_split);
+        const uint32_t acc = local % NBUF, use = local / NBUF;
+        // the epilogue must have emptied these accumulators (their previous use)
+        if (__any_sync(0xffffffffu, *bail != 0) ||
+            (use > 0 && !__all_sync(0xffffffffu, lane != 0 || mbar_wait(acc_free + acc, (use - 1) & 1, status, kStuckTmemFree)))) {
+          *bail = 1;
+          break;
+        }
+        const uint32_t tmem_d = tmem + acc * SET;
+        for (int kb = 0; kb < num_kb;) {
+          const int ready = min(ring_ready<STAGES>(full, it, lane, status, kStuckFull), num_kb - kb);
+          if (ready == 0) {
+            *bail = 1;
+            going = false;
+            break;
+          }
+          tc_fence_after();
+          for (const int until = kb + ready; kb < until; ++kb, ++it) {
+            const int s = it % STAGES;
+            const uint32_t a = ring + s * STAGE_BYTES, b = a + A_BYTES;
+            if (chosen) {
+#pragma unroll
+              for (int k = 0; k < BK / UMMA_K; ++k)
+#pragma unroll
+                for (int i = 0; i < MT; ++i)  // the 128-row blocks of X share the tile of W
+                  umma_bf16(tmem_d + i * BN, smem_desc(a + i * BM * BK * 2 + k * UMMA_K * 2),
+                            smem_desc(b + k * UMMA_K * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+              umma_commit(empty + s);  // arrives when these MMAs have finished reading the stage
+            }
+            __syncwarp();
+          }
+        }
+        if (chosen) umma_commit(acc_full + acc);  // arrives when every MMA issued so far has completed
+        __syncwarp();
+        ++local;
+      }
+    } else if (lane == 0) {
       // ---- issuer: one thread drives the tensor core
       constexpr uint32_t idesc = umma_idesc(BM, BN);  // both operands K-major
       uint32_t it = 0, local = 0;

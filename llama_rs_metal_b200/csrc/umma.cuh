@@ -49,6 +49,29 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   if (status != nullptr) atomicCAS(status, 0, where);
   return false;
 }
+// How many of a ring's "full" barriers in a row, from that of block `it` on, have completed their block's phase; at least 1, or 0
+// where a bounded wait for the first gave up. A whole warp calls it, on the same `it`. A question costs some 200 cycles whatever
+// the answer, so one is asked for all stages together, and one lane alone waits where none is there (32 lanes waiting on a barrier
+// take turns).
+template <int STAGES>
+__device__ __forceinline__ int ring_ready(uint64_t* bars, uint32_t it, int lane, int* status, int where) {
+  const uint32_t block = it + lane;
+  uint32_t done = 0;
+  if (lane < STAGES)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(smem_u32(bars + block % STAGES)), "r"((block / STAGES) & 1)
+        : "memory");
+  const uint32_t all = __ballot_sync(0xffffffffu, done != 0);
+  __syncwarp();
+  if (all & 1u) return __ffs(~all) - 1;
+  const bool there = __all_sync(0xffffffffu, lane != 0 || mbar_wait(bars + it % STAGES, (it / STAGES) & 1, status, where));
+  __syncwarp();
+  return there ? 1 : 0;
+}
 // One tile of a 2-D tensor map into shared memory; (x, y) = (innermost, outer) element coordinates.
 // x times the element size must be a multiple of 16 bytes.
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
