@@ -52,12 +52,18 @@ enum : int { kStuckEmpty = 1, kStuckFull = 2, kStuckAccumulator = 3, kStuckDrain
 // epilogue of one item runs under the MMAs of the next; a 256 x 256 tile fills it alone.
 // EXPERTS: row tile m multiplies the W of expert tile_experts[m] (-1: no tile, nothing is done), which begins w_rows rows
 // and w_cols columns after the W of the expert before.
+// GATED as well: W holds an expert's ff gate rows and then its ff up rows; a column tile takes BN / 2 of each, and its epilogue
+// writes weight * act(gate, up) in bfloat16 to out [M, ff], 0 where the row has no pair or no weight (moe_sorted.cu).
 struct ExpertArgs {
   const int* tile_experts;
   int w_rows, w_cols;
+  const int* rows;       // GATED from here on
+  const float* weights;  // of a row's pair
+  int ff, act;
+  float limit, alpha;
 };
 
-template <int BN, int STAGES, int MT, bool EXPERTS = false>
+template <int BN, int STAGES, int MT, bool EXPERTS = false, bool GATED = false>
 __global__ __launch_bounds__(kUmmaThreads, 1) void gemm_bf16_umma_kernel(
     const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
     void* __restrict__ out, int M, int N, int K, int mode, int kb_per_split, int splits,
@@ -136,8 +142,11 @@ __global__ __launch_bounds__(kUmmaThreads, 1) void gemm_bf16_umma_kernel(
           for (int i = 0; i < MT; ++i)  // 128 rows of X per accumulator (rows beyond M read as zero)
             tma_load_2d(tiles + s * STAGE_BYTES + i * BM * BK * 2, &map_x, full + s, (kb_begin + kb) * BK,
                         x0 + i * BM);
+          const int w_row = (GATED ? n0 / 2 : n0) + (EXPERTS ? e * experts.w_rows : 0);
           tma_load_2d(tiles + s * STAGE_BYTES + A_BYTES, &map_w, full + s, (kb_begin + kb) * BK + (EXPERTS ? e * experts.w_cols : 0),
-                      n0 + (EXPERTS ? e * experts.w_rows : 0));
+                      w_row);
+          if (GATED)  // (gate rows beyond ff are up rows, up rows beyond ff the next expert's or zeros: columns that are not stored)
+            tma_load_2d(tiles + s * STAGE_BYTES + A_BYTES + B_BYTES / 2, &map_w, full + s, (kb_begin + kb) * BK, w_row + experts.ff);
         }
       }
       if (*bail) {
@@ -256,7 +265,18 @@ __global__ __launch_bounds__(kUmmaThreads, 1) void gemm_bf16_umma_kernel(
       void* plane = mode == 4 ? static_cast<void*>(static_cast<float*>(out) +
                                                    static_cast<size_t>(item / (m_tiles * n_tiles)) * M * N)
                               : out;
-      if (mode == 5) {  // whole heads of a q|k|v projection: rotate, store packed and into the cache
+      if (GATED) {
+        const int row = m0 + quarter * 32, p = experts.rows[row + lane];
+        const float weight = p < 0 ? 0.f : experts.weights[p];
+        const uint32_t gates = tmem_base + acc * SET + (static_cast<uint32_t>(quarter * 32) << 16);
+#pragma unroll 1
+        for (int c = side * (BN / 4); c < (side + 1) * (BN / 4); c += 32) {
+          const int f = n0 / 2 + c;
+          if (f >= experts.ff) break;  // (ff a multiple of 64: pieces of 32 lie on one side)
+          store_gated(gates + c, gates + BN / 2 + c, stage, static_cast<__nv_bfloat16*>(out) + f, row, lane, weight, experts.ff,
+                      experts.act, experts.limit, experts.alpha);
+        }
+      } else if (mode == 5) {  // whole heads of a q|k|v projection: rotate, store packed and into the cache
         // the first of the two warps of a row takes the first half of the tile's heads (rounded up)
         const int heads = BN / qkv.head_dim, cut = ((heads + 1) >> 1) * qkv.head_dim;
 #pragma unroll 1
@@ -284,17 +304,17 @@ __global__ __launch_bounds__(kUmmaThreads, 1) void gemm_bf16_umma_kernel(
 }
 
 // ------------------------------------------------------------------------- host side
-template <int BN, int STAGES, int MT = 1, bool EXPERTS = false>
+template <int BN, int STAGES, int MT = 1, bool EXPERTS = false, bool GATED = false>
 int launch_umma(const void* X, const void* W, void* out, int M, int x_rows, int N, int K, int mode, int splits,
                 int* status, cudaStream_t stream, const QkvArgs& qkv = QkvArgs{}, int group_cols = 0,
                 int group_rows = 0, const SplitArgs& parts = SplitArgs{}, const ExpertArgs& experts = ExpertArgs{},
                 long long w_height = 0, long long w_width = 0) {
   CUtensorMap map_x, map_w;
   if (!make_map_bf16(&map_x, X, x_rows, K, BM) ||
-      !make_map_bf16(&map_w, W, EXPERTS ? w_height : N, EXPERTS ? w_width : K, BN))
+      !make_map_bf16(&map_w, W, EXPERTS ? w_height : N, EXPERTS ? w_width : K, GATED ? BN / 2 : BN))
     return LRM_UNSUPPORTED;
   constexpr int smem = STAGES * (MT * BM * BK * 2 + BN * BK * 2) + 1024 + 256 + 8 * kStageBytes;
-  auto kernel = gemm_bf16_umma_kernel<BN, STAGES, MT, EXPERTS>;
+  auto kernel = gemm_bf16_umma_kernel<BN, STAGES, MT, EXPERTS, GATED>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return static_cast<int>(e);
   const int k_blocks = (K + BK - 1) / BK;
@@ -439,7 +459,25 @@ LRM_API int lrm_gemm_bf16_umma_experts(const void* X, const void* W, void* out, 
     return LRM_UNSUPPORTED;
   if (tile_experts == nullptr || status == nullptr || w_rows < 0 || w_cols < 0) return LRM_BAD_ARGUMENT;
   if (reinterpret_cast<uintptr_t>(X) % 16 || reinterpret_cast<uintptr_t>(W) % 16) return LRM_UNSUPPORTED;
-  const ExpertArgs experts{tile_experts, w_rows, w_cols};
+  const ExpertArgs experts{tile_experts, w_rows, w_cols, nullptr, nullptr, 0, 0, 0.f, 0.f};
   return launch_umma<256, 4, 1, true>(X, W, out, M, M, N, K, 1, 1, status, stream, QkvArgs{}, 0, 0, SplitArgs{}, experts, w_height,
                                       w_width);
+}
+
+// The first product of a prompt's sorted experts with the gate in its epilogue: out bfloat16 [M, ff] = weights[rows[m]] *
+// act(x . gate_e^T, x . up_e^T), 0 where rows[m] < 0; W [w_height, K] holds 2 ff rows per expert (gate, then up). K and ff
+// multiples of 64. Against the product in float32 and the gate in a launch of its own: the same bits without 8 ff bytes
+// written and read per row.
+LRM_API int lrm_gemm_bf16_umma_experts_gated(const void* X, const void* W, void* out, int M, int ff, int K, long long w_height,
+                                             const int* tile_experts, const int* rows, const float* weights, float limit,
+                                             float alpha, int act, int* status, cudaStream_t stream) {
+  if (M <= 0 || ff <= 0) return 0;
+  if (!lrm_gemm_bf16_umma_supports(M, 2 * ff, K) || K % BK || M % BM || ff % 64 || w_height >= (1ll << 31)) return LRM_UNSUPPORTED;
+  if (tile_experts == nullptr || rows == nullptr || weights == nullptr || status == nullptr || (act != 0 && act != 1))
+    return LRM_BAD_ARGUMENT;
+  if (reinterpret_cast<uintptr_t>(X) % 16 || reinterpret_cast<uintptr_t>(W) % 16 || reinterpret_cast<uintptr_t>(out) % 16)
+    return LRM_UNSUPPORTED;
+  const ExpertArgs experts{tile_experts, 2 * ff, 0, rows, weights, ff, act, limit, alpha};
+  return launch_umma<256, 4, 1, true, true>(X, W, out, M, M, (ff + 127) / 128 * 256, K, 1, 1, status, stream, QkvArgs{}, 0, 0,
+                                            SplitArgs{}, experts, w_height, K);
 }

@@ -11,20 +11,20 @@
 
 namespace {
 
-// g / (1 + exp(-g)) of COUNT values. A division of its own for each, with its test for the rare operands, leaves a warp with
+// g / (1 + exp(-alpha g)) of COUNT values. A division of its own for each, with its test for the rare operands, leaves a warp with
 // one chain of some 80 cycles after the other (5.6 us for a 128 x 256 tile, staged 5.7); here the quotients of a thread go side by side:
 // Newton's step for the reciprocal of a denominator between 1 and 2^116, then Markstein's correction of the quotient by its
-// remainder (IBM J. Res. Dev. 34, 1990), which rounds as the division does. Beyond 80 the denominator is 1, and below -80 one
-// plus it is it.
+// remainder (IBM J. Res. Dev. 34, 1990), which rounds as the division does. With alpha g beyond 80 the denominator is 1, and below
+// -80 one plus it is it.
 template <int COUNT>
-__device__ __forceinline__ void silu_all(float (&g)[COUNT]) {
+__device__ __forceinline__ void silu_all(float (&g)[COUNT], float alpha = 1.f) {
   float v[COUNT];
   bool plain = true;
 #pragma unroll
-  for (int i = 0; i < COUNT; ++i) plain &= fabsf(g[i]) <= 80.f;  // not for NaN
+  for (int i = 0; i < COUNT; ++i) plain &= fabsf(alpha * g[i]) <= 80.f;  // not for NaN
 #pragma unroll
   for (int i = 0; i < COUNT; ++i) {
-    const float d = 1.0f + expf(-g[i]);
+    const float d = 1.0f + expf(-alpha * g[i]);
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     r = fmaf(r, fmaf(-d, r, 1.0f), r);
@@ -33,7 +33,10 @@ __device__ __forceinline__ void silu_all(float (&g)[COUNT]) {
   }
   if (!__all_sync(0xffffffffu, plain)) {
 #pragma unroll
-    for (int i = 0; i < COUNT; ++i) v[i] = g[i] > 80.f ? g[i] : g[i] < -80.f ? g[i] * expf(g[i]) : v[i];
+    for (int i = 0; i < COUNT; ++i) {
+      const float z = alpha * g[i];
+      v[i] = z > 80.f ? g[i] : z < -80.f ? g[i] * expf(z) : v[i];
+    }
   }
 #pragma unroll
   for (int i = 0; i < COUNT; ++i) g[i] = v[i];
@@ -170,6 +173,35 @@ __device__ __forceinline__ void store_piece(const uint32_t (&r)[32], unsigned ch
       }
     }
   }
+}
+
+// 32 gate columns and the 32 up columns beside them, at these places of tensor memory, of a warp's 32 rows (m0 ..): weight *
+// act(gate, up) to out [.., pitch]. Act 0: min(g, limit) sigmoid(alpha g) (clamp(u, -limit, limit) + 1); 1: silu(g) u.
+__device__ __forceinline__ void store_gated(uint32_t gates, uint32_t ups, unsigned char* stage, __nv_bfloat16* out, int m0,
+                                            int lane, float weight, int pitch, int act, float limit, float alpha) {
+  uint32_t packed[16];
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    uint32_t raw[16], up[16];
+    tmem_load16(gates + 16 * half, raw);
+    tmem_load16(ups + 16 * half, up);
+    float g[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) g[i] = act == 1 ? __uint_as_float(raw[i]) : fminf(__uint_as_float(raw[i]), limit);
+    silu_all(g, act == 1 ? 1.f : alpha);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      float u = __uint_as_float(up[i]);
+      if (act != 1) u = fminf(fmaxf(u, -limit), limit) + 1.f;
+      g[i] = weight != 0.f ? g[i] * u * weight : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) packed[8 * half + i] = pack_bf16(g[2 * i], g[2 * i + 1]);
+  }
+  stage_row<64>(stage, lane, packed);
+  unstage<64>(stage, lane, [&](int row, int byte, const uint4& v) {
+    *reinterpret_cast<uint4*>(out + static_cast<size_t>(m0 + row) * pitch + byte / 2) = v;
+  });
 }
 
 // What epilogue 5 needs: the product is a prompt's fused q|k|v projection [T, (Hq + 2 Hk) d], and

@@ -184,13 +184,82 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, const float* 
   for (int c = 0; c < top; ++c) w[c] /= mass;
 }
 
+// A warp chooses the `top` largest of z [E] (shared memory), the lower index on a tie, and weighs them by the softmax over the
+// chosen: the same numbers as one thread going through z for each choice, which spends a microsecond and more on it (its choices
+// come back to it through memory). A NaN, which is chosen only where it comes first, and more than 32 choices are left to that
+// thread.
+__device__ __forceinline__ void choose_top(const float* z, int E, int top, int lane, int* ids, float* weights) {
+  bool odd = top > 32;
+  for (int e = lane; e < E; e += 32) odd |= z[e] != z[e];
+  if (!__any_sync(0xffffffffu, odd)) {
+    float last = INFINITY, best = 0.f, mass = 0.f, share = 0.f;  // the choice before, in the order of (value, index)
+    int last_at = -1;
+    for (int c = 0; c < top; ++c) {
+      float val = -INFINITY;
+      int arg = E;  // none
+      for (int e = lane; e < E; e += 32) {
+        const float v = z[e];
+        const bool taken = v > last || (v == last && e <= last_at);
+        if (!taken && (arg == E || v > val)) {
+          val = v;
+          arg = e;
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float other = __shfl_xor_sync(0xffffffffu, val, o);
+        const int at = __shfl_xor_sync(0xffffffffu, arg, o);
+        if (other > val || (other == val && at < arg)) {
+          val = other;
+          arg = at;
+        }
+      }
+      last = val;
+      last_at = arg;
+      if (c == 0) best = val;
+      const float part = expf(val - best);
+      mass += part;
+      if (lane == c) {
+        ids[c] = arg;
+        share = part;
+      }
+    }
+    if (lane < top) weights[lane] = share / mass;
+    return;
+  }
+  if (lane != 0) return;
+  float best = -INFINITY, mass = 0.f;
+  for (int c = 0; c < top; ++c) {
+    int arg = -1;
+    float val = -INFINITY;
+    for (int e = 0; e < E; ++e) {
+      bool taken = false;
+      for (int p = 0; p < c; ++p) taken |= ids[p] == e;
+      if (!taken && (arg < 0 || z[e] > val)) {
+        arg = e;
+        val = z[e];
+      }
+    }
+    ids[c] = arg;
+    weights[c] = val;
+    if (c == 0) best = val;
+  }
+  for (int c = 0; c < top; ++c) {
+    weights[c] = expf(weights[c] - best);
+    mass += weights[c];
+  }
+  for (int c = 0; c < top; ++c) weights[c] /= mass;
+}
+
 // The router in one launch: a CTA per TOK tokens forms their E float32 logits (a warp per expert at a
 // time, the lanes across the row, each lane's products in ascending order and the lanes added by a
-// butterfly: a fixed order whatever the batch), then a warp per token chooses. A lane has 16 loads of
-// a router row under way together (8 tokens, 9 outputs, width 2048: 8 us, 15 with the loads one after
-// another); prompts share every load of the router's matrix between four tokens.
+// butterfly: a fixed order whatever the batch), then a warp per token chooses. Bound by what it waits for: a lane has
+// 16 to 32 loads of a router row under way, the first of them asked for ahead of the step before (the matrix is a weight).
+// Prompts share every load of the router's matrix between four tokens, which stand in shared memory side by side, so that one
+// load brings all four. 1,500 tokens, 8 outputs, width 2048: 11 us, 17 with a load
+// per token and one thread choosing; 8 tokens 4.1 (5.7).
 template <typename A, int TOK>
-__global__ void moe_router_kernel(const A* x, const float* __restrict__ w,
+__global__ __launch_bounds__(TOK == 1 ? 1024 : 256) void moe_router_kernel(const A* x, const float* __restrict__ w,
                                   const float* __restrict__ bias, int* __restrict__ ids,
                                   float* __restrict__ weights, float* __restrict__ logits, int tokens, int width, int E,
                                   int top, int scored, const float* __restrict__ correction, int groups, int keep,
@@ -198,42 +267,89 @@ __global__ void moe_router_kernel(const A* x, const float* __restrict__ w,
   extern __shared__ __align__(16) float smem[];
   pdl_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  constexpr int AHEAD = 16;
+  float r[AHEAD];
+  const bool begun = warp < E && width >= AHEAD * 32;
+  if (begun) {
+    const float* row = w + static_cast<size_t>(warp) * width;
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) r[u] = __ldg(row + lane + 32 * u);
+  }
   pdl_wait();
   const int t0 = blockIdx.x * TOK, live = min(TOK, tokens - t0);
-  float* xs = smem;  // [TOK][width]
+  float* xs = smem;  // [width][TOK]
   const A* rows = x + static_cast<size_t>(t0) * width;
-  constexpr int PIECE = 16 / sizeof(A);
-  if (width % PIECE == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0) {  // 16 bytes at a time
-    for (int i = threadIdx.x * PIECE; i < live * width; i += blockDim.x * PIECE) {
-      const uint4 raw = *reinterpret_cast<const uint4*>(rows + i);
-      const A* part = reinterpret_cast<const A*>(&raw);
+  if (TOK == 4) {
+    float4* quads = reinterpret_cast<float4*>(xs);
+    constexpr int PIECE = 4 / sizeof(A) > 1 ? 2 : 1;  // bfloat16: two numbers at a time
+    if (PIECE == 2 && (width % 2 != 0 || reinterpret_cast<uintptr_t>(x) % 4 != 0)) {
+      for (int i = threadIdx.x; i < width; i += blockDim.x) {
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int k = 0; k < live; ++k) v[k] = to_f32(rows[static_cast<size_t>(k) * width + i]);
+        quads[i] = make_float4(v[0], v[1], v[2], v[3]);
+      }
+    } else {
+#pragma unroll 4
+      for (int i = threadIdx.x * PIECE; i < width; i += blockDim.x * PIECE) {
+        float v[PIECE][4];
 #pragma unroll
-      for (int u = 0; u < PIECE; u += 4)
-        *reinterpret_cast<float4*>(xs + i + u) = make_float4(to_f32(part[u]), to_f32(part[u + 1]), to_f32(part[u + 2]), to_f32(part[u + 3]));
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t raw = k < live ? *reinterpret_cast<const uint32_t*>(rows + static_cast<size_t>(k) * width + i) : 0u;
+          const A* part = reinterpret_cast<const A*>(&raw);
+#pragma unroll
+          for (int u = 0; u < PIECE; ++u) v[u][k] = to_f32(part[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < PIECE; ++u) quads[i + u] = make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
+      }
     }
   } else {
-    for (int i = threadIdx.x; i < live * width; i += blockDim.x) xs[i] = to_f32(rows[i]);
+    constexpr int PIECE = 16 / sizeof(A);
+    if (width % PIECE == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0) {  // 16 bytes at a time
+      for (int i = threadIdx.x * PIECE; i < width; i += blockDim.x * PIECE) {
+        const uint4 raw = *reinterpret_cast<const uint4*>(rows + i);
+        const A* part = reinterpret_cast<const A*>(&raw);
+#pragma unroll
+        for (int u = 0; u < PIECE; u += 4)
+          *reinterpret_cast<float4*>(xs + i + u) = make_float4(to_f32(part[u]), to_f32(part[u + 1]), to_f32(part[u + 2]), to_f32(part[u + 3]));
+      }
+    } else {
+      for (int i = threadIdx.x; i < width; i += blockDim.x) xs[i] = to_f32(rows[i]);
+    }
   }
-  for (int i = live * width + threadIdx.x; i < TOK * width; i += blockDim.x) xs[i] = 0.f;
   __syncthreads();
   for (int e = warp; e < E; e += warps) {
     const float* row = w + static_cast<size_t>(e) * width;
     float acc[TOK];
 #pragma unroll
     for (int k = 0; k < TOK; ++k) acc[k] = 0.f;
+    const auto add = [&](float number, int i) {
+      if constexpr (TOK == 4) {
+        const float4 v = reinterpret_cast<const float4*>(xs)[i];
+        acc[0] = fmaf(number, v.x, acc[0]), acc[1] = fmaf(number, v.y, acc[1]);
+        acc[2] = fmaf(number, v.z, acc[2]), acc[3] = fmaf(number, v.w, acc[3]);
+      } else {
+        acc[0] = fmaf(number, xs[i], acc[0]);
+      }
+    };
     int i = lane;
-    for (; i + 15 * 32 < width; i += 16 * 32) {
-      float r[16];
+    const int whole = width / (AHEAD * 32);
+    if (whole > 0 && e != warp) {
 #pragma unroll
-      for (int u = 0; u < 16; ++u) r[u] = __ldg(row + i + 32 * u);
-#pragma unroll
-      for (int u = 0; u < 16; ++u)
-#pragma unroll
-        for (int k = 0; k < TOK; ++k) acc[k] = fmaf(r[u], xs[k * width + i + 32 * u], acc[k]);
+      for (int u = 0; u < AHEAD; ++u) r[u] = __ldg(row + i + 32 * u);
     }
-    for (; i < width; i += 32)
+    for (int part = 0; part < whole; ++part, i += AHEAD * 32) {
+      float next[AHEAD];
+      if (part + 1 < whole) {
 #pragma unroll
-      for (int k = 0; k < TOK; ++k) acc[k] = fmaf(row[i], xs[k * width + i], acc[k]);
+        for (int u = 0; u < AHEAD; ++u) next[u] = __ldg(row + i + (AHEAD + u) * 32);
+      }
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u) add(r[u], i + 32 * u);
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u) r[u] = next[u];
+    }
+    for (; i < width; i += 32) add(row[i], i);
 #pragma unroll
     for (int k = 0; k < TOK; ++k) {
       const float z = warp_sum(acc[k]);
@@ -256,28 +372,7 @@ __global__ void moe_router_kernel(const A* x, const float* __restrict__ w,
                     renormalize, mass_eps, weight_scale, mine, out);
     return;
   }
-  if (lane != 0) return;
-  float best = -INFINITY, mass = 0.f;
-  for (int c = 0; c < top; ++c) {
-    int arg = -1;
-    float val = -INFINITY;
-    for (int e = 0; e < E; ++e) {
-      bool taken = false;
-      for (int p = 0; p < c; ++p) taken |= mine[p] == e;
-      if (!taken && (arg < 0 || zs[e] > val)) {
-        arg = e;
-        val = zs[e];
-      }
-    }
-    mine[c] = arg;
-    out[c] = val;
-    if (c == 0) best = val;
-  }
-  for (int c = 0; c < top; ++c) {
-    out[c] = expf(out[c] - best);
-    mass += out[c];
-  }
-  for (int c = 0; c < top; ++c) out[c] /= mass;
+  choose_top(zs, E, top, lane, mine, out);
 }
 
 template <typename T> struct Pack8;

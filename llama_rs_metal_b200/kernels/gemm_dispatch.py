@@ -321,6 +321,7 @@ def gemm_bf16_qkv(x: torch.Tensor, weight: torch.Tensor, q: torch.Tensor, k: tor
 
 
 no_fused_rope = False  # tests: keep rotation and stores in their own launch
+no_fused_gate = False  # tests: keep the sorted experts' gate in its own launch
 
 
 def gemm_bf16(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, mode: int) -> None:

@@ -1675,13 +1675,19 @@ def moe_experts_sorted(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tenso
     _done(lib.lrm_moe_gather(_ptr(x), _ptr(rows), _ptr(tile_experts), top, width, tiles, _ptr(sorted_x), _stream()), "moe_gather")
     status = _ptr(gemm_dispatch._status_word(dev))
     gemm_dispatch.mark_status_dirty()
-    both = _f32((M, 2 * ff), dev)
-    _done(lib.lrm_gemm_bf16_umma_experts(_ptr(sorted_x), _ptr(gate_up), _ptr(both), M, 2 * ff, width,
-                                         ctypes.c_longlong(E * 2 * ff), ctypes.c_longlong(width), 2 * ff, 0, _ptr(tile_experts),
-                                         status, _stream()), "gemm_bf16_umma_experts")
     y = torch.empty((M, ff), dtype=torch.bfloat16, device=dev)
-    _done(lib.lrm_moe_sorted_gate(_ptr(both), _ptr(rows), _ptr(tile_experts), _ptr(weights), ff, tiles, ctypes.c_float(limit),
-                                  ctypes.c_float(alpha), act, _ptr(y), _stream()), "moe_sorted_gate")
+    if gemm_dispatch.no_fused_gate:
+        both = _f32((M, 2 * ff), dev)
+        _done(lib.lrm_gemm_bf16_umma_experts(_ptr(sorted_x), _ptr(gate_up), _ptr(both), M, 2 * ff, width,
+                                             ctypes.c_longlong(E * 2 * ff), ctypes.c_longlong(width), 2 * ff, 0, _ptr(tile_experts),
+                                             status, _stream()), "gemm_bf16_umma_experts")
+        _done(lib.lrm_moe_sorted_gate(_ptr(both), _ptr(rows), _ptr(tile_experts), _ptr(weights), ff, tiles, ctypes.c_float(limit),
+                                      ctypes.c_float(alpha), act, _ptr(y), _stream()), "moe_sorted_gate")
+    else:
+        _done(lib.lrm_gemm_bf16_umma_experts_gated(_ptr(sorted_x), _ptr(gate_up), _ptr(y), M, ff, width,
+                                                   ctypes.c_longlong(E * 2 * ff), _ptr(tile_experts), _ptr(rows), _ptr(weights),
+                                                   ctypes.c_float(limit), ctypes.c_float(alpha), act, status, _stream()),
+              "gemm_bf16_umma_experts_gated")
     part = _f32((M, width), dev)
     _done(lib.lrm_gemm_bf16_umma_experts(_ptr(y), _ptr(down), _ptr(part), M, width, ff, ctypes.c_longlong(width),
                                          ctypes.c_longlong(E * ff), 0, ff, _ptr(tile_experts), status, _stream()),

@@ -137,6 +137,7 @@ WORK: Dict[str, Callable[..., Tuple[float, float]]] = {
     "lrm_moe_experts_grouped": lambda a: (
         min(_v(a[7]) * _v(a[11]), _v(a[10])) * 6.0 * _v(a[9]) * _v(a[8]) + 4.0 * _v(a[7]) * _v(a[11]) * _v(a[8]),
         6.0 * _v(a[7]) * _v(a[11]) * _v(a[9]) * _v(a[8])),
+    "lrm_gemm_bf16_umma_experts_gated": lambda a: _gemm(_v(a[3]), 2 * _v(a[4]), _v(a[5]), 1, 2),
     "lrm_gemm_bf16_umma_experts": lambda a: _gemm(_v(a[3]), _v(a[4]), _v(a[5]), 4, 2),
     "lrm_moe_gather": lambda a: (_v(a[5]) * 128.0 * _v(a[4]) * 4.0, 0),
     "lrm_moe_sorted_gate": lambda a: (_v(a[5]) * 128.0 * _v(a[4]) * 10.0, 0),
