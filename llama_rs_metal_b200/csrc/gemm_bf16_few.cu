@@ -14,6 +14,7 @@
 //
 // Epilogues as in gemm_bf16_stream.cu: 0 bf16, 1 f32, 3 SiLU gate (blocks of 8 gate / 8 up rows alternate). Every mbarrier wait
 // is bounded. Its times beside those of the kernels it replaces stand at gemm_dispatch.few_takes.
+#include "silu.cuh"
 #include "umma.cuh"
 
 namespace {
@@ -30,26 +31,39 @@ struct Few {
   static constexpr size_t BYTES = 1024 + STAGES * STAGE_BYTES + 256;
 };
 
-__device__ __forceinline__ float silu_f32(float g) { return g / (1.0f + expf(-g)); }
-
-// Column n, activation row m. All lanes of a warp call it together (neighbouring columns).
+// Column n, activation row m.
 __device__ __forceinline__ void finish(float v, int m, int n, void* out, int N, int mode) {
-  if (mode == 3) {
-    const float up = __shfl_xor_sync(0xffffffffu, v, 8);
-    if ((n & 8) == 0 && n < N)
-      static_cast<__nv_bfloat16*>(out)[static_cast<size_t>(m) * (N >> 1) + (n >> 4) * 8 + (n & 7)] = __float2bfloat16_rn(silu_f32(v) * up);
-    return;
-  }
-  if (n >= N) return;
   const size_t o = static_cast<size_t>(m) * N + n;
   if (mode == 0) static_cast<__nv_bfloat16*>(out)[o] = __float2bfloat16_rn(v);
   else static_cast<float*>(out)[o] = v;
 }
 
+// The gate over rows m0 .. m0 + ROWS - 1, a column per lane, 8 gate and 8 up columns in turn. The two lanes of a pair take half of
+// the rows each, and their quotients go side by side. Every lane of the warp calls it; `stored`: this lane's column exists.
+template <int ROWS>
+__device__ __forceinline__ void finish_gated(const uint32_t (&r)[32], int m0, int M, int n, bool stored, __nv_bfloat16* out, int N) {
+  constexpr int HALF = ROWS / 2;
+  const bool is_up = n & 8;
+  float g[HALF], u[HALF];
+#pragma unroll
+  for (int i = 0; i < HALF; ++i) {
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, is_up ? r[i] : r[i + HALF], 8);
+    g[i] = __uint_as_float(is_up ? other : r[i]);
+    u[i] = __uint_as_float(is_up ? r[i + HALF] : other);
+  }
+  silu_all(g);
+  const int first = m0 + (is_up ? HALF : 0);
+  out += static_cast<size_t>(first) * (N >> 1) + (n >> 4) * 8 + (n & 7);
+#pragma unroll
+  for (int i = 0; i < HALF; ++i)
+    if (stored && first + i < M) out[static_cast<size_t>(i) * (N >> 1)] = __float2bfloat16_rn(g[i] * u[i]);
+}
+
 template <int NC>
 __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                     const __grid_constant__ CUtensorMap map_x, void* __restrict__ out,
-                                                                    int M, int N, int K, int mode, int* __restrict__ status) {
+                                                                    int M, int N, int K, int mode, int tile_rows,
+                                                                    int* __restrict__ status) {
   using F = Few<NC>;
   constexpr int STAGES = F::STAGES;
   pdl_trigger();
@@ -62,7 +76,8 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 2);
   volatile int* bail = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles = (N + kTileRows - 1) / kTileRows, k_blocks = (K + BK - 1) / BK;
+  const uint32_t stage_bytes = tile_rows * BK * 2 + F::STAGE_BYTES - F::W_BYTES;  // of the copies
+  const int tiles = (N + tile_rows - 1) / tile_rows, k_blocks = (K + BK - 1) / BK;
   const int first_tile = blockIdx.x, stride = gridDim.x, num_kb = k_blocks;
   const int early = min(num_kb, STAGES);  // stages of the first tile's weights asked for ahead of the wait
 
@@ -78,8 +93,8 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
     *bail = 0;
     mbar_fence_init();
     for (int kb = 0; kb < early; ++kb) {
-      mbar_expect_tx(full + kb, F::STAGE_BYTES);
-      tma_load_2d(ring + kb * F::STAGE_BYTES, &map_w, full + kb, kb * BK, first_tile * kTileRows);
+      mbar_expect_tx(full + kb, stage_bytes);
+      tma_load_2d(ring + kb * F::STAGE_BYTES, &map_w, full + kb, kb * BK, first_tile * tile_rows);
     }
   }
   if (warp == 1) {
@@ -106,8 +121,8 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
             *bail = 1;
             break;
           }
-          mbar_expect_tx(full + s, F::STAGE_BYTES);
-          tma_load_2d(ring + s * F::STAGE_BYTES, &map_w, full + s, kb * BK, tile * kTileRows);
+          mbar_expect_tx(full + s, stage_bytes);
+          tma_load_2d(ring + s * F::STAGE_BYTES, &map_w, full + s, kb * BK, tile * tile_rows);
           tma_load_2d(ring + s * F::STAGE_BYTES + F::W_BYTES, &map_x, full + s, kb * BK, 0);
         }
       }
@@ -117,32 +132,44 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc(kTileRows, NC);  // both operands K-major
-      uint32_t it = 0, local = 0;
-      for (int tile = first_tile; tile < tiles && !*bail; tile += stride, ++local) {
-        const uint32_t acc = local & 1, use = local >> 1;
-        if (use > 0 && !mbar_wait(acc_free + acc, (use - 1) & 1, status, kStuckTmemFree)) {
+    // The warp stays together around its issuing lane and goes through all blocks that are there with one question, as in
+    // gemm_bf16_umma.cu: a block's copies take some 600 cycles, a wait and four products by a lane of its own no fewer.
+    constexpr uint32_t idesc = umma_idesc(kTileRows, NC);  // both operands K-major
+    const uint32_t ring_at = __shfl_sync(0xffffffffu, smem_u32(ring), 0), tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+    const bool chosen = elect_one();
+    uint32_t it = 0, local = 0;
+    bool going = true;
+    for (int tile = first_tile; tile < tiles && going; tile += stride, ++local) {
+      const uint32_t acc = local & 1, use = local >> 1;
+      if (__any_sync(0xffffffffu, *bail != 0) ||
+          (use > 0 && !__all_sync(0xffffffffu, lane != 0 || mbar_wait(acc_free + acc, (use - 1) & 1, status, kStuckTmemFree)))) {
+        *bail = 1;
+        break;
+      }
+      tc_fence_after();
+      for (int kb = 0; kb < num_kb;) {
+        const int ready = min(ring_ready<STAGES>(full, it, lane, status, kStuckFull), num_kb - kb);
+        if (ready == 0) {
           *bail = 1;
+          going = false;
           break;
         }
         tc_fence_after();
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
+        for (const int until = kb + ready; kb < until; ++kb, ++it) {
           const uint32_t s = it % STAGES;
-          if (!mbar_wait(full + s, (it / STAGES) & 1, status, kStuckFull)) {
-            *bail = 1;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t a = smem_u32(ring + s * F::STAGE_BYTES), b = a + F::W_BYTES;
+          const uint32_t a = ring_at + s * F::STAGE_BYTES, b = a + F::W_BYTES;
+          if (chosen) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k)
-            umma_bf16(tmem_base + acc * F::SET, smem_desc(a + k * UMMA_K * 2), smem_desc(b + k * UMMA_K * 2), idesc,
-                      (kb > 0 || k > 0) ? 1u : 0u);
-          umma_commit(empty + s);
+            for (int k = 0; k < BK / UMMA_K; ++k)
+              umma_bf16(tmem + acc * F::SET, smem_desc(a + k * UMMA_K * 2), smem_desc(b + k * UMMA_K * 2), idesc,
+                        (kb > 0 || k > 0) ? 1u : 0u);
+            umma_commit(empty + s);
+          }
+          __syncwarp();
         }
-        umma_commit(acc_full + acc);
       }
+      if (chosen) umma_commit(acc_full + acc);
+      __syncwarp();
     }
   } else {
     const int quarter = warp & 3, place = quarter * 32 + lane;  // a warp may touch only this quarter of the lanes
@@ -154,17 +181,22 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
         break;
       }
       tc_fence_after();
-      const int n = tile * kTileRows + place;
+      const int n = tile * tile_rows + place;
+      const bool stored = place < tile_rows && n < N;
 #pragma unroll 1
       for (int c = 0; c < (NC + 31) / 32; ++c) {
         uint32_t r[32];
         tmem_load32(tmem_base + acc * F::SET + (static_cast<uint32_t>(quarter * 32) << 16) + c * 32, r);
+        constexpr int ROWS = NC < 32 ? NC : 32;
+        if (mode == 3) {
+          finish_gated<ROWS>(r, c * 32, M, n, stored, static_cast<__nv_bfloat16*>(out), N);
+          continue;
+        }
 #pragma unroll
-        for (int i = 0; i < (NC < 32 ? NC : 32); ++i) {
+        for (int i = 0; i < ROWS; ++i) {
           const int m = c * 32 + i;
-          if (m >= M) break;
-          const float v = __uint_as_float(r[i]);
-          finish(v, m, n, out, N, mode);
+          if (m >= M || !stored) break;
+          finish(__uint_as_float(r[i]), m, n, out, N, mode);
         }
       }
       tc_fence_before();
@@ -179,14 +211,26 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
 
 template <int NC>
 int launch(const void* X, const void* W, void* out, int M, int x_rows, int N, int K, int mode, int* status, cudaStream_t stream) {
+  // Fewer weight rows to a tile where that leaves the CTA with the most tiles fewer rows to read (the others wait for it, and a part
+  // of the SMs does not draw the whole bandwidth). The products work on 128 rows either way; those beyond are not stored. (8 rows:
+  // what a tile costs beside its reads.) With the whole warp issuing and the gate's quotients side by side, us, 32 rows: 28672 x
+  // 4096 43.1 -> 40.3 (gated 53.3 -> 41.0), 9472 x 22000 103 -> 84.
+  int tile_rows = kTileRows, least = 0;
+  for (int rows = kTileRows; rows >= 64; rows -= 16) {
+    const int cost = ((N + rows - 1) / rows + kSmCount - 1) / kSmCount * (rows + 8);
+    if (least == 0 || cost < least) {
+      least = cost;
+      tile_rows = rows;
+    }
+  }
   CUtensorMap map_w, map_x;
-  if (!make_map_bf16(&map_w, W, N, K, kTileRows) || !make_map_bf16(&map_x, X, x_rows, K, NC)) return LRM_UNSUPPORTED;
+  if (!make_map_bf16(&map_w, W, N, K, tile_rows) || !make_map_bf16(&map_x, X, x_rows, K, NC)) return LRM_UNSUPPORTED;
   auto kernel = gemm_bf16_few_kernel<NC>;
   constexpr int smem = static_cast<int>(Few<NC>::BYTES);
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return static_cast<int>(e);
-  const int tiles = (N + kTileRows - 1) / kTileRows;
-  LRM_LAUNCH(kernel, dim3(tiles < kSmCount ? tiles : kSmCount), kThreads, smem, stream, map_w, map_x, out, M, N, K, mode, status);
+  const int tiles = (N + tile_rows - 1) / tile_rows;
+  LRM_LAUNCH(kernel, dim3(tiles < kSmCount ? tiles : kSmCount), kThreads, smem, stream, map_w, map_x, out, M, N, K, mode, tile_rows, status);
   return 0;
 }
 

@@ -163,22 +163,20 @@ def _few_rows_plan(M: int, N: int, K: int, mode: int):
 
 
 def few_takes(M: int, N: int, K: int, mode: int) -> bool:
-    """Where the kernel with the weights as the wide tcgen05 operand is the faster one: 13 to 64 rows of products with tiles
-    enough, which the tile kernel reads at 5.5 TB/s; its ring holds 200 KB per SM on their way and reads at 6.2, but its
-    epilogue grows with the rows, most of all the SiLU gate's. us in a chain of products over more weights than L2 holds, in
-    brackets the kernel that else runs. bfloat16 results: 16384 x 2048 16 rows 13.7 (21.3), 28672 x 4096 16 rows 44.7
-    (50.4), 32 rows 45.6 (51.4), 49408 x 4096 33 rows 71.8 (78.4), 64 rows 73.8 (79.1), 128256 x 2048 64 rows 87.0 (94.4).
-    Gated: 16384 x 2048 16 rows 16.4 (24.4), 28672 x 4096 32 rows 53.3 (57.8), 49408 x 4096 33 rows 79.5 (84.1), 48 rows 84.1
-    (85.4), 64 rows 87.8 (85.2), 128256 x 2048 64 rows 101.1 (96.4). A tile for half the SMs only, 9472 x 22000: 32 rows
-    103.4 (105.3), 48 rows 107.2 (106.3), gated 118.4 (111.8). Smaller products of more rows would gain too (28672 x 4096 64
-    rows 48.1 against 51.7; gated 63.2 against 59.2). Up to 12 rows the streaming kernel stays although 28672 x 4096 alone
-    is faster here (8 rows 44.4 against 49.5): its like beside it live off the L1 that this kernel's ring takes from them (3
-    sequences, one layer of the 8B shape: 231 us a step against 177)."""
+    """Where the kernel with the weights as the wide tcgen05 operand runs: 13 to 64 rows of products with tiles enough. Its ring
+    holds 200 KB per SM on their way and reads at 6 TB/s. us in a chain of products over more weights than L2 holds, in
+    brackets the tile kernel. bfloat16 results: 16384 x 2048 16 rows 12.2 (14.8), 32 rows 13.0 (15.0), 28672 x 4096 16 rows
+    39.1 (46.9), 32 rows 40.3 (47.5), 49408 x 4096 32 rows 65.9 (72.3), 64 rows 70.4 (73.4), 128256 x 2048 64 rows 84.1 (88.9),
+    a tile for half the SMs only, 9472 x 22000 32 rows 84.1 (103.4). Gated: 16384 x 2048 16 rows 12.4 (15.5), 32 rows 13.5
+    (15.4), 28672 x 4096 32 rows 41.0 (48.2), 49408 x 4096 48 rows 70.9 (73.2). The line for more than 32 rows is that of both
+    kernels' earlier epilogues: below it lie a few per cent either way (28672 x 4096 64 rows 43.5 against 47.9, gated 44.9
+    against 48.4; gated 16384 x 3072 48 rows 21.6 against 21.4). Up to 12 rows the streaming kernel stays: its like beside it
+    live off the L1 that this kernel's ring takes from them (3 sequences, one layer of the 8B shape: 231 us a step against 177,
+    with this kernel's former times)."""
     if not 12 < M <= (48 if mode == 3 else 64):
         return False
-    least = 30e6 if M <= 16 else 100e6 if M <= 32 else 200e6
     tiles = -(-N // 128)
-    return mode in (0, 1, 3) and tiles >= (SM_COUNT // 2 if M <= 32 else SM_COUNT) and N * K >= least
+    return mode in (0, 1, 3) and tiles >= (SM_COUNT // 2 if M <= 32 else SM_COUNT) and N * K >= (30e6 if M <= 32 else 200e6)
 
 
 def _few(x: torch.Tensor, weight: torch.Tensor, mode: int, lib) -> bool:

@@ -43,3 +43,10 @@ def test_the_rule_takes_it_and_agrees_with_the_other_kernels(monkeypatch, M, N, 
     other = ops.linear(x, w).double()
     # both round a float32 sum to bfloat16: at most one step of it apart, and the sums' own difference
     assert bool(((got - other).abs() <= 2.0 ** -7 * other.abs() + K * 2.0 ** -22 * (x.double().abs() @ w.double().abs().T)).all())
+
+
+# columns for which tiles of fewer than 128 weight rows are taken: 64, 80, 96 and 112 of them, the last one ragged
+@pytest.mark.parametrize("N", [9472, 11600, 14032, 16384, 16528])
+@pytest.mark.parametrize("M,mode", [(13, 0), (29, 3), (50, 1), (64, 3)])
+def test_tiles_of_fewer_rows(N, M, mode):
+    test_matches_float64(M, N, 136, mode)
