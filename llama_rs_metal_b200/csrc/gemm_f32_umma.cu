@@ -1,11 +1,10 @@
 // float32 matrix product on the 5th-generation tensor cores: C[M,N] = X[M,K] . W[N,K]^T, for the larger matrices
-// (gemm_dispatch.f32_takes_umma). Every float32 number is cut into three bfloat16 parts of 8 bits, which hold all of it, and six of the
-// nine products of parts are added: what is left out is below 2^-24 of a product.
+// (gemm_dispatch.f32_takes_umma). Every float32 number is cut into three bfloat16 parts of 8 bits, which hold all of it, and six of
+// the nine products of parts are added: what is left out is at most 2^-22 of a product, of either sign.
 //
 // The tensor core truncates where it adds (measured: to 2^-23 of the sum), with a bias towards zero that grows with the terms: 1.2e-7
 // after 128, 2e-6 after 2,048. So an accumulator runs over 64 of K only, from zero, the small products ahead of the large one, and
-// the sums over K are float32 additions on the CUDA cores. Distance from 64 bits, relative,
-// normal numbers: 1.1e-7 at K 2,048 and 1.4e-7 at 8,192; float32 FMAs in ascending order 8.1e-7 and 1.6e-6.
+// the sums over K are float32 additions on the CUDA cores. Distance from 64 bits, relative, normal numbers: 1.1e-7 at K 2,048 and 1.4e-7 at 8,192; float32 FMAs in ascending order 8.1e-7 and 1.6e-6.
 //
 // A tile of 128 weight rows is the A operand; the rows of X, in equal tiles of up to 128, are its columns. One thread brings the
 // weights' blocks of 64 of K to shared memory by TMA, as float32. Eight or sixteen warps cut them, a row a lane, and put the parts into tensor

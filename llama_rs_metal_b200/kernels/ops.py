@@ -1629,8 +1629,8 @@ def moe_experts_rows(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor,
 def moe_prefers_sorted(tokens: int, width: int, ff: int, experts: int, top: int) -> bool:
     """Whether a prompt's experts are computed on rows sorted by expert instead of all of them for every token: where the
     sorted rows, each expert's filled up to tiles of 128, are at most half as many and the products large enough to pay for
-    six launches (30 us of nothing else). us, sorted against all, without the router. 2048 x 1024: 2 of 8 experts 500 tokens
-    60 and 92, 1,500 101 and 155, 4,096 192 and 358; 1 of 3 600 tokens 48 and 51; 4 of 8, more than half, 1,000 tokens 130 and
+    five launches. us, sorted against all, without the router and with the gate still in a launch of its own (with the router
+    1,500 tokens of the first size took 118 then and take 89 now; the line has stayed). 2048 x 1024: 2 of 8 experts 500 tokens 60 and 92, 1,500 101 and 155, 4,096 192 and 358; 1 of 3 600 tokens 48 and 51; 4 of 8, more than half, 1,000 tokens 130 and
     124. 1024 x 512: 2 of 8 500 tokens 38 and 46; 1 of 4 500 tokens 34 and 30, 1,000 37 and 36, 1,500 40 and 44; 1 of 3 1,500
     tokens 39 and 36, 2,048 43 and 45. 512 x 256: 2 of 8 500 tokens 33 and 28, 2,048 46 and 44; 1 of 4 4,096 tokens 46 and
     42; 8 of 32 4,096 tokens 243 and 231 (1,500 110 and 119)."""
