@@ -989,6 +989,15 @@ __global__ __launch_bounds__(256, DP > 128 ? 1 : 2) void block_scan_kernel(
 // tokens, in the kernels, so that its bits do not hang on the lengths of the others.
 inline bool takes_walk(int d, int tokens) { return tokens >= kWalkTokens && d <= 256; }
 inline int walking(int seqs, int tokens) { return seqs < tokens / kWalkTokens ? seqs : tokens / kWalkTokens; }  // at most
+// CTAs of the step's walks, for the choice of the way and its layout: as many whole walks as its tokens would make of the longest
+// one, which is what the step waits for. Where that is not known: all sequences where they bring kWalkTokens on average, else one.
+// us, counted so and by how many sequences could walk at most: 2,048 tokens beside 31 sequences of one, delta rule, 8 heads of 128 x 128
+// 187 and 361 (alone 167), head decay with a delta, 16 heads 226 and 544 (194), a bonus 191 and 329 (155); 297 beside three of one 50 and 95.
+inline long long walk_ctas(int seqs, int H, int dv, int tokens, int longest) {
+  const long long one = static_cast<long long>((dv + kBlockCols - 1) / kBlockCols) * H;
+  if (longest > 0) return longest < tokens ? one * tokens / longest : one;
+  return tokens >= static_cast<long long>(seqs) * kWalkTokens ? one * seqs : one;
+}
 
 // Floats of a stage in the workspace: its vectors, its numbers per head, and its tiles' (each behind those of all stages).
 template <int MODE>
@@ -1010,21 +1019,21 @@ long long block_stage_floats(int H, int KH, int d, int dv) {
 // and 282, head decay with a delta 252 and 214, a decay per token 185 and 172. With one decay a token and heads of up to 128 the
 // tensor cores are the faster way throughout (four of 1,024, 16 heads of 128 x 128 209 and 222).
 template <int MODE>
-bool block_takes_fma(int seqs, int H, int d, int dv, int tokens) {
-  const long long ctas = static_cast<long long>((dv + kBlockCols - 1) / kBlockCols) * H * walking(seqs, tokens);
+bool block_takes_fma(int seqs, int H, int d, int dv, int tokens, int longest) {
+  const long long ctas = walk_ctas(seqs, H, dv, tokens, longest);
   if (d > 128) return 2 * ctas > 3 * kSmCount;
   return BlockShape<64, MODE>::DELTA ? 2 * ctas > 5 * kSmCount : BlockShape<64, MODE>::BONUS && ctas > 3 * kSmCount;
 }
 
 template <int MODE>
-long long floats_per_stage(int seqs, int H, int KH, int d, int dv, int tokens) {
-  return block_takes_fma<MODE>(seqs, H, d, dv, tokens) ? walk_stage_floats<MODE>(H, KH, d) : block_stage_floats<MODE>(H, KH, d, dv);
+long long floats_per_stage(int seqs, int H, int KH, int d, int dv, int tokens, int longest) {
+  return block_takes_fma<MODE>(seqs, H, d, dv, tokens, longest) ? walk_stage_floats<MODE>(H, KH, d) : block_stage_floats<MODE>(H, KH, d, dv);
 }
 
 // Floats of a workspace that holds a step whole, 0 where the token-by-token kernel runs.
 template <int MODE>
-long long walk_floats(int seqs, int H, int KH, int d, int dv, int tokens) {
-  return takes_walk(d, tokens) ? walk_stages(tokens, seqs) * floats_per_stage<MODE>(seqs, H, KH, d, dv, tokens) : 0;
+long long walk_floats(int seqs, int H, int KH, int d, int dv, int tokens, int longest) {
+  return takes_walk(d, tokens) ? walk_stages(tokens, seqs) * floats_per_stage<MODE>(seqs, H, KH, d, dv, tokens, longest) : 0;
 }
 
 template <int DP, int MODE>
@@ -1039,7 +1048,7 @@ int launch_block(const WalkArgs& a) {
     return buffers;
   };
   constexpr int ALONE = fit(1), BESIDE = fit(2);
-  const bool alone = static_cast<long long>(tiles) * a.H * walkers <= kSmCount;
+  const bool alone = walk_ctas(a.seqs, a.H, a.dv, a.rows.tokens, a.rows.longest) <= kSmCount;
   auto kernel = alone ? (plain ? block_scan_kernel<DP, MODE, true, ALONE> : block_scan_kernel<DP, MODE, false, ALONE>)
                       : (plain ? block_scan_kernel<DP, MODE, true, BESIDE> : block_scan_kernel<DP, MODE, false, BESIDE>);
   const size_t bytes = K::bytes(alone ? ALONE : BESIDE);
@@ -1084,7 +1093,7 @@ int dispatch_walk(const float* q, const float* k, const float* v, const float* g
                   const float* look, const float* put, float* state, float* out, const int* cu_seqlens, const int* slots, int seqs,
                   int H, int KH, int d, int dv, const Workspace& workspace, cudaStream_t stream, const Rows& rows) {
   WalkArgs a{q, k, v, g, head_decay, beta, look, put, state, out, cu_seqlens, slots, seqs, H, KH, d, dv, workspace, stream, rows, 0, walking(seqs, rows.tokens)};
-  const long long stage = floats_per_stage<MODE>(seqs, H, KH, d, dv, rows.tokens);
+  const long long stage = floats_per_stage<MODE>(seqs, H, KH, d, dv, rows.tokens, rows.longest);
   if (reinterpret_cast<uintptr_t>(workspace.at) % 16 || workspace.floats < stage) return LRM_BAD_ARGUMENT;
   const bool pieces = workspace.floats / stage < walk_stages(rows.tokens, seqs);
   if (seqs > 1 || pieces) {  // the sequences that bring fewer tokens, one after another
@@ -1095,7 +1104,7 @@ int dispatch_walk(const float* q, const float* k, const float* v, const float* g
                                          stream, few);
     if (code != 0) return code;
   }
-  if (block_takes_fma<MODE>(seqs, H, d, dv, rows.tokens)) return launch_walk<MODE>(a);
+  if (block_takes_fma<MODE>(seqs, H, d, dv, rows.tokens, rows.longest)) return launch_walk<MODE>(a);
   if (d > 128) return launch_block<256, MODE>(a);
   if (d > 64) return launch_block<128, MODE>(a);
   return launch_block<64, MODE>(a);

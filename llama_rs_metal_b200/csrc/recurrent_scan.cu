@@ -7,8 +7,8 @@ int g_scan_rows = 16;
 extern "C" int lrm_scan_gated_delta(const float* q, const float* k, const float* v, const float* g, const float* beta,
                                     float* state, float* out, const int* cu_seqlens, const int* slots, int seqs, int H,
                                     int KH, int d, int dv, int tokens, float* workspace, long long floats,
-                                    cudaStream_t stream);
-extern "C" long long lrm_walk_floats_gated_delta(int seqs, int H, int KH, int d, int dv, int tokens);  // recurrent_scan_delta.cu
+                                    int longest, cudaStream_t stream);
+extern "C" long long lrm_walk_floats_gated_delta(int seqs, int H, int KH, int d, int dv, int tokens, int longest);  // recurrent_scan_delta.cu
 
 namespace {
 
@@ -248,10 +248,10 @@ LRM_API int lrm_linear_state_scan_rows(int rows) {
 // Floats of workspace that lrm_linear_state_scan wants to go in blocks, all of the step at once (0: it does not go so). With
 // fewer, but at least a stage's (this over tokens / 16 + seqs), it goes in pieces; without a workspace token by token.
 // rule 0: a decay per head, 1: the gated delta rule, 2: a decay per head and token.
-LRM_API long long lrm_linear_state_scan_floats(int rule, int seqs, int H, int KH, int d, int dv, int tokens) {
-  return rule == 0   ? walk_floats<0>(seqs, H, KH, d, dv, tokens)
-         : rule == 1 ? lrm_walk_floats_gated_delta(seqs, H, KH, d, dv, tokens)
-                     : walk_floats<2>(seqs, H, KH, d, dv, tokens);
+LRM_API long long lrm_linear_state_scan_floats(int rule, int seqs, int H, int KH, int d, int dv, int tokens, int longest) {
+  return rule == 0   ? walk_floats<0>(seqs, H, KH, d, dv, tokens, longest)
+         : rule == 1 ? lrm_walk_floats_gated_delta(seqs, H, KH, d, dv, tokens, longest)
+                     : walk_floats<2>(seqs, H, KH, d, dv, tokens, longest);
 }
 
 // q, k float32 [T, KH, d]; v float32 [T, H, dv]; out float32 [T, H, dv]; state float32
@@ -261,25 +261,25 @@ LRM_API long long lrm_linear_state_scan_floats(int rule, int seqs, int H, int KH
 LRM_API int lrm_linear_state_scan(const float* q, const float* k, const float* v, const float* g,
                                   const float* head_decay, const float* beta, float* state, float* out,
                                   const int* cu_seqlens, const int* slots, int seqs, int H, int KH, int d,
-                                  int dv, int tokens, float* workspace, long long floats, cudaStream_t stream) {
+                                  int dv, int tokens, float* workspace, long long floats, int longest, cudaStream_t stream) {
   if (seqs <= 0) return 0;
   if (H <= 0 || KH <= 0 || H % KH || d <= 0 || dv <= 0 || seqs > 65535 || H > 65535) return LRM_BAD_ARGUMENT;
   if (d > 2048) return LRM_UNSUPPORTED;
   if (g != nullptr) {
     if (beta == nullptr) return LRM_BAD_ARGUMENT;
-    return lrm_scan_gated_delta(q, k, v, g, beta, state, out, cu_seqlens, slots, seqs, H, KH, d, dv, tokens, workspace, floats,
+    return lrm_scan_gated_delta(q, k, v, g, beta, state, out, cu_seqlens, slots, seqs, H, KH, d, dv, tokens, workspace, floats, longest,
                                 stream);
   }
   if (head_decay == nullptr) {  // one decay per head and token, where beta would be
     if (beta == nullptr) return LRM_BAD_ARGUMENT;
     if (workspace != nullptr && takes_walk(d, tokens))
       return dispatch_walk<2>(q, k, v, nullptr, nullptr, beta, nullptr, nullptr, state, out, cu_seqlens, slots, seqs, H, KH, d, dv,
-                              Workspace{workspace, floats}, stream, Rows{tokens});
+                              Workspace{workspace, floats}, stream, Rows{tokens, 0, 0, longest});
     return dispatch_scan<2>(q, k, v, nullptr, nullptr, beta, nullptr, nullptr, state, out, cu_seqlens, slots, seqs, H, KH, d, dv, stream, Rows{tokens});
   }
   if (workspace != nullptr && takes_walk(d, tokens))
     return dispatch_walk<0>(q, k, v, nullptr, head_decay, nullptr, nullptr, nullptr, state, out, cu_seqlens, slots, seqs, H, KH, d,
-                            dv, Workspace{workspace, floats}, stream, Rows{tokens});
+                            dv, Workspace{workspace, floats}, stream, Rows{tokens, 0, 0, longest});
   return dispatch_scan<0>(q, k, v, nullptr, head_decay, nullptr, nullptr, nullptr, state, out, cu_seqlens, slots, seqs, H, KH, d,
                           dv, stream, Rows{tokens});
 }

@@ -319,6 +319,7 @@ __global__ __launch_bounds__(kScanThreads) void linear_scan_kernel(
 struct Rows {
   int tokens;
   long long q = 0, v = 0;
+  int longest = 0;                               // most tokens of a sequence, or more; 0: not known
   int below = INT_MAX, below_padding = INT_MAX;  // sequences (of padding) of as many tokens and more are left alone
 };
 

@@ -20,7 +20,7 @@ LRM_API int lrm_general_delta_scan(const float* q, const float* k, const float* 
 LRM_API int lrm_bonus_state_scan(const float* q, const float* k, long long q_stride, const float* v,
                                  long long v_stride, const float* g, const float* bonus, float* state, float* out,
                                  const int* cu_seqlens, const int* slots, int seqs, int H, int d, int dv,
-                                 int tokens, float* workspace, long long floats, cudaStream_t stream) {
+                                 int tokens, float* workspace, long long floats, int longest, cudaStream_t stream) {
   if (seqs <= 0) return 0;
   if (H <= 0 || d <= 0 || dv <= 0 || seqs > 65535 || H > 65535) return LRM_BAD_ARGUMENT;
   if (g == nullptr || bonus == nullptr || q_stride < static_cast<long long>(H) * d || v_stride < static_cast<long long>(H) * dv)
@@ -28,12 +28,12 @@ LRM_API int lrm_bonus_state_scan(const float* q, const float* k, long long q_str
   if (d > 2048) return LRM_UNSUPPORTED;
   if (workspace != nullptr && takes_walk(d, tokens))
     return dispatch_walk<4>(q, k, v, g, nullptr, nullptr, bonus, nullptr, state, out, cu_seqlens, slots, seqs, H, H, d, dv,
-                            Workspace{workspace, floats}, stream, Rows{tokens, q_stride, v_stride});
+                            Workspace{workspace, floats}, stream, Rows{tokens, q_stride, v_stride, longest});
   return dispatch_scan<4>(q, k, v, g, nullptr, nullptr, bonus, nullptr, state, out, cu_seqlens, slots, seqs, H, H, d,
                           dv, stream, Rows{tokens, q_stride, v_stride});
 }
 
 // Floats of workspace that lrm_bonus_state_scan wants to go in blocks, as lrm_linear_state_scan_floats.
-LRM_API long long lrm_bonus_state_scan_floats(int seqs, int H, int d, int dv, int tokens) {
-  return walk_floats<4>(seqs, H, H, d, dv, tokens);
+LRM_API long long lrm_bonus_state_scan_floats(int seqs, int H, int d, int dv, int tokens, int longest) {
+  return walk_floats<4>(seqs, H, H, d, dv, tokens, longest);
 }

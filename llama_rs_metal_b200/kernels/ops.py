@@ -826,17 +826,18 @@ SCAN_FLOATS = 64 << 20  # most floats of such a scan's workspace; a step that wa
 
 def _walk_workspace(entry: str, blocks: bool, tokens: int, longest: Optional[int], device, seqs: int, *sizes) -> Optional[torch.Tensor]:
     """float32 scratch of a state scan's blocked form; None where it goes token by token. `longest`: tokens of the longest
-    sequence, where the caller knows (no kernel is launched for long ones that a step cannot hold)."""
+    sequence, where the caller knows (no kernel is launched for long ones that a step cannot hold, and a step of one long
+    sequence among short ones is laid out for the one)."""
     if not blocks or min(tokens, tokens if longest is None else longest) < WALK_TOKENS:
         return None
     rule = sizes[:1] if entry == "lrm_linear_state_scan_floats" else ()
-    floats = getattr(_lib(), entry)(*rule, seqs, *sizes[len(rule):], tokens)
+    floats = getattr(_lib(), entry)(*rule, seqs, *sizes[len(rule):], tokens, longest or 0)
     stage = floats // (tokens // 16 + seqs)
     return torch.empty(max(stage, min(floats, SCAN_FLOATS)), dtype=torch.float32, device=device) if floats else None
 
 
-def _walk_args(work: Optional[torch.Tensor]):
-    return _ptr(work), ctypes.c_longlong(0 if work is None else work.numel())
+def _walk_args(work: Optional[torch.Tensor], longest: Optional[int]):
+    return _ptr(work), ctypes.c_longlong(0 if work is None else work.numel()), longest or 0
 
 
 def _walk_launches(work: Optional[torch.Tensor], seqs: int) -> int:
@@ -952,7 +953,7 @@ def linear_state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: 
     work = _walk_workspace("lrm_linear_state_scan_floats", blocks, T, longest, q.device, slots.numel(), rule, H, KH, d, dv)
     _done(_lib().lrm_linear_state_scan(_ptr(q), _ptr(k), _ptr(v), _ptr(g), _ptr(head_decay), _ptr(beta), _ptr(state),
                                        _ptr(out), _ptr(cu_seqlens), _ptr(slots), slots.numel(), H, KH, d, dv, T,
-                                       *_walk_args(work), _stream()), "linear_state_scan", launches=_walk_launches(work, slots.numel()))
+                                       *_walk_args(work, longest), _stream()), "linear_state_scan", launches=_walk_launches(work, slots.numel()))
     return out
 
 
@@ -1035,7 +1036,7 @@ def bonus_state_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, g: 
     _done(_lib().lrm_bonus_state_scan(_column_ptr(proj, q_off), _column_ptr(proj, k_off), ctypes.c_longlong(W),
                                       _column_ptr(proj, v_off), ctypes.c_longlong(W), _ptr(g), _ptr(bonus), _ptr(state),
                                       _ptr(out), _ptr(cu_seqlens), _ptr(slots), slots.numel(), H, d, value_dim, T,
-                                      *_walk_args(work), _stream()), "bonus_state_scan", launches=_walk_launches(work, slots.numel()))
+                                      *_walk_args(work, longest), _stream()), "bonus_state_scan", launches=_walk_launches(work, slots.numel()))
     return out
 
 
@@ -1056,7 +1057,7 @@ def head_decay_delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, dec
     out = _f32((T, H, dv), q.device)
     work = _walk_workspace("lrm_head_decay_delta_scan_floats", blocks, T, longest, q.device, slots.numel(), H, KH, d, dv)
     _done(_lib().lrm_head_decay_delta_scan(_ptr(q), _ptr(k), _ptr(v), _ptr(decay), _ptr(step), _ptr(state), _ptr(out),
-                                           _ptr(cu_seqlens), _ptr(slots), slots.numel(), H, KH, d, dv, T, *_walk_args(work), _stream()),
+                                           _ptr(cu_seqlens), _ptr(slots), slots.numel(), H, KH, d, dv, T, *_walk_args(work, longest), _stream()),
           "head_decay_delta_scan", launches=_walk_launches(work, slots.numel()))
     return out
 

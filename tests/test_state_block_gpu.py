@@ -69,3 +69,16 @@ def test_what_is_not_finite_shows_where_it_does_token_by_token(rule, name, value
         assert not bool(a[~whole].isfinite().any())
     assert torch.equal(got[:16], clean[:16]) and torch.equal(got[130:], clean[130:])
     assert _distance(got[16:token], clean[16:token].double()) <= 2e-6
+
+
+# one long sequence among short ones: on the tensor cores where its CTAs alone fit, whatever the step could hold
+@pytest.mark.parametrize("lengths", [[300] + [1] * 31, [1, 5, 200, 3], [130, 7, 120, 1, 1]])
+@pytest.mark.parametrize("H,d,dv", [(16, 128, 128), (32, 64, 64), (6, 160, 40)])
+@pytest.mark.parametrize("rule", RULES)
+def test_a_long_sequence_among_short_ones(rule, H, d, dv, lengths):
+    x = _inputs(H, H, d, dv, lengths, seed=H + len(lengths))
+    slots = [len(lengths) - i for i in range(len(lengths))]
+    want = _reference(rule, x, lengths, slots)
+    for longest in (max(lengths), 320, None):
+        for a, b in zip(_run(rule, x, lengths, slots, longest=longest), want):
+            assert _distance(a, b) <= 2e-6

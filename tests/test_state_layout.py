@@ -1,0 +1,41 @@
+"""Which way a step's state scans go (csrc/recurrent_block.cuh block_takes_fma): read off the workspace the library asks for."""
+import pytest
+
+WALK, STAGE = 96, 16
+
+
+def _stage_floats(rule, H, d, dv, lengths, longest):
+    """Floats of a stage of 16 tokens, which differ between the tensor cores' blocks and those with FMAs."""
+    from llama_rs_metal_b200.kernels import library
+    lib, tokens = library.load(), sum(lengths)
+    if rule == "bonus":
+        floats = lib.lrm_bonus_state_scan_floats(len(lengths), H, d, dv, tokens, longest)
+    elif rule == "head_delta":
+        floats = lib.lrm_head_decay_delta_scan_floats(len(lengths), H, H, d, dv, tokens, longest)
+    else:
+        floats = lib.lrm_linear_state_scan_floats({"head_decay": 0, "delta": 1, "token_decay": 2}[rule], len(lengths), H, H, d, dv, tokens, longest)
+    stages = tokens // STAGE + len(lengths)
+    assert floats > 0 and floats % stages == 0
+    return floats // stages
+
+
+# heads whose lone walk fits the SMs; per rule, among them heads beyond 128
+HEADS = [("delta", 8, 128, 128), ("delta", 16, 128, 128), ("delta", 16, 200, 64), ("head_delta", 16, 128, 128), ("head_delta", 8, 256, 64),
+         ("bonus", 32, 64, 64), ("bonus", 16, 128, 128), ("token_decay", 16, 256, 64), ("head_decay", 16, 129, 64)]
+
+
+@pytest.mark.parametrize("rule,H,d,dv", HEADS)
+@pytest.mark.parametrize("short", [[1] * 31, [1] * 3, [1], [95, 40, 1], [20] * 60])
+def test_a_long_sequence_goes_as_it_does_alone_whatever_stands_beside_it(rule, H, d, dv, short):
+    lone = _stage_floats(rule, H, d, dv, [2048], 2048)
+    assert _stage_floats(rule, H, d, dv, [2048] + short, 2048) == lone
+    assert _stage_floats(rule, H, d, dv, [1] + [2048] + short, 2112) == lone  # a bound of the longest, as padded steps know it
+    if 2048 + sum(short) < (len(short) + 1) * WALK:  # not known: told by the average
+        assert _stage_floats(rule, H, d, dv, [2048] + short, 0) == lone
+
+
+@pytest.mark.parametrize("rule,H,d,dv", HEADS)
+def test_many_long_sequences_go_with_fmas(rule, H, d, dv):
+    lone = _stage_floats(rule, H, d, dv, [2048], 2048)
+    for longest in (256, 0):
+        assert _stage_floats(rule, H, d, dv, [256] * 16, longest) != lone
