@@ -466,8 +466,8 @@ LRM_API int lrm_gemm_bf16_umma_experts(const void* X, const void* W, void* out, 
 
 // The first product of a prompt's sorted experts with the gate in its epilogue: out bfloat16 [M, ff] = weights[rows[m]] *
 // act(x . gate_e^T, x . up_e^T), 0 where rows[m] < 0; W [w_height, K] holds 2 ff rows per expert (gate, then up). K and ff
-// multiples of 64. Against the product in float32 and the gate in a launch of its own: the same bits without 8 ff bytes
-// written and read per row.
+// multiples of 64. Against the product in float32 and the gate in a launch of its own: the same bits (but for gates below -80,
+// silu.cuh) without 8 ff bytes written and read per row.
 LRM_API int lrm_gemm_bf16_umma_experts_gated(const void* X, const void* W, void* out, int M, int ff, int K, long long w_height,
                                              const int* tile_experts, const int* rows, const float* weights, float limit,
                                              float alpha, int act, int* status, cudaStream_t stream) {

@@ -4,8 +4,8 @@
 //   sort     the (token, choice) pairs in the order of their experts, each expert's on whole tiles of 128 rows
 //   gather   x of every row's token
 //   gate     y = weight(t, c) * act(gate, up) in the products' float32, rounded to bfloat16 as on the way over all
-//            experts (moe.cu): in the first product's epilogue; the launch below makes the same bits and is what tests
-//            compare with. 1,500 tokens, 2 of 8 experts of 2048 x 1024: product and gate 38 us (38 + 7 in two launches,
+//            experts (moe.cu): in the first product's epilogue; the launch below makes the same bits (but for gates below -80,
+//            silu.cuh) and is what tests compare with. 1,500 tokens, 2 of 8 experts of 2048 x 1024: product and gate 38 us (38 + 7 in two launches,
 //            and 29 MB of float32 less to write and read)
 //   combine  out[t] (+)= sum over a token's choices in their order
 //
