@@ -10,6 +10,9 @@
 // meanwhile. Bound by a CTA's chain of blocks. The 1B shape in float32, us: a prompt of 333 tokens 62 (160 key by key, each of which
 // waited for the sum of its dot product over the warp), a decode step of two layers with 3,000 keys, four sequences, 593 (6,287),
 // 300 tokens onto 1,000 1,207 (7,570). 32 rows a CTA 509 a layer's prompt against 495, 8 rows 494 and 1,247 for the portion.
+// Heads that share no keys, a query per sequence, us, in brackets key by key, then four and sixteen sequences to a CTA one after
+// another: 256 of 300 keys, 16 heads of 128 322 (339, 352, 774), 32 heads of 64 336 (625, 324, 762); 128 of 500 283 (522, 285, 1,146)
+// and 266 (530, 330, 612); four of 3,000 keys 316 (2,929, 1,204) and 195 (2,903, 750).
 //
 // It is the attention of the float32 path for prompts and for decoding, and
 // the bfloat16 path's fallback for sizes its tiled kernels refuse (head sizes up to 1024). The two
@@ -167,7 +170,8 @@ struct RowsArgs {
   int queries, q_heads, kv_heads, d, dv, page_size, table_stride, window, temp_every, v_stride;
   float scale, out_scale, temp_coef;
   const float *slopes, *sinks;
-  int aligned;  // rows of q, k and v begin on four elements
+  int aligned;    // rows of q, k and v begin on four elements
+  int per_query;  // CTAs of a query and key/value head where no two queries share a sequence; 0: a CTA's rows run on over queries
 };
 
 template <typename A>
@@ -202,7 +206,9 @@ __global__ __launch_bounds__(WARPS * 32) void attention_rows_kernel(const RowsAr
   float(*vs)[DP] = reinterpret_cast<float(*)[DP]>(rows_smem + ROWS * DP + kKeys * KP);
   float(*ps)[kKeys] = reinterpret_cast<float(*)[kKeys]>(rows_smem + ROWS * DP + kKeys * KP + kKeys * DP);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kh = blockIdx.y, group = a.q_heads / a.kv_heads;
-  const int row0 = static_cast<int>(gridDim.x - 1 - blockIdx.x) * ROWS, count = min(ROWS, a.queries * group - row0);
+  const int block_at = static_cast<int>(gridDim.x - 1 - blockIdx.x), of_query = a.per_query > 0 ? block_at % a.per_query * ROWS : 0;
+  const int row0 = a.per_query > 0 ? block_at / a.per_query * group + of_query : block_at * ROWS;
+  const int count = min(ROWS, a.per_query > 0 ? group - of_query : a.queries * group - row0);
   const bool aligned = a.aligned != 0;
 
   // Lane r of every warp knows row r: its sequence, position and first key.
@@ -349,15 +355,19 @@ int launch_rows(const RowsArgs& a, cudaStream_t stream) {
     if (e != cudaSuccess) return static_cast<int>(e);
   }
   const long long rows = static_cast<long long>(a.queries) * (a.q_heads / a.kv_heads);
-  attention_rows_kernel<A, DP, RW, WARPS, PAGED><<<dim3(static_cast<unsigned>((rows + ROWS - 1) / ROWS), a.kv_heads), WARPS * 32, bytes, stream>>>(a);
+  const long long ctas = a.per_query > 0 ? static_cast<long long>(a.queries) * a.per_query : (rows + ROWS - 1) / ROWS;
+  attention_rows_kernel<A, DP, RW, WARPS, PAGED><<<dim3(static_cast<unsigned>(ctas), a.kv_heads), WARPS * 32, bytes, stream>>>(a);
   LRM_LAUNCH_CHECK();
   return 0;
 }
 
-// 16 rows a CTA for prompts, which share their keys; 4 where a query is its sequence's only one, or few may be.
+// 16 rows a CTA for prompts, which share their keys; 4 where few may, and no two sequences in a CTA where every query is its
+// sequence's only one: a CTA goes through its sequences one after another.
 template <typename A, bool PAGED>
-int dispatch_rows(const RowsArgs& a, cudaStream_t stream) {
-  const bool many = PAGED ? a.positions != nullptr && a.queries >= 128 : true;
+int dispatch_rows(RowsArgs a, int seqs, cudaStream_t stream) {
+  const int group = a.q_heads / a.kv_heads;
+  if (PAGED && seqs == a.queries) a.per_query = (group + 3) / 4;
+  const bool many = PAGED ? a.queries >= 128 && a.per_query == 0 && static_cast<long long>(a.queries) * group >= 4ll * seqs : true;
   if (a.d <= 64 && a.dv <= 64)
     return many ? launch_rows<A, 64, 2, 8, PAGED>(a, stream) : launch_rows<A, 64, 1, 4, PAGED>(a, stream);
   return many ? launch_rows<A, 128, 2, 8, PAGED>(a, stream) : launch_rows<A, 128, 1, 4, PAGED>(a, stream);
@@ -388,10 +398,10 @@ LRM_API int lrm_attention_packed_rowwise(const void* q, const void* k, const voi
   const int widest = d > dv ? d : dv;
   if (widest <= kBlocked) {
     RowsArgs a{q, k, v, out, cu_seqlens, seq_of_token, nullptr, nullptr, nullptr, nullptr, tokens, q_heads, kv_heads, d, dv, 1, 0, window,
-               temp_every, v_stride, scale, out_scale, temp_coef, slopes, sinks, 0};
+               temp_every, v_stride, scale, out_scale, temp_coef, slopes, sinks, 0, 0};
     a.aligned = rows_alignment(a, dtype);
-    return dtype == LRM_F32    ? dispatch_rows<float, false>(a, stream)
-           : dtype == LRM_BF16 ? dispatch_rows<__nv_bfloat16, false>(a, stream)
+    return dtype == LRM_F32    ? dispatch_rows<float, false>(a, 0, stream)
+           : dtype == LRM_BF16 ? dispatch_rows<__nv_bfloat16, false>(a, 0, stream)
                                : LRM_BAD_ARGUMENT;
   }
 #define LRM_PACKED(AT, PER)                                                                                      \
@@ -418,7 +428,7 @@ LRM_API int lrm_attention_packed_rowwise(const void* q, const void* k, const voi
 
 // `queries` rows of q. With seq_of_token and positions (int32 [queries]) query t belongs to
 // sequence seq_of_token[t] and sees keys up to positions[t]; with both null there is one query
-// per sequence, at position kv_lens[b] - 1.
+// per sequence, at position kv_lens[b] - 1. `seqs`: sequences that bring queries (for the layout).
 LRM_API int lrm_attention_paged_rowwise(const void* q, const void* k_pages, const void* v_pages,
                                         void* out, int dtype, const int* page_table,
                                         int table_stride, const int* slots, const int* kv_lens,
@@ -426,9 +436,10 @@ LRM_API int lrm_attention_paged_rowwise(const void* q, const void* k_pages, cons
                                         int queries, int q_heads, int kv_heads, int d, int dv,
                                         int page_size, float scale, int window, const float* slopes,
                                         float out_scale, const float* sinks, float temp_coef,
-                                        int temp_every, int v_stride, cudaStream_t stream) {
+                                        int temp_every, int v_stride, int seqs, cudaStream_t stream) {
   if (queries <= 0) return 0;
   if (v_stride <= 0) v_stride = dv;
+  if (positions == nullptr) seqs = queries;
   if (bad_geometry(q_heads, kv_heads, d, dv) || page_size <= 0) return LRM_BAD_ARGUMENT;
   if ((seq_of_token == nullptr) != (positions == nullptr)) return LRM_BAD_ARGUMENT;
   if (positions == nullptr && kv_lens == nullptr) return LRM_BAD_ARGUMENT;
@@ -437,10 +448,10 @@ LRM_API int lrm_attention_paged_rowwise(const void* q, const void* k_pages, cons
   const int widest = d > dv ? d : dv;
   if (widest <= kBlocked) {
     RowsArgs a{q, k_pages, v_pages, out, nullptr, seq_of_token, page_table, slots, kv_lens, positions, queries, q_heads, kv_heads, d, dv,
-               page_size, table_stride, window, temp_every, v_stride, scale, out_scale, temp_coef, slopes, sinks, 0};
+               page_size, table_stride, window, temp_every, v_stride, scale, out_scale, temp_coef, slopes, sinks, 0, 0};
     a.aligned = rows_alignment(a, dtype);
-    return dtype == LRM_F32    ? dispatch_rows<float, true>(a, stream)
-           : dtype == LRM_BF16 ? dispatch_rows<__nv_bfloat16, true>(a, stream)
+    return dtype == LRM_F32    ? dispatch_rows<float, true>(a, seqs, stream)
+           : dtype == LRM_BF16 ? dispatch_rows<__nv_bfloat16, true>(a, seqs, stream)
                                : LRM_BAD_ARGUMENT;
   }
 #define LRM_PAGED(AT, PER)                                                                                       \

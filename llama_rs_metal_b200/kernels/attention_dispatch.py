@@ -233,7 +233,7 @@ def decode(q, kv, out, slots, kv_lens, max_kv_len: int, scale: float, window: in
                                           _ptr(kv_lens), None, None, B, Hq, kv.kv_heads, d, dv, kv.page_size,
                                           ctypes.c_float(scale), window, _ptr(slopes),
                                           ctypes.c_float(out_scale), *extras.arguments(), _value_stride(kv),
-                                          _stream()),
+                                          B, _stream()),
           "attention_paged_rowwise")
 
 
@@ -310,7 +310,7 @@ def extend(q, kv, out, cu_seqlens, seq_of_token, positions, slots, kv_lens, max_
                                           _ptr(kv_lens), _ptr(seq_of_token), _ptr(positions), T, Hq,
                                           kv.kv_heads, d, dv, kv.page_size, ctypes.c_float(scale), window,
                                           _ptr(slopes), ctypes.c_float(out_scale), *extras.arguments(),
-                                          _value_stride(kv), _stream()),
+                                          _value_stride(kv), cu_seqlens.numel() - 1, _stream()),
           "attention_paged_rowwise")
 
 
