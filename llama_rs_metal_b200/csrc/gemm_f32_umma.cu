@@ -18,7 +18,8 @@
 // else is in the batch.
 //
 // Both operands count 2^16 fold, so that parts of the smallest numbers are not lost, and the result is brought back. A row with a
-// number of 2^40 or more, an infinity or a NaN is marked, and the elements of marked rows are added once more with float32 FMAs.
+// number of 2^40 or more or an infinity in a slice of K is marked for that slice, and its elements' sums over the slice are added once
+// more with float32 FMAs.
 //
 // Bound by the chain of a block: 0.85 us with few rows (5.1 TB/s of weights), 1.1 with 112 of X a tile, of which the 24 products take
 // 0.75; and by 6 us of start-up and drain a CTA. us, in brackets gemm_f32.cu's kernels: 1 row, 3072 x 2048 11.6 (24.8), 16384 x 2048
@@ -102,24 +103,29 @@ __device__ __noinline__ float add_fma(const float* x, const float* w, int begin,
   return sum;
 }
 
-// X [rows, K] cut ahead: parts [3][rows][K], and which rows are marked. A CTA per row.
-__global__ __launch_bounds__(256) void cut_rows_kernel(const float* X, uint2* __restrict__ parts, int* __restrict__ marks, int rows, int K) {
+// X [rows, K] cut ahead: parts [3][rows][K], and for which slices of `of_slice` numbers a row is marked, a bit each. A CTA per row.
+__global__ __launch_bounds__(256) void cut_rows_kernel(const float* X, uint2* __restrict__ parts, int* __restrict__ marks, int rows, int K,
+                                                       int of_slice) {
+  __shared__ int marked;
   pdl_trigger();
+  if (threadIdx.x == 0) marked = 0;
+  __syncthreads();
   pdl_wait();
   const int row = blockIdx.x;
   const float4* from = reinterpret_cast<const float4*>(X + static_cast<size_t>(row) * K);
   const size_t plane = static_cast<size_t>(rows) * (K / 4);
-  float most = 0.f;
 #pragma unroll 4
   for (int i = threadIdx.x; i < K / 4; i += 256) {
     const float4 x = from[i];
+    float most = 0.f;
     uint2 part[3];
     cut2(x.x, x.y, part[0].x, part[1].x, part[2].x, most);
     cut2(x.z, x.w, part[0].y, part[1].y, part[2].y, most);
 #pragma unroll
     for (int p = 0; p < 3; ++p) parts[p * plane + static_cast<size_t>(row) * (K / 4) + i] = part[p];
+    if (most >= kTooLarge) atomicOr(&marked, 1 << (4 * i / of_slice));
   }
-  const int marked = __syncthreads_or(most >= kTooLarge);
+  __syncthreads();
   if (threadIdx.x == 0) marks[row] = marked;
 }
 
@@ -174,7 +180,7 @@ __global__ __launch_bounds__(Cut<MAXC, RAW, AHEAD, WW>::THREADS, 1) void gemm_f3
   pdl_wait();
   if (AHEAD && warp == 3)
     for (int i = lane; i < columns; i += 32)
-      if (m0 + i < M && marks[x_row0 + i]) marked[kRows + i] = *any_marked = 1;
+      if (m0 + i < M && (marks[x_row0 + i] >> slice & 1)) marked[kRows + i] = *any_marked = 1;
   auto all_meet = []() { asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory"); };
 
   if (warp == kLoader) {
@@ -428,7 +434,7 @@ int launch(const float* X, const float* W, float* C, int M, int N, int K, int mo
   if (e != cudaSuccess) return static_cast<int>(e);
   if (AHEAD)
     LRM_LAUNCH(cut_rows_kernel, dim3(static_cast<unsigned>(x_rows)), 256, 0, stream, X, static_cast<uint2*>(parts), marks,
-               static_cast<int>(x_rows), K);
+               static_cast<int>(x_rows), K, ((K + BK - 1) / BK + slices - 1) / slices * BK);
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(static_cast<unsigned>(items));
   config.blockDim = dim3(T::THREADS);

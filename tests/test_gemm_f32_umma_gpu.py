@@ -70,6 +70,21 @@ def test_numbers_out_of_the_parts_range(M):
     assert bool(((got.double() - want).abs() <= bound)[whole].all())
 
 
+# slices of K: 4, 2, 1; numbers beyond the range in the first slice, in the last and in two, where the weights are zero or not
+@pytest.mark.parametrize("N,K", [(1000, 2056), (512, 1024), (12416, 1088)])
+def test_a_row_out_of_range_does_not_depend_on_the_batch(N, K):
+    from llama_rs_metal_b200.kernels import ops
+    x, w = _randn(140, K, seed=3), _randn(N, K, seed=4)
+    x[0, 5] = x[1, K - 3] = x[2, 9] = x[2, K // 2 + 40] = 2.0 ** 41
+    x[3, 70] = float("inf")
+    w[::2, 5] = w[::2, K - 3] = w[::2, 9] = 0.0
+    w[7, K - 1] = 2.0 ** 50
+    got = ops.linear(x, w)
+    for rows in (1, 5, 20, 33):
+        few = ops.linear(x[:rows].contiguous(), w)
+        assert torch.equal(few.isnan(), got[:rows].isnan()) and torch.equal(few.nan_to_num(), got[:rows].nan_to_num())
+
+
 def test_rows_off_16_bytes_go_to_the_other_kernels():
     from llama_rs_metal_b200.kernels import ops
     room = torch.empty(9 * 1024 + 1, device=DEV)
