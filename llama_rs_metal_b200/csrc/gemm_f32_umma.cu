@@ -18,7 +18,7 @@
 // else is in the batch.
 //
 // Both operands count 2^16 fold, so that parts of the smallest numbers are not lost, and the result is brought back. A row with a
-// number of 2^40 or more or an infinity in a slice of K is marked for that slice, and its elements' sums over the slice are added once
+// number of 2^32 or more or an infinity in a slice of K is marked for that slice, and its elements' sums over the slice are added once
 // more with float32 FMAs.
 //
 // Bound by the chain of a block: 0.85 us with few rows (5.1 TB/s of weights), 1.1 with 112 of X a tile, of which the 24 products take
@@ -62,7 +62,7 @@ __device__ __forceinline__ void cut2(float x, float y, uint32_t& high, uint32_t&
   const float sa = ra - __uint_as_float(middle << 16), sb = rb - __uint_as_float(middle & 0xffff0000u);
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(low) : "f"(sb), "f"(sa));
 }
-constexpr float kTooLarge = 72057594037927936.f;  // 2^40 2^16: from here a product of two, K times over, could leave the range
+constexpr float kTooLarge = 281474976710656.f;  // 2^32 2^16: products of smaller ones are below 2^96 and no sum over K leaves the range
 
 // A bounded wait that also ends when another role of the CTA has given up.
 __device__ __forceinline__ bool wait_or_bail(uint64_t* bar, uint32_t parity, int* status, int where, volatile int* bail) {

@@ -49,7 +49,7 @@ def test_grouped_inputs_match_single_ones(T):
 
 @pytest.mark.parametrize("M", [20, 140])
 def test_numbers_out_of_the_parts_range(M):
-    """Infinities, NaNs and numbers of 2^40 and more are added with float32 FMAs, in their row and column alone; the smallest numbers
+    """Infinities, NaNs and numbers of 2^32 and more are added with float32 FMAs, in their row and column alone; the smallest numbers
     keep their bits."""
     from llama_rs_metal_b200.kernels import ops
     x, w = _randn(M, 1024), _randn(640, 1024, seed=1)
@@ -83,6 +83,15 @@ def test_a_row_out_of_range_does_not_depend_on_the_batch(N, K):
     for rows in (1, 5, 20, 33):
         few = ops.linear(x[:rows].contiguous(), w)
         assert torch.equal(few.isnan(), got[:rows].isnan()) and torch.equal(few.nan_to_num(), got[:rows].nan_to_num())
+
+
+def test_long_sums_of_large_numbers_stay_in_range():
+    """Numbers below 2^40 whose products, brought back, float32 holds, over so long a K in one slice that the sum of the scaled ones was infinite."""
+    from llama_rs_metal_b200.kernels import ops
+    N, K, number = 12288, 81920, 2.0 ** 39.9
+    got = ops.linear(torch.full((2, K), number, device=DEV), torch.full((1, 1), number, device=DEV).expand(N, K).contiguous())
+    want = K * torch.tensor(number).double().item() ** 2
+    assert bool(((got.double() - want).abs() <= K * 2.0 ** -24 * want).all())  # a rounding per FMA
 
 
 def test_rows_off_16_bytes_go_to_the_other_kernels():
