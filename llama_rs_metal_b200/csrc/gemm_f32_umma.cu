@@ -1,18 +1,22 @@
 // float32 matrix product on the 5th-generation tensor cores: C[M,N] = X[M,K] . W[N,K]^T, for the larger matrices
-// (gemm_dispatch.f32_takes_umma). Every float32 number is cut into three bfloat16 parts of 8 bits, which hold all of it, and six of
-// the nine products of parts are added: what is left out is at most 2^-22 of a product, of either sign.
+// (gemm_dispatch.f32_takes_umma). Every float32 number is cut into three bfloat16 parts, each rounded, which hold all of it, and eight of
+// the nine products of parts are added: the one left out is below 2^-34 of a product.
 //
 // The tensor core truncates where it adds (measured: to 2^-23 of the sum), with a bias towards zero that grows with the terms: 1.2e-7
-// after 128, 2e-6 after 2,048. So an accumulator runs over 64 of K only, from zero, the small products ahead of the large one, and
-// the sums over K are float32 additions on the CUDA cores. Distance from 64 bits, relative, normal numbers: 1.1e-7 at K 2,048 and 1.4e-7 at 8,192; float32 FMAs in ascending order 8.1e-7 and 1.6e-6.
+// after 128, 2e-6 after 2,048. So the large products (of the first parts, 16 bits each) are added over 64 of K only, from zero, and the
+// sums over K are float32 additions on the CUDA cores. The seven small ones have an accumulator of their own, over all of K, whose
+// truncation is 2^-8 of that, and are added once, at the end. So a single product is rounded as a float32 FMA rounds it, and sums of
+// any number of terms are no further off than with FMAs in ascending order. Distance from 64 bits, relative, normal numbers, rows with
+// n of them (FMAs): 1 2.5e-8 (2.5e-8), 2 2.5e-8 (3.1e-8), 16 3.3e-8 (7.3e-8), 2,048 9.9e-8 (8.1e-7), 8,192 1.4e-7 (1.6e-6). (Six products,
+// the first part cut off, all in one accumulator: 5.5e-8, 6.2e-8, 7.9e-8, 1.1e-7, 1.4e-7.)
 //
 // A tile of 128 weight rows is the A operand; the rows of X, in equal tiles of up to 128, are its columns. One thread brings the
 // weights' blocks of 64 of K to shared memory by TMA, as float32. Eight or sixteen warps cut them, a row a lane, and put the parts into tensor
-// memory (A from there leaves shared memory, which bounds this kernel, to the other operand). X's parts lie in shared memory in the
+// memory (A from there leaves shared memory to the other operand). X's parts lie in shared memory in the
 // swizzled layout of the instruction: up to 32 rows are cut there by four more warps; more rows, which many tiles share, have been cut by
-// a launch ahead and come by TMA. One warp issues 24 products a block, and four or twelve add a finished accumulator (two in turn) to
-// their registers, a thread per weight row and up to 48 rows of X. A matrix with few tiles is cut along K into slices of a
-// cluster's CTAs, whose sums meet in distributed shared memory, in order.
+// a launch ahead and come by TMA. One warp issues 32 products a block, the four large ones first, and four or twelve warps add those to
+// their registers under the small ones, a thread per weight row and up to 48 rows of X. A matrix with few tiles is cut along K into
+// slices of a cluster's CTAs, whose large and small sums meet in distributed shared memory, in order.
 //
 // An element's blocks and slices follow from N and K alone, so its value does not depend on M, on the tile it falls in, or on what
 // else is in the batch.
@@ -21,11 +25,14 @@
 // number of 2^32 or more or an infinity in a slice of K is marked for that slice, and its elements' sums over the slice are added once
 // more with float32 FMAs.
 //
-// Bound by the chain of a block: 0.85 us with few rows (5.1 TB/s of weights), 1.1 with 112 of X a tile, of which the 24 products take
-// 0.75; and by 6 us of start-up and drain a CTA. us, in brackets gemm_f32.cu's kernels: 1 row, 3072 x 2048 11.6 (24.8), 16384 x 2048
-// 28 (35), 2048 x 8192 28 (94), 128256 x 2048 193 (177; 4 rows 194 and 237); 32 rows 13 (71), 32 (141), 32 (227); 333 rows 46 (127),
-// 118 (592), 76 (500); 512 rows 51 (176), 166 (699), 93 (493). Tried: operands through registers (loads under way share scoreboards, so a use
-// waits for the newest: 16384 x 2048 333 rows 189), the weights' parts in shared memory, three waits of the issuer a block (158).
+// Bound, with many rows, by the tensor pipe: a block's 32 products take 72 cycles each with 112 rows of X a tile (56 by the
+// instruction's size), and 6 us of start-up and drain a CTA beside that; with few rows by the chain of a block, 0.85 us (5.1 TB/s of weights).
+// us, in brackets gemm_f32.cu's kernels: 1 row, 3072 x 2048 12.1 (24.8), 16384 x 2048 28 (36), 2048 x 8192 28 (94), 128256 x 2048 196
+// (175; 4 rows 197 and 240); 32 rows 14 (66), 33 (147), 32 (221); 333 rows 60 (128), 139 (597), 99 (499); 512 rows 68, 202, 113. (With six
+// products 333 rows 46, 115, 77.) Tried, 16384 x 2048, 333 rows: operands through registers (loads under way share scoreboards, so a
+// use waits for the newest) 189 with six products; the large products behind the small ones, with a second wait of the issuer 169
+// against 152; a look at the next barrier ahead of the last eight products 153, of the last sixteen 173; three stages of parts 154; sixteen
+// warps cutting 185.
 //
 // Every wait is bounded (see umma.cuh).
 #include "umma.cuh"
@@ -43,21 +50,20 @@ struct Cut {
   static constexpr uint32_t W_RAW = kRows * BK * 4, X_RAW = AHEAD ? 0 : MAXC * BK * 4, RAW_STAGE = W_RAW + X_RAW;
   static constexpr uint32_t PART = MAXC * BK * 2, STAGE = 3 * PART;
   static constexpr uint32_t AT_PARTS = RAW * RAW_STAGE, AT_BARRIERS = AT_PARTS + 2 * STAGE;
-  static constexpr uint32_t WEIGHTS_AT = 2 * MAXC, COLUMNS = MAXC == 32 ? 256 : 512;  // of tensor memory: accumulators, weights
+  static constexpr uint32_t WEIGHTS_AT = 2 * MAXC, COLUMNS = MAXC == 32 ? 256 : 512;  // of tensor memory: two accumulators, weights
   static constexpr size_t BYTES = 1024 + AT_BARRIERS + 256 + (kRows + MAXC) * sizeof(int);
   static constexpr int CHUNKS = (MAXC / 16 + ADDERS / 4 - 1) / (ADDERS / 4);  // pieces of 16 rows of X that an adding thread has
-  static_assert(WEIGHTS_AT + 2 * 3 * kHeld <= COLUMNS && MAXC * kRows * 4 <= AT_PARTS && BYTES <= 227 * 1024, "room");
+  static_assert(WEIGHTS_AT + 2 * 3 * kHeld <= COLUMNS && 2 * MAXC * kRows * 4 <= AT_PARTS && BYTES <= 227 * 1024, "room");
 };
 
-enum : int { kStuckEmpty = 61, kStuckFull = 62, kStuckAccumulator = 63, kStuckRaw = 64, kStuckDrain = 65, kStuckRawEmpty = 66 };
+enum : int { kStuckEmpty = 61, kStuckFull = 62, kStuckAccumulator = 63, kStuckRaw = 64, kStuckDrain = 65, kStuckRawEmpty = 66, kStuckSmall = 67 };
 
 // Two numbers, 2^16 fold, as three pairs of bfloat16; `most` collects the largest.
 __device__ __forceinline__ void cut2(float x, float y, uint32_t& high, uint32_t& middle, uint32_t& low, float& most) {
   x *= 65536.f, y *= 65536.f;
   most = fmaxf(most, fmaxf(fabsf(x), fabsf(y)));  // (a NaN needs no mark: it is one in every product)
-  const uint32_t a = __float_as_uint(x), b = __float_as_uint(y);
-  high = __byte_perm(a, b, 0x7632);
-  const float ra = x - __uint_as_float(a & 0xffff0000u), rb = y - __uint_as_float(b & 0xffff0000u);
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(high) : "f"(y), "f"(x));
+  const float ra = x - __uint_as_float(high << 16), rb = y - __uint_as_float(high & 0xffff0000u);
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(middle) : "f"(rb), "f"(ra));
   const float sa = ra - __uint_as_float(middle << 16), sb = rb - __uint_as_float(middle & 0xffff0000u);
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(low) : "f"(sb), "f"(sa));
@@ -143,12 +149,12 @@ __global__ __launch_bounds__(Cut<MAXC, RAW, AHEAD, WW>::THREADS, 1) void gemm_f3
   unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint64_t* raw_full = reinterpret_cast<uint64_t*>(ring + T::AT_BARRIERS);
   uint64_t* raw_empty = raw_full + RAW;
-  // A block's parts are there and its accumulator has been added: one barrier, since a wait costs 200 cycles even when it is over
-  // (behind the shared-memory traffic), and the issuer's are not hidden.
+  // A block's parts are there and the block before's large products have been added: one barrier, since each wait of the issuer
+  // leaves the tensor pipe idle for some 500 cycles.
   uint64_t* full = raw_empty + RAW;      // [2]
-  uint64_t* empty = full + 2;            // [2]
-  uint64_t* acc_full = empty + 2;        // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 2);
+  uint64_t* empty = full + 2;            // [2] a block's products are done with its parts
+  uint64_t* acc_full = empty + 2;        // its large products are in their accumulator
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile int* bail = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* any_marked = reinterpret_cast<int*>(tmem_slot + 2);
   int* marked = reinterpret_cast<int*>(ring + T::AT_BARRIERS + 256);  // [128 rows of W | rows of X]
@@ -162,8 +168,9 @@ __global__ __launch_bounds__(Cut<MAXC, RAW, AHEAD, WW>::THREADS, 1) void gemm_f3
   if (tid == 0) {
     for (int s = 0; s < RAW; ++s) mbar_init(raw_full + s, 1), mbar_init(raw_empty + s, kWeightWarps + kInputWarps);
     for (int s = 0; s < 2; ++s) {
-      mbar_init(full + s, kWeightWarps + (AHEAD ? 1 : kInputWarps) + kAdders), mbar_init(empty + s, 1), mbar_init(acc_full + s, 1);
+      mbar_init(full + s, kWeightWarps + (AHEAD ? 1 : kInputWarps) + kAdders), mbar_init(empty + s, 1);
     }
+    mbar_init(acc_full, 1);
     *bail = 0;
     *any_marked = 0;
     mbar_fence_init();
@@ -229,16 +236,19 @@ __global__ __launch_bounds__(Cut<MAXC, RAW, AHEAD, WW>::THREADS, 1) void gemm_f3
       const int s = block & 1;
       if (!ready && !__all_sync(0xffffffffu, wait_or_bail(full + s, (block >> 1) & 1, status, kStuckFull, bail))) break;
       tc_fence_after();
-      const uint32_t a = tmem + T::WEIGHTS_AT + s * 3 * kHeld, b = parts_at + s * T::STAGE, d = tmem + s * MAXC;
-      constexpr int of_w[6] = {2, 0, 1, 1, 0, 0}, of_x[6] = {0, 2, 1, 0, 1, 0};  // the small products first
-      if (leader) {
+      const uint32_t a = tmem + T::WEIGHTS_AT + s * 3 * kHeld, b = parts_at + s * T::STAGE;
+      constexpr int kSmall = 7, of_w[kSmall] = {1, 2, 2, 0, 1, 1, 0}, of_x[kSmall] = {2, 1, 0, 2, 1, 0, 1};
+      if (leader) {  // the large products first: they are added under the small ones
 #pragma unroll
-        for (int p = 0; p < 6; ++p)
+        for (int k = 0; k < BK / 16; ++k) umma_bf16_a_tmem(tmem, a + k * 8, smem_desc(b + k * 32), idesc, k > 0 ? 1u : 0u);
+        umma_commit(acc_full);
+#pragma unroll
+        for (int p = 0; p < kSmall; ++p)
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k)
-            umma_bf16_a_tmem(d, a + of_w[p] * kHeld + k * 8, smem_desc(b + of_x[p] * T::PART + k * 32), idesc, p > 0 || k > 0 ? 1u : 0u);
+            umma_bf16_a_tmem(tmem + MAXC, a + of_w[p] * kHeld + k * 8, smem_desc(b + of_x[p] * T::PART + k * 32), idesc,
+                             block > 0 || p > 0 || k > 0 ? 1u : 0u);
         umma_commit(empty + s);
-        umma_commit(acc_full + s);
       }
       __syncwarp();
       ready = block + 1 < blocks && __all_sync(0xffffffffu, mbar_try_wait(full + (s ^ 1), ((block + 1) >> 1) & 1));
@@ -320,12 +330,13 @@ __global__ __launch_bounds__(Cut<MAXC, RAW, AHEAD, WW>::THREADS, 1) void gemm_f3
     for (int i = 0; i < CHUNKS * 16; ++i) acc[i >> 4][i & 15] = 0.f;
     const int quarter = warp & 3, side = (warp - 4 - kWeightWarps - kInputWarps) >> 2;  // lanes of tensor memory, columns
     const int c0 = side * CHUNKS * 16, place = quarter * 32 + lane, n = n0 + place;
-    if (lane == 0) mbar_arrive(full), mbar_arrive(full + 1);  // both accumulators are free
+    constexpr float kBack = 2.3283064365386963e-10f;  // 2^-32
+    float* sums = reinterpret_cast<float*>(ring);       // slices: [columns][128] of the large products, then of the small ones
+    const uint32_t at = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + c0;
+    if (lane == 0) mbar_arrive(full);  // the accumulator is free
     for (int block = 0; block < blocks; ++block) {
-      const int s = block & 1;
-      if (!wait_or_bail(acc_full + s, (block >> 1) & 1, status, kStuckAccumulator, bail)) break;
+      if (!wait_or_bail(acc_full, block & 1, status, kStuckAccumulator, bail)) break;
       tc_fence_after();
-      const uint32_t at = tmem + s * MAXC + (static_cast<uint32_t>(quarter * 32) << 16) + c0;
 #pragma unroll
       for (int i = 0; i < CHUNKS; ++i) {
         if (c0 + i * 16 >= columns) break;
@@ -336,18 +347,34 @@ __global__ __launch_bounds__(Cut<MAXC, RAW, AHEAD, WW>::THREADS, 1) void gemm_f3
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(full + s);
+      if (lane == 0) mbar_arrive(full + ((block + 1) & 1));
+    }
+    if (wait_or_bail(empty + ((blocks - 1) & 1), ((blocks - 1) >> 1) & 1, status, kStuckSmall, bail)) {  // (every block has been read)
+      tc_fence_after();
+#pragma unroll
+      for (int i = 0; i < CHUNKS; ++i) {
+        if (c0 + i * 16 >= columns) break;
+        uint32_t r[16];
+        tmem_load16(at + MAXC + i * 16, r);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          if (slices == 1) acc[i][j] += __uint_as_float(r[j]);
+          else sums[(MAXC + c0 + i * 16 + j) * kRows + place] = __uint_as_float(r[j]) * kBack;
+        }
+      }
     }
     all_meet();  // all marks are made
 #pragma unroll
-    for (int i = 0; i < CHUNKS * 16; ++i) acc[i >> 4][i & 15] *= 2.3283064365386963e-10f;  // 2^-32
+    for (int i = 0; i < CHUNKS * 16; ++i) acc[i >> 4][i & 15] *= kBack;
     if (*any_marked && n < N) {
       const int k_end = min(K, (first + blocks) * BK);
 #pragma unroll
       for (int i = 0; i < CHUNKS * 16; ++i) {
         const int c = c0 + i;
-        if (c < columns && m0 + c < M && (marked[place] || marked[kRows + c]))
+        if (c < columns && m0 + c < M && (marked[place] || marked[kRows + c])) {
           acc[i >> 4][i & 15] = add_fma(X + static_cast<size_t>(x_row0 + c) * K, W + static_cast<size_t>(n) * K, first * BK, k_end);
+          if (slices > 1) sums[(MAXC + c) * kRows + place] = 0.f;
+        }
       }
     }
     if (slices == 1) {
@@ -362,7 +389,6 @@ __global__ __launch_bounds__(Cut<MAXC, RAW, AHEAD, WW>::THREADS, 1) void gemm_f3
         }
       }
     } else {
-      float* sums = reinterpret_cast<float*>(ring);  // [columns][128]: every block has been read
 #pragma unroll
       for (int i = 0; i < CHUNKS * 16; ++i)
         if (c0 + i < columns) sums[(c0 + i) * kRows + place] = acc[i >> 4][i & 15];
@@ -376,11 +402,13 @@ __global__ __launch_bounds__(Cut<MAXC, RAW, AHEAD, WW>::THREADS, 1) void gemm_f3
   const bool wide = N % 4 == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0;
   for (int i = tid; i < (rows - static_cast<int>(rank) + slices - 1) / slices * (kRows / 4); i += kThreads) {  // rows rank, rank + slices, ...
     const int c = static_cast<int>(rank) + i / (kRows / 4) * slices, col = i % (kRows / 4) * 4;
-    float4 v = load_from_rank(smem_u32(sums + c * kRows + col), 0);
+    float4 v = load_from_rank(smem_u32(sums + c * kRows + col), 0), small = load_from_rank(smem_u32(sums + (MAXC + c) * kRows + col), 0);
     for (int s = 1; s < slices; ++s) {
-      const float4 more = load_from_rank(smem_u32(sums + c * kRows + col), s);
+      const float4 more = load_from_rank(smem_u32(sums + c * kRows + col), s), less = load_from_rank(smem_u32(sums + (MAXC + c) * kRows + col), s);
       v.x += more.x, v.y += more.y, v.z += more.z, v.w += more.w;
+      small.x += less.x, small.y += less.y, small.z += less.z, small.w += less.w;
     }
+    v.x += small.x, v.y += small.y, v.z += small.z, v.w += small.w;
     float* to = C + static_cast<size_t>(m0 + c) * N + n0 + col;
     const float out[4] = {v.x, v.y, v.z, v.w};
     if (wide && n0 + col < N) {

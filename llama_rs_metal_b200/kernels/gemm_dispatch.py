@@ -74,7 +74,7 @@ def check_status() -> None:
             names.update({51: "a free stage", 52: "operand tiles", 53: "the accumulator", 54: "copies in flight",
                           55: "a free accumulator"})
             names.update({61: "a free stage", 62: "operand parts", 63: "the accumulator", 64: "operand tiles", 65: "copies in flight",
-                          66: "a free tile"})
+                          66: "a free tile", 67: "the small products"})
             kernel = "gemm_f32_umma" if code >= 61 else "gemm_bf16_few" if code >= 51 else "attention_gated_umma" if code >= 41 else "gemm_bf16_umma_pair" \
                 if code >= 31 else "attention_prefill_pingpong" if code >= 21 else "gemm_bf16_umma"
             raise LlamaError(f"{kernel} gave up waiting for {names.get(code, code)}; its result is invalid")
@@ -361,9 +361,8 @@ def gemm_bf16(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, mode: in
 def f32_takes_umma(N: int, K: int) -> bool:
     """Whether a float32 product goes to the tensor cores in three-part splits (csrc/gemm_f32_umma.cu) or to the FMA kernels
     (csrc/gemm_f32.cu). A matter of the matrix alone, so that a row gives the same bits however many there are. us for 1, 32 and 333
-    rows, in brackets the FMA kernels: 1024 x 1024 9.3 (12.7), 10.7 (28.8), 14.9 (39.4); 512 x 2048 9.7 (23.9), 11.3 (56.3), 16.6
-    (76.9); 2048 x 512, below the line, 9.1 (6.9), 9.7 (15.3), 21.0 (32.7). Of larger matrices a single row of 128256 x 2048 alone is slower
-    (193 against 177). Rows on 32 bytes (K a multiple of 8), as the parts' copies want them."""
+    rows, in brackets the FMA kernels: 1024 x 1024 9.9 (12.7), 11.1 (28.7), 18.2 (40.0); 512 x 2048 9.9 (24.2), 11.6 (56.2), 21.0
+    (76.2). Of larger matrices a single row of 128256 x 2048 alone is slower (196 against 175; 4 rows 197 against 240). Rows on 32 bytes (K a multiple of 8), as the parts' copies want them."""
     return K % 8 == 0 and K >= 1024 and N >= 512
 
 

@@ -15,8 +15,8 @@ def _randn(*shape, seed=0):
 
 
 def _bound(x, w):
-    """Left-out products 2^-22 of the numbers' (2^-7 2^-16 twice), four large truncated additions a block at 2^-22 each, and a rounding
-    of 2^-24 for each of the K / 64 additions between blocks."""
+    """Four large truncated additions a block at 2^-22 each, as many times seven of the small products at 2^-7 of that (over all blocks,
+    in the K 2^-30), and a rounding of 2^-24 for each of the K / 64 additions between blocks."""
     K = x.shape[1]
     return (5 * 2.0 ** -22 + K * 2.0 ** -30) * (x.double().abs() @ w.double().abs().T)
 
@@ -92,6 +92,25 @@ def test_long_sums_of_large_numbers_stay_in_range():
     got = ops.linear(torch.full((2, K), number, device=DEV), torch.full((1, 1), number, device=DEV).expand(N, K).contiguous())
     want = K * torch.tensor(number).double().item() ** 2
     assert bool(((got.double() - want).abs() <= K * 2.0 ** -24 * want).all())  # a rounding per FMA
+
+
+# one slice of K, two and four; rows cut in the kernel and ahead of it
+@pytest.mark.parametrize("N,K", [(12416, 2048), (1537, 1088), (512, 2048), (600, 8192)])
+@pytest.mark.parametrize("M", [30, 140])
+@pytest.mark.parametrize("numbers", [1, 2, 3, 4, 8, 20, None])
+def test_rows_of_few_numbers_are_no_further_off_than_with_fmas(monkeypatch, M, N, K, numbers):
+    from llama_rs_metal_b200.kernels import gemm_dispatch, ops
+    gen = torch.Generator(device=DEV).manual_seed(K + N)
+    x, w = _randn(M, K, seed=5), _randn(N, K, seed=6)
+    if numbers is not None:
+        x *= torch.rand((M, K), generator=gen, device=DEV).argsort(1) < numbers
+    want, got = x.double() @ w.double().T, ops.linear(x, w)
+    monkeypatch.setattr(gemm_dispatch, "force_tiled", True)
+    other = ops.linear(x, w)
+    off, other_off = float((got.double() - want).norm()), float((other.double() - want).norm())
+    assert off <= 1.02 * other_off  # (the spread of so many roundings' sum is under 1 %)
+    if numbers == 1:  # one rounding, the three low products left out (2^-34) and the small ones' truncated sum (2^-31)
+        assert bool(((got.double() - want).abs() <= (2.0 ** -24 + 2.0 ** -30) * want.abs()).all())
 
 
 def test_rows_off_16_bytes_go_to_the_other_kernels():
