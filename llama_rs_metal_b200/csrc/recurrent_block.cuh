@@ -14,12 +14,14 @@
 // In the walk the rules with a delta use p'_j = sum_i (T k G)_ji S_i, u = T v - p', and the read-outs o = D T v + (q G - D T k G) S,
 // so that nothing waits for T or D; the others o = D v + q G S.
 //
-// Precision: the sums over i and m are bfloat16 products of float32 numbers cut into three parts of 8 bits, which hold every
-// bit; of the nine products the three below 2^-24 are left out. The tensor core cuts sums off where it should round (measured:
+// Precision: the sums over i and m are bfloat16 products of float32 numbers cut into three parts, each rounded, which hold every bit;
+// of the nine products the lowest, below 2^-34, is left out. The tensor core cuts sums off where it should round (measured:
 // at 2^-23 of the largest term, up to 2^-25 of it kept within a product), so each runs over at most 64 terms from zero, the
 // small products apart from the large ones; what is longer than that, the state itself first of all, is added in float32 on the
-// CUDA cores. Distance from 64 bits, relative, over 2,048 tokens of the shapes below (float32 FMAs, blocks of 8 or 4, in
-// brackets): delta rule 1.8e-7 to 2.1e-7 (1.9e-7 to 2.2e-7), a decay per token 1.4e-7 to 1.6e-7 (2.1e-7 to 2.4e-7).
+// CUDA cores. A read of one number is rounded once, as an FMA is. Distance from 64 bits, relative, read-outs and state, 16 heads of
+// 128 x 128 that forget at 1e-3 to 0.3 a token (in brackets float32 FMAs, blocks of 8 or 4): delta rule, 96 tokens 1.4e-7 and
+// 1.3e-7 (1.5e-7, 1.4e-7), 1,500 2.0e-7 and 1.9e-7 (2.1e-7, 2.0e-7); a decay per token 1.1e-7 and 6.6e-8 (1.2e-7, 9.3e-8), 1.3e-7 and 1.1e-7
+// (2.0e-7, 2.0e-7); of these the states of the heads that forget the fastest 7.3e-8 (6.5e-8) and 5.5e-8 (4.8e-8): few terms, cut off.
 //
 // Two launches (behind one for a step's sequences that go token by token). What does not depend on the column is made first,
 // for all blocks at once, into a workspace, cut into its parts: the vectors T k G, q G - D T k G (or q G), k (G_L / G_m) and G_L
@@ -31,16 +33,18 @@
 // warps' shares of p' meet in shared memory, once a block. Four more warps bring the stages and make the read-outs from the
 // state's parts, off the chain.
 //
-// What bounds it: the chain of a block (cut the state, p', its exchange, cut u, the update) is 1.05 us under a delta rule and
-// 0.8 us without, with a CTA of eight warps per SM; the tensor pipe is 31 % busy, the shared-memory pipe some 55 %. us, in
-// brackets float32 FMAs in blocks of 8 or 4 tokens: delta rule, 16 heads of 128 x 128, 2,048 tokens 187 (262), 8 heads 163 (231),
-// 16 heads of 64 x 64 137 (229); a decay per token 136 (203), 133 (168), 94 (160); 32 heads of 128 x 64, 1,500 and 777 tokens 131
-// (187). One sequence of 96 tokens is within 1 us of the FMAs on both rules (17 and 18 us, 16 heads of 128 x 128), 256 29 (37).
+// What bounds it: the chain of a block (cut the state, p', its exchange, cut u, the update) is 1.15 us under a delta rule and
+// 0.87 us without, with a CTA of eight warps per SM; the tensor pipe is 38 % busy meanwhile (profiles/state_block_scan_2048.md). us, in
+// brackets float32 FMAs in blocks of 8 or 4 tokens: delta rule, 16 heads of 128 x 128, 2,048 tokens 200 (262), 8 heads 175 (231),
+// 16 heads of 64 x 64 148 (229); a decay per token 146 (203), 143 (168), 100 (160); 32 heads of 128 x 64, 1,500 and 777 tokens 145
+// (187). One sequence of 96 tokens is within 2 us of the FMAs on both rules (16 heads of 128 x 128), 256 8 us below. (With six products
+// of parts cut off, less exact for reads of few numbers: 187, 163, 137; 136, 133, 94; 131.)
 // The shares as a second product of all eight warps' halves of the rows, and tiles of 32 columns a CTA, gave nothing.
 //
 // Numbers that are not finite: a product with a zero would spread them to tokens ahead of them. They are taken out (zero
 // instead), and the columns of the state that they reach are done once more with float32 FMAs from the token they come with
-// (BlockAgain), so an infinity or a NaN shows where the formulas above let it and nowhere else.
+// (BlockAgain), so an infinity or a NaN shows where the formulas above let it and nowhere else. So do vectors' numbers of 2^24 and more
+// and states' of 2^64, whose products, 2^32 fold, could leave the range.
 //
 // Which sequences walk is each one's own matter, but this way or with FMAs follows the step's size, and with it the order of the
 // sums: the same sequence gives other bits, within float32 rounding, in another step. Who needs the bits goes without a
@@ -61,7 +65,7 @@ struct BlockShape {
   static constexpr int PLANE = L * DP;                       // bfloat16 numbers of a part of a block's vectors
   static constexpr int AT_K = 0, AT_Q = BONUS ? 0 : 1, AT_W = BY_HEAD ? AT_Q + 1 : 0, VECTORS = (BY_HEAD ? AT_W : AT_Q) + 1;
   static constexpr int AT_G = VECTORS * 3 * PLANE / 2, STAGE = AT_G + (ROW_DECAY ? DP : 0);  // in floats
-  // numbers of a block and head: G_j [L] | G_L, what its rounding lost, whether all numbers are finite
+  // numbers of a block and head: G_j [L] | G_L, what its rounding lost, whether a vector's number is out of range
   static constexpr int AT_ALL = L, AT_BAD = AT_ALL + 2, SCALARS = AT_ALL + 4;
   // and of a tile of columns, each in the order of block_lane_at: what the tokens write but for what they read of the state |
   // what their read-outs are but for that
@@ -69,27 +73,35 @@ struct BlockShape {
   static_assert(STAGE % 4 == 0 && SCALARS % 4 == 0, "pieces of 16 bytes");
 };
 
-// Two finite numbers as the sums of three pairs of bfloat16 (8 bits each, the first cut off, so that it does not overflow):
-// parts[0] + parts[1] + parts[2] is exact but for what lies below bfloat16's smallest number.
+// Numbers are cut 2^16 fold, so that parts of the smallest are not lost; products of parts are brought back by 2^-32. Vectors' and
+// states' numbers beyond these lines could leave the range in a product's sum.
+constexpr float kBlockVector = 16777216.f, kBlockState = 18446744073709551616.f;  // 2^24, 2^64
+constexpr float kBlockBack = 2.3283064365386963e-10f;                             // 2^-32
+__device__ __forceinline__ void block_most(float& most, float x) { asm("max.NaN.f32 %0, %0, %1;" : "+f"(most) : "f"(fabsf(x))); }
+__device__ __forceinline__ bool block_out(float x, float line) { return !(fabsf(x) < line); }  // (a NaN is out)
+// Two numbers as the sums of three pairs of bfloat16, each rounded, exact.
 __device__ __forceinline__ void block_split(float x, float y, uint32_t& high, uint32_t& middle, uint32_t& low) {
-  const uint32_t a = __float_as_uint(x), b = __float_as_uint(y);
-  high = __byte_perm(a, b, 0x7632);
-  const float rx = x - __uint_as_float(a & 0xffff0000u), ry = y - __uint_as_float(b & 0xffff0000u);
+  x *= 65536.f, y *= 65536.f;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(high) : "f"(y), "f"(x));
+  const float rx = x - __uint_as_float(high << 16), ry = y - __uint_as_float(high & 0xffff0000u);
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(middle) : "f"(ry), "f"(rx));
   const float sx = rx - __uint_as_float(middle << 16), sy = ry - __uint_as_float(middle & 0xffff0000u);
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(low) : "f"(sy), "f"(sx));
 }
-// One number that need not be finite: its three parts (the first keeps an infinity or a NaN).
+// One number of a block that goes by FMAs: as above, or its own bits and a mark.
+constexpr uint16_t kBlockWhole = 0x7fc0;
 __device__ __forceinline__ void block_split_any(float x, uint16_t (&part)[3]) {
   uint32_t high, middle, low;
   block_split(x, 0.f, high, middle, low);
-  const bool finite = isfinite(x);
-  part[0] = finite ? high & 0xffff : isnan(x) ? 0x7fc0 : __float_as_uint(x) >> 16;
-  part[1] = finite ? middle & 0xffff : 0, part[2] = finite ? low & 0xffff : 0;
+  const bool whole = block_out(x, kBlockVector);
+  part[0] = whole ? __float_as_uint(x) >> 16 : high & 0xffff;
+  part[1] = whole ? __float_as_uint(x) & 0xffff : middle & 0xffff;
+  part[2] = whole ? kBlockWhole : low & 0xffff;
 }
 __device__ __forceinline__ float block_join(const uint16_t* at, int plane) {
-  return __uint_as_float(static_cast<uint32_t>(at[0]) << 16) + __uint_as_float(static_cast<uint32_t>(at[plane]) << 16) +
-         __uint_as_float(static_cast<uint32_t>(at[2 * plane]) << 16);
+  const uint32_t high = at[0], middle = at[plane], low = at[2 * plane];
+  if (low == kBlockWhole) return __uint_as_float(high << 16 | middle);
+  return (__uint_as_float(high << 16) + (__uint_as_float(middle << 16) + __uint_as_float(low << 16))) * (1.f / 65536.f);
 }
 // Where row r of token t's vector lies in a part's [L][DP]: pieces of 8 rows change places so that eight tokens' pieces lie in
 // different banks.
@@ -98,14 +110,14 @@ __device__ __forceinline__ int block_at(int t, int r) {
   return t * DP + ((((r >> 3) ^ (t & 7)) << 3) | (r & 7));
 }
 
-// Where a block's vectors are cut and stored: rows r and r + 1 of token t's vector `which` at a time. What is not finite is
-// counted in `check` and stored once more at the end (block_store_again).
+// Where a block's vectors are cut and stored: rows r and r + 1 of token t's vector `which` at a time. `most` collects the largest;
+// what is out of range is stored once more at the end (block_store_again).
 template <int DP, int MODE>
-__device__ __forceinline__ void block_store(uint16_t* planes, int which, int t, int r, float x, float y, float& check) {
+__device__ __forceinline__ void block_store(uint16_t* planes, int which, int t, int r, float x, float y, float& most) {
   using W = BlockShape<DP, MODE>;
   uint32_t part[3];
   block_split(x, y, part[0], part[1], part[2]);
-  check = fmaf(x, 0.f, fmaf(y, 0.f, check));
+  block_most(most, x), block_most(most, y);
   const int at = block_at<DP>(t, r);
 #pragma unroll
   for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(planes + (which * 3 + i) * W::PLANE + at) = part[i];
@@ -116,14 +128,14 @@ __device__ __noinline__ void block_store_again(uint16_t* at, int plane, float x,
 #pragma unroll
   for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(at + i * plane) = a[i] | static_cast<uint32_t>(b[i]) << 16;
 }
-// Vector `which` of COUNT tokens from t0 on; -> whether all is finite.
+// Vector `which` of COUNT tokens from t0 on; -> whether all is in range.
 template <int DP, int MODE, int COUNT, int SIZE>
 __device__ __forceinline__ bool block_store_all(uint16_t* planes, int which, int t0, int r, const float2 (&x)[SIZE]) {
   using W = BlockShape<DP, MODE>;
-  float check = 0.f;
+  float most = 0.f;
 #pragma unroll
-  for (int t = 0; t < COUNT; ++t) block_store<DP, MODE>(planes, which, t0 + t, r, x[t].x, x[t].y, check);
-  if (check == 0.f) return true;
+  for (int t = 0; t < COUNT; ++t) block_store<DP, MODE>(planes, which, t0 + t, r, x[t].x, x[t].y, most);
+  if (!block_out(most, kBlockVector)) return true;
 #pragma unroll
   for (int t = 0; t < COUNT; ++t) block_store_again(planes + which * 3 * W::PLANE + block_at<DP>(t0 + t, r), W::PLANE, x[t].x, x[t].y);
   return false;
@@ -494,7 +506,7 @@ __global__ __launch_bounds__(128) void block_prepare_shared_kernel(BlockPrepare 
   for (int j = 0; j < L; ++j)
     decay[j] = j < tokens.count ? (MODE == 0 ? a.head_decay[h] : a.beta[static_cast<size_t>(tokens.start + j) * a.H + h]) : 1.f;
   uint16_t* planes = reinterpret_cast<uint16_t*>(a.vectors + (static_cast<size_t>(stage) * a.KH + kh) * W::STAGE);
-  float check = 0.f;
+  float most = 0.f;
   constexpr int PER = 2 * L * PAIRS / 128;
   float2 both[PER];
 #pragma unroll
@@ -512,10 +524,10 @@ __global__ __launch_bounds__(128) void block_prepare_shared_kernel(BlockPrepare 
   for (int n = 0; n < PER; ++n) {
     const int i = tid + n * 128, row = i / PAIRS, j = row % L, r = i % PAIRS * 2, which = row < L ? W::AT_K : W::AT_Q;
     *reinterpret_cast<float2*>(&rows[row][r]) = both[n];
-    if (blockIdx.z == 0) block_store<DP, MODE>(planes, which, j, r, both[n].x, both[n].y, check);
-    else check = fmaf(both[n].x, 0.f, fmaf(both[n].y, 0.f, check));
+    if (blockIdx.z == 0) block_store<DP, MODE>(planes, which, j, r, both[n].x, both[n].y, most);
+    else block_most(most, both[n].x), block_most(most, both[n].y);
   }
-  if (check != 0.f) {
+  if (block_out(most, kBlockVector)) {
     spoilt = 1;
     if (blockIdx.z == 0) {
 #pragma unroll
@@ -541,13 +553,17 @@ __global__ __launch_bounds__(128) void block_prepare_shared_kernel(BlockPrepare 
   }
   __syncthreads();
   if (hh < heads) {
-    float upto = 1.f, lost = 0.f, rest = 1.f, mine = 1.f;
+    float upto = 1.f, lost = 0.f, behind = 1.f, gone = 0.f, rest = 1.f, mine = 1.f;  // products with what their rounding lost
 #pragma unroll
     for (int j = 0; j < L; ++j) {
       const float x = decay[j], next = upto * x;
       lost = fmaf(lost, x, fmaf(upto, x, -next)), upto = next;
-      if (j == m) mine = upto;
-      if (j > m) rest *= x;
+      if (j == m) mine = isfinite(lost) ? upto + lost : upto;
+      if (j > m) {
+        const float more = behind * x;
+        gone = fmaf(gone, x, fmaf(behind, x, -more)), behind = more;
+        rest = isfinite(gone) ? behind + gone : behind;
+      }
       const float value = j >= m ? totals[j][m] * rest : 0.f;
       D[hh][j][m] = make_float2(value, value);
     }
@@ -609,32 +625,24 @@ struct BlockParts {
   }
 };
 
-// Two 16 x 8 products of a 16 x 16 operand x, side by side, all six products of parts that count: the large one into `large`,
-// the small ones into `small`. `b`: the second operand's parts, for the two products in turn.
-template <bool FIRST>
-__device__ __forceinline__ void block_product(float (&large)[2][4], float (&small)[2][4], const BlockParts& x, const uint32_t (&b)[3][4]) {
+// COUNT (1 or 2) 16 x 8 products of a 16 x 16 operand x, side by side, all products of parts but the two low ones: the large one
+// into `large`, the small ones into `small`. `b`: the second operand's parts, for the products in turn, from `at` on.
+template <bool FIRST, int COUNT>
+__device__ __forceinline__ void block_products(float (&large)[COUNT][4], float (&small)[COUNT][4], const BlockParts& x, const uint32_t (&b)[3][4],
+                                               int at = 0) {
+  constexpr int of_x[7] = {1, 2, 2, 0, 1, 1, 0}, of_b[7] = {2, 1, 0, 2, 1, 0, 1};
 #pragma unroll
-  for (int i = 0; i < 2; ++i) block_mma<FIRST>(small[i], x.part[2], b[0][2 * i], b[0][2 * i + 1]);
+  for (int p = 0; p < 7; ++p) {
 #pragma unroll
-  for (int i = 0; i < 2; ++i) block_mma<FIRST>(large[i], x.part[0], b[0][2 * i], b[0][2 * i + 1]);
+    for (int i = 0; i < COUNT; ++i) {
+      if (FIRST && p == 0) block_mma<true>(small[i], x.part[of_x[p]], b[of_b[p]][at + 2 * i], b[of_b[p]][at + 2 * i + 1]);
+      else block_mma<false>(small[i], x.part[of_x[p]], b[of_b[p]][at + 2 * i], b[of_b[p]][at + 2 * i + 1]);
+    }
+    if (p == 0) {
 #pragma unroll
-  for (int i = 0; i < 2; ++i) block_mma<false>(small[i], x.part[0], b[2][2 * i], b[2][2 * i + 1]);
-#pragma unroll
-  for (int i = 0; i < 2; ++i) block_mma<false>(small[i], x.part[1], b[1][2 * i], b[1][2 * i + 1]);
-#pragma unroll
-  for (int i = 0; i < 2; ++i) block_mma<false>(small[i], x.part[1], b[0][2 * i], b[0][2 * i + 1]);
-#pragma unroll
-  for (int i = 0; i < 2; ++i) block_mma<false>(small[i], x.part[0], b[1][2 * i], b[1][2 * i + 1]);
-}
-// The same for one 16 x 8 product.
-template <bool FIRST>
-__device__ __forceinline__ void block_product(float (&large)[4], float (&small)[4], const BlockParts& x, const uint32_t (&b)[3][4], int at) {
-  block_mma<FIRST>(small, x.part[2], b[0][at], b[0][at + 1]);
-  block_mma<FIRST>(large, x.part[0], b[0][at], b[0][at + 1]);
-  block_mma<false>(small, x.part[0], b[2][at], b[2][at + 1]);
-  block_mma<false>(small, x.part[1], b[1][at], b[1][at + 1]);
-  block_mma<false>(small, x.part[1], b[0][at], b[0][at + 1]);
-  block_mma<false>(small, x.part[0], b[1][at], b[1][at + 1]);
+      for (int i = 0; i < COUNT; ++i) block_mma<FIRST>(large[i], x.part[0], b[0][at + 2 * i], b[0][at + 2 * i + 1]);
+    }
+  }
 }
 
 template <int DP, int MODE>
@@ -649,7 +657,7 @@ struct BlockWalk {
   static_assert(STATE >= kBlockCols * (DP + 4), "room for the state as it is, for columns that are done once more");
 };
 
-// What eight neighbouring threads of a column do with float32 FMAs where a number is not finite.
+// What eight neighbouring threads of a column do with float32 FMAs where a number is out of range.
 template <int DP, int MODE>
 struct BlockAgain {
   using W = BlockShape<DP, MODE>;
@@ -690,7 +698,7 @@ __global__ __launch_bounds__(256, DP > 128 ? 1 : 2) void block_scan_kernel(
   float* parts_at = smem + BUFFERS * K::BUFFER;             // [2][16 rows of the state each][3][32 lanes][4 pairs]
   float* shares = parts_at + 2 * K::STATE;                  // [2][4 warps][2][32 lanes][4]
   float* halves = shares + (DELTA ? K::SHARES : 512);       // [2][32 lanes][4]
-  int* state_bad = reinterpret_cast<int*>(halves + K::HALVES);  // [2] the block whose state is not finite
+  int* state_bad = reinterpret_cast<int*>(halves + K::HALVES);  // [2] the block whose state is out of range
   const int h = blockIdx.y, b = ALL ? blockIdx.z : walking_sequence(cu_seqlens, seqs, least, blockIdx.z);
   const int vh = BY_HEAD ? h : h / (H / KH), VH = BY_HEAD ? H : KH, col0 = blockIdx.x * kBlockCols;
   if (!ALL && b < 0) return;
@@ -786,13 +794,14 @@ __global__ __launch_bounds__(256, DP > 128 ? 1 : 2) void block_scan_kernel(
           BlockParts x;
 #pragma unroll
           for (int i = 0; i < 3; ++i) x.part[i] = parts[((step + e) * 3 + i) * 32];
-          if (s == 0) block_product<true>(large[e], small[e], x, operand, 2 * e);
-          else block_product<false>(large[e], small[e], x, operand, 2 * e);
+          float(&l)[1][4] = reinterpret_cast<float(&)[1][4]>(large[e]), (&m)[1][4] = reinterpret_cast<float(&)[1][4]>(small[e]);
+          if (s == 0) block_products<true, 1>(l, m, x, operand, 2 * e);
+          else block_products<false, 1>(l, m, x, operand, 2 * e);
         }
       }
       float sum[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) sum[e] = (large[0][e] + large[1][e]) + (small[0][e] + small[1][e]);
+      for (int e = 0; e < 4; ++e) sum[e] = ((large[0][e] + large[1][e]) + (small[0][e] + small[1][e])) * kBlockBack;
       float4* meet = reinterpret_cast<float4*>(halves) + eight * 32 + lane;
       if (half == 1) *meet = make_float4(sum[0], sum[1], sum[2], sum[3]);
       asm volatile("bar.sync %0, 64;" ::"r"(1 + eight) : "memory");
@@ -823,7 +832,7 @@ __global__ __launch_bounds__(256, DP > 128 ? 1 : 2) void block_scan_kernel(
     }
   const int along_t = (lane >> 4) * 8 + (lane & 7), along_c = warp * ROWS / 8 + ((lane >> 3) & 1);
   const int across_t = ((lane >> 3) & 1) * 8 + (lane & 7), across_c = warp * ROWS / 8 + (lane >> 4);
-  // The state's parts, ahead of `block`, for its readers; whether it is finite; and under the delta rules the share of this
+  // The state's parts, ahead of `block`, for its readers; whether it is in range; and under the delta rules the share of this
   // warp's rows in what the block's tokens read.
   auto present = [&](int block) {
     uint4* to = reinterpret_cast<uint4*>(parts_at + (block & 1) * K::STATE) + warp * STEPS * 3 * 32 + lane;
@@ -840,21 +849,22 @@ __global__ __launch_bounds__(256, DP > 128 ? 1 : 2) void block_scan_kernel(
         const int at = ((along_c + 2 * s) ^ (along_t & 7)) << 3;
 #pragma unroll
         for (int i = 0; i < 3; ++i) block_ldmatrix<false>(operand[i], planes + i * W::PLANE + at);
-        if (s == 0) block_product<true>(large, small, x, operand);
-        else block_product<false>(large, small, x, operand);
+        if (s == 0) block_products<true, 2>(large, small, x, operand);
+        else block_products<false, 2>(large, small, x, operand);
       }
     }
-    float sums[4] = {0.f, 0.f, 0.f, 0.f};
+    float most[2] = {0.f, 0.f};
 #pragma unroll
     for (int t = 0; t < 2 * STEPS; ++t)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) sums[e] = fmaf(S[t][e], 0.f, sums[e]);
-    if ((sums[0] + sums[1]) + (sums[2] + sums[3]) != 0.f) state_bad[block & 1] = block;
+      for (int e = 0; e < 4; ++e) block_most(most[e & 1], S[t][e]);
+    if (block_out(most[0], kBlockState) || block_out(most[1], kBlockState)) state_bad[block & 1] = block;
     if (DELTA) {
       float4* share = reinterpret_cast<float4*>(shares + ((block & 1) * 4 + warp) * 256) + lane;
 #pragma unroll
       for (int i = 0; i < 2; ++i)
-        share[i * 32] = make_float4(large[i][0] + small[i][0], large[i][1] + small[i][1], large[i][2] + small[i][2], large[i][3] + small[i][3]);
+        share[i * 32] = make_float4((large[i][0] + small[i][0]) * kBlockBack, (large[i][1] + small[i][1]) * kBlockBack,
+                                    (large[i][2] + small[i][2]) * kBlockBack, (large[i][3] + small[i][3]) * kBlockBack);
     }
   };
   auto again_state = [&](float* held) {
@@ -911,10 +921,10 @@ __global__ __launch_bounds__(256, DP > 128 ? 1 : 2) void block_scan_kernel(
           u[i][2] -= (x.z + y.z) + (z.z + w.z), u[i][3] -= (x.w + y.w) + (z.w + w.w);
         }
       }
-      float sums[2] = {0.f, 0.f};
+      float most = 0.f;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) sums[0] = fmaf(u[0][e], 0.f, sums[0]), sums[1] = fmaf(u[1][e], 0.f, sums[1]);
-      const bool spoilt = __any_sync(0xffffffffu, sums[0] + sums[1] != 0.f);  // the same in all four warps
+      for (int e = 0; e < 4; ++e) block_most(most, u[0][e]), block_most(most, u[1][e]);
+      const bool spoilt = __any_sync(0xffffffffu, block_out(most, kBlockState));  // the same in all four warps
       float* writes = shares + ((block + 1) & 1) * (DELTA ? 4 * 256 : 256);
       if (spoilt) {
         again_state(held);
@@ -923,11 +933,11 @@ __global__ __launch_bounds__(256, DP > 128 ? 1 : 2) void block_scan_kernel(
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             if (warp == 0) writes[(gid + (e >> 1) * 8) * L + 8 * i + 2 * tig + (e & 1)] = u[i][e];
-            if (!isfinite(u[i][e])) u[i][e] = 0.f;
+            if (block_out(u[i][e], kBlockState)) u[i][e] = 0.f;
           }
         states_meet();
         bool mine_spoilt = false;
-        for (int t = 0; t < count; ++t) mine_spoilt = mine_spoilt || !isfinite(writes[again_c * L + t]);
+        for (int t = 0; t < count; ++t) mine_spoilt = mine_spoilt || block_out(writes[again_c * L + t], kBlockState);
         const BlockAgain<DP, MODE> again{at_stage, scalars};
         if (mine_spoilt) again.move(held + again_c * HP, writes + again_c * L, count);
         states_meet();
@@ -942,7 +952,7 @@ __global__ __launch_bounds__(256, DP > 128 ? 1 : 2) void block_scan_kernel(
 #pragma unroll
         for (int i = 0; i < 3; ++i) block_ldmatrix<true>(operand[i], planes + i * W::PLANE + at);
         float large[2][4], small[2][4];
-        block_product<true>(large, small, x, operand);
+        block_products<true, 2>(large, small, x, operand);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           float2 decay;
@@ -951,7 +961,7 @@ __global__ __launch_bounds__(256, DP > 128 ? 1 : 2) void block_scan_kernel(
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             float& y = S[2 * s + i][e];
-            float more = large[i][e] + small[i][e];
+            float more = (large[i][e] + small[i][e]) * kBlockBack;
             if (!ROW_DECAY) more = fmaf(y, scalars[W::AT_ALL + 1], more);
             y = fmaf(y, e & 1 ? decay.y : decay.x, more);
           }
@@ -961,7 +971,7 @@ __global__ __launch_bounds__(256, DP > 128 ? 1 : 2) void block_scan_kernel(
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           bool lost = false;
-          for (int t = 0; t < count; ++t) lost = lost || !isfinite(writes[(gid + 8 * c) * L + t]);
+          for (int t = 0; t < count; ++t) lost = lost || block_out(writes[(gid + 8 * c) * L + t], kBlockState);
           if (lost) {
 #pragma unroll
             for (int t = 0; t < 2 * STEPS; ++t)

@@ -26,7 +26,7 @@ def test_edges_match_the_recurrence_no_further_off_than_token_by_token(rule, H, 
     want, single = _reference(rule, x, lengths, slots), _run(rule, x, lengths, slots, blocks=False)
     for a, b, c in zip(_run(rule, x, lengths, slots), want, single):
         assert _distance(a, b) <= 2e-6                             # float32 sums, forgotten at the decays' rate
-        assert _distance(a, b) <= 2 * _distance(c, b) + 2.0 ** -24  # both are sums of roundings of 2^-24
+        assert _distance(a, b) <= 1.5 * _distance(c, b) + 2.0 ** -26  # both are sums of roundings of 2^-24, those of 16 tokens cut off
 
 
 # CTAs (tiles x heads x sequences) on both sides of the line: 370 for delta rules, 444 with a bonus, 222 for heads beyond 128
@@ -82,3 +82,52 @@ def test_a_long_sequence_among_short_ones(rule, H, d, dv, lengths):
     for longest in (max(lengths), 320, None):
         for a, b in zip(_run(rule, x, lengths, slots, longest=longest), want):
             assert _distance(a, b) <= 2e-6
+
+
+def _still(x, lengths, decay=1.0):
+    """Inputs under which nothing is written and the state decays by `decay` alone."""
+    for name in ("g", "decay", "head"):
+        x[name].fill_(decay)
+    x["step"].zero_()
+    x["v"].zero_()
+    return x
+
+
+@pytest.mark.parametrize("H,d,dv", [(2, 64, 20), (1, 128, 33), (1, 256, 16)])
+@pytest.mark.parametrize("rule", RULES)
+def test_a_read_of_one_number_is_rounded_once(rule, H, d, dv):
+    """Queries with one number each against a state that stays: single products of float32 numbers."""
+    x, T = _still(_inputs(H, H, d, dv, [112], seed=d), [112]), 112
+    x["q"] = torch.randn(T, H, d, device=DEV) * (torch.arange(d, device=DEV) == torch.arange(T, device=DEV)[:, None] * 5 % d)[:, None]
+    (out, state), (want, _) = _run(rule, x, [112], [1]), _reference(rule, x, [112], [1])
+    # the product's rounding; the low parts' product, 2^-34 of it, and the small ones' truncated sum, 2^-31, are left out
+    assert bool(((out.double() - want).abs() <= (2.0 ** -24 + 2.0 ** -30) * want.abs()).all())
+    assert torch.equal(state, x["state"])
+
+
+@pytest.mark.parametrize("scale", [2.0 ** -116, 2.0 ** 70])
+@pytest.mark.parametrize("H,d,dv", [(2, 64, 20), (1, 128, 33)])
+@pytest.mark.parametrize("rule", RULES)
+def test_very_small_and_very_large_states(rule, H, d, dv, scale):
+    """What is written and held, times a power of two: the same relative distance as token by token."""
+    x = _inputs(H, H, d, dv, [120], seed=d + 1)
+    x["v"] *= scale
+    x["state"] *= scale
+    want, single = _reference(rule, x, [120], [1]), _run(rule, x, [120], [1], blocks=False)
+    for a, b, c in zip(_run(rule, x, [120], [1]), want, single):
+        assert _distance(a / scale, b / scale) <= 1.25 * _distance(c / scale, b / scale) + 2.0 ** -24
+
+
+@pytest.mark.parametrize("rule", RULES)
+def test_keys_and_queries_out_of_the_parts_range(rule):
+    """A key and a query of 2^30 and more are read and written with FMAs, the tokens around them as ever."""
+    x = _inputs(2, 2, 64, 20, [130], seed=3)
+    x["q"][40, 1, 3], x["q"][77, 0, 9] = 2.0 ** 30, 2.0 ** 120
+    if rule not in ("delta", "head_delta"):  # (a delta rule's state would grow by the key's square)
+        x["k"][55, 0, 5] = 2.0 ** 31
+    got, single = _run(rule, x, [130], [1]), _run(rule, x, [130], [1], blocks=False)
+    want = _reference(rule, x, [130], [1])
+    for a, b, c in zip(got, want, single):
+        whole = c.isfinite() & (b.abs() < 2.0 ** 60)
+        assert torch.equal(a.isfinite(), c.isfinite())
+        assert float((a[whole].double() - b[whole]).norm() / b[whole].norm()) <= 2e-6
