@@ -1023,16 +1023,18 @@ long long block_stage_floats(int H, int KH, int d, int dv) {
 }
 
 // Whether the step goes with float32 FMAs (recurrent_walk.cuh): once its CTAs pass what the SMs hold at once the preparation per
-// head weighs more. us, tensor cores and FMAs: delta rule, 16 heads of 128 x 128, two sequences of 700 (256 CTAs) 97 and 123, three
-// of 400 (384) 118 and 123, four of 1,024 (512) 339 and 303; 32 heads of 128 x 64, the same 122 and 132, 141 and 133, 417 and 332;
-// a bonus, 32 heads of 64 x 64, four of 600 (512) 122 and 101; heads of 256 x 64, 16 of them, four of 600 (256) delta rule 255
-// and 282, head decay with a delta 252 and 214, a decay per token 185 and 172. With one decay a token and heads of up to 128 the
-// tensor cores are the faster way throughout (four of 1,024, 16 heads of 128 x 128 209 and 222).
+// head weighs more. us, tensor cores and FMAs, n sequences of so many tokens (CTAs): delta rule, 16 heads of 128 x 128, two of 600 (256)
+// 126 and 122, three of 1,024 (384) 304 and 310, four (512) 361 and 318; head decay with a delta 126 and 167, 306 and 335, 372 and
+// 341; a bonus, 32 heads of 64 x 64, three of 600 (384) 110 and 103, four (512) 134 and 110; one decay a token, 16 heads of 128 x 128, four of
+// 1,024 (512) 263 and 249, five of 600 (640) 210 and 230, eight of 600 (1,024) 294 and 292, eight of 1,024 521 and 472, 32 heads of 64 x 64
+// 384 CTAs 161 and 167, 512 194 and 173, 1,024 384 and 325. Heads of 256 x 64, 16 of them, three of 1,024 (192) delta rule 404 and 456, head
+// decay with a delta 394 and 345, a decay per token 292 and 280; four (256) 457 and 476, 448 and 359, 314 and 290.
 template <int MODE>
 bool block_takes_fma(int seqs, int H, int d, int dv, int tokens, int longest) {
   const long long ctas = walk_ctas(seqs, H, dv, tokens, longest);
   if (d > 128) return 2 * ctas > 3 * kSmCount;
-  return BlockShape<64, MODE>::DELTA ? 2 * ctas > 5 * kSmCount : BlockShape<64, MODE>::BONUS && ctas > 3 * kSmCount;
+  if (BlockShape<64, MODE>::DELTA) return 2 * ctas > 5 * kSmCount;
+  return ctas > (BlockShape<64, MODE>::BONUS || d <= 64 ? 3 : 6) * kSmCount;
 }
 
 template <int MODE>

@@ -543,11 +543,8 @@ template <int MODE>
 int launch_walk(const WalkArgs& a) {
   constexpr int LONG = walk_block<MODE>(256);
   if (a.d > 128) return launch_walk<(LONG == 8 ? 4 : 2), (LONG == 8 ? 2 : 4), 256, MODE, LONG>(a);
-  if constexpr (MODE != 0 && MODE != 2) {  // (where the tensor path is always the faster one)
-    if (a.d > 64) return launch_walk<2, 4, 128, MODE, 4>(a);
-    return launch_walk<1, 4, 64, MODE, 4>(a);
-  }
-  return LRM_UNSUPPORTED;
+  if (a.d > 64) return launch_walk<2, 4, 128, MODE, 4>(a);
+  return launch_walk<1, 4, 64, MODE, 4>(a);
 }
 
 }  // namespace

@@ -29,8 +29,10 @@ def test_edges_match_the_recurrence_no_further_off_than_token_by_token(rule, H, 
         assert _distance(a, b) <= 1.5 * _distance(c, b) + 2.0 ** -26  # both are sums of roundings of 2^-24, those of 16 tokens cut off
 
 
-# CTAs (tiles x heads x sequences) on both sides of the line: 370 for delta rules, 444 with a bonus, 222 for heads beyond 128
-@pytest.mark.parametrize("H,d,dv,seqs", [(46, 64, 64, 2), (47, 64, 64, 2), (55, 64, 64, 2), (56, 64, 64, 2), (37, 160, 48, 2), (38, 160, 48, 2)])
+# CTAs (tiles x heads x sequences) on both sides of the line: 370 for delta rules, 444 with a bonus or heads of up to 64, 888 with one decay and
+# heads of up to 128, 222 for heads beyond
+@pytest.mark.parametrize("H,d,dv,seqs", [(46, 64, 64, 2), (47, 64, 64, 2), (55, 64, 64, 2), (56, 64, 64, 2), (37, 160, 48, 2), (38, 160, 48, 2),
+                                         (148, 100, 48, 2), (149, 100, 48, 2)])
 @pytest.mark.parametrize("rule", RULES)
 def test_both_sides_of_the_line_to_the_blocks_with_fmas(rule, H, d, dv, seqs):
     lengths = [97 + 16 * i for i in range(seqs)]

@@ -19,9 +19,10 @@ def _stage_floats(rule, H, d, dv, lengths, longest):
     return floats // stages
 
 
-# heads whose lone walk fits the SMs; per rule, among them heads beyond 128
+# heads whose lone walk fits the SMs; per rule, of each padded size
 HEADS = [("delta", 8, 128, 128), ("delta", 16, 128, 128), ("delta", 16, 200, 64), ("head_delta", 16, 128, 128), ("head_delta", 8, 256, 64),
-         ("bonus", 32, 64, 64), ("bonus", 16, 128, 128), ("token_decay", 16, 256, 64), ("head_decay", 16, 129, 64)]
+         ("bonus", 32, 64, 64), ("bonus", 16, 128, 128), ("token_decay", 16, 256, 64), ("head_decay", 16, 129, 64),
+         ("token_decay", 16, 128, 128), ("head_decay", 32, 64, 64)]
 
 
 @pytest.mark.parametrize("rule,H,d,dv", HEADS)
