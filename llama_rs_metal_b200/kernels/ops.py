@@ -821,7 +821,9 @@ def _f32(shape, device) -> torch.Tensor:
 WALK_TOKENS = 96  # the state scans' sequences of as many tokens go in blocks (kWalkTokens in csrc/recurrent_walk.cuh)
 
 
-SCAN_FLOATS = 64 << 20  # most floats of such a scan's workspace; a step that wants more goes in pieces
+# Most floats of such a scan's workspace; a step that wants more goes in pieces, and sequences of different pieces one after another: two
+# of 2,048 tokens, head decay with a delta, 16 heads of 256 x 64, whole 439 us, in two pieces 715 (with 64 Mi floats).
+SCAN_FLOATS = 128 << 20
 
 
 def _walk_workspace(entry: str, blocks: bool, tokens: int, longest: Optional[int], device, seqs: int, *sizes) -> Optional[torch.Tensor]:

@@ -40,3 +40,11 @@ def test_many_long_sequences_go_with_fmas(rule, H, d, dv):
     lone = _stage_floats(rule, H, d, dv, [2048], 2048)
     for longest in (256, 0):
         assert _stage_floats(rule, H, d, dv, [256] * 16, longest) != lone
+
+
+# two prompts of 2,048 tokens beside one another: what the blocks with FMAs held in 64 Mi floats, the tensor cores' larger stages hold too
+@pytest.mark.parametrize("rule,H,d,dv", HEADS)
+def test_two_prompts_go_whole(rule, H, d, dv):
+    from llama_rs_metal_b200.kernels import ops
+    lengths = [2048, 2048, 1, 1]
+    assert _stage_floats(rule, H, d, dv, lengths, 2048) * (sum(lengths) // STAGE + len(lengths)) <= ops.SCAN_FLOATS
