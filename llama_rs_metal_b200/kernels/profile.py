@@ -252,7 +252,7 @@ WORK: Dict[str, Callable[..., Tuple[float, float]]] = {
     "lrm_tanh_columns": lambda a: (_v(a[5]) * _v(a[6]) * (_ELEM[_v(a[1])] + _ELEM[_v(a[4])]), 0),
 }
 # entry points that only answer questions and launch nothing
-_QUERIES = ("_supports", "_ctas_per_sm", "_slices", "_pieces", "_resident", "_floats", "_error", "_room", "lrm_set_pdl", "lrm_set_norm_ranks", "lrm_pick_pieces", "lrm_linear_state_scan_rows")
+_QUERIES = ("_supports", "_ctas_per_sm", "_slices", "_pieces", "_resident", "_floats", "lrm_gemm_f32_umma_scratch", "_error", "_room", "lrm_set_pdl", "lrm_set_norm_ranks", "lrm_pick_pieces", "lrm_linear_state_scan_rows")
 
 
 class _Row:
