@@ -34,7 +34,7 @@
 // state's parts, off the chain.
 //
 // What bounds it: the chain of a block (cut the state, p', its exchange, cut u, the update) is 1.15 us under a delta rule and
-// 0.87 us without, with a CTA of eight warps per SM; the tensor pipe is 38 % busy meanwhile (profiles/state_block_scan_2048.md). us, in
+// 0.87 us without, with a CTA of eight warps per SM; the tensor pipe is 38 % busy meanwhile. us, in
 // brackets float32 FMAs in blocks of 8 or 4 tokens: delta rule, 16 heads of 128 x 128, 2,048 tokens 200 (262), 8 heads 175 (231),
 // 16 heads of 64 x 64 148 (229); a decay per token 146 (203), 143 (168), 100 (160); 32 heads of 128 x 64, 1,500 and 777 tokens 145
 // (187). One sequence of 96 tokens is within 2 us of the FMAs on both rules (16 heads of 128 x 128), 256 8 us below. (With six products
@@ -1002,7 +1002,7 @@ inline int walking(int seqs, int tokens) { return seqs < tokens / kWalkTokens ? 
 // CTAs of the step's walks, for the choice of the way and its layout: as many whole walks as its tokens would make of the longest
 // one, which is what the step waits for. Where that is not known: all sequences where they bring kWalkTokens on average, else one.
 // us, counted so and by how many sequences could walk at most: 2,048 tokens beside 31 sequences of one, delta rule, 8 heads of 128 x 128
-// 187 and 361 (alone 167), head decay with a delta, 16 heads 226 and 544 (194), a bonus 191 and 329 (155); 297 beside three of one 50 and 95.
+// 200 and 361 (alone 181), head decay with a delta, 16 heads 241 and 544 (210), a bonus 206 and 329 (165); 297 beside three of one 52 and 95.
 inline long long walk_ctas(int seqs, int H, int dv, int tokens, int longest) {
   const long long one = static_cast<long long>((dv + kBlockCols - 1) / kBlockCols) * H;
   if (longest > 0) return longest < tokens ? one * tokens / longest : one;
@@ -1026,7 +1026,9 @@ long long block_stage_floats(int H, int KH, int d, int dv) {
 // head weighs more. us, tensor cores and FMAs, n sequences of so many tokens (CTAs): delta rule, 16 heads of 128 x 128, two of 600 (256)
 // 126 and 122, three of 1,024 (384) 304 and 310, four (512) 361 and 318; head decay with a delta 126 and 167, 306 and 335, 372 and
 // 341; a bonus, 32 heads of 64 x 64, three of 600 (384) 110 and 103, four (512) 134 and 110; one decay a token, 16 heads of 128 x 128, four of
-// 1,024 (512) 263 and 249, five of 600 (640) 210 and 230, eight of 600 (1,024) 294 and 292, eight of 1,024 521 and 472, 32 heads of 64 x 64
+// 1,024 (512) 263 and 249, five of 600 (640) 210 and 230, eight of 600 (1,024) 294 and 292, eight of 1,024 521 and 472 (the FMAs' CTAs have 32
+// columns, two to an SM: four SMs' worth of 16 columns fill them once; sequences whose longest is not known are seldom equal, and then
+// the tensor cores are ahead: 1,000, 700, 400 and 300 tokens 167 and 187), 32 heads of 64 x 64
 // 384 CTAs 161 and 167, 512 194 and 173, 1,024 384 and 325. Heads of 256 x 64, 16 of them, three of 1,024 (192) delta rule 404 and 456, head
 // decay with a delta 394 and 345, a decay per token 292 and 280; four (256) 457 and 476, 448 and 359, 314 and 290.
 template <int MODE>
@@ -1034,7 +1036,8 @@ bool block_takes_fma(int seqs, int H, int d, int dv, int tokens, int longest) {
   const long long ctas = walk_ctas(seqs, H, dv, tokens, longest);
   if (d > 128) return 2 * ctas > 3 * kSmCount;
   if (BlockShape<64, MODE>::DELTA) return 2 * ctas > 5 * kSmCount;
-  return ctas > (BlockShape<64, MODE>::BONUS || d <= 64 ? 3 : 6) * kSmCount;
+  if (BlockShape<64, MODE>::BONUS || d <= 64) return ctas > 3 * kSmCount;
+  return (longest > 0 && ctas > 3 * kSmCount && ctas <= 4 * kSmCount) || ctas > 6 * kSmCount;
 }
 
 template <int MODE>

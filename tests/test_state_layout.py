@@ -42,6 +42,14 @@ def test_many_long_sequences_go_with_fmas(rule, H, d, dv):
         assert _stage_floats(rule, H, d, dv, [256] * 16, longest) != lone
 
 
+@pytest.mark.parametrize("rule", ["token_decay", "head_decay"])
+def test_one_decay_a_token_goes_with_fmas_where_their_ctas_fill_the_sms(rule):
+    way = lambda seqs, longest=600: _stage_floats(rule, 16, 128, 128, [600] * seqs, longest)  # noqa: E731
+    lone = way(1)
+    assert [way(n) != lone for n in (2, 3, 4, 5, 6, 8)] == [False, False, True, False, False, True]
+    assert way(4, 0) == lone
+
+
 # two prompts of 2,048 tokens beside one another: what the blocks with FMAs held in 64 Mi floats, the tensor cores' larger stages hold too
 @pytest.mark.parametrize("rule,H,d,dv", HEADS)
 def test_two_prompts_go_whole(rule, H, d, dv):
