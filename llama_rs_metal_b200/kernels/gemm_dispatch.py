@@ -169,8 +169,8 @@ def few_takes(M: int, N: int, K: int, mode: int) -> bool:
     39.1 (46.9), 32 rows 40.3 (47.5), 49408 x 4096 32 rows 65.9 (72.3), 64 rows 70.4 (73.4), 128256 x 2048 64 rows 84.1 (88.9),
     a tile for half the SMs only, 9472 x 22000 32 rows 84.1 (103.4). Gated: 16384 x 2048 16 rows 12.4 (15.5), 32 rows 13.5
     (15.4), 28672 x 4096 32 rows 41.0 (48.2), 49408 x 4096 48 rows 70.9 (73.2). The line for more than 32 rows is that of both
-    kernels' earlier epilogues: below it lie a few per cent either way (28672 x 4096 64 rows 43.5 against 47.9, gated 44.9
-    against 48.4; gated 16384 x 3072 48 rows 21.6 against 21.4). Up to 12 rows the streaming kernel stays: its like beside it
+    kernels' earlier epilogues and leaves up to 9 % behind: 28672 x 4096 33 rows 43.0 against 47.0, 64 rows 44.1 against 47.7, gated 45.7
+    against 47.6 and 47.3 against 48.0; 16384 x 3072 64 rows 21.0 against 21.7, gated 24.3 against 21.9. Up to 12 rows the streaming kernel stays: its like beside it
     live off the L1 that this kernel's ring takes from them (3 sequences, one layer of the 8B shape: 231 us a step against 177,
     with this kernel's former times)."""
     if not 12 < M <= (48 if mode == 3 else 64):
@@ -362,7 +362,7 @@ def f32_takes_umma(N: int, K: int) -> bool:
     """Whether a float32 product goes to the tensor cores in three-part splits (csrc/gemm_f32_umma.cu) or to the FMA kernels
     (csrc/gemm_f32.cu). A matter of the matrix alone, so that a row gives the same bits however many there are. us for 1, 32 and 333
     rows, in brackets the FMA kernels: 1024 x 1024 9.9 (12.7), 11.1 (28.7), 18.2 (40.0); 512 x 2048 9.9 (24.2), 11.6 (56.2), 21.0
-    (76.2). Of larger matrices a single row of 128256 x 2048 alone is slower (196 against 175; 4 rows 197 against 240). Rows on 32 bytes (K a multiple of 8), as the parts' copies want them."""
+    (76.2); 2048 x 512, below the line, 9.2 (6.9), 10.6 (17.4), 18.9 (33.2). Of larger matrices a single row of 128256 x 2048 alone is slower (196 against 175; 4 rows 197 against 240). Rows on 32 bytes (K a multiple of 8), as the parts' copies want them."""
     return K % 8 == 0 and K >= 1024 and N >= 512
 
 

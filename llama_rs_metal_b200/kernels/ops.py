@@ -821,8 +821,9 @@ def _f32(shape, device) -> torch.Tensor:
 WALK_TOKENS = 96  # the state scans' sequences of as many tokens go in blocks (kWalkTokens in csrc/recurrent_walk.cuh)
 
 
-# Most floats of such a scan's workspace; a step that wants more goes in pieces, and sequences of different pieces one after another: two
-# of 2,048 tokens, head decay with a delta, 16 heads of 256 x 64, whole 439 us, in two pieces 715 (with 64 Mi floats).
+# Most floats of such a scan's workspace; a step that wants more goes in pieces, and sequences of different pieces one after another. us,
+# with 64 Mi floats, with these and with twice as many: two of 2,048 tokens, head decay with a delta, 16 heads of 256 x 64 710, 433,
+# 433; two of 4,096, 16 heads of 128 x 128, delta rule 1,072, 718, 720, a decay per token 752, 505, 505; one of 16,384 1,545, 1,553, 1,574.
 SCAN_FLOATS = 128 << 20
 
 
@@ -1632,11 +1633,13 @@ def moe_experts_rows(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor,
 def moe_prefers_sorted(tokens: int, width: int, ff: int, experts: int, top: int) -> bool:
     """Whether a prompt's experts are computed on rows sorted by expert instead of all of them for every token: where the
     sorted rows, each expert's filled up to tiles of 128, are at most half as many and the products large enough to pay for
-    five launches. us, sorted against all, without the router and with the gate still in a launch of its own (with the router
-    1,500 tokens of the first size took 118 then and take 89 now; the line has stayed). 2048 x 1024: 2 of 8 experts 500 tokens 60 and 92, 1,500 101 and 155, 4,096 192 and 358; 1 of 3 600 tokens 48 and 51; 4 of 8, more than half, 1,000 tokens 130 and
+    five launches. us, sorted against all, without the router and with the gate still in a launch of its own; the line is that of
+    these figures. 2048 x 1024: 2 of 8 experts 500 tokens 60 and 92, 1,500 101 and 155, 4,096 192 and 358; 1 of 3 600 tokens 48 and 51; 4 of 8, more than half, 1,000 tokens 130 and
     124. 1024 x 512: 2 of 8 500 tokens 38 and 46; 1 of 4 500 tokens 34 and 30, 1,000 37 and 36, 1,500 40 and 44; 1 of 3 1,500
     tokens 39 and 36, 2,048 43 and 45. 512 x 256: 2 of 8 500 tokens 33 and 28, 2,048 46 and 44; 1 of 4 4,096 tokens 46 and
-    42; 8 of 32 4,096 tokens 243 and 231 (1,500 110 and 119)."""
+    42; 8 of 32 4,096 tokens 243 and 231 (1,500 110 and 119). With the gate in the first product's
+    epilogue, and the router, 2048 x 1024 2 of 8 1,500 tokens 97 and 151, 4,096 175 and 327; beyond the line 4 of 8 1,000 tokens 116 and 123,
+    512 x 256 8 of 32 4,096 tokens 229 and 244."""
     rows = 128 * int(_lib().lrm_moe_sorted_tiles_room(tokens * top, experts))
     large = width * ff >= 1 << 19 and (experts * ff >= 3072 or tokens * experts * width * ff >= 3e9)
     return 2 * rows <= tokens * experts and large and width % 64 == 0 and ff % 64 == 0
