@@ -1027,7 +1027,7 @@ long long block_stage_floats(int H, int KH, int d, int dv) {
 // 126 and 122, three of 1,024 (384) 304 and 310, four (512) 361 and 318; head decay with a delta 126 and 167, 306 and 335, 372 and
 // 341; a bonus, 32 heads of 64 x 64, three of 600 (384) 110 and 103, four (512) 134 and 110; one decay a token, 16 heads of 128 x 128, four of
 // 1,024 (512) 263 and 249, five of 600 (640) 210 and 230, eight of 600 (1,024) 294 and 292, eight of 1,024 521 and 472 (the FMAs' CTAs have 32
-// columns, two to an SM: four SMs' worth of 16 columns fill them once; sequences whose longest is not known are seldom equal, and then
+// columns, two to an SM, and fill the SMs once at 592 of 16; sequences whose longest is not known are seldom equal, and then
 // the tensor cores are ahead: 1,000, 700, 400 and 300 tokens 167 and 187), 32 heads of 64 x 64
 // 384 CTAs 161 and 167, 512 194 and 173, 1,024 384 and 325. Heads of 256 x 64, 16 of them, three of 1,024 (192) delta rule 404 and 456, head
 // decay with a delta 394 and 345, a decay per token 292 and 280; four (256) 457 and 476, 448 and 359, 314 and 290.
