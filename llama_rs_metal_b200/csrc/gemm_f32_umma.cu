@@ -362,6 +362,7 @@ __global__ __launch_bounds__(Cut<MAXC, RAW, AHEAD, WW>::THREADS, 1) void gemm_f3
           else sums[(MAXC + c0 + i * 16 + j) * kRows + place] = __uint_as_float(r[j]) * kBack;
         }
       }
+      tc_fence_before();
     }
     all_meet();  // all marks are made
 #pragma unroll
