@@ -58,8 +58,6 @@ class StateView:
 
 
 class KeyValueGroup:
-    STAGED = 4  # copies of the page table that may be under way
-
     def __init__(self, request: KeyValueRequest, entries: List[int], pages: int, max_slots: int,
                  pages_per_sequence: int, page_size: int, dtype, device):
         self.request, self.entries, self.page_size = request, entries, page_size
@@ -68,12 +66,7 @@ class KeyValueGroup:
         self.table_device = torch.full((max_slots, pages_per_sequence), -1, dtype=torch.int32,
                                        device=device)
         self.dirty = False
-        if self.table_device.is_cuda:  # pinned tables that copies leave from, by turns, the events behind them, the last one's stream
-            self.staged = torch.empty((self.STAGED, max_slots, pages_per_sequence), dtype=torch.int32, pin_memory=True)
-            self.copied = [torch.cuda.Event() for _ in range(self.STAGED)]
-            for event in self.copied:  # an event comes into being with its first record
-                event.record(torch.cuda.current_stream(self.table_device.device))
-            self.turn, self.copied_on = 0, None
+        self.copied, self.copied_on = None, None  # the event behind the table's last copy, and the stream that is behind it
         shape = (pages, request.kv_heads, page_size, request.head_dim)
         value_shape = (pages, request.kv_heads, page_size, request.value_dim or request.head_dim)
         # zeroed once: a kernel may load rows of a page that no token was ever stored in (they are
@@ -151,27 +144,23 @@ class KeyValueGroup:
             self.dirty = True
 
     def sync(self) -> None:
-        """Bring the device's page table up to date, in the stream's order. The copy leaves from pinned memory, so the host
-        goes on while earlier steps run (a copy from pageable memory waits for the whole stream first: the device then idled
-        while the host prepared and launched a prompt, 4,690 us a pass against 4,510 at 2,048 tokens of the 1B shape, 2,020
-        against 1,800 for 4,353 packed ones on two layers of the 3B shape, 568 against 499 where the step is a captured one). A step on another stream than
-        the last copy's waits for that copy, so the table is there for every stream, and copies keep their order."""
-        if not self.table_device.is_cuda:
-            if self.dirty:
-                self.table_device.copy_(torch.from_numpy(self.table_host))
-                self.dirty = False
-            return
-        stream = torch.cuda.current_stream(self.table_device.device)
+        """Bring the device's page table up to date, in the stream's order, without waiting for the device: the asynchronous copy
+        from pageable memory takes the table as it is into a buffer of the driver's before it returns. (A copy that waits for the
+        whole stream left the device idle while the host prepared and launched a prompt: 4,690 us a pass against 4,510 at 2,048
+        tokens of the 1B shape, 2,020 against 1,800 for 4,353 packed ones on two layers of the 3B shape, 568 against 499 where the
+        step is a captured one.) A step on another stream than the last copy's waits for that copy, so the table is there for
+        every stream, and copies keep their order."""
+        stream = torch.cuda.current_stream(self.table_device.device) if self.table_device.is_cuda else None
         if self.copied_on is not None and self.copied_on != stream:
-            stream.wait_event(self.copied[self.turn])
+            stream.wait_event(self.copied)
             self.copied_on = stream  # what follows on this stream is behind the copy
         if self.dirty:
-            self.turn = (self.turn + 1) % self.STAGED
-            self.copied[self.turn].synchronize()  # the copy that last left from this buffer is done
-            self.staged[self.turn].copy_(torch.from_numpy(self.table_host))
-            self.table_device.copy_(self.staged[self.turn], non_blocking=True)
-            self.copied[self.turn].record(stream)
-            self.copied_on = stream
+            self.table_device.copy_(torch.from_numpy(self.table_host), non_blocking=True)
+            if stream is not None:
+                if self.copied is None:
+                    self.copied = torch.cuda.Event()
+                self.copied.record(stream)
+                self.copied_on = stream
             self.dirty = False
 
     def bytes(self) -> int:
