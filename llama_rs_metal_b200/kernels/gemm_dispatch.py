@@ -5,7 +5,9 @@
   leave most SMs idle and cannot split K (few output columns, epilogue other than "add");
 * 13 to 64 rows of products large enough: tcgen05 with the weights as its wide operand
   (csrc/gemm_bf16_few.cu; few_takes says where it is the faster one);
-* more rows (prompts, larger decode batches): the TMA + tcgen05 kernel
+* 65 to some 1,300 rows, wherever its tiles waste less: tcgen05 over pairs of SMs with the weights as
+  the wide operand (csrc/gemm_bf16_wide.cu; wide_plan);
+* more rows (prompts): the TMA + tcgen05 kernel
   (csrc/gemm_bf16_umma.cu), with 128 x 128, 128 x 256 or 256 x 256 tiles, whichever needs less
   time by a count of rounds over the SMs and the measured cost of a tile;
 * a narrow product that is to be added to the residual stream may be cut into K slices so that
@@ -18,6 +20,7 @@
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Dict, Optional
 
 import torch
@@ -28,6 +31,8 @@ from .ops import _done, _ptr, _stream  # noqa: PLC2701  (same package)
 
 SM_COUNT = 148
 force_tiled = False  # tests switch the fast kernels off to compare both paths
+no_wide = False  # tests: products of more than 64 rows stay off the kernel with the weights as the wide operand
+wide_shape = None  # tests and tuning: (activation rows of a tile, K slices) of that kernel instead of its own rule
 umma_width: Optional[int] = None  # tests pin the tile: 128 (128 x 128), 256 (128 x 256), 512 (256 x 256), 192 (128 x 192)
 
 _status: Dict[int, torch.Tensor] = {}
@@ -75,7 +80,8 @@ def check_status() -> None:
                           55: "a free accumulator"})
             names.update({61: "a free stage", 62: "operand parts", 63: "the accumulator", 64: "operand tiles", 65: "copies in flight",
                           66: "a free tile", 67: "the small products"})
-            kernel = "gemm_f32_umma" if code >= 61 else "gemm_bf16_few" if code >= 51 else "attention_gated_umma" if code >= 41 else "gemm_bf16_umma_pair" \
+            names.update({71: "a free stage", 72: "operand tiles", 73: "the accumulator", 74: "copies in flight", 75: "a free accumulator"})
+            kernel = "gemm_bf16_wide" if code >= 71 else "gemm_f32_umma" if code >= 61 else "gemm_bf16_few" if code >= 51 else "attention_gated_umma" if code >= 41 else "gemm_bf16_umma_pair" \
                 if code >= 31 else "attention_prefill_pingpong" if code >= 21 else "gemm_bf16_umma"
             raise LlamaError(f"{kernel} gave up waiting for {names.get(code, code)}; its result is invalid")
 
@@ -136,8 +142,71 @@ def tile_choice(M: int, N: int, K: int = 2048, mode: int = 0, pairs: int = 0, mu
     return best
 
 
-def _wide(M: int, N: int) -> bool:
-    return tile_choice(M, N) >= 1
+def _tile_time(M: int, N: int, K: int, mode: int, pairs: int) -> float:
+    """us that tile_choice's tile is estimated to take, on the scale of wide_plan: 0.3 us for 64 of K of a 128 x 128 tile."""
+    k_blocks = -(-K // 64)
+    costs = [-(-(-(-M // rows) * -(-N // columns)) // SM_COUNT) * cost for index, (rows, columns, cost) in enumerate(_tile_costs(K, mode))
+             if not (pairs > 0 and index == 2)]
+    if pairs > 0:
+        costs.append(_pair_cost(K, -(-(-(-M // 256) * -(-N // 256)) // pairs)))
+    return max(min(costs) * k_blocks * 0.3, N * K * 2 / 6e6) + 4.0
+
+
+# us for 64 of K of a tile of 256 weight rows and so many activation rows on a pair of SMs
+WIDE_BLOCK = {64: 0.21, 96: 0.215, 128: 0.23, 160: 0.265, 192: 0.29, 224: 0.345, 256: 0.40}
+
+
+@functools.lru_cache(maxsize=4096)
+def wide_plan(M: int, N: int, K: int, mode: int, pairs: int):
+    """(activation rows of a tile, K slices) on the kernel with the weights as the wide operand, or None where the other tiles are
+    estimated to be faster. Mode 2 may be cut into K slices, whose planes the next norm adds; the others never are.
+
+    An item's time is its blocks of 64 of K times WIDE_BLOCK, as measured in steady state (389 cycles at 192 rows, whose products take
+    384; the clock falls with the width under the power cap), 5 us a product for start-up and the last epilogue, and the weights come
+    at 6.2 TB/s at best. A plane costs its write and the norm's read. us, in brackets the tiles with the activations as the wide operand, in
+    chains over more weights than L2 holds: 3072 x 2048 128 rows 9.2 (12.1), 529 rows 11.5 (12.2); 6144 x 4096 128 rows 16.7 (21.1), 529 rows
+    23.4 (27.4), 1,024 rows 40.6 (44.7); gated 16384 x 2048 180 rows 17.2 (20.0), 529 rows 32.0 (37.8); gated 28672 x 4096 300 rows 72.5
+    (84.9), 529 rows 99.8 (115.9); 2048 x 2048 529 rows 10.4 (13.0), 2,500 rows 20.0 (26.0); 4096 x 14336 300 rows 35.0 in two planes
+    (41.4 in three), 600 rows 61.2 (74.6), 1,280 rows 121 (171). Where full tiles of 256 x 256 on the pairs fill their rounds they are as
+    good or better: gated 28672 x 4096 1,024 rows 169 against 180, 4096 x 14336 2,048 rows 170 against 173."""
+    k_blocks, columns = -(-K // 64), -(-N // 256)
+    best = None
+    for rows, block in WIDE_BLOCK.items():
+        tiles = columns * -(-M // rows)
+        for wanted in range(1, 9 if mode == 2 else 2):
+            per_slice = -(-k_blocks // wanted)
+            slices = -(-k_blocks // per_slice)
+            if slices != wanted or (slices > 1 and per_slice < 4):
+                continue
+            time = max(-(-tiles * slices // pairs) * per_slice * block, N * K * 2 / 6.2e6) + 5.0
+            if slices > 1:
+                time += slices * (2.0 * M * N * 4 / 3.5e6)
+            if best is None or time < best[0]:
+                best = (time, rows, slices)
+    sliced = mode == 2 and best[2] > 1
+    if not sliced and 0.97 * _tile_time(M, N, K, mode, pairs) <= best[0]:
+        return None
+    return best[1], best[2]
+
+
+def _wide(x: torch.Tensor, weight: torch.Tensor, mode: int, umma_ok: bool):
+    """wide_plan where that kernel takes the product at all."""
+    M, K = x.shape
+    N = weight.shape[0]
+    if M <= 64 or not umma_ok or no_wide or umma_width is not None or N % 2 or (mode == 3 and N % 16):
+        return None
+    pairs = pair_room()
+    if pairs == 0:
+        return None
+    return wide_shape or wide_plan(M, N, K, mode, pairs)
+
+
+def gemm_bf16_wide(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, mode: int, rows: int, slices: int = 1) -> None:
+    """gemm_bf16 (modes 0 to 3), or K slices as planes [slices, M, N] (mode 4), in tiles of 256 weight rows and `rows` rows of x."""
+    M, K = x.shape
+    mark_status_dirty()
+    _done(library.load().lrm_gemm_bf16_wide(_ptr(x), _ptr(weight), _ptr(out), M, weight.shape[0], K, mode, rows, slices,
+                                            _ptr(_status_word(x.device)), _stream()), "gemm_bf16_wide")
 
 
 STREAM_ROWS = 8  # up to this many rows the streaming kernel is always the faster one
@@ -257,6 +326,13 @@ def gemm_bf16_slices(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Te
         # A short prompt (a few hundred rows): few tiles and a long K leave most SMs idle (the 2048 x
         # 8192 product of a 128-token prompt: 16 CTAs, 42 us), so K is cut until the items fill the
         # SMs once, no slice shorter than 256 (the same product in 9 slices: 12 us).
+        wide = _wide(x, weight, 2, umma_ok)
+        if wide is not None:
+            if wide[1] == 1:
+                return None
+            out = torch.empty((wide[1], M, N), dtype=torch.float32, device=x.device)
+            gemm_bf16_wide(x, weight, out, 4, *wide)
+            return out
         tile, splits = _sliced_plan(M, N, K)
         planes = lib.lrm_gemm_bf16_umma_slices(K, splits) if splits > 1 else 1
         if planes <= 1:
@@ -331,6 +407,11 @@ def gemm_bf16(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, mode: in
         gemm_bf16_few(x, weight, out, mode)
         return
     stream_ok, umma_ok = _fast_kernels(x, weight, lib)
+    if M > 64 and mode <= 3 and out.data_ptr() % 4 == 0:
+        wide = _wide(x, weight, 1 if mode == 2 else mode, umma_ok)  # whole: out takes no planes
+        if wide is not None:
+            gemm_bf16_wide(x, weight, out, mode, wide[0])
+            return
     tile, splits = tile_choice(M, N, K, mode, pair_room() if umma_ok and M > 64 else 0), 1
     if stream_ok and umma_ok and M > STREAM_ROWS and not force_stream:
         use_umma, splits = _few_rows_plan(M, N, K, mode)
