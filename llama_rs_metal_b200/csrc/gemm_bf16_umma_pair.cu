@@ -150,13 +150,12 @@ __global__ __launch_bounds__(kPairThreads, 1) void gemm_bf16_umma_pair_kernel(
               for (int k = 0; k < PK / P_UMMA_K; ++k)
                 umma_bf16_pair(tmem_d, smem_desc(a + k * P_UMMA_K * 2), smem_desc(b + k * P_UMMA_K * 2), idesc,
                                (kb > 0 || k > 0) ? 1u : 0u);
-              umma_commit_pair(empty + s, 3);  // both CTAs' loaders may refill the stage
+              if (kb + 1 == k_blocks) umma_commit_pair(acc_full + acc, 3);  // both CTAs' epilogues may read (as in gemm_bf16_umma.cu)
+              umma_commit_pair(empty + s, 3);                         // both CTAs' loaders may refill the stage
             }
             __syncwarp();
           }
         }
-        if (chosen) umma_commit_pair(acc_full + acc, 3);  // both CTAs' epilogues may read
-        __syncwarp();
       }
     }
   } else {

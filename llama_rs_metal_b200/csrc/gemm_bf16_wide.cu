@@ -214,13 +214,12 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_wide_kernel(const __gri
 #pragma unroll
               for (int k = 0; k < BK / UMMA_K; ++k)
                 umma_bf16_pair(tmem_d, smem_desc(a + k * UMMA_K * 2), smem_desc(b + k * UMMA_K * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-              umma_commit_pair(empty + s, 3);  // both CTAs' loaders may refill the stage
+              if (kb + 1 == count) umma_commit_pair(acc_full + acc, 3);  // both CTAs' epilogues may read (as in gemm_bf16_umma.cu)
+              umma_commit_pair(empty + s, 3);                         // both CTAs' loaders may refill the stage
             }
             __syncwarp();
           }
         }
-        if (chosen) umma_commit_pair(acc_full + acc, 3);  // both CTAs' epilogues may read
-        __syncwarp();
       }
     }
   } else {
