@@ -12,7 +12,8 @@
 // wait before it leaves. Nothing goes through global memory between the split and the merge,
 // and no second kernel runs. A cluster of one CTA writes its output without any of this.
 //
-// The step's fused q|k|v projection is the input. The CTA that owns the sequence's last page
+// The step's fused q|k|v projection is the input: bfloat16, or the float32 planes of its K slices, whose sum is rounded to
+// bfloat16 here, by every CTA for the rows it needs. The CTA that owns the sequence's last page
 // rotates the new k row, writes it and the v row to the cache and places both in its shared
 // tile, so the first cache pages are in flight while q and the new row are rotated.
 //
@@ -69,7 +70,8 @@ __global__ __launch_bounds__(kThreads) void attention_decode_cluster_kernel(
     __nv_bfloat16* __restrict__ v_pages, const int* __restrict__ dest_rows,
     __nv_bfloat16* __restrict__ out, const int* __restrict__ page_table, int table_stride,
     const int* __restrict__ slots, const int* __restrict__ kv_lens, int q_heads, int kv_heads,
-    int row_groups, float scale_log2, const int* __restrict__ order) {
+    int row_groups, float scale_log2, const int* __restrict__ order, const float* __restrict__ planes, int n_planes,
+    long long plane_stride, int fresh_at) {
   constexpr int STRIDE = D + 8, TILE = kTile * STRIDE, PART = D + 2, kStages = stages_of<D>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float cs_tab[D / 2], sn_tab[D / 2];
@@ -140,24 +142,44 @@ __global__ __launch_bounds__(kThreads) void attention_decode_cluster_kernel(
   float ka = 0.f, kb = 0.f;
   int ia = 0, ib = 0;
   __nv_bfloat16 v_new = __float2bfloat16_rn(0.f);
-  if (owner) {
-    const __nv_bfloat16* k_src = src + static_cast<size_t>(q_heads + kh) * D;
-    if (threadIdx.x < D / 2) {
-      const int i = threadIdx.x;
-      if (rotate && i < half) {
-        ia = i;
-        ib = i + half;
-      } else {
-        ia = (rotate ? rotary : 0) + 2 * (i - (rotate ? half : 0));
-        ib = ia + 1;
+  auto take = [&](const __nv_bfloat16* q_src, const __nv_bfloat16* k_src, const __nv_bfloat16* v_src) {
+    if (owner) {
+      if (threadIdx.x < D / 2) {
+        const int i = threadIdx.x;
+        if (rotate && i < half) {
+          ia = i;
+          ib = i + half;
+        } else {
+          ia = (rotate ? rotary : 0) + 2 * (i - (rotate ? half : 0));
+          ib = ia + 1;
+        }
+        ka = __bfloat162float(k_src[ia]);
+        kb = __bfloat162float(k_src[ib]);
       }
-      ka = __bfloat162float(k_src[ia]);
-      kb = __bfloat162float(k_src[ib]);
+      if (threadIdx.x < D) v_new = v_src[threadIdx.x];
     }
-    if (threadIdx.x < D) v_new = src[static_cast<size_t>(q_heads + kv_heads + kh) * D + threadIdx.x];
+    load_q<D>(qa, q_src, D, rows);
+  };
+  __nv_bfloat16* fresh = reinterpret_cast<__nv_bfloat16*>(smem_raw + fresh_at);  // planes: q rows, the new k, the new v
+  if (planes == nullptr) {
+    take(src + static_cast<size_t>(head0) * D, src + static_cast<size_t>(q_heads + kh) * D,
+         src + static_cast<size_t>(q_heads + kv_heads + kh) * D);
+  } else {
+    const float* from = planes + b * qkv_row;
+    for (int i = threadIdx.x; i < (rows + (owner ? 2 : 0)) * (D / 2); i += kThreads) {
+      const int r = i / (D / 2), c = 2 * (i % (D / 2));
+      const float* at = from + static_cast<size_t>(r < rows ? head0 + r : q_heads + (r - rows) * kv_heads + kh) * D + c;
+      float2 sum = *reinterpret_cast<const float2*>(at);
+#pragma unroll 4
+      for (int p = 1; p < n_planes; ++p) {
+        const float2 more = *reinterpret_cast<const float2*>(at + p * plane_stride);
+        sum.x += more.x, sum.y += more.y;
+      }
+      *reinterpret_cast<uint32_t*>(fresh + r * D + c) = pack_bf16(sum.x, sum.y);
+    }
   }
-  load_q<D>(qa, src + static_cast<size_t>(head0) * D, D, rows);
-  __syncthreads();  // the table is complete
+  __syncthreads();  // the table (and what the planes gave) is complete
+  if (planes != nullptr) take(fresh, fresh + rows * D, fresh + (rows + 1) * D);
   if (rotate) {
     // the partner of column c is column c + half: fragment ks + half / 16
     if (half == 16) rotate_q<D, 1>(qa, cs_tab, sn_tab);
@@ -339,12 +361,14 @@ template <int D> int smem_bytes(int cluster, int rows) {
   const int runs = (rows * D + 127) / 128, runs_each = (runs + cluster - 1) / cluster;
   return ring + cluster * (runs_each * 128 + 32) * 4;
 }
+// and behind it, for a projection that comes as planes, the rows that a CTA needs of it.
+template <int D> int fresh_bytes(int rows) { return (rows + 2) * D * 2; }
 
 
 template <int D> int prepare(int cluster) {
   auto kernel = attention_decode_cluster_kernel<D>;
   int most = 0;  // over every cluster size and up to 16 query heads per kv head
-  for (int c = 1; c <= 16; ++c) most = max(most, smem_bytes<D>(c, 16));
+  for (int c = 1; c <= 16; ++c) most = max(most, smem_bytes<D>(c, 16) + fresh_bytes<D>(16));
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
   if (e != cudaSuccess) return static_cast<int>(e);
   if (cluster > 8) {
@@ -358,7 +382,7 @@ template <int D> void fill_config(cudaLaunchConfig_t& config, cudaLaunchAttribut
                                   int cluster, int rows, cudaStream_t stream) {
   config.gridDim = dim3(pairs * cluster);
   config.blockDim = dim3(kThreads);
-  config.dynamicSmemBytes = smem_bytes<D>(cluster, rows);
+  config.dynamicSmemBytes = smem_bytes<D>(cluster, rows) + fresh_bytes<D>(rows);
   config.stream = stream;
   attributes[0].id = cudaLaunchAttributeClusterDimension;
   attributes[0].val.clusterDim.x = cluster;
@@ -397,7 +421,7 @@ template <int D> int launch(const void* qkv, const int* positions, const float* 
                             void* k_pages, void* v_pages, const int* dest_rows, void* out,
                             const int* page_table, int table_stride, const int* slots, const int* kv_lens,
                             int seqs, int q_heads, int kv_heads, float scale, int cluster,
-                            cudaStream_t stream, const int* order = nullptr) {
+                            cudaStream_t stream, const int* order, const float* planes, int n_planes) {
   int code = prepare<D>(cluster);
   if (code != 0) return code;
   const int group = q_heads / kv_heads, row_groups = (group + 15) / 16;
@@ -408,7 +432,8 @@ template <int D> int launch(const void* qkv, const int* positions, const float* 
       &config, attention_decode_cluster_kernel<D>, static_cast<const __nv_bfloat16*>(qkv), positions,
       inv_freq, rotary, static_cast<__nv_bfloat16*>(k_pages), static_cast<__nv_bfloat16*>(v_pages),
       dest_rows, static_cast<__nv_bfloat16*>(out), page_table, table_stride, slots, kv_lens, q_heads,
-      kv_heads, row_groups, scale * 1.4426950408889634f, order);
+      kv_heads, row_groups, scale * 1.4426950408889634f, order, planes, n_planes,
+      static_cast<long long>(seqs) * (q_heads + 2 * kv_heads) * D, smem_bytes<D>(cluster, min(group, 16)));
   return e == cudaSuccess ? 0 : static_cast<int>(e);
 }
 
@@ -430,12 +455,13 @@ LRM_API int lrm_attention_decode_cluster_resident(int head_dim, int cluster, int
   return 0;
 }
 
-// qkv: [seqs, (q_heads + 2 kv_heads) * d] bfloat16, this step's fused projection, unrotated.
+// qkv: [seqs, (q_heads + 2 kv_heads) * d] bfloat16, this step's fused projection, unrotated; or, with n_planes > 0, float32
+// [n_planes, seqs, (q_heads + 2 kv_heads) * d], whose sum over the planes, rounded to bfloat16, is the projection.
 // positions, dest_rows, slots, kv_lens: int32 [seqs]; kv_lens counts the new token;
 // dest_rows[b] = page * 64 + row where the new key/value row is stored. out: [seqs, q_heads, d].
 // order: int32 [seqs] or nullptr: the sequences in the order their clusters are to start (the longest
 // first: clusters beyond what the device holds at once then are those of the short sequences).
-LRM_API int lrm_attention_decode_cluster(const void* qkv, const int* positions, const float* inv_freq,
+LRM_API int lrm_attention_decode_cluster(const void* qkv, int n_planes, const int* positions, const float* inv_freq,
                                          int rotary, void* k_pages, void* v_pages, const int* dest_rows,
                                          void* out, const int* page_table, int table_stride,
                                          const int* slots, const int* kv_lens, int seqs, int q_heads,
@@ -444,12 +470,14 @@ LRM_API int lrm_attention_decode_cluster(const void* qkv, const int* positions, 
   if (seqs <= 0) return 0;
   if (q_heads <= 0 || kv_heads <= 0 || q_heads % kv_heads != 0 || cluster < 1 || cluster > 16)
     return LRM_BAD_ARGUMENT;
+  if (n_planes < 0) return LRM_BAD_ARGUMENT;
+  const float* planes = n_planes > 0 ? static_cast<const float*>(qkv) : nullptr;
   if (inv_freq == nullptr) rotary = 0;
   if (!lrm_attention_decode_cluster_supports(head_dim, page_size, rotary)) return LRM_UNSUPPORTED;
 #define LRM_CASE(DIM)                                                                                  \
   if (head_dim == DIM)                                                                                 \
     return launch<DIM>(qkv, positions, inv_freq, rotary, k_pages, v_pages, dest_rows, out, page_table, \
-                       table_stride, slots, kv_lens, seqs, q_heads, kv_heads, scale, cluster, stream, order);
+                       table_stride, slots, kv_lens, seqs, q_heads, kv_heads, scale, cluster, stream, order, planes, n_planes);
   LRM_CASE(32)
   LRM_CASE(64)
   LRM_CASE(128)

@@ -7,13 +7,14 @@
 // accumulator's lanes are weight rows: a thread has one output column for all activation rows, and neighbouring threads
 // neighbouring columns.
 //
-// Persistent: CTA b works on tiles b, b + gridDim.x, ..., two accumulators in turn, so a tile's epilogue runs under the next
-// tile's reads. No atomics: the result is the same every time. (Narrow products, a cluster of CTAs to a tile with the partial
-// sums meeting in distributed shared memory: 6144 x 4096, 32 rows, 20.6 us against the streaming kernel's 22.2 alone, but a
-// whole step got slower, since the streaming kernels beside it need the shared memory for their L1.)
+// Persistent: CTA b works on items b, b + gridDim.x, ...; an item is a (K slice, tile) with the tiles fastest, two accumulators in
+// turn, so an item's epilogue runs under the next one's reads. Narrow products, whose tiles leave SMs idle, are cut into K slices, each
+// a float32 plane that the reader adds up in order (the next norm, or decode attention for q|k|v): 6144 x 4096, 32 rows, 10.3 us in three
+// planes against 16.4 whole. No atomics: the result is the same every time. (A cluster of CTAs to a tile with the partial sums meeting
+// in distributed shared memory was slower: 20.6 us.)
 //
-// Epilogues as in gemm_bf16_stream.cu: 0 bf16, 1 f32, 3 SiLU gate (blocks of 8 gate / 8 up rows alternate). Every mbarrier wait
-// is bounded. Its times beside those of the kernels it replaces stand at gemm_dispatch.few_takes.
+// Epilogues as in gemm_bf16_stream.cu: 0 bf16, 1 f32, 3 SiLU gate (blocks of 8 gate / 8 up rows alternate), 4 f32 planes of K slices.
+// Every mbarrier wait is bounded. Its times beside those of the kernels it replaces stand at gemm_dispatch.few_takes and few_plan.
 #include "silu.cuh"
 #include "umma.cuh"
 
@@ -62,8 +63,8 @@ __device__ __forceinline__ void finish_gated(const uint32_t (&r)[32], int m0, in
 template <int NC>
 __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                     const __grid_constant__ CUtensorMap map_x, void* __restrict__ out,
-                                                                    int M, int N, int K, int mode, int tile_rows,
-                                                                    int* __restrict__ status) {
+                                                                    int M, int N, int K, int mode, int tile_rows, int kb_per_split,
+                                                                    int splits, int* __restrict__ status) {
   using F = Few<NC>;
   constexpr int STAGES = F::STAGES;
   pdl_trigger();
@@ -78,8 +79,8 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t stage_bytes = tile_rows * BK * 2 + F::STAGE_BYTES - F::W_BYTES;  // of the copies
   const int tiles = (N + tile_rows - 1) / tile_rows, k_blocks = (K + BK - 1) / BK;
-  const int first_tile = blockIdx.x, stride = gridDim.x, num_kb = k_blocks;
-  const int early = min(num_kb, STAGES);  // stages of the first tile's weights asked for ahead of the wait
+  const int items = tiles * splits, first_item = blockIdx.x, stride = gridDim.x;  // an item: (K slice, tile), the tiles fastest
+  const int early = min(min(kb_per_split, k_blocks - first_item / tiles * kb_per_split), STAGES);  // stages of the first item's weights asked for ahead of the wait
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -94,7 +95,7 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
     mbar_fence_init();
     for (int kb = 0; kb < early; ++kb) {
       mbar_expect_tx(full + kb, stage_bytes);
-      tma_load_2d(ring + kb * F::STAGE_BYTES, &map_w, full + kb, kb * BK, first_tile * tile_rows);
+      tma_load_2d(ring + kb * F::STAGE_BYTES, &map_w, full + kb, (first_item / tiles * kb_per_split + kb) * BK, first_item % tiles * tile_rows);
     }
   }
   if (warp == 1) {
@@ -111,10 +112,12 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
     if (lane == 0) {
       // The early stages' activations first, whatever happens: copies into those stages are under way.
       for (int kb = 0; kb < early; ++kb)
-        tma_load_2d(ring + kb * F::STAGE_BYTES + F::W_BYTES, &map_x, full + kb, kb * BK, 0);
+        tma_load_2d(ring + kb * F::STAGE_BYTES + F::W_BYTES, &map_x, full + kb, (first_item / tiles * kb_per_split + kb) * BK, 0);
       uint32_t it = early;  // blocks asked for so far
       int from = early;
-      for (int tile = first_tile; tile < tiles && !*bail; tile += stride, from = 0) {
+      for (int item = first_item; item < items && !*bail; item += stride, from = 0) {
+        const int slice = item / tiles, w_row = (item - slice * tiles) * tile_rows, kb0 = slice * kb_per_split;
+        const int num_kb = min(kb_per_split, k_blocks - kb0);
         for (int kb = from; kb < num_kb; ++kb, ++it) {
           const uint32_t s = it % STAGES, round = it / STAGES;
           if (round > 0 && !mbar_wait(empty + s, (round - 1) & 1, status, kStuckEmpty)) {
@@ -122,8 +125,8 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
             break;
           }
           mbar_expect_tx(full + s, stage_bytes);
-          tma_load_2d(ring + s * F::STAGE_BYTES, &map_w, full + s, kb * BK, tile * tile_rows);
-          tma_load_2d(ring + s * F::STAGE_BYTES + F::W_BYTES, &map_x, full + s, kb * BK, 0);
+          tma_load_2d(ring + s * F::STAGE_BYTES, &map_w, full + s, (kb0 + kb) * BK, w_row);
+          tma_load_2d(ring + s * F::STAGE_BYTES + F::W_BYTES, &map_x, full + s, (kb0 + kb) * BK, 0);
         }
       }
       if (*bail) {  // wait (bounded) for the copies already in flight before the CTA may exit
@@ -139,7 +142,8 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
     const bool chosen = elect_one();
     uint32_t it = 0, local = 0;
     bool going = true;
-    for (int tile = first_tile; tile < tiles && going; tile += stride, ++local) {
+    for (int item = first_item; item < items && going; item += stride, ++local) {
+      const int num_kb = min(kb_per_split, k_blocks - item / tiles * kb_per_split);
       const uint32_t acc = local & 1, use = local >> 1;
       if (__any_sync(0xffffffffu, *bail != 0) ||
           (use > 0 && !__all_sync(0xffffffffu, lane != 0 || mbar_wait(acc_free + acc, (use - 1) & 1, status, kStuckTmemFree)))) {
@@ -163,18 +167,19 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
             for (int k = 0; k < BK / UMMA_K; ++k)
               umma_bf16(tmem + acc * F::SET, smem_desc(a + k * UMMA_K * 2), smem_desc(b + k * UMMA_K * 2), idesc,
                         (kb > 0 || k > 0) ? 1u : 0u);
+            if (kb + 1 == num_kb) umma_commit(acc_full + acc);  // (as in gemm_bf16_umma.cu)
             umma_commit(empty + s);
           }
           __syncwarp();
         }
       }
-      if (chosen) umma_commit(acc_full + acc);
-      __syncwarp();
     }
   } else {
     const int quarter = warp & 3, place = quarter * 32 + lane;  // a warp may touch only this quarter of the lanes
     uint32_t local = 0;
-    for (int tile = first_tile; tile < tiles; tile += stride, ++local) {
+    for (int item = first_item; item < items; item += stride, ++local) {
+      const int slice = item / tiles, tile = item - slice * tiles;
+      void* plane = mode == 4 ? static_cast<void*>(static_cast<float*>(out) + static_cast<size_t>(slice) * M * N) : out;
       const uint32_t acc = local & 1;
       if (*bail || !mbar_wait(acc_full + acc, (local >> 1) & 1, status, kStuckAccumulator)) {
         *bail = 1;
@@ -196,7 +201,7 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
         for (int i = 0; i < ROWS; ++i) {
           const int m = c * 32 + i;
           if (m >= M || !stored) break;
-          finish(__uint_as_float(r[i]), m, n, out, N, mode);
+          finish(__uint_as_float(r[i]), m, n, plane, N, mode);
         }
       }
       tc_fence_before();
@@ -210,27 +215,29 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
 }
 
 template <int NC>
-int launch(const void* X, const void* W, void* out, int M, int x_rows, int N, int K, int mode, int* status, cudaStream_t stream) {
+int launch(const void* X, const void* W, void* out, int M, int x_rows, int N, int K, int mode, int splits, int rows_wanted, int* status, cudaStream_t stream) {
   // Fewer weight rows to a tile where that leaves the CTA with the most tiles fewer rows to read (the others wait for it, and a part
   // of the SMs does not draw the whole bandwidth). The products work on 128 rows either way; those beyond are not stored. (8 rows:
   // what a tile costs beside its reads.) With the whole warp issuing and the gate's quotients side by side, us, 32 rows: 28672 x
   // 4096 43.1 -> 40.3 (gated 53.3 -> 41.0), 9472 x 22000 103 -> 84.
   int tile_rows = kTileRows, least = 0;
   for (int rows = kTileRows; rows >= 64; rows -= 16) {
-    const int cost = ((N + rows - 1) / rows + kSmCount - 1) / kSmCount * (rows + 8);
+    const int cost = ((N + rows - 1) / rows * splits + kSmCount - 1) / kSmCount * (rows + 8);
     if (least == 0 || cost < least) {
       least = cost;
       tile_rows = rows;
     }
   }
+  if (rows_wanted > 0) tile_rows = rows_wanted;
   CUtensorMap map_w, map_x;
   if (!make_map_bf16(&map_w, W, N, K, tile_rows) || !make_map_bf16(&map_x, X, x_rows, K, NC)) return LRM_UNSUPPORTED;
   auto kernel = gemm_bf16_few_kernel<NC>;
   constexpr int smem = static_cast<int>(Few<NC>::BYTES);
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return static_cast<int>(e);
-  const int tiles = (N + tile_rows - 1) / tile_rows;
-  LRM_LAUNCH(kernel, dim3(tiles < kSmCount ? tiles : kSmCount), kThreads, smem, stream, map_w, map_x, out, M, N, K, mode, tile_rows, status);
+  const int items = (N + tile_rows - 1) / tile_rows * splits, k_blocks = (K + BK - 1) / BK;
+  LRM_LAUNCH(kernel, dim3(items < kSmCount ? items : kSmCount), kThreads, smem, stream, map_w, map_x, out, M, N, K, mode, tile_rows,
+             (k_blocks + splits - 1) / splits, splits, status);
   return 0;
 }
 
@@ -241,15 +248,23 @@ LRM_API int lrm_gemm_bf16_few_supports(int M, int N, int K) {
   return M >= 1 && M <= 64 && N >= 1 && K >= 8 && K % 8 == 0 && encode_tiled() != nullptr ? 1 : 0;
 }
 
-// `x_rows` >= M: rows of X that may be read (TMA was measured slower on maps of fewer than 32 rows). `status`: one int in device memory, 0 before the launch.
-LRM_API int lrm_gemm_bf16_few(const void* X, const void* W, void* out, int M, int x_rows, int N, int K, int mode,
+// K slices a product in `wanted` slices really has: none is empty.
+LRM_API int lrm_gemm_bf16_few_slices(int K, int wanted) {
+  const int k_blocks = (K + BK - 1) / BK, per_split = (k_blocks + wanted - 1) / wanted;
+  return (k_blocks + per_split - 1) / per_split;
+}
+
+// `x_rows` >= M: rows of X that may be read (TMA was measured slower on maps of fewer than 32 rows). `splits` (mode 4): as
+// lrm_gemm_bf16_few_slices says; out is [splits, M, N]. `status`: one int in device memory, 0 before the launch.
+LRM_API int lrm_gemm_bf16_few(const void* X, const void* W, void* out, int M, int x_rows, int N, int K, int mode, int splits, int tile_rows,
                               int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (!lrm_gemm_bf16_few_supports(M, N, K)) return LRM_UNSUPPORTED;
-  if ((mode != 0 && mode != 1 && mode != 3) || (mode == 3 && N % 16 != 0) || x_rows < M || status == nullptr)
+  if ((mode != 0 && mode != 1 && mode != 3 && mode != 4) || (mode == 3 && N % 16 != 0) || x_rows < M || status == nullptr || splits < 1 ||
+      (splits > 1 && mode != 4) || splits != lrm_gemm_bf16_few_slices(K, splits) || tile_rows < 0 || tile_rows > kTileRows || tile_rows % 16)
     return LRM_BAD_ARGUMENT;
   if (reinterpret_cast<uintptr_t>(X) % 16 || reinterpret_cast<uintptr_t>(W) % 16) return LRM_UNSUPPORTED;
-  if (M <= 16) return launch<16>(X, W, out, M, x_rows, N, K, mode, status, stream);
-  if (M <= 32) return launch<32>(X, W, out, M, x_rows, N, K, mode, status, stream);
-  return launch<64>(X, W, out, M, x_rows, N, K, mode, status, stream);
+  if (M <= 16) return launch<16>(X, W, out, M, x_rows, N, K, mode, splits, tile_rows, status, stream);
+  if (M <= 32) return launch<32>(X, W, out, M, x_rows, N, K, mode, splits, tile_rows, status, stream);
+  return launch<64>(X, W, out, M, x_rows, N, K, mode, splits, tile_rows, status, stream);
 }

@@ -489,11 +489,11 @@ def decode_cluster_size(seqs: int, kv_heads: int, group: int, head_dim: int, max
 
 def decode_fused(qkv, positions, inv_freq, rotary: int, kv, dest_rows, out, slots, kv_lens, max_kv_len: int,
                  q_heads: int, scale: float, order=None, fill: int = 4) -> None:
-    B = qkv.shape[0]
+    planes, B = (qkv.shape[0], qkv.shape[1]) if qkv.dim() == 3 else (0, qkv.shape[0])
     d = kv.head_dim
     cluster = decode_cluster_size(B, kv.kv_heads, q_heads // kv.kv_heads, d, max_kv_len, fill if order is not None else 4)
     _done(library.load().lrm_attention_decode_cluster(
-        _ptr(qkv), _ptr(positions), _ptr(inv_freq), rotary, _ptr(kv.k), _ptr(kv.v), _ptr(dest_rows), _ptr(out),
+        _ptr(qkv), planes, _ptr(positions), _ptr(inv_freq), rotary, _ptr(kv.k), _ptr(kv.v), _ptr(dest_rows), _ptr(out),
         _ptr(kv.page_table), kv.page_table.shape[1], _ptr(slots), _ptr(kv_lens), B, q_heads, kv.kv_heads, d,
         kv.page_size, ctypes.c_float(scale), cluster, _ptr(order), _stream()), "attention_decode_cluster")
 
@@ -606,19 +606,26 @@ def attend(projected, *, q_heads: int, kv_heads: int, head_dim: int, rotary, ctx
                 q, k, v = fused
                 ctx.fresh_kv[cache_entry] = (k, v)
                 return ops.attention_prefill(q, k, v, ctx.cu_seqlens, ctx.seq_of_token, ctx.max_seq_len, scale, window)
-        projected = ops.linear(x, weight)
     if writes_cache:
-        if (phase == "decode" and cache is not None and projected.dtype == torch.bfloat16
-                and decode_fused_supported(projected.dtype, head_dim, cache.page_size, width,
+        source = projection[0] if projection is not None else projected
+        if (phase == "decode" and cache is not None and source.dtype == torch.bfloat16
+                and decode_fused_supported(source.dtype, head_dim, cache.page_size, width,
                                            window or cache.window)
-                and decode_prefers_fused(projected.shape[0], kv_heads, q_heads // kv_heads, head_dim,
+                and decode_prefers_fused(source.shape[0], kv_heads, q_heads // kv_heads, head_dim,
                                          ctx.max_kv_len, ctx.kv_fill)):
             # rotation, cache write, attention and the merge of the splits in one launch
             # the order comes with the step's arrays: the kernel reads it before it waits
-            order = ctx.longest_first if projected.shape[0] > 1 else None
+            order = ctx.longest_first if source.shape[0] > 1 else None
+            if projection is not None:  # a narrow product's K slices are added up in that launch too
+                projected = ops.linear_few_slices(*projection)
+                if projected is None:
+                    projected = ops.linear(*projection)
             return ops.attention_decode_fused(projected, q_heads, inv_freq, width, ctx.positions, cache,
                                               ctx.dest_rows[cache.group], ctx.slots, ctx.kv_lens,
                                               ctx.max_kv_len, scale, order, ctx.kv_fill)
+    if projection is not None:
+        projected = ops.linear(*projection)
+    if writes_cache:
         prefill = phase == "prefill"
         q, k, v = ops.rope_store(projected, q_heads, kv_heads, head_dim, inv_freq, width, ctx.positions,
                                  kv=cache, dest_rows=ctx.dest_rows[cache.group] if cache is not None else None,

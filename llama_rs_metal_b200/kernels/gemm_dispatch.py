@@ -1,10 +1,10 @@
 """Which bfloat16 matrix-product kernel runs for a shape.
 
-* up to 8 rows (small decode batches): the weight-streaming kernel
-  (csrc/gemm_bf16_stream.cu); it also takes 9-64 rows when the tensor-core kernel would
-  leave most SMs idle and cannot split K (few output columns, epilogue other than "add");
-* 13 to 64 rows of products large enough: tcgen05 with the weights as its wide operand
-  (csrc/gemm_bf16_few.cu; few_takes says where it is the faster one);
+* up to 64 rows (decode steps): tcgen05 with the weights as its wide operand (csrc/gemm_bf16_few.cu),
+  in K slices where the product is narrow and its reader adds planes; few_plan says where it is the
+  faster one;
+* up to 8 rows of smaller matrices, and what is narrow and cannot be cut: the weight-streaming kernel
+  (csrc/gemm_bf16_stream.cu);
 * 65 to some 1,300 rows, wherever its tiles waste less: tcgen05 over pairs of SMs with the weights as
   the wide operand (csrc/gemm_bf16_wide.cu; wide_plan);
 * more rows (prompts): the TMA + tcgen05 kernel
@@ -209,7 +209,7 @@ def gemm_bf16_wide(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, mod
                                             _ptr(_status_word(x.device)), _stream()), "gemm_bf16_wide")
 
 
-STREAM_ROWS = 8  # up to this many rows the streaming kernel is always the faster one
+STREAM_ROWS = 8  # up to this many rows the streaming kernel is faster than the tiles with the rows as the wide operand
 force_stream = False  # tests: keep 17-64 rows on the streaming kernel
 stream_shape = None  # tests and tuning: (warps per CTA, K slices) of the streaming kernel instead of its own rule
 
@@ -232,27 +232,70 @@ def _few_rows_plan(M: int, N: int, K: int, mode: int):
 
 
 def few_takes(M: int, N: int, K: int, mode: int) -> bool:
-    """Where the kernel with the weights as the wide tcgen05 operand runs: 13 to 64 rows of products with tiles enough. Its ring
-    holds 200 KB per SM on their way and reads at 6 TB/s. us in a chain of products over more weights than L2 holds, in
-    brackets the tile kernel. bfloat16 results: 16384 x 2048 16 rows 12.2 (14.8), 32 rows 13.0 (15.0), 28672 x 4096 16 rows
-    39.1 (46.9), 32 rows 40.3 (47.5), 49408 x 4096 32 rows 65.9 (72.3), 64 rows 70.4 (73.4), 128256 x 2048 64 rows 84.1 (88.9),
-    a tile for half the SMs only, 9472 x 22000 32 rows 84.1 (103.4). Gated: 16384 x 2048 16 rows 12.4 (15.5), 32 rows 13.5
-    (15.4), 28672 x 4096 32 rows 41.0 (48.2), 49408 x 4096 48 rows 70.9 (73.2). The line for more than 32 rows is that of both
-    kernels' earlier epilogues and leaves up to 9 % behind: 28672 x 4096 33 rows 43.0 against 47.0, 64 rows 44.1 against 47.7, gated 45.7
-    against 47.6 and 47.3 against 48.0; 16384 x 3072 64 rows 21.0 against 21.7, gated 24.3 against 21.9. Up to 12 rows the streaming kernel stays: its like beside it
-    live off the L1 that this kernel's ring takes from them (3 sequences, one layer of the 8B shape: 231 us a step against 177,
-    with this kernel's former times)."""
+    """Whole products of 13 to 64 rows that were timed on the kernel with the weights as the wide tcgen05 operand against the tile
+    kernel first (few_plan goes on from here): its ring holds 200 KB per SM on their way and reads at 6 TB/s. us in a chain of products
+    over more weights than L2 holds, in brackets the tile kernel. bfloat16 results: 16384 x 2048 16 rows 12.2 (14.8), 32 rows 13.0 (15.0),
+    28672 x 4096 16 rows 39.1 (46.9), 32 rows 40.3 (47.5), 49408 x 4096 32 rows 65.9 (72.3), 64 rows 70.4 (73.4), 128256 x 2048 64 rows
+    84.1 (88.9), 9472 x 22000 32 rows 84.1 (103.4). Gated: 16384 x 2048 16 rows 12.4 (15.5), 32 rows 13.5 (15.4), 28672 x 4096 32 rows 41.0
+    (48.2), 49408 x 4096 48 rows 70.9 (73.2)."""
     if not 12 < M <= (48 if mode == 3 else 64):
         return False
     tiles = -(-N // 128)
     return mode in (0, 1, 3) and tiles >= (SM_COUNT // 2 if M <= 32 else SM_COUNT) and N * K >= (30e6 if M <= 32 else 200e6)
 
 
-def _few(x: torch.Tensor, weight: torch.Tensor, mode: int, lib) -> bool:
+def few_plan(M: int, N: int, K: int, mode: int, added: bool = False) -> int:
+    """K slices (1: whole) on the kernel with the weights as the wide operand, 0 where another kernel is the faster one. Mode 4 may be
+    cut; the others never are. `added`: the slices go to a norm, which adds them to the residual stream.
+
+    Narrow products are cut until their items fill the SMs. us in chains of products, in brackets the streaming or the tile kernel:
+    6144 x 4096 in three slices 8 rows 9.7 (11.9), 32 rows 10.3 (22.4), 64 rows 11.5 (40.7); 5120 x 3072 9 rows 7.7 (12.2), 48 rows 9.0
+    (28.2); 4096 x 14336 in four 8 rows 20.5 (25.5), 32 rows 21.4 (24.2); 2048 x 8192 in nine 12 rows 7.7 (9.8), 64 rows 9.0 (10.3). Whole:
+    28672 x 4096 gated 8 rows 39.4 (49.7), 12 rows 39.3 (62.1), 64 rows 44.5 (47.7); 32768 x 4096 8 rows 43.2 (51.6), 12 rows 43.5 (66.1);
+    8192 x 2048 24 rows 10.1 (13.1), 12 rows 9.8 (9.3); 5120 x 3072 12 rows 12.5 (12.7), 64 rows 15.0 (31.5).
+
+    A norm that adds planes takes 2 to 4 us more than one behind a product that was added in place (4096 x 4096 with its norm, 8 rows:
+    11.4 against 9.8 streamed; 3072 x 3072 9.2 against 6.8; 2048 x 2048 16 rows 6.6 against 6.0, 64 rows 8.1 against 10.3), so small
+    products of few rows that go to one stream. Up to 8 rows the products of small matrices stream too, which then keep their L1 from
+    layer to layer. Whole steps of two layers and a head of 32,768, all streamed / by this rule: 3B shape 4 sequences 179.6 / 172.1 us,
+    8B shape 4 283 / 258, 8 299 / 267; before this rule / by it: 1B shape 9 sequences 165 / 141, 48 196 / 182, 3B shape 12 268 / 190, 48
+    288 / 246, 8B shape 12 373 / 274, 48 400 / 343."""
+    if M > 64 or mode not in (0, 1, 3, 4):
+        return 0
+    if few_takes(M, N, K, mode):
+        return 1
+    large, head = min(N, K) >= 3072, N >= 32768
+    if M <= STREAM_ROWS and not large and not head:
+        return 0
+    if added and (M <= 32 and N * K <= 4 * 1024 * 1024 or M <= STREAM_ROWS and N * K <= 16 * 1024 * 1024):
+        return 0
+    tiles = -(-N // 128)
+    if mode == 4:
+        k_blocks = -(-K // 64)
+        per_slice = max(4, -(-k_blocks // max(1, SM_COUNT // tiles)))
+        return -(-k_blocks // per_slice)
+    return 1 if tiles >= SM_COUNT // 2 or (large and tiles >= 64) or (M > 16 and tiles >= 40) else 0
+
+
+def _few(x: torch.Tensor, weight: torch.Tensor, mode: int, lib, added: bool = False) -> int:
+    """few_plan where the kernel takes the product at all."""
     M, K = x.shape
     N = weight.shape[0]
-    return (few_takes(M, N, K, mode) and not force_tiled and not force_stream and stream_shape is None and umma_width is None
-            and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0 and bool(lib.lrm_gemm_bf16_few_supports(M, N, K)))
+    if (M > 64 or force_tiled or force_stream or stream_shape is not None or umma_width is not None or x.data_ptr() % 16
+            or weight.data_ptr() % 16 or (mode == 3 and N % 16)):
+        return 0
+    slices = few_plan(M, N, K, mode, added)
+    return slices if slices and lib.lrm_gemm_bf16_few_supports(M, N, K) else 0
+
+
+def gemm_bf16_few_slices(x: torch.Tensor, weight: torch.Tensor, added: bool = False) -> Optional[torch.Tensor]:
+    """x . weight^T as planes over K slices from that kernel, or None where it is not to be cut there."""
+    slices = _few(x, weight, 4, library.load(), added)
+    if slices <= 1:
+        return None
+    out = torch.empty((slices, x.shape[0], weight.shape[0]), dtype=torch.float32, device=x.device)
+    gemm_bf16_few(x, weight, out, 4, slices)
+    return out
 
 
 def _held_rows(x: torch.Tensor) -> int:
@@ -262,12 +305,12 @@ def _held_rows(x: torch.Tensor) -> int:
     return min(max(M, 32), max(M, held))
 
 
-def gemm_bf16_few(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, mode: int) -> None:
-    """gemm_bf16 (modes 0, 1, 3) for up to 64 rows on the kernel with the weights as the wide operand."""
+def gemm_bf16_few(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, mode: int, slices: int = 1, rows: int = 0) -> None:
+    """gemm_bf16 (modes 0, 1, 3), or K slices as planes (mode 4), for up to 64 rows on the kernel with the weights as the wide operand."""
     M, K = x.shape
     lib = library.load()
     mark_status_dirty()
-    _done(lib.lrm_gemm_bf16_few(_ptr(x), _ptr(weight), _ptr(out), M, _held_rows(x), weight.shape[0], K, mode,
+    _done(lib.lrm_gemm_bf16_few(_ptr(x), _ptr(weight), _ptr(out), M, _held_rows(x), weight.shape[0], K, mode, slices, rows,
                                 _ptr(_status_word(x.device)), _stream()), "gemm_bf16_few")
 
 
@@ -319,6 +362,9 @@ def gemm_bf16_slices(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Te
     M, K = x.shape
     N = weight.shape[0]
     lib = library.load()
+    planes = gemm_bf16_few_slices(x, weight, added=True)
+    if planes is not None:
+        return planes
     stream_ok, umma_ok = _fast_kernels(x, weight, lib)
     if not stream_ok:
         if not umma_ok or M <= 64:
@@ -403,7 +449,7 @@ def gemm_bf16(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, mode: in
     M, K = x.shape
     N = weight.shape[0]
     lib = library.load()
-    if 12 < M <= 64 and _few(x, weight, mode, lib):
+    if M <= 64 and _few(x, weight, mode, lib):
         gemm_bf16_few(x, weight, out, mode)
         return
     stream_ok, umma_ok = _fast_kernels(x, weight, lib)

@@ -387,6 +387,19 @@ def linear_slices(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Tenso
     return gemm_dispatch.gemm_bf16_slices(x, weight)
 
 
+def linear_few_slices(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Tensor]:
+    """x . weight^T of a few rows as float32 planes over K slices [slices, M, N], for a reader that adds them up itself, or None
+    where the whole product (linear) is the better one."""
+    _check(x, "x", dims=2)
+    _check(weight, "weight", dims=2)
+    if weight.shape[1] != x.shape[1]:
+        raise InvalidError(f"linear: x has {x.shape[1]} columns, weight has {weight.shape[1]}")
+    if x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16:
+        return None
+    from . import gemm_dispatch
+    return gemm_dispatch.gemm_bf16_few_slices(x, weight)
+
+
 def add_planes_(x: torch.Tensor, planes: torch.Tensor) -> torch.Tensor:
     """x += planes[0] + planes[1] + ... (in that order); x float32, planes [n, *x.shape] float32."""
     _check(x, "x", torch.float32)
@@ -2029,17 +2042,21 @@ def attention_decode_fused(qkv: torch.Tensor, q_heads: int, inv_freq: Optional[t
     token) and merges the splits, in one launch. -> [B, Hq*d]. `order` (int32 [B], made on the host and
     copied before the step, because the kernel reads it before it waits for the kernels ahead of
     it): the sequences' work is handed out in this order, longest first when lengths are unequal;
-    `fill`: their mean length in quarters of the longest (launch geometry only)."""
-    _check(qkv, "qkv", torch.bfloat16, 2)
+    `fill`: their mean length in quarters of the longest (launch geometry only). `qkv` may also be the projection's
+    K slices, float32 [slices, B, (Hq+2Hk)*d]: their sum, rounded to bfloat16, is the projection."""
+    if qkv.dim() == 3:
+        _check(qkv, "qkv", torch.float32, 3)
+    else:
+        _check(qkv, "qkv", torch.bfloat16, 2)
     d, Hk = kv.head_dim, kv.kv_heads
-    if qkv.shape[1] != (q_heads + 2 * Hk) * d or q_heads % Hk:
+    if qkv.shape[-1] != (q_heads + 2 * Hk) * d or q_heads % Hk:
         raise InvalidError("attention_decode_fused: qkv width does not match the head geometry")
-    _check(kv.k, "k pages", qkv.dtype, 4)
-    _check(kv.v, "v pages", qkv.dtype, 4)
+    _check(kv.k, "k pages", torch.bfloat16, 4)
+    _check(kv.v, "v pages", torch.bfloat16, 4)
     if tuple(kv.k.shape[1:]) != (Hk, kv.page_size, d):
         raise InvalidError("attention_decode_fused: cache pages do not match the head geometry")
     _check(kv.page_table, "page table", torch.int32, 2)
-    B = qkv.shape[0]
+    B = qkv.shape[-2]
     for name, t in (("positions", positions), ("dest_rows", dest_rows), ("slots", slots), ("kv_lens", kv_lens)):
         _check(t, name, torch.int32, 1)
         if t.numel() != B:
@@ -2050,9 +2067,9 @@ def attention_decode_fused(qkv: torch.Tensor, q_heads: int, inv_freq: Optional[t
             raise InvalidError("attention_decode_fused: inv_freq must have rotary/2 entries")
     else:
         rotary = 0
-    if not attention_decode_fused_supported(qkv.dtype, d, kv.page_size, rotary, kv.window):
+    if not attention_decode_fused_supported(torch.bfloat16, d, kv.page_size, rotary, kv.window):
         raise UnsupportedError("attention_decode_fused: geometry not supported; use rope_store and attention_decode")
-    out = _activation(B, q_heads * d, qkv.dtype, qkv.device)
+    out = _activation(B, q_heads * d, torch.bfloat16, qkv.device)
     from . import attention_dispatch
     if order is not None:
         _check(order, "order", torch.int32, 1)

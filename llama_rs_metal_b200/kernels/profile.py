@@ -102,7 +102,7 @@ WORK: Dict[str, Callable[..., Tuple[float, float]]] = {
     "lrm_attention_packed_rowwise": lambda a: (0, 4.0 * hints["pairs"] * _v(a[8]) * _v(a[10])),
     # over the cache: every cached key and value of the live sequences once
     "lrm_attention_decode_tiled": lambda a: (2.0 * hints["kv_tokens"] * _v(a[11]) * _v(a[12]) * 2, 0),
-    "lrm_attention_decode_cluster": lambda a: (2.0 * hints["kv_tokens"] * _v(a[14]) * _v(a[15]) * 2, 0),
+    "lrm_attention_decode_cluster": lambda a: (2.0 * hints["kv_tokens"] * _v(a[15]) * _v(a[16]) * 2, 0),
     "lrm_attention_paged_rowwise": lambda a: (2.0 * hints["kv_tokens"] * _v(a[13]) * _v(a[14]) * _ELEM[_v(a[4])], 0),
     "lrm_attention_extend_umma": lambda a: (2.0 * hints["kv_tokens"] * _v(a[14]) * _v(a[15]) * 2,
                                             4.0 * hints["pairs"] * _v(a[13]) * _v(a[15])),
