@@ -130,6 +130,39 @@ __global__ void rms_norm_vec_kernel(float* __restrict__ x, const W* __restrict__
   }
 }
 
+// The plain norm with a warp per row, for steps of many rows: a lane has up to PER4 groups of four under way at once, nothing waits for
+// a block, and the weights come behind the sum, from L1. The order of the sum differs from the one-CTA kernel's: used where the output
+// is bfloat16 only. See launch_norm for the times.
+template <typename W, typename O, int PER4>
+__global__ __launch_bounds__(128) void rms_norm_rows_kernel(const float* x, const W* __restrict__ w, O* __restrict__ out, int n_rows,
+                                                            int hidden, float eps) {
+  const int r = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, groups = hidden >> 2;
+  pdl_trigger();
+  pdl_wait();
+  if (r >= n_rows) return;
+  const float* xr = x + static_cast<size_t>(r) * hidden;
+  O* yr = out + static_cast<size_t>(r) * hidden;
+  float4 xv[PER4];
+#pragma unroll
+  for (int e = 0; e < PER4; ++e) {
+    const int c = lane + 32 * e;
+    xv[e] = c < groups ? load4(xr + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  float ss[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int e = 0; e < PER4; ++e)
+    ss[e & 3] = fmaf(xv[e].x, xv[e].x, fmaf(xv[e].y, xv[e].y, fmaf(xv[e].z, xv[e].z, fmaf(xv[e].w, xv[e].w, ss[e & 3]))));
+  const float total = warp_sum((ss[0] + ss[1]) + (ss[2] + ss[3]));
+  const float inv = 1.0f / sqrtf(total / static_cast<float>(hidden) + eps);
+#pragma unroll
+  for (int e = 0; e < PER4; ++e) {
+    const int c = lane + 32 * e;
+    if (c >= groups) continue;
+    const float4 wv = load4(w + 4 * c);
+    store4(yr + 4 * c, make_float4((xv[e].x * inv) * wv.x, (xv[e].y * inv) * wv.y, (xv[e].z * inv) * wv.z, (xv[e].w * inv) * wv.w));
+  }
+}
+
 // The same row cut among the CTAs of a thread-block cluster (`ranks` of them, each with its share of
 // the columns): for few rows with several slices to fold, where one CTA per row leaves most SMs
 // idle and each of the busy ones reads (slices + 1) rows. Every CTA sends its share of the sum of
@@ -238,10 +271,11 @@ static int launch_norm(float* x, const void* w, void* out, const int* rows, cons
     // Few rows of 40 KB or more to read each (the row and the slices to fold), bfloat16 out: a cluster
     // of eight CTAs per row (see the kernel). Whole decode steps, one CTA per row against clusters
     // of 8: 3B sizes at batch 16 2.98 -> 2.86 ms, 8B at batch 8 4.56 -> 4.48, 1B at batch 64 2.10 ->
-    // 2.08; rows of 8-24 KB (1B at batch 8) lose 2 % to the cluster's barrier and stay as they were.
+    // 2.08; rows of 8-24 KB (1B at batch 8) lose 2 % to the cluster's barrier and stay as they were. 128
+    // rows of 4,096 with two slices 4.4 us against 5.9, 256 rows 8.0 against 6.6.
     int ranks = g_lrm_norm_ranks;
     if (ranks == 0)
-      ranks = sizeof(O) == 2 && n_rows <= 74 && static_cast<long long>(n_partials + 1) * hidden >= 10240 ? 8 : 1;
+      ranks = sizeof(O) == 2 && n_rows <= kSmCount && static_cast<long long>(n_partials + 1) * hidden >= 10240 ? 8 : 1;
     if (ranks > 1 && sizeof(O) == 2 && groups >= 32 * ranks) {
       const int per_cta = (groups + ranks - 1) / ranks;
       const int cthreads = per_cta >= 256 ? 256 : 128;
@@ -254,8 +288,24 @@ static int launch_norm(float* x, const void* w, void* out, const int* rows, cons
       if (cper4 <= 4) LRM_NORM_CLUSTER(4);
 #undef LRM_NORM_CLUSTER
     }
+    // Many rows without slices to fold: a warp per row. us, in brackets a CTA per row (with as many groups of four per thread as the
+    // row has): 2,048 rows of 2,048 4.9 (7.2), 1,024 rows of 3,072 5.1 (5.3), 2,048 7.8 (8.7), 1,500 rows of 4,096 8.4 (8.0),
+    // 2,048 9.7 (10.0); 700 rows of 2,048 3.6 (4.0). With slices the CTA's loads of all of them at once are the better way.
+    if (sizeof(O) == 2 && rows == nullptr && n_partials == 0 && n_rows >= 1024 && groups <= 1024) {
+#define LRM_NORM_ROWS(P4)                                                                                                   \
+  return static_cast<int>(lrm_launch(rms_norm_rows_kernel<W, O, P4>, (n_rows + 3) / 4, 128, 0, stream,                      \
+                                     static_cast<const float*>(x), static_cast<const W*>(w), static_cast<O*>(out), n_rows,  \
+                                     hidden, eps))
+      if (groups <= 256) LRM_NORM_ROWS(8);
+      if (groups <= 512) LRM_NORM_ROWS(16);
+      if (groups <= 768) LRM_NORM_ROWS(24);
+      LRM_NORM_ROWS(32);
+#undef LRM_NORM_ROWS
+    }
     // up to eight groups of four per thread: 256 threads reach rows of 8,192 elements (a block of
-    // 1,024 threads per row was measured at a third of the memory rate at 4,096 elements)
+    // 1,024 threads per row was measured at a third of the memory rate at 4,096 elements). Room for
+    // four groups where a thread has no more: with room for eight fewer CTAs fit on an SM (529 rows
+    // of 4,096 5.0 us against 3.6, with two slices 11.4 against 8.1; 2,048 rows 15.2 against 10.0).
     const int vthreads = groups > 2048 ? 1024 : (groups >= 512 ? 256 : (groups >= 64 ? 128 : 32));
     const int per4 = (groups + vthreads - 1) / vthreads;
 #define LRM_NORM_VEC(P4)                                                                               \
@@ -263,6 +313,7 @@ static int launch_norm(float* x, const void* w, void* out, const int* rows, cons
                                      static_cast<const W*>(w), static_cast<O*>(out), rows, partials,  \
                                      n_partials, partial_stride, hidden, eps))
     if (per4 <= 2) LRM_NORM_VEC(2);
+    if (per4 <= 4) LRM_NORM_VEC(4);
     if (per4 <= 8) LRM_NORM_VEC(8);
 #undef LRM_NORM_VEC
   }
