@@ -10,7 +10,9 @@
 // are added up in float32.
 //
 // blockIdx.y numbers the distinct experts of the step, found by every CTA from the ids, and the list of the expert's
-// pairs is in ascending order, so a result depends on nothing else in the batch.
+// pairs is in ascending order, so a result depends on nothing else in the batch. Where there are twice as many pairs as experts (at
+// least 86 % of the experts are then chosen, on average) blockIdx.y is the expert itself, so that the first product's CTAs ask for
+// their weights while the router still runs: 8 rows, 2 of 8 experts of 3 x 1024 x 2048, router to sum 37.7 -> 35.0 us.
 #include "common.cuh"
 
 namespace {
@@ -58,9 +60,8 @@ __device__ __forceinline__ int chosen_expert_of_few(const int* ids, int n, int e
   return e;
 }
 
-// The same for any number, by the whole block (experts numbered by their ids). words: [32] shared, list: [n] shared.
-__device__ int chosen_expert(const int* ids, int n, int experts, int nth, unsigned* words, int* list, int* count,
-                             int* picked) {
+// The same expert for any number of pairs, by the whole block (experts numbered by their ids). words: [32] shared.
+__device__ int chosen_expert(const int* ids, int n, int experts, int nth, unsigned* words, int* picked) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid < 32) words[tid] = 0u;
   __syncthreads();
@@ -88,7 +89,19 @@ __device__ int chosen_expert(const int* ids, int n, int experts, int nth, unsign
   __syncthreads();
   const int e = *picked;
   if (e < 0) return -1;
-  if (warp == 0) {
+  return e;
+}
+
+// The pairs of ids [0 .. n) that chose expert e, in ascending order, by the whole block; `list` [n] shared.
+__device__ __forceinline__ int pairs_of(const int* ids, int n, int e, int* list, int* count) {
+  const int lane = threadIdx.x & 31;
+  if (n <= 32) {  // every warp for itself, all writing the same
+    const unsigned mine = __ballot_sync(0xffffffffu, lane < n && ids[lane] == e);
+    if (mine >> lane & 1u) list[__popc(mine & ((1u << lane) - 1u))] = lane;
+    __syncwarp();
+    return __popc(mine);
+  }
+  if (threadIdx.x < 32) {
     int held = 0;
     for (int i0 = 0; i0 < n; i0 += 128) {  // four loads under way together
       int id[4];
@@ -104,7 +117,7 @@ __device__ int chosen_expert(const int* ids, int n, int experts, int nth, unsign
     if (lane == 0) *count = held;
   }
   __syncthreads();
-  return e;
+  return *count;
 }
 
 // DOWN false: rows f (gate) and ff + f (up) of gate_up, right operand x rows [tokens, width], K = width;
@@ -114,7 +127,7 @@ __device__ int chosen_expert(const int* ids, int n, int experts, int nth, unsign
 template <int NT, int WARPS, bool DOWN>
 __global__ __launch_bounds__(WARPS * 32, 16 / WARPS) void moe_grouped_kernel(
     const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ W, const int* ids, const float* weights, __nv_bfloat16* y3,
-    float* planes, int tokens, int width, int ff, int experts, int top, float limit, float alpha, int act, const float* x32) {
+    float* planes, int tokens, int width, int ff, int experts, int top, float limit, float alpha, int act, const float* x32, int by_id) {
   extern __shared__ __align__(16) unsigned char shared[];
   __shared__ unsigned words[32];
   __shared__ int count_of, picked;
@@ -123,9 +136,10 @@ __global__ __launch_bounds__(WARPS * 32, 16 / WARPS) void moe_grouped_kernel(
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int pairs = tokens * top, row0 = blockIdx.x * (DOWN ? 16 : 8);
   // The second product's CTAs are let in when all of the first one's are past their wait, so the ids are there: they
-  // find their expert and ask for its first weights before they wait for the first product.
-  if (!DOWN) pdl_wait();
-  pdl_trigger();
+  // find their expert and ask for its first weights before they wait for the first product. The first product's CTAs do
+  // before they wait for the router where blockIdx.y is the expert.
+  if (!DOWN && !by_id) pdl_wait();
+  if (DOWN || !by_id) pdl_trigger();
   if (DOWN && blockIdx.y == gridDim.y - 1) {  // the identity experts: their output is their input
     pdl_wait();
     for (int p = warp; p < pairs; p += WARPS) {
@@ -136,14 +150,16 @@ __global__ __launch_bounds__(WARPS * 32, 16 / WARPS) void moe_grouped_kernel(
     }
     return;
   }
-  int count = 0, e;
-  if (pairs <= 32) {
-    e = chosen_expert_of_few(ids, pairs, experts, blockIdx.y, list, &count);
-  } else {
-    e = chosen_expert(ids, pairs, experts, blockIdx.y, words, list, &count_of, &picked);
-    count = count_of;
+  int count = 0, e = blockIdx.y;
+  if (!by_id) {
+    if (pairs <= 32) {
+      e = chosen_expert_of_few(ids, pairs, experts, blockIdx.y, list, &count);
+    } else {
+      e = chosen_expert(ids, pairs, experts, blockIdx.y, words, &picked);
+      if (e >= 0) count = pairs_of(ids, pairs, e, list, &count_of);
+    }
+    if (e < 0) return;
   }
-  if (e < 0) return;
   const int K = DOWN ? ff : width, rows = DOWN ? width : ff;
   const int row_a = row0 + g, row_b = DOWN ? row0 + g + 8 : row0 + g;
   const bool ok_a = row_a < rows, ok_b = row_b < rows;
@@ -172,6 +188,14 @@ __global__ __launch_bounds__(WARPS * 32, 16 / WARPS) void moe_grouped_kernel(
   uint4 wa_at[kDepth][kPieces], wb_at[kDepth][kPieces];  // kDepth chunks of weights under way
 #pragma unroll
   for (int i = 0; i < kDepth; ++i) load_w(k_begin + i * kStep, wa_at[i], wb_at[i]);
+  if (!DOWN && by_id) {
+    pdl_wait();
+    pdl_trigger();
+  }
+  if (by_id) {
+    count = pairs_of(ids, pairs, e, list, &count_of);
+    if (count == 0) return;
+  }
   if (DOWN) pdl_wait();
   for (int base = 0; base < count; base += 8 * NT) {
     int right[NT];  // element where this thread's column of every tile begins (-1: no pair)
@@ -261,9 +285,10 @@ int launch_grouped(const void* x, const void* W, const int* ids, const float* we
   const int rows = DOWN ? width : ff, per = DOWN ? 16 : 8, pairs = tokens * top;
   const size_t bytes = sizeof(float) * WARPS * NT * 128 + sizeof(int) * (pairs < 32 ? 32 : pairs);
   const dim3 grid((rows + per - 1) / per, (experts < pairs ? experts : pairs) + (DOWN ? 1 : 0));
+  const int by_id = pairs >= 2 * experts;
   LRM_LAUNCH((moe_grouped_kernel<NT, WARPS, DOWN>), grid, WARPS * 32, bytes, stream, static_cast<const __nv_bfloat16*>(x),
              static_cast<const __nv_bfloat16*>(W), ids, weights, static_cast<__nv_bfloat16*>(y3), planes, tokens, width, ff,
-             experts, top, limit, alpha, act, x32);
+             experts, top, limit, alpha, act, x32, by_id);
   return 0;
 }
 
@@ -303,5 +328,37 @@ LRM_API int lrm_moe_experts_grouped(const void* x, const void* gate_up, const vo
   else if (tokens <= 16) LRM_GROUPED(2);
   else LRM_GROUPED(4);
 #undef LRM_GROUPED
+  return code;
+}
+
+LRM_API int lrm_moe_router(const void* x, int x_dtype, const float* w, const float* bias, int* ids, float* weights, float* logits,
+                           int tokens, int width, int E, int top, int scored, const float* correction, int groups, int keep,
+                           int renormalize, float mass_eps, float weight_scale, cudaStream_t stream);
+LRM_API int lrm_add_planes(float* x, const float* planes, int count, long long n, cudaStream_t stream);
+
+// Bytes of scratch that lrm_moe_rows_step wants: y's terms, the choices and their weights.
+LRM_API long long lrm_moe_rows_step_floats(int tokens, int ff, int top) {  // in floats
+  const long long pairs = static_cast<long long>(tokens) * top;
+  return (3 * pairs * ff + 7) / 8 * 4 + (pairs + 3) / 4 * 4 + pairs;
+}
+
+// The whole part for a step of few rows in one call: lrm_moe_router (w [outputs, width], its arguments from `scored` on), then
+// lrm_moe_experts_grouped, then, with `sum`, all planes into the first one. `scratch`: on 16 bytes, lrm_moe_rows_step_floats floats.
+LRM_API int lrm_moe_rows_step(const void* x, const float* w, const float* bias, const void* gate_up, const void* down, float* scratch,
+                              float* planes, int tokens, int width, int ff, int experts, int outputs, int top, float limit, float alpha,
+                              int act, const float* x32, int sum, int scored, const float* correction, int groups, int keep,
+                              int renormalize, float mass_eps, float weight_scale, cudaStream_t stream) {
+  if (tokens <= 0) return 0;
+  if (top <= 0 || scratch == nullptr || !lrm_moe_experts_grouped_supports(tokens, width, ff, experts, top)) return LRM_BAD_ARGUMENT;
+  const long long pairs = static_cast<long long>(tokens) * top;
+  int* ids = reinterpret_cast<int*>(scratch + (3 * pairs * ff + 7) / 8 * 4);
+  float* weights = reinterpret_cast<float*>(ids + (pairs + 3) / 4 * 4);
+  int code = lrm_moe_router(x, LRM_BF16, w, bias, ids, weights, nullptr, tokens, width, outputs, top, scored, correction, groups, keep,
+                            renormalize, mass_eps, weight_scale, stream);
+  if (code == 0)
+    code = lrm_moe_experts_grouped(x, gate_up, down, ids, weights, scratch, planes, tokens, width, ff, experts, top, limit, alpha, act, x32,
+                                   stream);
+  const long long numbers = static_cast<long long>(tokens) * width;
+  if (code == 0 && sum && top > 1) code = lrm_add_planes(planes, planes + numbers, top - 1, numbers, stream);
   return code;
 }

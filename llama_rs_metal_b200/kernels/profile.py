@@ -135,6 +135,9 @@ WORK: Dict[str, Callable[..., Tuple[float, float]]] = {
         + 4.0 * _v(a[8]) * _v(a[12]) * _v(a[13]) * _v(a[9]),
         6.0 * _v(a[8]) * _v(a[12]) * _v(a[10]) * _v(a[9])),
     # every chosen expert's matrices once
+    "lrm_moe_rows_step": lambda a: (
+        min(_v(a[7]) * _v(a[12]), _v(a[10])) * 6.0 * _v(a[9]) * _v(a[8]) + 4.0 * (_v(a[7]) * _v(a[12]) + _v(a[11])) * _v(a[8]),
+        6.0 * _v(a[7]) * _v(a[12]) * _v(a[9]) * _v(a[8])),
     "lrm_moe_experts_grouped": lambda a: (
         min(_v(a[7]) * _v(a[11]), _v(a[10])) * 6.0 * _v(a[9]) * _v(a[8]) + 4.0 * _v(a[7]) * _v(a[11]) * _v(a[8]),
         6.0 * _v(a[7]) * _v(a[11]) * _v(a[9]) * _v(a[8])),

@@ -136,6 +136,13 @@ class MixtureOfExperts(FeedForward):
                 else ops.moe_route(logits, self.bias, self.top)
         return routed
 
+    def _rows(self, x, x32, sum_planes: bool):
+        """Router and experts of a step of few rows in one call: the planes (their sum with `sum_planes`), or None."""
+        if x.shape[0] > self.ROUTER_ROWS and self.outputs > 16:
+            return None
+        return ops.moe_rows_step(x, self.router.weight, self.bias, self.top, self.scoring, self.gate_up, self.down, self.limit, self.alpha,
+                                 self.act, x32, sum_planes)
+
     def _sorted(self, x, ids, weights, out):
         """The experts of a prompt on rows sorted by expert, added to `out` (None: returned), or None where all experts
         for every token are the faster way or the only one."""
@@ -144,11 +151,15 @@ class MixtureOfExperts(FeedForward):
         return ops.moe_experts_sorted(x, self.gate_up, self.down, ids, weights, self.limit, self.alpha, self.act, out)
 
     def forward(self, x, ctx, residual):
-        ids, weights = self.route(x)
         # identity experts pass the input on: the float32 stream itself where x is its rounding
         x32 = ctx.stream if self.identity and x.dtype != torch.float32 else None
         dense = (x.dtype == torch.bfloat16 and self.gate_up.dtype == torch.bfloat16 and x.shape[0] >= self.DENSE_ROWS
                  and self.num_experts <= self.DENSE_RATIO * self.top)
+        if not dense and self.shared is None:
+            planes = self._rows(x, x32, residual is None)
+            if planes is not None:
+                return planes if residual is None else self._add_planes(residual, planes, ctx)
+        ids, weights = self.route(x)
         if residual is None:
             # a block that puts a norm between this part and the stream: the shared part's float32
             # output (or the all-experts product's) is what everything else is added to
@@ -198,7 +209,11 @@ class MixtureOfExperts(FeedForward):
                 ctx.settle(residual)
                 ops.moe_identity_add_(residual, x32 if x32 is not None else x, ids, weights, self.num_experts)
             return self.down_all(y, epilogue=ops.ADD, out=residual, ctx=ctx)
-        planes = ops.moe_experts_rows(x, self.gate_up, self.down, ids, weights, self.limit, self.alpha, self.act, x32)
+        return self._add_planes(residual, ops.moe_experts_rows(x, self.gate_up, self.down, ids, weights, self.limit, self.alpha,
+                                                               self.act, x32), ctx)
+
+    @staticmethod
+    def _add_planes(residual, planes, ctx):
         if ctx.may_defer:
             ctx.settle(residual)  # at most one set of partial sums is pending at a time
             ctx.pending = planes
