@@ -1,5 +1,5 @@
 // A prompt's experts, rows sorted by expert, bfloat16: the passes around the two tensor-core products
-// (lrm_gemm_bf16_umma_experts, gemm_bf16_umma.cu) in which every row multiplies its own expert only.
+// (gemm_bf16_wide.cu, or gemm_bf16_umma.cu where there are no pairs of SMs) in which every row multiplies its own expert only.
 //
 //   sort     the (token, choice) pairs in the order of their experts, each expert's on whole tiles of 128 rows
 //   gather   x of every row's token
@@ -184,4 +184,60 @@ LRM_API int lrm_moe_combine(const float* part, const int* places, int tokens, in
   if (width <= 0 || width % 4 || top <= 0) return LRM_BAD_ARGUMENT;
   LRM_LAUNCH(moe_combine_kernel, tokens, 256, 0, stream, part, places, top, width, add, out);
   return 0;
+}
+
+LRM_API int lrm_gemm_bf16_wide_experts(const void* X, const void* W, void* out, int M, int N, int K, long long w_height, long long w_width,
+                                       int w_rows, int w_cols, const int* tile_experts, int* status, cudaStream_t stream);
+LRM_API int lrm_gemm_bf16_wide_experts_gated(const void* X, const void* W, void* out, int M, int ff, int K, long long w_height,
+                                             const int* tile_experts, const int* rows, const float* weights, float limit, float alpha,
+                                             int act, int* status, cudaStream_t stream);
+
+namespace {
+
+// How lrm_moe_sorted_step divides its scratch, in bytes from its start; M rows in `tiles` tiles.
+struct SortedScratch {
+  int tiles;
+  long long M, y, part, rows, places, tile_experts, end;
+  SortedScratch(int tokens, int width, int ff, int experts, int top) {
+    const long long pairs = static_cast<long long>(tokens) * top;
+    tiles = static_cast<int>(pairs / kTileRows) + experts, M = static_cast<long long>(tiles) * kTileRows;
+    y = M * width * 2, part = y + M * ff * 2, rows = part + M * width * 4, places = rows + M * 4;
+    tile_experts = places + (pairs + 3) / 4 * 16, end = tile_experts + (tiles + 3) / 4 * 16ll;
+  }
+};
+
+}  // namespace
+
+// Bytes of scratch that lrm_moe_sorted_step wants.
+LRM_API long long lrm_moe_sorted_step_bytes(int tokens, int width, int ff, int experts, int top) {
+  return SortedScratch(tokens, width, ff, experts, top).end;
+}
+
+// The five launches in one call, with the products on pairs of SMs: out float32 [T, width] (added to with `add`) from bfloat16 x
+// [T, width], gate_up [experts, 2 ff, width], down [width, experts, ff] and the choices ids, weights [T, top]. width and ff multiples of
+// 64; x, gate_up, down and scratch on 16 bytes.
+LRM_API int lrm_moe_sorted_step(const void* x, const void* gate_up, const void* down, const int* ids, const float* weights, void* scratch,
+                                float* out, int tokens, int width, int ff, int experts, int top, float limit, float alpha, int act, int add,
+                                int* status, cudaStream_t stream) {
+  if (tokens <= 0) return 0;
+  if (width <= 0 || width % 64 || ff <= 0 || ff % 64 || top <= 0 || experts <= 0 || experts > 8192 || (act != 0 && act != 1) ||
+      scratch == nullptr || status == nullptr || static_cast<long long>(tokens) * top >= 1ll << 28)
+    return LRM_BAD_ARGUMENT;
+  const SortedScratch at(tokens, width, ff, experts, top);
+  if (at.M >= 1ll << 31 || 2ll * experts * ff >= 1ll << 31) return LRM_UNSUPPORTED;
+  char* const base = static_cast<char*>(scratch);
+  int *rows = reinterpret_cast<int*>(base + at.rows), *places = reinterpret_cast<int*>(base + at.places);
+  int* tile_experts = reinterpret_cast<int*>(base + at.tile_experts);
+  float* part = reinterpret_cast<float*>(base + at.part);
+  const int M = static_cast<int>(at.M);
+  LRM_LAUNCH(moe_sort_kernel, experts, kSortThreads, sizeof(int) * experts, stream, ids, tokens * top, experts, rows, places, tile_experts,
+             at.tiles);
+  LRM_LAUNCH(moe_gather_kernel, M, 256, 0, stream, static_cast<const uint4*>(x), rows, tile_experts, top, width / 8,
+             reinterpret_cast<uint4*>(base));
+  int code = lrm_gemm_bf16_wide_experts_gated(base, gate_up, base + at.y, M, ff, width, 2ll * experts * ff, tile_experts, rows, weights, limit,
+                                              alpha, act, status, stream);
+  if (code == 0)
+    code = lrm_gemm_bf16_wide_experts(base + at.y, down, part, M, width, ff, width, static_cast<long long>(experts) * ff, 0, ff, tile_experts,
+                                      status, stream);
+  return code != 0 ? code : lrm_moe_combine(part, places, tokens, top, width, add, out, stream);
 }

@@ -80,7 +80,8 @@ def check_status() -> None:
                           55: "a free accumulator"})
             names.update({61: "a free stage", 62: "operand parts", 63: "the accumulator", 64: "operand tiles", 65: "copies in flight",
                           66: "a free tile", 67: "the small products"})
-            names.update({71: "a free stage", 72: "operand tiles", 73: "the accumulator", 74: "copies in flight", 75: "a free accumulator"})
+            names.update({71: "a free stage", 72: "operand tiles", 73: "the accumulator", 74: "copies in flight", 75: "a free accumulator",
+                          76: "gates and ups"})
             kernel = "gemm_bf16_wide" if code >= 71 else "gemm_f32_umma" if code >= 61 else "gemm_bf16_few" if code >= 51 else "attention_gated_umma" if code >= 41 else "gemm_bf16_umma_pair" \
                 if code >= 31 else "attention_prefill_pingpong" if code >= 21 else "gemm_bf16_umma"
             raise LlamaError(f"{kernel} gave up waiting for {names.get(code, code)}; its result is invalid")
@@ -199,6 +200,13 @@ def _wide(x: torch.Tensor, weight: torch.Tensor, mode: int, umma_ok: bool):
     if pairs == 0:
         return None
     return wide_shape or wide_plan(M, N, K, mode, pairs)
+
+
+def sorted_on_pairs() -> bool:
+    """Whether a prompt's sorted experts go through pairs of SMs with the weights as the wide operand: wherever those are to be had. us
+    over router and experts, in brackets 128 x 256 tiles of one SM each: 2048 x 1024, 2 of 8 experts 408 tokens 67 (85), 1,500 82.7 (87.4),
+    2,048 103 (117), 4 of 16 1,000 tokens 120 (123); 1024 x 512 2 of 8 520 tokens 31.8 (34.8), 2,000 54.2 (60.9)."""
+    return not (no_wide or no_fused_gate) and umma_width is None and pair_room() > 0
 
 
 def gemm_bf16_wide(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, mode: int, rows: int, slices: int = 1) -> None:

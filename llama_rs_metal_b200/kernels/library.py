@@ -151,7 +151,7 @@ def load() -> ctypes.CDLL:
             # let their successor start at once, large ones after their main loop (letting every
             # kernel do so at once made the whole step slower). LRM_PDL=0 switches it off.
             for name in ("lrm_linear_state_scan_floats", "lrm_bonus_state_scan_floats", "lrm_head_decay_delta_scan_floats",
-                         "lrm_gemm_f32_umma_scratch", "lrm_moe_rows_step_floats"):
+                         "lrm_gemm_f32_umma_scratch", "lrm_moe_rows_step_floats", "lrm_moe_sorted_step_bytes"):
                 getattr(_library, name).restype = ctypes.c_longlong  # a long prompt's workspace passes 2^31
             _library.lrm_set_pdl(0 if os.environ.get("LRM_PDL", "1") == "0" else 1)
             from . import profile

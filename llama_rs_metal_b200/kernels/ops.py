@@ -1723,8 +1723,17 @@ def moe_experts_sorted(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tenso
     if (gemm_dispatch.force_tiled or width % 64 or ff % 64 or E > 8192 or T * top >= 1 << 28
             or any(t.data_ptr() % 16 for t in (x, gate_up, down)) or not lib.lrm_gemm_bf16_umma_supports(128, width, ff)):
         return None
+    dev = x.device
+    if T and top and gemm_dispatch.sorted_on_pairs():
+        scratch = torch.empty(lib.lrm_moe_sorted_step_bytes(T, width, ff, E, top), dtype=torch.uint8, device=dev)
+        total = _f32((T, width), dev) if out is None else out
+        gemm_dispatch.mark_status_dirty()
+        _done(lib.lrm_moe_sorted_step(_ptr(x), _ptr(gate_up), _ptr(down), _ptr(ids), _ptr(weights), _ptr(scratch), _ptr(total), T, width, ff,
+                                      E, top, ctypes.c_float(limit), ctypes.c_float(alpha), act, int(out is not None),
+                                      _ptr(gemm_dispatch._status_word(dev)), _stream()), "moe_sorted_step", launches=5)
+        return total
     tiles = int(lib.lrm_moe_sorted_tiles_room(T * top, E))
-    M, dev = 128 * tiles, x.device
+    M = 128 * tiles
     rows = torch.empty(M, dtype=torch.int32, device=dev)
     places = torch.empty(T * top, dtype=torch.int32, device=dev)
     tile_experts = torch.empty(tiles, dtype=torch.int32, device=dev)

@@ -141,8 +141,14 @@ WORK: Dict[str, Callable[..., Tuple[float, float]]] = {
     "lrm_moe_experts_grouped": lambda a: (
         min(_v(a[7]) * _v(a[11]), _v(a[10])) * 6.0 * _v(a[9]) * _v(a[8]) + 4.0 * _v(a[7]) * _v(a[11]) * _v(a[8]),
         6.0 * _v(a[7]) * _v(a[11]) * _v(a[9]) * _v(a[8])),
+    "lrm_gemm_bf16_wide_experts_gated": lambda a: _gemm(_v(a[3]), 2 * _v(a[4]), _v(a[5]), 1, 2),
+    "lrm_gemm_bf16_wide_experts": lambda a: _gemm(_v(a[3]), _v(a[4]), _v(a[5]), 4, 2),
     "lrm_gemm_bf16_umma_experts_gated": lambda a: _gemm(_v(a[3]), 2 * _v(a[4]), _v(a[5]), 1, 2),
     "lrm_gemm_bf16_umma_experts": lambda a: _gemm(_v(a[3]), _v(a[4]), _v(a[5]), 4, 2),
+    # every expert's matrices once; the sorted rows, their gated values and terms written and read, without what fills up tiles
+    "lrm_moe_sorted_step": lambda a: (
+        _v(a[10]) * 6.0 * _v(a[9]) * _v(a[8]) + _v(a[7]) * (_v(a[11]) * (14.0 * _v(a[8]) + 4.0 * _v(a[9])) + 4.0 * _v(a[8])),
+        6.0 * _v(a[7]) * _v(a[11]) * _v(a[9]) * _v(a[8])),
     "lrm_moe_gather": lambda a: (_v(a[5]) * 128.0 * _v(a[4]) * 4.0, 0),
     "lrm_moe_sorted_gate": lambda a: (_v(a[5]) * 128.0 * _v(a[4]) * 10.0, 0),
     "lrm_moe_combine": lambda a: (_v(a[2]) * (_v(a[3]) + 1.0) * _v(a[4]) * 4.0, 0),
@@ -256,7 +262,7 @@ WORK: Dict[str, Callable[..., Tuple[float, float]]] = {
     "lrm_tanh_columns": lambda a: (_v(a[5]) * _v(a[6]) * (_ELEM[_v(a[1])] + _ELEM[_v(a[4])]), 0),
 }
 # entry points that only answer questions and launch nothing
-_QUERIES = ("_supports", "_ctas_per_sm", "_slices", "_pieces", "_resident", "_floats", "lrm_gemm_f32_umma_scratch", "_error", "_room", "lrm_set_pdl", "lrm_set_norm_ranks", "lrm_pick_pieces", "lrm_linear_state_scan_rows")
+_QUERIES = ("_supports", "_ctas_per_sm", "_slices", "_pieces", "_resident", "_floats", "_bytes", "lrm_gemm_f32_umma_scratch", "_error", "_room", "lrm_set_pdl", "lrm_set_norm_ranks", "lrm_pick_pieces", "lrm_linear_state_scan_rows")
 
 
 class _Row:
