@@ -17,6 +17,30 @@ __global__ void silu_mul_kernel(const A* __restrict__ gate_up, A* __restrict__ o
   out[idx] = from_f32<A>(g / (1.0f + expf(-g)) * u);
 }
 
+// The same 16 bytes at a time, where blocks and addresses allow it. Bound by memory and the launch: 333 rows of 8,192 float32
+// 6 us beside the launches around it, 14.8 a number at a time with three divisions of its index each.
+template <typename A>
+__global__ __launch_bounds__(256) void silu_mul_vec_kernel(const A* gate_up, A* __restrict__ out, unsigned pieces, unsigned per_block) {
+  pdl_trigger();
+  pdl_wait();
+  constexpr int N = 16 / sizeof(A);
+  const unsigned idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= pieces) return;
+  // rows are whole numbers of blocks: every block ahead, of this row or others, stands there twice
+  const unsigned at = idx / per_block * 2 * per_block + idx % per_block;
+  union Piece {
+    uint4 raw;
+    A v[N];
+  } g, u, y;
+  g.raw = reinterpret_cast<const uint4*>(gate_up)[at], u.raw = reinterpret_cast<const uint4*>(gate_up)[at + per_block];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const float gate = to_f32(g.v[i]);
+    y.v[i] = from_f32<A>(gate / (1.0f + expf(-gate)) * to_f32(u.v[i]));
+  }
+  reinterpret_cast<uint4*>(out)[idx] = y.raw;
+}
+
 // The clamped gate: g = min(gate, limit), u = clamp(up, -limit, limit),
 // out = g * sigmoid(alpha * g) * (u + 1), from the same column layout. The input may be float32
 // while the output has the activation type (a product that keeps its sums until the activation).
@@ -118,6 +142,18 @@ LRM_API int lrm_silu_mul(const void* gate_up, void* out, int dtype, long long ro
   if (rows <= 0) return 0;
   if (inter <= 0 || block <= 0 || inter % block != 0) return LRM_BAD_ARGUMENT;
   const size_t total = static_cast<size_t>(rows) * inter;
+  const int piece = dtype == LRM_F32 ? 4 : 8;
+  if ((dtype == LRM_F32 || dtype == LRM_BF16) && block % piece == 0 && total / piece < 1ull << 30 &&
+      (reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(out)) % 16 == 0) {
+    const unsigned pieces = static_cast<unsigned>(total / piece), per_block = block / piece;
+    if (dtype == LRM_F32)
+      LRM_LAUNCH(silu_mul_vec_kernel<float>, blocks_for(pieces), 256, 0, stream, static_cast<const float*>(gate_up), static_cast<float*>(out),
+                 pieces, per_block);
+    else
+      LRM_LAUNCH(silu_mul_vec_kernel<__nv_bfloat16>, blocks_for(pieces), 256, 0, stream, static_cast<const __nv_bfloat16*>(gate_up),
+                 static_cast<__nv_bfloat16*>(out), pieces, per_block);
+    return 0;
+  }
   if (dtype == LRM_F32)
     silu_mul_kernel<float><<<blocks_for(total), 256, 0, stream>>>(
         static_cast<const float*>(gate_up), static_cast<float*>(out), total, inter, block);
