@@ -204,7 +204,7 @@ def _wide(x: torch.Tensor, weight: torch.Tensor, mode: int, umma_ok: bool):
 
 def sorted_on_pairs() -> bool:
     """Whether a prompt's sorted experts go through pairs of SMs with the weights as the wide operand: wherever those are to be had. us
-    over router and experts, in brackets 128 x 256 tiles of one SM each: 2048 x 1024, 2 of 8 experts 408 tokens 67 (85), 1,500 82.7 (87.4),
+    over router and experts, in brackets 128 x 256 tiles of one SM each, before the passes around them became shorter: 2048 x 1024, 2 of 8 experts 408 tokens 67 (85), 1,500 82.7 (87.4),
     2,048 103 (117), 4 of 16 1,000 tokens 120 (123); 1024 x 512 2 of 8 520 tokens 31.8 (34.8), 2,000 54.2 (60.9)."""
     return not (no_wide or no_fused_gate) and umma_width is None and pair_room() > 0
 
