@@ -15,8 +15,8 @@
 // tokens 112 (120); 1024 x 512, 2 of 8 520 tokens 30.5 (31.8), 2,000 46.3 (54.2).
 //
 // Against the products over all experts (E / top times the arithmetic, E 2 ff float32 columns per token between them)
-// this pays where the sorted rows are half as many as T E and the products large: ops.moe_prefers_sorted has the line and
-// what both sides measured.
+// this pays where experts are large or many: ops.moe_prefers_sorted and ops.moe_prefers_pairs have the lines and what both sides
+// measured.
 // What the launches before write is read through plain pointers: loads through `const __restrict__` ones may be moved ahead of
 // the wait for those launches.
 #include <climits>

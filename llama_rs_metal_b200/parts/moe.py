@@ -6,7 +6,7 @@ from typing import Dict, Optional, Tuple
 import torch
 
 from ..errors import InvalidError, UnsupportedError
-from ..kernels import ops
+from ..kernels import gemm_dispatch, ops
 from ..registry import FEED_FORWARDS, build_part, register_feed_forward
 from ..weights.loader import TensorSpec
 from .base import FeedForward, PartSpec
@@ -30,8 +30,8 @@ class MixtureOfExperts(FeedForward):
     to the stream in a fixed order (by the next norm where it folds them). All experts at once
     (bfloat16 steps of DENSE_ROWS tokens and more when at most DENSE_RATIO experts exist per chosen
     one): two tensor-core products over every expert, with the weights of the experts a token did not
-    choose set to zero between them. Sorted (such steps of large experts once they have tokens enough to
-    fill tiles of 128 rows per expert, csrc/moe_sorted.cu): the same two products with every row in its
+    choose set to zero between them. Sorted (such steps of large or many experts, ops.moe_prefers_pairs
+    and ops.moe_prefers_sorted, csrc/moe_sorted.cu): the same two products with every row in its
     own expert's tile.
 
     Options beyond that router and that expert. `activation` "silu": an expert is W_down (silu(W_gate
@@ -146,7 +146,8 @@ class MixtureOfExperts(FeedForward):
     def _sorted(self, x, ids, weights, out):
         """The experts of a prompt on rows sorted by expert, added to `out` (None: returned), or None where all experts
         for every token are the faster way or the only one."""
-        if not ops.moe_prefers_sorted(x.shape[0], self.hidden_size, self.intermediate_size, self.num_experts, self.top):
+        prefers = ops.moe_prefers_pairs if gemm_dispatch.sorted_on_pairs() else ops.moe_prefers_sorted
+        if not prefers(x.shape[0], self.hidden_size, self.intermediate_size, self.num_experts, self.top):
             return None
         return ops.moe_experts_sorted(x, self.gate_up, self.down, ids, weights, self.limit, self.alpha, self.act, out)
 
