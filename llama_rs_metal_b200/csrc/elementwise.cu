@@ -128,6 +128,24 @@ __global__ void add_planes_kernel(float* __restrict__ x, const float* __restrict
   for (int p = 0; p < count; ++p) v += planes[p * n + idx];
   x[idx] = v;
 }
+// The same 16 bytes at a time, eight planes' loads under way: the time is that of memory and of one wait for it.
+__global__ __launch_bounds__(256) void add_planes_vec_kernel(float4* x, const float4* planes, int count, size_t n) {
+  pdl_trigger();
+  pdl_wait();
+  const size_t idx = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
+  if (idx >= n) return;
+  float4 v = x[idx];
+  for (int p0 = 0; p0 < count; p0 += 8) {
+    float4 part[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (p0 + u < count) part[u] = planes[(p0 + u) * n + idx];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (p0 + u < count) v.x += part[u].x, v.y += part[u].y, v.z += part[u].z, v.w += part[u].w;
+  }
+  x[idx] = v;
+}
 
 template <typename S, typename D>
 __global__ void cast_kernel(const S* __restrict__ src, D* __restrict__ dst, size_t n) {
@@ -265,7 +283,11 @@ LRM_API int lrm_add_row(float* x, const float* row, long long rows, int width, c
 LRM_API int lrm_add_planes(float* x, const float* planes, int count, long long n, cudaStream_t stream) {
   if (n <= 0 || count <= 0) return 0;
   if (x == nullptr || planes == nullptr) return LRM_BAD_ARGUMENT;
-  LRM_LAUNCH(add_planes_kernel, blocks_for(n), 256, 0, stream, x, planes, count, static_cast<size_t>(n));
+  if (n % 4 == 0 && (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(planes)) % 16 == 0)
+    LRM_LAUNCH(add_planes_vec_kernel, blocks_for(n / 4), 256, 0, stream, reinterpret_cast<float4*>(x), reinterpret_cast<const float4*>(planes),
+               count, static_cast<size_t>(n / 4));
+  else
+    LRM_LAUNCH(add_planes_kernel, blocks_for(n), 256, 0, stream, x, planes, count, static_cast<size_t>(n));
   return 0;
 }
 

@@ -170,11 +170,20 @@ def wide_plan(M: int, N: int, K: int, mode: int, pairs: int):
     (84.9), 529 rows 99.8 (115.9); 2048 x 2048 529 rows 10.4 (13.0), 2,500 rows 20.0 (26.0); 4096 x 14336 300 rows 35.0 in two planes
     (41.4 in three), 600 rows 61.2 (74.6), 1,280 rows 121 (171). Where full tiles of 256 x 256 on the pairs fill their rounds they are as
     good or better: gated 28672 x 4096 1,024 rows 169 against 180, 4096 x 14336 2,048 rows 170 against 173."""
+    best = _wide_best(M, N, K, 8 if mode == 2 else 1, pairs)
+    sliced = mode == 2 and best[2] > 1
+    if not sliced and 0.97 * _tile_time(M, N, K, mode, pairs) <= best[0]:
+        return None
+    return best[1], best[2]
+
+
+def _wide_best(M: int, N: int, K: int, most: int, pairs: int):
+    """(us, activation rows of a tile, K slices, at most `most`) of the best tiles there by wide_plan's estimate."""
     k_blocks, columns = -(-K // 64), -(-N // 256)
     best = None
     for rows, block in WIDE_BLOCK.items():
         tiles = columns * -(-M // rows)
-        for wanted in range(1, 9 if mode == 2 else 2):
+        for wanted in range(1, most + 1):
             per_slice = -(-k_blocks // wanted)
             slices = -(-k_blocks // per_slice)
             if slices != wanted or (slices > 1 and per_slice < 4):
@@ -184,10 +193,27 @@ def wide_plan(M: int, N: int, K: int, mode: int, pairs: int):
                 time += slices * (2.0 * M * N * 4 / 3.5e6)
             if best is None or time < best[0]:
                 best = (time, rows, slices)
-    sliced = mode == 2 and best[2] > 1
-    if not sliced and 0.97 * _tile_time(M, N, K, mode, pairs) <= best[0]:
-        return None
-    return best[1], best[2]
+    return best
+
+
+@functools.lru_cache(maxsize=4096)
+def cut_plan(M: int, N: int, K: int, pairs: int) -> bool:
+    """Whether a product whose float32 result is wanted at once (no norm behind it adds planes) is cut into K slices all the same, the
+    planes of few_plan or wide_plan, with a launch that adds them up: where a long K leaves most SMs idle or one after another.
+
+    us, whole and cut with the addition, weights from memory: up to 64 rows, 2048 x 8192 16 rows 16 and 10, 64 rows 40 and 11; 4096 x 14336 8
+    rows 24 and 23, 16 rows 32 and 24, 64 rows 76 and 27; 1024 x 4096 16 rows 7 and 6, 64 rows 17 and 8; 3072 x 2048 32 rows 9 and 6; under the
+    line 2048 x 2048 16 rows 5 and 6, 4096 x 8192 8 rows 14 and 15, 8192 x 2048 48 rows 13 and 14. More rows, by wide_plan's estimate and 3 us for
+    the launch: 2048 x 8192 100 rows 27 and 14, 500 rows 29 and 25; 4096 x 14336 100 rows 45 and 30, 300 rows 48 and 40; under the line 2048 x 2048 300
+    rows 10 and 12, 6144 x 4096 100 rows 17 and 18."""
+    if M > 64:
+        best = _wide_best(M, N, K, 8, pairs)
+        return best[2] > 1 and best[0] + 3.0 < min(_wide_best(M, N, K, 1, pairs)[0], _tile_time(M, N, K, 2, pairs))
+    if M <= STREAM_ROWS:
+        return N * K >= 40e6
+    if M <= 16:
+        return K >= 6144
+    return K >= (4096 if M <= 32 and N < 3072 else 2048) and (K > 2048 or N < 8192)
 
 
 def _wide(x: torch.Tensor, weight: torch.Tensor, mode: int, umma_ok: bool):
@@ -204,8 +230,9 @@ def _wide(x: torch.Tensor, weight: torch.Tensor, mode: int, umma_ok: bool):
 
 def sorted_on_pairs() -> bool:
     """Whether a prompt's sorted experts go through pairs of SMs with the weights as the wide operand: wherever those are to be had. us
-    over router and experts, in brackets 128 x 256 tiles of one SM each, before the passes around them became shorter: 2048 x 1024, 2 of 8 experts 408 tokens 67 (85), 1,500 82.7 (87.4),
-    2,048 103 (117), 4 of 16 1,000 tokens 120 (123); 1024 x 512 2 of 8 520 tokens 31.8 (34.8), 2,000 54.2 (60.9)."""
+    over router and experts, in brackets 128 x 256 tiles of one SM each, before the passes around them became shorter: 2048 x 1024, 2 of
+    8 experts 1,500 tokens 82.7 (87.4), 2,048 103 (117), 4 of 16 1,000 tokens 120 (123); 1024 x 512 2 of 8 520 tokens 31.8 (34.8), 2,000 54.2
+    (60.9)."""
     return not (no_wide or no_fused_gate) and umma_width is None and pair_room() > 0
 
 
@@ -304,6 +331,17 @@ def gemm_bf16_few_slices(x: torch.Tensor, weight: torch.Tensor, added: bool = Fa
     out = torch.empty((slices, x.shape[0], weight.shape[0]), dtype=torch.float32, device=x.device)
     gemm_bf16_few(x, weight, out, 4, slices)
     return out
+
+
+def gemm_bf16_cut(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Tensor]:
+    """x . weight^T as planes over K slices that the caller adds up at once, or None where the whole product is the better one."""
+    M, K = x.shape
+    N = weight.shape[0]
+    if M > 64:
+        if no_wide or umma_width is not None or N % 2 or pair_room() == 0 or not cut_plan(M, N, K, pair_room()):
+            return None
+        return gemm_bf16_slices(x, weight)
+    return gemm_bf16_few_slices(x, weight) if cut_plan(M, N, K, 0) else None
 
 
 def _held_rows(x: torch.Tensor) -> int:

@@ -306,6 +306,11 @@ def linear(x: torch.Tensor, weight: torch.Tensor, epilogue: str = STORE,
         return out
     if x.dtype != torch.bfloat16:
         raise UnsupportedError(f"linear: dtype {x.dtype}")
+    from . import gemm_dispatch
+    if epilogue == ADD or (epilogue == STORE and out_dtype == torch.float32):
+        planes = gemm_dispatch.gemm_bf16_cut(x, weight) if M and N else None
+        if planes is not None:
+            return add_planes_(out, planes) if epilogue == ADD else add_planes_(planes[0], planes[1:])
     if epilogue == STORE:
         out_dtype = out_dtype or torch.bfloat16
         out = _activation(M, N, out_dtype, x.device)
@@ -321,7 +326,6 @@ def linear(x: torch.Tensor, weight: torch.Tensor, epilogue: str = STORE,
         mode = 3
     else:
         raise InvalidError(f"linear: unknown epilogue {epilogue!r}")
-    from . import gemm_dispatch
     gemm_dispatch.gemm_bf16(x, weight, out, mode)
     return out
 
