@@ -1702,19 +1702,21 @@ def moe_prefers_sorted(tokens: int, width: int, ff: int, experts: int, top: int)
 
 
 def moe_prefers_pairs(tokens: int, width: int, ff: int, experts: int, top: int) -> bool:
-    """The same where the sorted experts' products go through pairs of SMs: from some experts, or some work on top of the chosen, on.
-    Timed in graphs, router to sum, over nine widths, eleven counts of experts and 64 to 4,096 tokens: of 1,681 none slower by more than 3 %
-    than with the line above, 15 % less on average; within 1.3 % of the better way throughout. us, sorted and all: 2048 x 1024, 2 of 8
-    experts 96 tokens 49 and 57, 384 47 and 67; 4 of 16 64 tokens half, 384 71 and 121; 4 of 8 160 tokens 47 and 62, 2,048 156 and 180; 1 of 4 (under
-    the line) 160 tokens 39 and 36; 1024 x 512, 4 of 16 96 tokens 31 and 47, 1,024 57 and 80; 1 of 4 (by tokens) 384 30 and 25, 1,024 31 and 32;
-    1024 x 2048, 8 of 32 64 tokens 106 and 475; 768 x 384, 8 of 16 (by pairs) 512 tokens 0.81, 4,096 1.16 of the time; 4096 x 1024, 4 of 8 (by
-    width) 384 tokens 98 and 93."""
-    if moe_prefers_sorted(tokens, width, ff, experts, top):
-        return True
+    """The same where the sorted experts' products go through pairs of SMs: experts that are large or many, from some 200 tokens on.
+    Timed in graphs, router to sum, at 1,681 sizes (nine widths, eleven counts of experts, 64 to 4,096 tokens): 0.7 % above the better of the two
+    ways on average, 468 sizes answered otherwise than by the line above, up to half the time, one 8 % slower and eight up to 6 %. us, sorted
+    and all: 2048 x 1024, 2 of 8 experts 160 tokens 47 and 45, 256 49 and 53, 384 47 and 58; 4 of 16 256 tokens 68 and 84, 768 99 and 144; 4 of 8
+    (more than a third chosen) 320 tokens 57 and 55, 768 77 and 94; 1024 x 512, 1 of 4 (by tokens) 768 tokens 31 and 31, 1,500 33 and 37; 1024 x
+    2048, 4 of 16 (ff at least the width) 96 tokens 65 and 87, 384 68 and 117; 768 x 384, 8 of 16 4,096 tokens 185 and 163; 4096 x 1024, 4 of 16
+    (width four times ff) 200 tokens 118 and 109, 320 121 and 141."""
     if width % 64 or ff % 64:
         return False
+    if tokens < (256 if width >= 4 * ff else 200):
+        return tokens >= 80 and experts >= 8 and ff >= width and experts * ff >= 16384
+    if moe_prefers_sorted(tokens, width, ff, experts, top):
+        return True
     if 3 * top > experts:
-        return experts * ff >= 6144 and width < 4 * ff and (width * ff >= 1 << 20 or tokens * top <= 4096)
+        return experts * ff >= 6144 and (ff >= width or (tokens >= 400 and width < 4 * ff and (width * ff >= 1 << 20 or tokens * top <= 4096)))
     return experts * ff >= 6144 or tokens * (experts - top) * ff >= (1.5e6 if width * ff >= 1 << 19 else 2.4e6)
 
 
