@@ -592,9 +592,10 @@ def attend(projected, *, q_heads: int, kv_heads: int, head_dim: int, rotary, ctx
         return ops.attention_extend(q, cache, ctx.cu_seqlens, ctx.seq_of_token, ctx.positions, ctx.slots,
                                     ctx.kv_lens, ctx.max_seq_len, scale, window, slopes, out_scale, extras, ctx.max_kv_len)
     if projection is not None:
+        from . import gemm_dispatch
         x, weight = projection
         if (phase == "prefill" and writes_cache and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
-                and width in (0, head_dim)):
+                and width in (0, head_dim) and not gemm_dispatch.qkv_apart(x.shape[0], *weight.shape)):
             table = None
             if inv_freq is not None:   # one table of cosines and sines per step and rotation
                 table = ctx.scratch.get(("rope_table", id(inv_freq)))

@@ -458,6 +458,17 @@ def gemm_bf16_slices(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Te
     return out
 
 
+def qkv_apart(M: int, N: int, K: int) -> bool:
+    """Whether a prompt's q|k|v projection goes to the tiles with the weights as the wide operand and the rotation and the stores to a
+    launch of their own, instead of tiles with the activations as the wide operand that rotate and store in their epilogue (gemm_bf16_qkv;
+    the same bits): rows that leave those tiles half empty, and matrices whose gain is more than the host's time for the launch. us in
+    chains of weights from memory, apart and in one: 6144 x 4096 65 rows 18 and 25, 320 23 and 26, 529 28 and 31, 700 33 and 32; 5120 x 3072 65
+    rows 15 and 20, 529 23 and 27, 700 28 and 27; 10240 x 8192 192 rows 44 and 51, 256 53 and 51; 12288 x 4096 128 rows 29 and 32, 320 39 and 37;
+    3072 x 2048, below the line, 65 rows 12 and 15, 400 14 and 16."""
+    return (not no_wide and umma_width is None and 64 < M <= (560 if N * K <= 32e6 else 200) and N * K >= 12e6
+            and pair_room() > 0 and wide_plan(M, N, K, 0, pair_room()) is not None)
+
+
 def gemm_bf16_qkv(x: torch.Tensor, weight: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
                   kv, dest_rows: Optional[torch.Tensor], table: Optional[torch.Tensor]) -> bool:
     """A prompt's fused q|k|v projection with rotation and stores in the product's epilogue:
