@@ -7,7 +7,7 @@ DEV = "cuda"
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("M,heads,kv_heads,d,K", [(65, 32, 8, 128, 4096), (200, 64, 8, 128, 8192), (333, 24, 8, 128, 3072), (560, 32, 8, 128, 4096),
+@pytest.mark.parametrize("M,heads,kv_heads,d,K", [(65, 32, 8, 128, 4096), (100, 64, 8, 128, 8192), (333, 24, 8, 128, 3072), (560, 32, 8, 128, 4096),
                                                   (128, 40, 12, 64, 3072)])
 def test_the_bits_of_the_epilogue(M, heads, kv_heads, d, K):
     from llama_rs_metal_b200.kernels import gemm_dispatch, ops
