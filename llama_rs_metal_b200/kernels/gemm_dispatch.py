@@ -294,7 +294,9 @@ def few_plan(M: int, N: int, K: int, mode: int, added: bool = False) -> int:
     products of few rows that go to one stream. Up to 8 rows the products of small matrices stream too, which then keep their L1 from
     layer to layer. Whole steps of two layers and a head of 32,768, all streamed / by this rule: 3B shape 4 sequences 179.6 / 172.1 us,
     8B shape 4 283 / 258, 8 299 / 267; before this rule / by it: 1B shape 9 sequences 165 / 141, 48 196 / 182, 3B shape 12 268 / 190, 48
-    288 / 246, 8B shape 12 373 / 274, 48 400 / 343."""
+    288 / 246, 8B shape 12 373 / 274, 48 400 / 343. Gates of fewer than 74
+    tiles stream up to 8 rows: four layers, hidden 4,096, 8 sequences, inner width 4,096 (64 tiles) 326 / 355, 4 sequences of 5,120 (80) 320 /
+    311; hidden 3,072, inner 4,608 (72) 243 / 292; from 9 rows on 64 tiles are the better ones too, 359 / 327."""
     if M > 64 or mode not in (0, 1, 3, 4):
         return 0
     if few_takes(M, N, K, mode):
@@ -309,7 +311,7 @@ def few_plan(M: int, N: int, K: int, mode: int, added: bool = False) -> int:
         k_blocks = -(-K // 64)
         per_slice = max(4, -(-k_blocks // max(1, SM_COUNT // tiles)))
         return -(-k_blocks // per_slice)
-    return 1 if tiles >= SM_COUNT // 2 or (large and tiles >= 64) or (M > 16 and tiles >= 40) else 0
+    return 1 if tiles >= SM_COUNT // 2 or (large and tiles >= 64 and M > STREAM_ROWS) or (M > 16 and tiles >= 40) else 0
 
 
 def _few(x: torch.Tensor, weight: torch.Tensor, mode: int, lib, added: bool = False) -> int:
