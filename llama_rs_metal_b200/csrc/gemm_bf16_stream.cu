@@ -282,9 +282,25 @@ int launch_variant(const void* X, const void* W, void* out, int M, int N, int K,
   constexpr int kChunk = Chunk<NT>::kK;
   const int k_per_split = ((K + splits - 1) / splits + kChunk - 1) / kChunk * kChunk;
   const dim3 grid((N + 15) / 16, (K + k_per_split - 1) / k_per_split);
-  LRM_LAUNCH(kernel, grid, WARPS * 32, smem, stream, static_cast<const __nv_bfloat16*>(X),
-             static_cast<const __nv_bfloat16*>(W), out, M, N, K, mode, k_per_split, pick, grouped);
-  return 0;
+  // The rest of the SM's memory as L1, which the activations live off: behind a kernel with much shared memory the SMs else keep that
+  // kernel's division, as kernels overlap. Steps of four layers, hidden 4,096, 8 sequences, with the division left open 652 us (the product
+  // behind gemm_bf16_few.cu 83 to 114 us), asked for 536 (51 to 67); asked for no shared memory at all, which leaves a CTA an SM, 737.
+  constexpr int held = (MINB * (smem + 1024) * 100 + 228 * 1024 - 1) / (228 * 1024);
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = dim3(WARPS * 32);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attributes[2];
+  attributes[0].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  attributes[0].val.sharedMemCarveout = held < 100 ? held : 100;
+  attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attributes[1].val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = attributes;
+  config.numAttrs = g_lrm_pdl ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&config, kernel, static_cast<const __nv_bfloat16*>(X), static_cast<const __nv_bfloat16*>(W), out, M,
+                                           N, K, mode, k_per_split, pick, grouped);
+  return e == cudaSuccess ? 0 : static_cast<int>(e);
 }
 
 // Register budgets: 64 per thread for up to 16 activation rows (32 warps resident per SM),
