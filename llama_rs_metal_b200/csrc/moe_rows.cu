@@ -285,7 +285,8 @@ int launch_grouped(const void* x, const void* W, const int* ids, const float* we
   const int rows = DOWN ? width : ff, per = DOWN ? 16 : 8, pairs = tokens * top;
   const size_t bytes = sizeof(float) * WARPS * NT * 128 + sizeof(int) * (pairs < 32 ? 32 : pairs);
   const dim3 grid((rows + per - 1) / per, (experts < pairs ? experts : pairs) + (DOWN ? 1 : 0));
-  const int by_id = pairs >= 2 * experts;
+  // an expert a block row where nearly all are chosen: some choices are of identity experts where x32 is given
+  const int by_id = pairs >= 2 * experts && x32 == nullptr;
   LRM_LAUNCH((moe_grouped_kernel<NT, WARPS, DOWN>), grid, WARPS * 32, bytes, stream, static_cast<const __nv_bfloat16*>(x),
              static_cast<const __nv_bfloat16*>(W), ids, weights, static_cast<__nv_bfloat16*>(y3), planes, tokens, width, ff,
              experts, top, limit, alpha, act, x32, by_id);
