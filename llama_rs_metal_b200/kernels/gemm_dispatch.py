@@ -291,12 +291,13 @@ def few_plan(M: int, N: int, K: int, mode: int, added: bool = False) -> int:
 
     A norm that adds planes takes 2 to 4 us more than one behind a product that was added in place (4096 x 4096 with its norm, 8 rows:
     11.4 against 9.8 streamed; 3072 x 3072 9.2 against 6.8; 2048 x 2048 16 rows 6.6 against 6.0, 64 rows 8.1 against 10.3), so small
-    products of few rows that go to one stream. Up to 8 rows the products of small matrices stream too, which then keep their L1 from
-    layer to layer. Whole steps of two layers and a head of 32,768, all streamed / by this rule: 3B shape 4 sequences 179.6 / 172.1 us,
-    8B shape 4 283 / 258, 8 299 / 267; before this rule / by it: 1B shape 9 sequences 165 / 141, 48 196 / 182, 3B shape 12 268 / 190, 48
-    288 / 246, 8B shape 12 373 / 274, 48 400 / 343. Gates of fewer than 74
-    tiles stream up to 8 rows: four layers, hidden 4,096, 8 sequences, inner width 4,096 (64 tiles) 326 / 355, 4 sequences of 5,120 (80) 320 /
-    311; hidden 3,072, inner 4,608 (72) 243 / 292; from 9 rows on 64 tiles are the better ones too, 359 / 327."""
+    products of few rows that go to one stream. Up to 8 rows the products of small matrices stream too: eight
+    layers of the 1B shape and a head of 128,256, 1 sequence 387 us, with the down products in slices here 410, with the gates too 421; 8
+    sequences 452, 477 and 476; six of the 3B shape the same either way (523, 522, 523). Whole steps of two layers and a head of 32,768, all
+    streamed / by this rule: 3B shape 4 sequences 179.6 / 172.1 us, 8B shape 4 283 / 258, 8 299 / 267; before this rule / by it: 1B shape 9
+    sequences 165 / 141, 48 196 / 182, 3B shape 12 268 / 190, 48 288 / 246, 8B shape 12 373 / 274, 48 400 / 343. Gates of fewer than 74 tiles,
+    which leave half of the SMs idle here, stream up to 8 rows: four layers, hidden 4,096, 8 sequences, inner width 4,096 (64 tiles) 326 / 355,
+    4 sequences of 5,120 (80) 318 / 314; hidden 3,072, inner 4,608 (72) 243 / 292."""
     if M > 64 or mode not in (0, 1, 3, 4):
         return 0
     if few_takes(M, N, K, mode):
