@@ -272,17 +272,19 @@ void attention_prefill_pingpong_kernel(
         umma_commit(s_full + i);
       }
     };
-    auto weighted = [&](int i, int j) {  // O_i (+)= P_i V_j, P from tensor memory (8 columns per 16 keys)
+    // O_i (+)= P_i V_j, P from tensor memory (8 columns per 16 keys). `frees`: the last product that reads stage j; `ends`: the
+    // chain's last. The commits stand in the elected lane's block of products, like that of the scores: one in an `if` of its own was
+    // lost or came twice in a GEMM of this form (gemm_bf16_umma.cu). The one that is waited for before the CTA leaves is the last.
+    auto weighted = [&](int i, int j, bool frees, bool ends) {
       const uint32_t va = kv_at + (j % STAGES) * 2 * KV_TILE + KV_TILE;
       if (leader) {
 #pragma unroll
         for (int k = 0; k < BKV / UMMA_K; ++k)
           umma_bf16_a_tmem(tmem + CHAINS * BKV + i * D, tmem + i * BKV + k * (UMMA_K / 2),
                            smem_desc(va + k * UMMA_K * 128, KV_BLOCK), idesc_pv, (j >= CHAINS / NQ || k > 0) ? 1u : 0u);
+        if (frees) umma_commit(kv_free + j % STAGES);
+        if (ends) umma_commit(o_done + i);
       }
-    };
-    auto commit = [&](uint64_t* bar) {
-      if (leader) umma_commit(bar);
     };
     bool ok = wait(q_full, 0, kStuckQ) && wait(kv_full, 0, kStuckKV);
     if (ok) scores(0, 0);
@@ -296,10 +298,8 @@ void attention_prefill_pingpong_kernel(
         if (next < tiles) ok = wait(kv_full + next % STAGES, (next / STAGES) & 1, kStuckKV);
         ok = ok && wait(p_ready + i, (t / CHAINS) & 1, kStuckProbabilities);
         if (!ok) break;
-        weighted(i, t);
+        weighted(i, t, true, next >= tiles);
         if (next < tiles) scores(i, next);
-        else commit(o_done + i);
-        commit(kv_free + t % STAGES);
       }
     } else {
       if (ok && last1 >= 0) scores(1, 0);
@@ -307,8 +307,7 @@ void attention_prefill_pingpong_kernel(
         if (j <= last0) {
           ok = wait(p_ready + 0, j & 1, kStuckProbabilities);
           if (!ok) break;
-          weighted(0, j);
-          if (j == last0) commit(o_done + 0);
+          weighted(0, j, j > last1, j == last0);
         }
         if (j < last0 || j < last1) {  // the next key tile has to be here for the next scores
           ok = wait(kv_full + (j + 1) % STAGES, ((j + 1) / STAGES) & 1, kStuckKV);
@@ -318,10 +317,8 @@ void attention_prefill_pingpong_kernel(
         if (j <= last1) {
           ok = wait(p_ready + 1, j & 1, kStuckProbabilities);
           if (!ok) break;
-          weighted(1, j);
-          if (j == last1) commit(o_done + 1);
+          weighted(1, j, true, j == last1);
         }
-        commit(kv_free + j % STAGES);  // every product that reads stage j has been issued
         if (j < last1) scores(1, j + 1);
       }
     }
