@@ -167,8 +167,8 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_few_kernel(const __grid
             for (int k = 0; k < BK / UMMA_K; ++k)
               umma_bf16(tmem + acc * F::SET, smem_desc(a + k * UMMA_K * 2), smem_desc(b + k * UMMA_K * 2), idesc,
                         (kb > 0 || k > 0) ? 1u : 0u);
-            if (kb + 1 == num_kb) umma_commit(acc_full + acc);  // (as in gemm_bf16_umma.cu)
             umma_commit(empty + s);
+            if (kb + 1 == num_kb) umma_commit(acc_full + acc);  // (here and last: as in gemm_bf16_umma.cu)
           }
           __syncwarp();
         }

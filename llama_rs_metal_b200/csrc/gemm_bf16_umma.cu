@@ -199,10 +199,11 @@ __global__ __launch_bounds__(kUmmaThreads, 1) void gemm_bf16_umma_kernel(
                 for (int i = 0; i < MT; ++i)  // the 128-row blocks of X share the tile of W
                   umma_bf16(tmem_d + i * BN, smem_desc(a + i * BM * BK * 2 + k * UMMA_K * 2),
                             smem_desc(b + k * UMMA_K * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+              umma_commit(empty + s);  // arrives when these MMAs have finished reading the stage
               if (kb + 1 == num_kb) umma_commit(acc_full + acc);  // arrives when every MMA issued so far has completed
               // (In the lane's block of products, like the other: in an `if` of its own behind the loop it did not reach the waiting
-              // warps, or twice, in one of 20 launches of 700 x 40000 x 72 added in place, whose epilogue gave up then.)
-              umma_commit(empty + s);  // arrives when these MMAs have finished reading the stage
+              // warps, or twice, in one of 20 launches of 700 x 40000 x 72 added in place, whose epilogue gave up then. Behind the
+              // stage's: nobody waits for the last stage's arrival, and the CTA may leave when this one has come.)
             }
             __syncwarp();
           }

@@ -115,6 +115,9 @@ __global__ __launch_bounds__(kPairThreads, 1) void gemm_bf16_umma_pair_kernel(
         for (uint32_t i = first; i < it; ++i)
           mbar_wait(full + i % STAGES, (i / STAGES) & 1, status, kPairStuckDrain);
       }
+      // Nobody waits for the last stages to refill them, but the leader's commits signal them here all the same: not to leave before.
+      for (uint32_t i = it > STAGES ? it - STAGES : 0; i < it && !*bail; ++i)
+        if (!mbar_wait(empty + i % STAGES, (i / STAGES) & 1, status, kPairStuckEmpty)) *bail = 1;
     }
   } else if (warp == 1) {
     if (leader) {
@@ -150,8 +153,8 @@ __global__ __launch_bounds__(kPairThreads, 1) void gemm_bf16_umma_pair_kernel(
               for (int k = 0; k < PK / P_UMMA_K; ++k)
                 umma_bf16_pair(tmem_d, smem_desc(a + k * P_UMMA_K * 2), smem_desc(b + k * P_UMMA_K * 2), idesc,
                                (kb > 0 || k > 0) ? 1u : 0u);
-              if (kb + 1 == k_blocks) umma_commit_pair(acc_full + acc, 3);  // both CTAs' epilogues may read (as in gemm_bf16_umma.cu)
-              umma_commit_pair(empty + s, 3);                         // both CTAs' loaders may refill the stage
+              umma_commit_pair(empty + s, 3);                               // both CTAs' loaders may refill the stage
+              if (kb + 1 == k_blocks) umma_commit_pair(acc_full + acc, 3);  // both CTAs' epilogues may read (here and last: as in gemm_bf16_umma.cu)
             }
             __syncwarp();
           }

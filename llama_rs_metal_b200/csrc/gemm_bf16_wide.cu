@@ -260,6 +260,10 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_wide_kernel(const __gri
       for (uint32_t i = first; i < it; ++i)
         if ((i & 1) == mine) mbar_wait(full + i % STAGES, (i / STAGES) & 1, status, kStuckDrain);
     }
+    // Nobody waits for the last stages to refill them, but the leader's commits signal them here all the same: not to leave before.
+    if (lane == 0)
+      for (uint32_t i = it > STAGES ? it - STAGES : 0; i < it && !*bail; ++i)
+        if ((i & 1) == mine && !mbar_wait(empty + i % STAGES, (i / STAGES) & 1, status, kStuckEmpty)) *bail = 1;
   } else if (warp == 1) {
     if (leader) {
       // One lane of the leader drives the tensor cores of both SMs; the warp stays together around it, as in gemm_bf16_umma_pair.cu.
@@ -293,8 +297,8 @@ __global__ __launch_bounds__(kThreads, 1) void gemm_bf16_wide_kernel(const __gri
 #pragma unroll
               for (int k = 0; k < BK / UMMA_K; ++k)
                 umma_bf16_pair(tmem_d, smem_desc(a + k * UMMA_K * 2), smem_desc(b + k * UMMA_K * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-              if (kb + 1 == count) umma_commit_pair(acc_full + acc, 3);  // both CTAs' epilogues may read (as in gemm_bf16_umma.cu)
-              umma_commit_pair(empty + s, 3);                         // both CTAs' loaders may refill the stage
+              umma_commit_pair(empty + s, 3);                            // both CTAs' loaders may refill the stage
+              if (kb + 1 == count) umma_commit_pair(acc_full + acc, 3);  // both CTAs' epilogues may read (here and last: as in gemm_bf16_umma.cu)
             }
             __syncwarp();
           }

@@ -60,3 +60,26 @@ def test_commits_stand_with_their_products(name, source):
             assert name == "gemm_bf16_umma.cu" and not head.startswith(("if", "else")), f"{name}: a commit under {head!r}"
             lane_of_its_own += 1
     assert lane_of_its_own == (2 if name == "gemm_bf16_umma.cu" else 0)
+
+
+@pytest.mark.parametrize("name,source", KERNELS, ids=[name for name, _ in KERNELS])
+def test_the_arrival_that_is_waited_for_is_the_last(name, source):
+    """Nobody waits for the last arrival at a stage, and a CTA leaves when its results have: theirs has to be behind it."""
+    both = 0
+    for at in commits(source):
+        _, body = block_around(source, at)
+        told = re.findall(r"\bumma_commit(?:_pair)?\((\w+)", body)
+        stages = [i for i, bar in enumerate(told) if bar in ("empty", "kv_free")]
+        results = [i for i, bar in enumerate(told) if bar in ("acc_full", "o_done")]
+        if stages and results and name != "gemm_f32_umma.cu":  # (there the stage's commit stands for later products, and is waited for)
+            both += 1
+            assert max(stages) < min(results), f"{name}: {told}"
+    assert both or name == "gemm_f32_umma.cu"
+
+
+@pytest.mark.parametrize("name", ["gemm_bf16_umma_pair.cu", "gemm_bf16_wide.cu"])
+def test_no_cta_of_a_pair_leaves_before_its_stages_were_signalled(name):
+    """What the leader's commits signal in the other CTA's memory has come before the pair meets for the last time."""
+    source = dict(KERNELS)[name]
+    last = re.search(r"for \(uint32_t i = it > STAGES \? it - STAGES : 0; i < it && !\*bail; \+\+i\)\s*if \(([^;]*)\) \*bail = 1;", source)
+    assert last and "mbar_wait(empty + i % STAGES, (i / STAGES) & 1" in last.group(1)
