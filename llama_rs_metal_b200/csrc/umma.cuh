@@ -49,9 +49,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   if (status != nullptr) atomicCAS(status, 0, where);
   return false;
 }
-// A whole warp's wait: the `chosen` lane alone polls, all get the answer.
+// A whole warp's wait: the `chosen` lane alone polls, all get the answer, and what the barrier guards is there for all (a vote
+// alone orders no memory).
 __device__ __forceinline__ bool mbar_wait_warp(bool chosen, uint64_t* bar, uint32_t parity, int* status, int where) {
-  return __all_sync(0xffffffffu, !chosen || mbar_wait(bar, parity, status, where));
+  const bool there = __all_sync(0xffffffffu, !chosen || mbar_wait(bar, parity, status, where));
+  __syncwarp();
+  return there;
 }
 // How many of a ring's "full" barriers in a row, from that of block `it` on, have completed their block's phase; at least 1, or 0
 // where a bounded wait for the first gave up. A whole warp calls it, on the same `it`. A question costs some 200 cycles whatever

@@ -1,5 +1,7 @@
-"""Commits of kernels whose issuing warp stays together around an elected lane (no GPU needed): each stands in the lane's block of the
-products it stands for. One in an `if` of its own was lost, or came twice, in one of 20 launches of one product."""
+"""Barriers of the tensor-core kernels, as their sources have them (no GPU needed).
+
+Commits of kernels whose issuing warp stays together around an elected lane: each stands in the lane's block of the products it stands
+for. One in an `if` of its own was lost, or came twice, in one of 20 launches of one product. And waits of one lane for its warp."""
 import os
 import re
 
@@ -83,3 +85,14 @@ def test_no_cta_of_a_pair_leaves_before_its_stages_were_signalled(name):
     source = dict(KERNELS)[name]
     last = re.search(r"for \(uint32_t i = it > STAGES \? it - STAGES : 0; i < it && !\*bail; \+\+i\)\s*if \(([^;]*)\) \*bail = 1;", source)
     assert last and "mbar_wait(empty + i % STAGES, (i / STAGES) & 1" in last.group(1)
+
+
+@pytest.mark.parametrize("function", ["mbar_wait_warp", "ring_ready"])
+def test_a_lane_that_waits_for_its_warp_orders_the_others_reads(function):
+    """One lane has seen the barrier; a vote tells the others, but only __syncwarp() puts their reads behind what it saw."""
+    with open(os.path.join(CSRC, "umma.cuh")) as handle:
+        source = handle.read()
+    begin = source.index(" %s(" % function)
+    body = source[begin:source.index("\n}\n", begin)]
+    for vote in re.finditer(r"__(all|ballot|any)_sync\(", body):
+        assert "__syncwarp();" in body[vote.end():] and "return __all_sync" not in body
