@@ -63,14 +63,15 @@ __device__ __forceinline__ void rotate_q(uint32_t (&qa)[D / 16][4], const float*
   }
 }
 
+// (qkv and planes are what the launch before writes: plain pointers, or their loads might move ahead of the wait.)
 template <int D>
 __global__ __launch_bounds__(kThreads) void attention_decode_cluster_kernel(
-    const __nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions,
+    const __nv_bfloat16* qkv, const int* __restrict__ positions,
     const float* __restrict__ inv_freq, int rotary, __nv_bfloat16* __restrict__ k_pages,
     __nv_bfloat16* __restrict__ v_pages, const int* __restrict__ dest_rows,
     __nv_bfloat16* __restrict__ out, const int* __restrict__ page_table, int table_stride,
     const int* __restrict__ slots, const int* __restrict__ kv_lens, int q_heads, int kv_heads,
-    int row_groups, float scale_log2, const int* __restrict__ order, const float* __restrict__ planes, int n_planes,
+    int row_groups, float scale_log2, const int* __restrict__ order, const float* planes, int n_planes,
     long long plane_stride, int fresh_at) {
   constexpr int STRIDE = D + 8, TILE = kTile * STRIDE, PART = D + 2, kStages = stages_of<D>();
   extern __shared__ __align__(16) unsigned char smem_raw[];

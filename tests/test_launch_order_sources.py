@@ -19,6 +19,8 @@ KERNELS = [
     ("moe.cu", "moe_router_kernel", {"w", "bias", "correction"}),
     ("moe.cu", "moe_dense_gate_wide_kernel", set()),
     ("recurrent_walk.cuh", "walk_prepare_kernel", {"head_decay", "look", "cu_seqlens"}),
+    ("attention_decode_cluster.cu", "attention_decode_cluster_kernel",
+     {"positions", "inv_freq", "dest_rows", "page_table", "slots", "kv_lens", "order"}),
 ]
 
 
