@@ -99,10 +99,11 @@ __global__ void rope_store_kernel(const A* __restrict__ qkv, A* __restrict__ q_o
 // chunk, or a chunk of v. Needs R/2 and d to be multiples of VEC. A CTA makes its token's sines and cosines once, for all heads, while
 // its first rows are on the way. Bound by the latency of that and of the stores. us, in brackets with the sines of every head made
 // anew: 529 tokens of 40 heads of 128 4.7 (4.9; in a step behind the product 6.1 to 6.8, 7.9), 333 of 40 of 64 2.9 (4.2), 1,200 4.5 (5.1).
+// (qkv is what the launch before writes: a plain pointer, or its loads might move ahead of the wait.)
 template <typename A> struct alignas(16) Vec16 { A v[16 / sizeof(A)]; };
 
 template <typename A>
-__global__ void rope_store_vec_kernel(const A* __restrict__ qkv, A* __restrict__ q_out,
+__global__ void rope_store_vec_kernel(const A* qkv, A* __restrict__ q_out,
                                       A* __restrict__ k_out, A* __restrict__ v_out,
                                       A* __restrict__ k_pages, A* __restrict__ v_pages,
                                       const int* __restrict__ dest_rows,
