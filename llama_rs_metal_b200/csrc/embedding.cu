@@ -25,9 +25,9 @@ __global__ void embed_rows_kernel(const W* __restrict__ table, const int* __rest
 // The same 16 bytes of a row at a time, a piece of the row per thread and `pieces` CTAs per token, so that all of a step's loads are
 // under way together (a thread that walks the row four bytes at a time waits for HBM as often as it loads): 32 tokens of 4,096
 // bfloat16 numbers 10.1 -> 2.2 us, one of 2,048 3.8 -> 1.7, 4,353 tokens of 3,072 30 -> 21 us (3.8 TB/s of rows read and written).
-// Rows and both tensors lie on 16 bytes.
+// Rows and both tensors lie on 16 bytes. (ids may be what a launch before chose: a plain pointer, or their load might move ahead of the wait.)
 template <typename W>
-__global__ __launch_bounds__(256) void embed_rows_vec_kernel(const W* __restrict__ table, const int* __restrict__ ids,
+__global__ __launch_bounds__(256) void embed_rows_vec_kernel(const W* __restrict__ table, const int* ids,
                                                              float* __restrict__ out, int hidden, int vocab, int pieces, float scale) {
   constexpr int PER = 16 / sizeof(W);
   pdl_trigger();
@@ -36,7 +36,7 @@ __global__ __launch_bounds__(256) void embed_rows_vec_kernel(const W* __restrict
   if (i >= hidden) return;
   const int id = ids[t];
   const bool ok = id >= 0 && id < vocab;
-  const uint4 raw = ok ? __ldg(reinterpret_cast<const uint4*>(table + static_cast<size_t>(id) * hidden + i)) : make_uint4(0u, 0u, 0u, 0u);
+  const uint4 raw = ok ? *reinterpret_cast<const uint4*>(table + static_cast<size_t>(id) * hidden + i) : make_uint4(0u, 0u, 0u, 0u);
   const W* from = reinterpret_cast<const W*>(&raw);
   float* to = out + static_cast<size_t>(t) * hidden + i;
 #pragma unroll

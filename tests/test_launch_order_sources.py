@@ -22,6 +22,7 @@ KERNELS = [
     ("attention_decode_cluster.cu", "attention_decode_cluster_kernel",
      {"positions", "inv_freq", "dest_rows", "page_table", "slots", "kv_lens", "order"}),
     ("rope_store.cu", "rope_store_vec_kernel", {"dest_rows", "positions", "inv_freq"}),
+    ("embedding.cu", "embed_rows_vec_kernel", {"table"}),
     ("elementwise.cu", "silu_mul_vec_kernel", set()),
     ("elementwise.cu", "add_planes_vec_kernel", set()),
     ("norm.cu", "rms_norm_rows_kernel", {"w"}),
