@@ -61,7 +61,8 @@ __global__ void rms_norm_kernel(float* __restrict__ x, const W* __restrict__ w, 
 }
 
 // The same with 16-byte accesses: a thread keeps PER4 groups of four consecutive elements.
-// Needs hidden % 4 == 0 and 16-byte aligned rows.
+// Needs hidden % 4 == 0 and 16-byte aligned rows. (partials are what the launch before writes, and the weights are
+// loaded ahead of the wait for it on purpose: a plain pointer, or those loads might go with them. x is written here.)
 __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
   const uint2 raw = *reinterpret_cast<const uint2*>(p);
@@ -80,7 +81,7 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
 
 template <typename W, typename O, int PER4>
 __global__ void rms_norm_vec_kernel(float* __restrict__ x, const W* __restrict__ w, O* __restrict__ out,
-                                    const int* __restrict__ rows, const float* __restrict__ partials,
+                                    const int* __restrict__ rows, const float* partials,
                                     int n_partials, size_t partial_stride, int hidden, float eps) {
   __shared__ float scratch[32];
   const int groups = hidden >> 2;
@@ -177,7 +178,7 @@ __device__ __forceinline__ uint32_t norm_cluster_rank() {
 
 template <typename W, typename O, int PER4>
 __global__ void rms_norm_cluster_kernel(float* __restrict__ x, const W* __restrict__ w, O* __restrict__ out,
-                                        const int* __restrict__ rows, const float* __restrict__ partials,
+                                        const int* __restrict__ rows, const float* partials,
                                         int n_partials, size_t partial_stride, int hidden, float eps, int ranks) {
   __shared__ float scratch[32];
   __shared__ float shares[8];  // shares[k]: rank k's part of the sum of squares, written by rank k

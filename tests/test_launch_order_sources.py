@@ -26,6 +26,8 @@ KERNELS = [
     ("elementwise.cu", "silu_mul_vec_kernel", set()),
     ("elementwise.cu", "add_planes_vec_kernel", set()),
     ("norm.cu", "rms_norm_rows_kernel", {"w"}),
+    ("norm.cu", "rms_norm_vec_kernel", {"w", "rows"}),
+    ("norm.cu", "rms_norm_cluster_kernel", {"w", "rows"}),
 ]
 
 
