@@ -72,7 +72,7 @@ __global__ __launch_bounds__(kThreads) void attention_decode_cluster_kernel(
     __nv_bfloat16* __restrict__ out, const int* __restrict__ page_table, int table_stride,
     const int* __restrict__ slots, const int* __restrict__ kv_lens, int q_heads, int kv_heads,
     int row_groups, float scale_log2, const int* __restrict__ order, const float* planes, int n_planes,
-    long long plane_stride, int fresh_at) {
+    long long plane_stride, int fresh_from) {
   constexpr int STRIDE = D + 8, TILE = kTile * STRIDE, PART = D + 2, kStages = stages_of<D>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float cs_tab[D / 2], sn_tab[D / 2];
@@ -161,7 +161,7 @@ __global__ __launch_bounds__(kThreads) void attention_decode_cluster_kernel(
     }
     load_q<D>(qa, q_src, D, rows);
   };
-  __nv_bfloat16* fresh = reinterpret_cast<__nv_bfloat16*>(smem_raw + fresh_at);  // planes: q rows, the new k, the new v
+  __nv_bfloat16* fresh = reinterpret_cast<__nv_bfloat16*>(smem_raw + fresh_from);  // planes: q rows, the new k, the new v
   if (planes == nullptr) {
     take(src + static_cast<size_t>(head0) * D, src + static_cast<size_t>(q_heads + kh) * D,
          src + static_cast<size_t>(q_heads + kv_heads + kh) * D);
@@ -362,14 +362,21 @@ template <int D> int smem_bytes(int cluster, int rows) {
   const int runs = (rows * D + 127) / 128, runs_each = (runs + cluster - 1) / cluster;
   return ring + cluster * (runs_each * 128 + 32) * 4;
 }
-// and behind it, for a projection that comes as planes, the rows that a CTA needs of it.
-template <int D> int fresh_bytes(int rows) { return (rows + 2) * D * 2; }
 
+// Where a CTA puts the rows that it adds up from planes: the ring's last slot, which is first asked for in the walk's first turn,
+// behind a barrier that everybody reaches with those rows taken. (Room of their own behind the ring cost head size 64 one CTA of four an SM
+// with clusters of 2, and head size 128 one of three with eight query heads per kv head: 24 sequences of 64 / 8 heads of 128, 3,000
+// keys, 65 us against 55; whole steps of the 1B shape, 8 layers, 28 sequences of 1,000 keys 527 against 498, 32 of 3,000 780 against 700, 37
+// of 3,000 815 against 770. An argument of the kernel: known to the compiler, 40 sequences took 47.5 us against 45.6, planes or not.)
+template <int D> constexpr int fresh_at() {
+  static_assert(18 * D <= kTile * (D + 8), "16 query rows, k and v");
+  return (stages_of<D>() - 1) * kTile * (D + 8) * 2;
+}
 
 template <int D> int prepare(int cluster) {
   auto kernel = attention_decode_cluster_kernel<D>;
   int most = 0;  // over every cluster size and up to 16 query heads per kv head
-  for (int c = 1; c <= 16; ++c) most = max(most, smem_bytes<D>(c, 16) + fresh_bytes<D>(16));
+  for (int c = 1; c <= 16; ++c) most = max(most, smem_bytes<D>(c, 16));
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
   if (e != cudaSuccess) return static_cast<int>(e);
   if (cluster > 8) {
@@ -383,7 +390,7 @@ template <int D> void fill_config(cudaLaunchConfig_t& config, cudaLaunchAttribut
                                   int cluster, int rows, cudaStream_t stream) {
   config.gridDim = dim3(pairs * cluster);
   config.blockDim = dim3(kThreads);
-  config.dynamicSmemBytes = smem_bytes<D>(cluster, rows) + fresh_bytes<D>(rows);
+  config.dynamicSmemBytes = smem_bytes<D>(cluster, rows);
   config.stream = stream;
   attributes[0].id = cudaLaunchAttributeClusterDimension;
   attributes[0].val.clusterDim.x = cluster;
@@ -434,7 +441,7 @@ template <int D> int launch(const void* qkv, const int* positions, const float* 
       inv_freq, rotary, static_cast<__nv_bfloat16*>(k_pages), static_cast<__nv_bfloat16*>(v_pages),
       dest_rows, static_cast<__nv_bfloat16*>(out), page_table, table_stride, slots, kv_lens, q_heads,
       kv_heads, row_groups, scale * 1.4426950408889634f, order, planes, n_planes,
-      static_cast<long long>(seqs) * (q_heads + 2 * kv_heads) * D, smem_bytes<D>(cluster, min(group, 16)));
+      static_cast<long long>(seqs) * (q_heads + 2 * kv_heads) * D, fresh_at<D>());
   return e == cudaSuccess ? 0 : static_cast<int>(e);
 }
 
