@@ -14,7 +14,7 @@ from typing import Optional, Tuple
 import torch
 
 from ..errors import InvalidError, KernelUnavailableError, UnsupportedError
-from . import library
+from . import library, profile
 
 F32, BF16 = 0, 1
 _CODES = {torch.float32: F32, torch.bfloat16: BF16}
@@ -1652,8 +1652,9 @@ def moe_rows_step(x: torch.Tensor, router: torch.Tensor, bias: Optional[torch.Te
                   x32: Optional[torch.Tensor] = None, sum_planes: bool = False) -> Optional[torch.Tensor]:
     """moe_router and moe_experts_rows in one call for a step of few rows (bfloat16): the planes [top, T, width], or with
     `sum_planes` their sum [T, width]. One trip through the bindings and one scratch tensor instead of three and five: the host took
-    41 us for 8 rows, longer than the device. None where the kernels do not take the sizes."""
-    if x.dtype != torch.bfloat16 or gate_up.dtype != torch.bfloat16:
+    41 us for 8 rows, longer than the device. None where the kernels do not take the sizes, and under the launch profile, which
+    times them apart (the same bits)."""
+    if x.dtype != torch.bfloat16 or gate_up.dtype != torch.bfloat16 or profile.enabled:
         return None
     _check(x, "x", torch.bfloat16, 2)
     _check(router, "router", torch.float32, 2)
@@ -1747,7 +1748,8 @@ def moe_experts_sorted(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tenso
             or any(t.data_ptr() % 16 for t in (x, gate_up, down)) or not lib.lrm_gemm_bf16_umma_supports(128, width, ff)):
         return None
     dev = x.device
-    if T and top and gemm_dispatch.sorted_on_pairs():
+    pairs = bool(T and top and gemm_dispatch.sorted_on_pairs())
+    if pairs and not profile.enabled:  # (the launch profile times the five kernels apart: the same bits)
         scratch = torch.empty(lib.lrm_moe_sorted_step_bytes(T, width, ff, E, top), dtype=torch.uint8, device=dev)
         total = _f32((T, width), dev) if out is None else out
         gemm_dispatch.mark_status_dirty()
@@ -1774,14 +1776,13 @@ def moe_experts_sorted(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tenso
         _done(lib.lrm_moe_sorted_gate(_ptr(both), _ptr(rows), _ptr(tile_experts), _ptr(weights), ff, tiles, ctypes.c_float(limit),
                                       ctypes.c_float(alpha), act, _ptr(y), _stream()), "moe_sorted_gate")
     else:
-        _done(lib.lrm_gemm_bf16_umma_experts_gated(_ptr(sorted_x), _ptr(gate_up), _ptr(y), M, ff, width,
-                                                   ctypes.c_longlong(E * 2 * ff), _ptr(tile_experts), _ptr(rows), _ptr(weights),
-                                                   ctypes.c_float(limit), ctypes.c_float(alpha), act, status, _stream()),
-              "gemm_bf16_umma_experts_gated")
+        gated = lib.lrm_gemm_bf16_wide_experts_gated if pairs else lib.lrm_gemm_bf16_umma_experts_gated
+        _done(gated(_ptr(sorted_x), _ptr(gate_up), _ptr(y), M, ff, width, ctypes.c_longlong(E * 2 * ff), _ptr(tile_experts), _ptr(rows),
+                    _ptr(weights), ctypes.c_float(limit), ctypes.c_float(alpha), act, status, _stream()), "gemm_bf16_experts_gated")
     part = _f32((M, width), dev)
-    _done(lib.lrm_gemm_bf16_umma_experts(_ptr(y), _ptr(down), _ptr(part), M, width, ff, ctypes.c_longlong(width),
-                                         ctypes.c_longlong(E * ff), 0, ff, _ptr(tile_experts), status, _stream()),
-          "gemm_bf16_umma_experts")
+    experts = lib.lrm_gemm_bf16_wide_experts if pairs else lib.lrm_gemm_bf16_umma_experts
+    _done(experts(_ptr(y), _ptr(down), _ptr(part), M, width, ff, ctypes.c_longlong(width), ctypes.c_longlong(E * ff), 0, ff,
+                  _ptr(tile_experts), status, _stream()), "gemm_bf16_experts")
     add = out is not None
     if out is None:
         out = _f32((T, width), dev)

@@ -12,3 +12,10 @@ def test_entry_points_that_return_sizes_are_not_timed():
     names = {n for f in sources.glob("*.cu") for n in re.findall(r'LRM_API long long (lrm_\w+)\(', f.read_text())}
     assert "lrm_gemm_f32_umma_scratch" in names
     assert all(any(q in name for q in profile._QUERIES) for name in names)
+
+
+def test_what_has_a_row_of_work_is_launched_from_here():
+    """The profile stands between the wrappers and the library: entry points that only other entry points call never pass it."""
+    kernels = Path(profile.__file__).parent
+    called = {n for f in kernels.glob("*.py") if f.name != "profile.py" for n in re.findall(r"\b(lrm_\w+)", f.read_text())}
+    assert set(profile.WORK) <= called, sorted(set(profile.WORK) - called)
