@@ -284,35 +284,59 @@ def few_plan(M: int, N: int, K: int, mode: int, added: bool = False) -> int:
     cut; the others never are. `added`: the slices go to a norm, which adds them to the residual stream.
 
     Narrow products are cut until their items fill the SMs. us in chains of products, in brackets the streaming or the tile kernel:
-    6144 x 4096 in three slices 8 rows 9.7 (11.9), 32 rows 10.3 (22.4), 64 rows 11.5 (40.7); 5120 x 3072 9 rows 7.7 (12.2), 48 rows 9.0
-    (28.2); 4096 x 14336 in four 8 rows 20.5 (25.5), 32 rows 21.4 (24.2); 2048 x 8192 in nine 12 rows 7.7 (9.8), 64 rows 9.0 (10.3). Whole:
-    28672 x 4096 gated 8 rows 39.4 (49.7), 12 rows 39.3 (62.1), 64 rows 44.5 (47.7); 32768 x 4096 8 rows 43.2 (51.6), 12 rows 43.5 (66.1);
-    8192 x 2048 24 rows 10.1 (13.1), 12 rows 9.8 (9.3); 5120 x 3072 12 rows 12.5 (12.7), 64 rows 15.0 (31.5).
-
-    A norm that adds planes takes 2 to 4 us more than one behind a product that was added in place (4096 x 4096 with its norm, 8 rows:
-    11.4 against 9.8 streamed; 3072 x 3072 9.2 against 6.8; 2048 x 2048 16 rows 6.6 against 6.0, 64 rows 8.1 against 10.3), so small
-    products of few rows that go to one stream. Up to 8 rows the products of small matrices stream too: eight
-    layers of the 1B shape and a head of 128,256, 1 sequence 387 us, with the down products in slices here 410, with the gates too 421; 8
-    sequences 452, 477 and 476; six of the 3B shape the same either way (523, 522, 523). Whole steps of two layers and a head of 32,768, all
-    streamed / by this rule: 3B shape 4 sequences 179.6 / 172.1 us, 8B shape 4 283 / 258, 8 299 / 267; before this rule / by it: 1B shape 9
-    sequences 165 / 141, 48 196 / 182, 3B shape 12 268 / 190, 48 288 / 246, 8B shape 12 373 / 274, 48 400 / 343. Gates of fewer than 74 tiles,
-    which leave half of the SMs idle here, stream up to 8 rows: four layers, hidden 4,096, 8 sequences, inner width 4,096 (64 tiles) 326 / 355,
-    4 sequences of 5,120 (80) 318 / 314; hidden 3,072, inner 4,608 (72) 243 / 292."""
+    6144 x 4096 in three slices 32 rows 10.3 (22.4), 64 rows 11.5 (40.7); 5120 x 3072 9 rows 7.7 (12.2), 48 rows 9.0 (28.2); 4096 x 14336
+    in four 32 rows 21.4 (24.2); 2048 x 8192 in nine 12 rows 7.7 (9.8), 64 rows 9.0 (10.3). Whole: 28672 x 4096 gated 12 rows 39.3 (62.1), 64
+    rows 44.5 (47.7); 32768 x 4096 12 rows 43.5 (66.1); 8192 x 2048 24 rows 10.1 (13.1), 12 rows 9.8 (9.3); 5120 x 3072 12 rows 12.5
+    (12.7), 64 rows 15.0 (31.5). A norm that adds planes takes 2 to 4 us more than one behind a product that was added in place (2048 x
+    2048 16 rows 6.6 against 6.0, 64 rows 8.1 against 10.3), so small products of few rows that go to one stream. Up to 8 rows:
+    _few_up_to_eight. Whole steps of two layers and a head of 32,768, before this rule / by it: 1B shape 9 sequences 165 / 141, 48 196 / 182, 3B
+    shape 12 268 / 190, 48 288 / 246, 8B shape 12 373 / 274, 48 400 / 343."""
     if M > 64 or mode not in (0, 1, 3, 4):
         return 0
     if few_takes(M, N, K, mode):
         return 1
-    large, head = min(N, K) >= 3072, N >= 32768
-    if M <= STREAM_ROWS and not large and not head:
-        return 0
-    if added and (M <= 32 and N * K <= 4 * 1024 * 1024 or M <= STREAM_ROWS and N * K <= 16 * 1024 * 1024):
-        return 0
     tiles = -(-N // 128)
+    if M <= STREAM_ROWS:
+        if not _few_up_to_eight(M, N, K, mode, added):
+            return 0
+    elif added and M <= 32 and N * K <= 4 * 1024 * 1024:
+        return 0
     if mode == 4:
         k_blocks = -(-K // 64)
         per_slice = max(4, -(-k_blocks // max(1, SM_COUNT // tiles)))
         return -(-k_blocks // per_slice)
-    return 1 if tiles >= SM_COUNT // 2 or (large and tiles >= 64 and M > STREAM_ROWS) or (M > 16 and tiles >= 40) else 0
+    if M <= STREAM_ROWS:
+        return 1
+    return 1 if tiles >= SM_COUNT // 2 or (min(N, K) >= 3072 and tiles >= 64) or (M > 16 and tiles >= 40) else 0
+
+
+def _few_up_to_eight(M: int, N: int, K: int, mode: int, added: bool) -> bool:
+    """Where up to 8 rows leave the streaming kernel, whose CTAs have 16 columns each. us a whole decode step, streamed / here, by what
+    the line is about:
+
+    * more columns than eight such CTAs an SM have (18,944): a second round of them. Gates, four layers, 1 and 8 sequences: hidden 2,048,
+      18,432 columns 172 / 180 and 193 / 195, 19,456 196 / 194 and 227 / 214, 28,672 227 / 222 and 249 / 242; hidden 2,560, 18,432 224 / 230 and
+      249 / 247, 19,456 260 / 248 and 296 / 269; hidden 1,024, 19,456 144 / 146 and 162 / 158.
+    * gates of fewer columns, but two tiles for every second SM: K above 3,072. 17,920 x 3,328 277 / 277 and 301 / 297, 18,432 x 3,584 279 / 278
+      and 305 / 297, 18,432 x 4,096 321 / 317 and 353 / 344; 16,384 x 3,072 248 / 252 and 278 / 279. (64 tiles: 4,096 wide, 8 sequences, 326 / 355.)
+    * heads, the same line. Two layers, 1, 4 and 8 sequences: 24,576 x 2,560 127 / 124, 133 / 130, 140 / 135; 98,304 x 2,048 151 / 150, 162 / 158,
+      170 / 163; 49,152 x 1,024 78 / 77, 86 / 84, 87 / 87. A single sequence of 2,048 of K may lose: 24,576 107 / 107, 32,768 110 / 112 (4 and 8
+      sequences 120 / 119, 124 / 122), six layers 251 / 255.
+    * whole bfloat16 results (a q|k|v projection of 74 tiles and more): both sides 3,072 and more, four layers of 12,288 x 4,096 343 / 336 and
+      389 / 377.
+    * slices that a norm adds up: K of 8,192 and more (which the streaming kernel cuts too) or a third CTA an SM, not where each SM has one.
+      A product and its norm, 1 and 8 rows: 2,048 x 8,192 9.8 / 11.9 and 10.5 / 12.3; 2,560 x 8,192 15.4 / 12.5 and 16.4 / 13.3, x 6,144 10.3 / 11.3
+      and 10.9 / 12.0; 4,096 x 6,144 12.5 / 14.1 and 13.4 / 14.5, x 8,192 17.3 / 17.0 and 19.0 / 17.3, x 14,336 27.7 / 25.4 and 29.2 / 26.3; 5,120 x
+      5,120 15.8 / 14.9 and 16.9 / 15.5; 8,192 x 8,192 31.0 / 27.7 and 32.2 / 28.3.
+    * slices that decode attention adds up, every CTA for the rows it needs: large products only. Four layers, 1 and 8 sequences: 3,840 x 3,328
+      (13 heads to a key head) 270 / 290 and 284 / 305, 4,608 x 3,584 277 / 292 and 293 / 310, two layers of 5,120 x 3,072 157.6 / 159.4 and 171.6 / 172.8;
+      6,144 x 4,096 269 / 269 and 300 / 296, 8,192 x 6,144 317 / 317 and 334 / 332."""
+    rounds = -(-N // (16 * SM_COUNT))  # CTAs of the streaming kernel to an SM
+    if mode == 4:
+        if added:
+            return rounds > 1 and (K >= 8192 or rounds > 2)
+        return min(N, K) >= 3072 and N * K >= 22e6
+    return rounds > 8 or (-(-N // 128) >= SM_COUNT // 2 and (K > 3072 if mode == 3 else min(N, K) >= 3072))
 
 
 def _few(x: torch.Tensor, weight: torch.Tensor, mode: int, lib, added: bool = False) -> int:
