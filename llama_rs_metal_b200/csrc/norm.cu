@@ -289,10 +289,12 @@ static int launch_norm(float* x, const void* w, void* out, const int* rows, cons
       if (cper4 <= 4) LRM_NORM_CLUSTER(4);
 #undef LRM_NORM_CLUSTER
     }
-    // Many rows without slices to fold: a warp per row. us, in brackets a CTA per row (with as many groups of four per thread as the
-    // row has): 2,048 rows of 2,048 4.9 (7.2), 1,024 rows of 3,072 5.1 (5.3), 2,048 7.8 (8.7), 1,500 rows of 4,096 8.4 (8.0),
-    // 2,048 9.7 (10.0); 700 rows of 2,048 3.6 (4.0). With slices the CTA's loads of all of them at once are the better way.
-    if (sizeof(O) == 2 && rows == nullptr && n_partials == 0 && n_rows >= 1024 && groups <= 1024) {
+    // Many rows without slices to fold: a warp per row, from a second round of CTAs of a row each on (eight of 256 threads an SM, of
+    // shorter rows some ten of 128). us, in brackets a CTA per row, input and output in L2: rows of 2,048 1,024 3.4 (3.1), 1,200 3.6
+    // (3.8), 2,048 4.1 (5.2), 8,192 12.4 (23.4); of 3,072 1,024 4.1 (3.8), 1,200 4.3 (4.5), 2,048 4.7 (6.4); of 4,096 1,024 4.6 (4.2), 1,200 5.0
+    // (5.0), 1,500 4.7 (5.6), 2,048 7.2 (7.1), 4,096 13.0 (17.2); of 1,024 1,200 2.9 (2.3), 1,500 3.1 (3.2), 4,096 3.7 (5.2). With slices
+    // the CTA's loads of all of them at once are the better way.
+    if (sizeof(O) == 2 && rows == nullptr && n_partials == 0 && n_rows > (groups >= 512 ? 8 : 10) * kSmCount && groups <= 1024) {
 #define LRM_NORM_ROWS(P4)                                                                                                   \
   return static_cast<int>(lrm_launch(rms_norm_rows_kernel<W, O, P4>, (n_rows + 3) / 4, 128, 0, stream,                      \
                                      static_cast<const float*>(x), static_cast<const W*>(w), static_cast<O*>(out), n_rows,  \

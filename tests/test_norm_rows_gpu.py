@@ -25,3 +25,17 @@ def test_against_float64(hidden, n_rows, planes, w_dtype):
     assert bool(((got.double().cpu() - want).abs() <= bound).all())
     if planes:
         assert bool(((stream.double().cpu() - total).abs() <= planes * 2.0 ** -23 * size).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("hidden,n_rows", [(1024, 1480), (1024, 1481), (2048, 1184), (2048, 1185), (3072, 1100), (4096, 1024), (4096, 1185)])
+def test_one_round_of_ctas_keeps_a_row_each(hidden, n_rows):
+    """Up to eight rows an SM (ten of short rows) have the bits that a few rows have; beyond, a warp's order of the sum."""
+    from llama_rs_metal_b200.kernels import ops
+    gen = torch.Generator(device=DEV).manual_seed(n_rows)
+    x, w = torch.randn(n_rows, hidden, generator=gen, device=DEV), torch.randn(hidden, generator=gen, device=DEV).bfloat16()
+    got = ops.rms_norm(x, w, 1e-5, torch.bfloat16)
+    few = torch.cat([ops.rms_norm(part.contiguous(), w, 1e-5, torch.bfloat16) for part in x.split(500)])
+    assert torch.equal(got, few) == (n_rows <= (1184 if hidden >= 2048 else 1480))
+    want = x.double() * (w.double() / (x.double().square().mean(-1, keepdim=True) + 1e-5).sqrt())
+    assert bool(((got.double() - want).abs() <= (2.0 ** -8 + 2.0 ** -20) * want.abs() + 1e-30).all())
