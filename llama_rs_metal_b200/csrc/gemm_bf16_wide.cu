@@ -1,4 +1,5 @@
-// bfloat16 products of some 65 to 1,100 rows on pairs of SMs, the weights as the wide operand: Y[M, N] = X[M, K] . W[N, K]^T.
+// bfloat16 products of more than 64 rows on pairs of SMs, the weights as the wide operand: Y[M, N] = X[M, K] . W[N, K]^T. Which products
+// come here is estimated (gemm_dispatch.wide_plan): mostly those of up to some 1,300 rows, narrow ones of any number.
 //
 // A cluster of two CTAs makes a tile of 256 weight rows and BN activation rows with tcgen05.mma.cta_group::2 (M 256, N = BN): the
 // weight rows are the A operand, so the activation rows are cut into tiles of any multiple of 32 up to 256 (529 rows: three of

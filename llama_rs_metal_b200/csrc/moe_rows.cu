@@ -337,8 +337,8 @@ LRM_API int lrm_moe_router(const void* x, int x_dtype, const float* w, const flo
                            int renormalize, float mass_eps, float weight_scale, cudaStream_t stream);
 LRM_API int lrm_add_planes(float* x, const float* planes, int count, long long n, cudaStream_t stream);
 
-// Bytes of scratch that lrm_moe_rows_step wants: y's terms, the choices and their weights.
-LRM_API long long lrm_moe_rows_step_floats(int tokens, int ff, int top) {  // in floats
+// Scratch that lrm_moe_rows_step wants, in floats: y's terms, the choices and their weights.
+LRM_API long long lrm_moe_rows_step_floats(int tokens, int ff, int top) {
   const long long pairs = static_cast<long long>(tokens) * top;
   return (3 * pairs * ff + 7) / 8 * 4 + (pairs + 3) / 4 * 4 + pairs;
 }

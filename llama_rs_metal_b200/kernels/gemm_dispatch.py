@@ -5,9 +5,9 @@
   faster one;
 * up to 8 rows of smaller matrices, and what is narrow and cannot be cut: the weight-streaming kernel
   (csrc/gemm_bf16_stream.cu);
-* 65 to some 1,300 rows, wherever its tiles waste less: tcgen05 over pairs of SMs with the weights as
-  the wide operand (csrc/gemm_bf16_wide.cu; wide_plan);
-* more rows (prompts): the TMA + tcgen05 kernel
+* more than 64 rows, wherever its tiles are estimated to waste less (no fixed number of rows): tcgen05
+  over pairs of SMs with the weights as the wide operand (csrc/gemm_bf16_wide.cu; wide_plan);
+* else (prompts): the TMA + tcgen05 kernel
   (csrc/gemm_bf16_umma.cu), with 128 x 128, 128 x 256 or 256 x 256 tiles, whichever needs less
   time by a count of rounds over the SMs and the measured cost of a tile;
 * a narrow product that is to be added to the residual stream may be cut into K slices so that
@@ -488,7 +488,9 @@ def gemm_bf16_slices(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Te
 def qkv_apart(M: int, N: int, K: int) -> bool:
     """Whether a prompt's q|k|v projection goes to the tiles with the weights as the wide operand and the rotation and the stores to a
     launch of their own, instead of tiles with the activations as the wide operand that rotate and store in their epilogue (gemm_bf16_qkv;
-    the same bits): rows that leave those tiles half empty, and matrices whose gain is more than the host's time for the launch. us in
+    the same bits): rows that leave those tiles half empty, and matrices whose gain is more than the host's time for the launch where a
+    length comes for the first time and is not replayed (3072 x 2048, four layers, 66 and 256 tokens: in one 860 and 890 us, apart 920 and
+    950; replayed 306 and 337, apart 294 and 319; 560 tokens 430 either way). us in
     chains of weights from memory, apart and in one: 6144 x 4096 65 rows 18 and 25, 320 23 and 26, 529 28 and 31, 700 33 and 32; 5120 x 3072 65
     rows 15 and 20, 529 23 and 27, 700 28 and 27; 10240 x 8192 192 rows 44 and 51, 256 53 and 51; 12288 x 4096 128 rows 29 and 32, 320 39 and 37;
     3072 x 2048, below the line, 65 rows 12 and 15, 400 14 and 16."""
